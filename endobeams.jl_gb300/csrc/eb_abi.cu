@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "../../include/endobeams_gb300.h"
+#include "eb_cond_plan.hpp"
 #include "eb_gmres.cuh"
 #include "eb_internal.cuh"
 #include "eb_output.cuh"
@@ -129,78 +130,6 @@ void prefilter_axis(double* c, const int64_t dims[3], int axis, std::vector<doub
       y[-stride] = y[0];
       y[n * stride] = y[(n - 1) * stride];
     }
-}
-
-// Reverse Cuthill-McKee order of one simulation's node graph (neighbours in
-// increasing degree, root a pseudo-peripheral node of each component).
-// adj holds local neighbour lists (self excluded).  Returns the half
-// bandwidth in nodes of the permuted graph; pos[i] is node i's position.
-int rcm_order(const std::vector<std::vector<int>>& adj, std::vector<int>& pos) {
-  const int n = (int)adj.size();
-  std::vector<int> order;
-  order.reserve(n);
-  std::vector<char> seen(n, 0);
-  std::vector<int> level(n, -1), queue;
-  auto bfs = [&](int root, std::vector<int>& visited) {
-    visited.clear();
-    visited.push_back(root);
-    level[root] = 0;
-    int last = 0;
-    for (size_t h = 0; h < visited.size(); ++h) {
-      int v = visited[h];
-      for (int w : adj[v])
-        if (level[w] < 0) {
-          level[w] = level[v] + 1;
-          last = std::max(last, level[w]);
-          visited.push_back(w);
-        }
-    }
-    return last;
-  };
-  std::vector<int> comp;
-  for (int start = 0; start < n; ++start) {
-    if (seen[start]) continue;
-    int root = start;
-    // pseudo-peripheral root (George-Liu iteration)
-    // (levels hold the BFS from `root` at the top of every iteration)
-    int ecc = bfs(root, comp);
-    for (int it = 0; it < 8; ++it) {
-      int best = -1;
-      for (int v : comp)
-        if (level[v] == ecc && (best < 0 || adj[v].size() < adj[best].size())) best = v;
-      for (int v : comp) level[v] = -1;
-      int e2 = bfs(best, comp);
-      if (e2 <= ecc) break;
-      ecc = e2;
-      root = best;
-    }
-    for (int v : comp) level[v] = -1;
-    // Cuthill-McKee from root
-    queue.clear();
-    queue.push_back(root);
-    seen[root] = 1;
-    for (size_t h = 0; h < queue.size(); ++h) {
-      int v = queue[h];
-      order.push_back(v);
-      std::vector<int> nb;
-      for (int w : adj[v])
-        if (!seen[w]) nb.push_back(w);
-      std::sort(nb.begin(), nb.end(), [&](int x, int y) {
-        return adj[x].size() != adj[y].size() ? adj[x].size() < adj[y].size() : x < y;
-      });
-      for (int w : nb) {
-        seen[w] = 1;
-        queue.push_back(w);
-      }
-    }
-  }
-  std::reverse(order.begin(), order.end());
-  pos.assign(n, 0);
-  for (int k = 0; k < n; ++k) pos[order[k]] = k;
-  int bw = 0;
-  for (int v = 0; v < n; ++v)
-    for (int w : adj[v]) bw = std::max(bw, std::abs(pos[v] - pos[w]));
-  return bw;
 }
 
 // The samples (sign flipped when `negate`) in the interior of the zero-padded
@@ -415,7 +344,8 @@ struct eb_handle {
   bool tc_lu = false;  // band LU trailing updates on the tensor cores
   size_t band_floats = 0;
   BandDev band{};
-  int* d_blk_row = nullptr;
+  CondFactor cond{};
+  std::vector<int64_t> cond_elim_off, cond_tgt_off;  // per level (all simulations): offsets of its lists
   std::vector<int> band_b;  // per sim half bandwidth (0: block-Jacobi)
   // factorisation reuse
   int* d_refactor = nullptr;
@@ -507,10 +437,12 @@ int launch_solve(eb_handle* h, bool refactor, const int* refactor_src, PhaseTime
   }
   if (refactor) {
     CK(cudaMemcpyAsync(h->d_refactor, refactor_src, sizeof(int) * h->n_sims, cudaMemcpyHostToDevice, h->stream));
-    launch_band_fill(h->d, h->band, h->d_blk_row, h->stream);
+    const CondLevels lv{h->cond_elim_off.data(), h->cond_tgt_off.data(), (int)h->cond_elim_off.size() - 1};
+    launch_cond_factor(h->d, h->cond, lv, h->d_refactor, h->stream);
+    launch_band_fill(h->d, h->band, h->cond, h->stream);
     if (h->tc_lu) CK(launch_band_lu_tc(h->d, h->band, h->max_b, h->band.lu_fail, h->stream));
     else CK(launch_band_lu(h->d, h->band, h->max_b, h->stream));
-    T.launches[EB_PHASE_PRECOND] += 3;
+    T.launches[EB_PHASE_PRECOND] += 3 + 2 + 2 * lv.n;
   }
   CK(cudaGetLastError());
   T.mark(EB_PHASE_PRECOND, h->stream);
@@ -922,31 +854,33 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
   }
   h->blk_off.assign(n_sims + 1, 0);
   for (int s = 0; s < n_sims; ++s) h->blk_off[s + 1] = row_ptr[h->node_off[s + 1]];
-  std::vector<int> blk_row(NB);
-  for (int64_t i = 0; i < NN; ++i)
-    for (int k = row_ptr[i]; k < row_ptr[i + 1]; ++k) blk_row[k] = (int)i;
 
-  // ---- band-LU preconditioner plan: reverse Cuthill-McKee order per simulation
-  std::vector<int> pos_all(NN), node_at(NN);
-  std::vector<int64_t> band_off(n_sims + 1, 0);
+  // ---- preconditioner plan per simulation: condensation levels, then the band of the kept nodes
+  std::vector<int64_t> band_off(n_sims + 1, 0), roff(n_sims + 1, 0);
   h->band_b.assign(n_sims, 0);
   const int bmax = (((227 * 1024) / 4 - 8) / kPanel - kPanel) / 2;  // shared-memory limit of k_band_lu
+  std::vector<CondPlan> plan(n_sims);
+  {
+    auto build = [&](int s) {
+      const int64_t no = h->node_off[s], n = h->node_off[s + 1] - no;
+      std::vector<std::vector<int>> la(n);
+      for (int64_t i = 0; i < n; ++i)
+        for (int g : adj[no + i])
+          if (g != (int)(no + i)) la[i].push_back((int)(g - no));
+      cond_plan(la, (bmax - 5) / 6, plan[s]);
+    };
+    const int nthr = std::max(1, std::min<int>({16, (int)std::thread::hardware_concurrency(), (int)n_sims}));
+    std::vector<std::thread> pool;
+    for (int k = 1; k < nthr; ++k)
+      pool.emplace_back([&, k] { for (int s = k; s < n_sims; s += nthr) build(s); });
+    for (int s = 0; s < n_sims; s += nthr) build(s);
+    for (auto& th : pool) th.join();
+  }
   for (int s = 0; s < n_sims; ++s) {
-    const int64_t no = h->node_off[s], n = h->node_off[s + 1] - no;
-    std::vector<std::vector<int>> la(n);
-    for (int64_t i = 0; i < n; ++i)
-      for (int g : adj[no + i])
-        if (g != (int)(no + i)) la[i].push_back((int)(g - no));
-    std::vector<int> pos;
-    const int w = rcm_order(la, pos);
-    int b = 6 * w + 5;
-    if (p->preconditioner == EB_PRECOND_BLOCK_JACOBI || b > bmax) b = 0;
-    h->band_b[s] = b;
-    for (int64_t i = 0; i < n; ++i) {
-      pos_all[no + i] = pos[i];
-      node_at[no + pos[i]] = (int)(no + i);
-    }
-    band_off[s + 1] = band_off[s] + (b ? band_floats(6 * n, b) : 0);
+    const int b = 6 * plan[s].w + 5, nr = plan[s].n - plan[s].ne;
+    if (p->preconditioner != EB_PRECOND_BLOCK_JACOBI && b <= bmax) h->band_b[s] = b;
+    band_off[s + 1] = band_off[s] + (h->band_b[s] ? band_floats(6 * (int64_t)nr, b) : 0);
+    roff[s + 1] = roff[s] + nr;
   }
 
   // ---- device arenas
@@ -1143,46 +1077,129 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
   {
     size_t fr = 0, tot = 0;
     CK(cudaMemGetInfo(&fr, &tot));
-    // the band, its diagonal-block inverses and the work vector must leave 2 GB free
-    const size_t inv_bytes = 2 * sizeof(float) * (size_t)inv_base(NN, n_sims);
+    // the band, its diagonal-block inverses and the condensation's blocks must leave 2 GB free
+    const size_t inv_bytes = 2 * sizeof(float) * (size_t)inv_base(roff[n_sims], n_sims);
     size_t need = sizeof(float) * (size_t)band_off[n_sims];
+    for (int s = 0; s < n_sims; ++s)
+      if (h->band_b[s]) need += (size_t)plan[s].n_blocks * (36 * sizeof(float) + 10 * sizeof(int));
     const size_t margin = (size_t)2 << 30;
     if (need + inv_bytes + margin > fr) {
       std::fill(h->band_b.begin(), h->band_b.end(), 0);
       std::fill(band_off.begin(), band_off.end(), 0);
-      need = 0;
     }
     for (int s = 0; s < n_sims; ++s) {
       h->max_b = std::max(h->max_b, h->band_b[s]);
       if (h->band_b[s]) h->any_band = true;
       else h->any_jacobi = true;
     }
+    // condensation lists of all simulations with a band: blocks simulation by simulation, the
+    // elimination and update lists level by level
+    CondFactor& cf = h->cond;
+    {
+      std::vector<int> node_at(NN), scol, src, rnode, cnode, ldiag, elim, elim_node, tgt, tptr, cl, cw, red, rpos;
+      std::vector<int> ne(n_sims, 0), lev_off(n_sims + 1, 0), lev_ptr;
+      std::vector<CondRange> range(NN, CondRange{0, 0, 0, 0});
+      std::vector<int64_t> base(n_sims + 1, 0);
+      size_t nlev = 0;
+      for (int s = 0; s < n_sims; ++s) {
+        const CondPlan& P = plan[s];
+        const int64_t no = h->node_off[s];
+        base[s + 1] = base[s];
+        lev_off[s + 1] = lev_off[s];
+        for (int i = 0; i < P.n; ++i) node_at[no + P.pos[i]] = (int)(no + i);
+        if (!h->band_b[s]) continue;
+        const int o = (int)base[s];
+        base[s + 1] += P.n_blocks;
+        if (base[s + 1] >= (1LL << 31)) return fail(EB_ERR_ARG, "problem too large for 32-bit block indices");
+        ne[s] = P.ne;
+        lev_ptr.insert(lev_ptr.end(), P.lev_ptr.begin(), P.lev_ptr.end());
+        lev_off[s + 1] += (int)P.lev_ptr.size();
+        nlev = std::max(nlev, P.tgt.size());
+        for (int q = 0; q < P.n; ++q)
+          range[no + q] = CondRange{q < P.ne ? o + P.wptr[q] : 0, q < P.ne ? o + P.wptr[q + 1] : 0, o + P.lptr[q],
+                                    o + P.lptr[q + 1]};
+        const int l0 = P.lptr[0];
+        for (int k = 0; k < P.n_blocks; ++k) {
+          const int r = node_at[no + P.srow[k]], c = node_at[no + P.scol[k]];
+          auto it = std::lower_bound(col.begin() + row_ptr[r], col.begin() + row_ptr[r + 1], c);
+          src.push_back(it != col.begin() + row_ptr[r + 1] && *it == c ? (int)(it - col.begin()) : -1);
+          rnode.push_back(r);
+          cnode.push_back(c);
+          scol.push_back(P.scol[k]);
+          ldiag.push_back(k >= l0 && k < P.red0 ? o + P.wptr[P.scol[k]] : -1);
+          if (k >= P.red0) {
+            red.push_back(o + k);
+            rpos.push_back(P.srow[k]);
+          }
+        }
+      }
+      h->cond_elim_off.assign(1, 0);
+      h->cond_tgt_off.assign(1, 0);
+      for (size_t l = 0; l < nlev; ++l) {
+        for (int s = 0; s < n_sims; ++s) {
+          const CondPlan& P = plan[s];
+          if (!h->band_b[s] || l >= P.tgt.size()) continue;
+          const int o = (int)base[s];
+          for (int q = P.lev_ptr[l]; q < P.lev_ptr[l + 1]; ++q) {
+            elim.push_back((int)(h->node_off[s] + q));
+            elim_node.push_back(node_at[h->node_off[s] + q]);
+          }
+          for (size_t k = 0; k < P.tgt[l].size(); ++k) {
+            tgt.push_back(o + P.tgt[l][k]);
+            tptr.push_back((int)cl.size());
+            for (int u = P.tptr[l][k]; u < P.tptr[l][k + 1]; ++u) {
+              cl.push_back(o + P.cl[l][u]);
+              cw.push_back(o + P.cw[l][u]);
+            }
+          }
+        }
+        h->cond_elim_off.push_back((int64_t)elim.size());
+        h->cond_tgt_off.push_back((int64_t)tgt.size());
+      }
+      tptr.push_back((int)cl.size());
+      int *p_scol, *p_ne, *p_lo, *p_lp, *p_src, *p_rn, *p_cn, *p_ld, *p_el, *p_en, *p_t, *p_tp, *p_cl, *p_cw, *p_red,
+          *p_rpos, *p_nat;
+      CondRange* p_range;
+      int64_t* p_roff;
+      CK(A.alloc(&cf.c.S, 36 * (size_t)base[n_sims]));
+      CK(A.upload(&p_scol, scol)); CK(A.upload(&p_ne, ne)); CK(A.upload(&p_lo, lev_off)); CK(A.upload(&p_lp, lev_ptr));
+      CK(A.upload(&p_src, src)); CK(A.upload(&p_rn, rnode)); CK(A.upload(&p_cn, cnode)); CK(A.upload(&p_ld, ldiag));
+      CK(A.upload(&p_el, elim)); CK(A.upload(&p_en, elim_node)); CK(A.upload(&p_t, tgt)); CK(A.upload(&p_tp, tptr));
+      CK(A.upload(&p_cl, cl)); CK(A.upload(&p_cw, cw)); CK(A.upload(&p_red, red)); CK(A.upload(&p_rpos, rpos));
+      CK(A.upload(&p_range, range)); CK(A.upload(&p_roff, roff)); CK(A.upload(&p_nat, node_at));
+      cf.c.scol = p_scol; cf.c.range = p_range; cf.c.ne = p_ne; cf.c.lev_off = p_lo; cf.c.lev_ptr = p_lp; cf.c.roff = p_roff;
+      cf.n_blocks = base[n_sims];
+      cf.src = p_src; cf.rnode = p_rn; cf.cnode = p_cn; cf.ldiag = p_ld; cf.elim = p_el; cf.elim_node = p_en;
+      cf.tgt = p_t; cf.tptr = p_tp; cf.cl = p_cl; cf.cw = p_cw;
+      cf.red_n = (int64_t)red.size();
+      cf.red = p_red; cf.rpos = p_rpos;
+      h->band.node_at = p_nat;
+      h->band.cond = cf.c;
+    }
     int64_t *p_boff;
-    int *p_bw, *p_pos, *p_nat;
+    int* p_bw;
     CK(A.upload(&p_boff, band_off));
     CK(A.upload(&p_bw, h->band_b));
-    CK(A.upload(&p_pos, pos_all));
-    CK(A.upload(&p_nat, node_at));
-    CK(A.upload(&h->d_blk_row, blk_row));
     h->band_floats = (size_t)band_off[n_sims];
     float *p_band, *p_work, *p_li, *p_ui;
     CK(A.alloc(&p_band, h->band_floats));
     CK(A.alloc(&p_work, ND));
-    const size_t inv = h->any_band ? (size_t)inv_base(NN, n_sims) : 1;
+    const size_t inv = h->any_band ? (size_t)inv_base(roff[n_sims], n_sims) : 1;
     CK(A.alloc(&p_li, inv));
     CK(A.alloc(&p_ui, inv));
     CK(A.alloc(&h->d_refactor, n_sims));
     int* p_lu_fail;
     CK(A.alloc(&p_lu_fail, n_sims));
     CK(cudaMemset(p_lu_fail, 0, sizeof(int) * n_sims));
-    // CTA order of the per-simulation kernels: decreasing n (b + 1) (band solve and LU work)
+    // CTA order of the per-simulation kernels: decreasing work of a solve (all DOFs, and the kept ones' band)
     std::vector<int> order(n_sims);
     for (int s = 0; s < n_sims; ++s) order[s] = s;
-    auto cost = [&](int s) { return (h->node_off[s + 1] - h->node_off[s]) * (int64_t)(h->band_b[s] + 6); };
+    auto kept = [&](int s) { return (int)(6 * (roff[s + 1] - roff[s])); };
+    auto cost = [&](int s) { return 6 * (h->node_off[s + 1] - h->node_off[s]) * (int64_t)64 + kept(s) * (int64_t)(h->band_b[s] + 6); };
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost(x) > cost(y); });
     int* p_order;
     CK(A.upload(&p_order, order));
-    h->band = BandDev{p_band, p_boff, p_bw, p_pos, p_nat, p_work, p_li, p_ui, h->d_refactor, p_order, p_lu_fail};
+    h->band = BandDev{p_band, p_boff, p_bw, h->band.cond, h->band.node_at, p_work, p_li, p_ui, h->d_refactor, p_order, p_lu_fail};
     // the tensor-core factorisation where its shared memory fits the widest band
     h->tc_lu = h->any_band && p->band_lu == EB_LU_TENSOR && band_lu_tc_smem(h->max_b) <= kLuTcSmemLimit;
     sa.band = h->band;
@@ -1197,7 +1214,7 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
     h->cur_dt.assign(n_sims, 0.0);
     h->cur_active.assign(n_sims, 0);
     int max_n = 0;
-    for (int s = 0; s < n_sims; ++s) max_n = std::max<int>(max_n, (int)(6 * (h->node_off[s + 1] - h->node_off[s])));
+    for (int s = 0; s < n_sims; ++s) max_n = std::max(max_n, kept(s));
     sa.max_n = max_n;
     sa.x_in_smem = h->any_band && gmres_smem(m) + sizeof(float) * (size_t)max_n <= 200 * 1024;
     // stage band blocks through shared memory when the two buffers fit beside the rest
@@ -1218,7 +1235,7 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
         int bmax = 0, nmax = 0;
         for (int s2 : sims) {
           bmax = std::max(bmax, h->band_b[s2]);
-          nmax = std::max<int>(nmax, (int)(6 * (h->node_off[s2 + 1] - h->node_off[s2])));
+          nmax = std::max(nmax, kept(s2));
         }
         c.n_sims = (int)sims.size();
         c.max_n = nmax;

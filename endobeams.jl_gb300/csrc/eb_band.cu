@@ -7,40 +7,37 @@
 
 namespace eb {
 
-// Thread per (block, entry): copies Ktan into the permuted FP32 band; fixed
-// DOFs become identity rows/columns (the free-DOF system of
-// extract_free_dofs!, src/utils_solver.jl:94-102, embedded in the full size).
-__global__ void k_band_fill(Dev d, BandDev B, const int* __restrict__ blk_row) {
+// Thread per (block among the kept nodes, entry): the condensed tangent (fixed DOFs are
+// identity rows/columns already) into the FP32 band.
+__global__ void k_band_fill(Dev d, BandDev B, CondFactor f) {
   int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= d.nnzb * 36) return;
-  const int blk = (int)(t / 36), k = (int)(t % 36);
-  const int s = d.blk_sim[blk];
+  if (t >= f.red_n * 36) return;
+  const int blk = f.red[t / 36], k = (int)(t % 36);
+  const int rn = f.rnode[blk];
+  const int s = d.node_sim[rn];
   if (!d.active[s] || !B.refactor[s]) return;
-  const int b = B.bw[s];
-  if (b == 0) return;
-  const int row = blk_row[blk], colnode = d.col[blk];
-  const int r = k % 6, c = k / 6;
-  const int i = 6 * B.pos[row] + r, j = 6 * B.pos[colnode] + c;
-  const int64_t gr = 6 * (int64_t)row + r, gc = 6 * (int64_t)colnode + c;
-  double v = d.Kt[t];
-  if (d.fixed[gr] || d.fixed[gc]) v = (gr == gc) ? 1.0 : 0.0;
-  const int n = (int)(6 * (d.sim_node_off[s + 1] - d.sim_node_off[s]));
-  band_view(B, s, n).at(i, j) = (float)v;
+  const int ne = B.cond.ne[s];
+  const int i = 6 * (f.rpos[t / 36] - ne) + k / 6, j = 6 * (B.cond.scol[blk] - ne) + k % 6;
+  band_view(B, s, band_n(B, s)).at(i, j) = B.cond.S[(int64_t)blk * 36 + k];
 }
 
-// Zeroes the bands of the simulations about to be refactorised (one CTA per simulation).
+constexpr int kZeroCtas = 16;  // CTAs per simulation (one took 165 us for a 33 x 33 net's 10.6 MB band)
+
+// Zeroes the bands of the simulations about to be refactorised.
 __global__ void k_band_zero(Dev d, BandDev B) {
-  const int s = blockIdx.x;
+  const int s = blockIdx.x / kZeroCtas;
   if (!d.active[s] || !B.refactor[s] || B.bw[s] == 0) return;
-  if (threadIdx.x == 0 && B.lu_fail) B.lu_fail[s] = 0;
-  float* A = B.A + B.off[s];
-  const int64_t len = band_floats(6 * (d.sim_node_off[s + 1] - d.sim_node_off[s]), B.bw[s]);
-  for (int64_t i = threadIdx.x; i < len; i += blockDim.x) A[i] = 0.f;
+  const int part = blockIdx.x % kZeroCtas;
+  if (threadIdx.x == 0 && part == 0 && B.lu_fail) B.lu_fail[s] = 0;
+  float4* A = reinterpret_cast<float4*>(B.A + B.off[s]);  // offsets and lengths are multiples of 32 floats
+  const int64_t len = band_floats(band_n(B, s), B.bw[s]) / 4;
+  for (int64_t i = (int64_t)part * blockDim.x + threadIdx.x; i < len; i += kZeroCtas * (int64_t)blockDim.x)
+    A[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
-void launch_band_fill(const Dev& d, const BandDev& B, const int* blk_row, cudaStream_t s) {
-  k_band_zero<<<d.n_sims, 512, 0, s>>>(d, B);
-  if (d.nnzb) k_band_fill<<<nblocks(d.nnzb * 36, 256), 256, 0, s>>>(d, B, blk_row);
+void launch_band_fill(const Dev& d, const BandDev& B, const CondFactor& f, cudaStream_t s) {
+  k_band_zero<<<d.n_sims * kZeroCtas, 256, 0, s>>>(d, B);
+  if (f.red_n) k_band_fill<<<nblocks(f.red_n * 36, 256), 256, 0, s>>>(d, B, f);
 }
 
 // Blocked right-looking LU without pivoting of one simulation's band (one CTA
@@ -56,11 +53,10 @@ __global__ void __launch_bounds__(kLuThreads) k_band_lu(Dev d, BandDev B) {
   if (!d.active[s] || !B.refactor[s]) return;
   const int b = B.bw[s];
   if (b == 0) return;
-  const int64_t n0 = d.sim_node_off[s];
-  const int n = (int)(6 * (d.sim_node_off[s + 1] - n0));
+  const int n = band_n(B, s);
   const BandView V = band_view(B, s, n);
-  float* Li = B.Linv + inv_base(n0, s);  // per panel: kPanel x kPanel, column-major
-  float* Ui = B.Uinv + inv_base(n0, s);
+  float* Li = B.Linv + inv_base(B.cond.roff[s], s);  // per panel: kPanel x kPanel, column-major
+  float* Ui = B.Uinv + inv_base(B.cond.roff[s], s);
   extern __shared__ float smf[];
   const int ldp = kPanel + b;             // odd: column stride avoids bank conflicts
   float* P = smf;                         // panel, ldp x kPanel column-major

@@ -2,14 +2,15 @@
 //
 // The reference factorises Ktan_free exactly with MKL PARDISO on every
 // Newton iteration (src/linearsolvers.jl:15-23).  Here each simulation's
-// tangent is permuted (reverse Cuthill-McKee on the node graph, 6 DOFs per
+// tangent is condensed (eb_cond.cuh) onto the nodes that the condensation keeps,
+// these are permuted (reverse Cuthill-McKee on their graph, 6 DOFs per
 // node), copied into band storage in FP32 and factorised by one CTA
 // (blocked right-looking LU, no pivoting: the dynamic tangent carries the
 // positive mass term 1/(βΔt²)M on its diagonal).  The FP32 factors are the
 // GMRES preconditioner; GMRES itself measures and drives the FP64 residual,
 // so the factorisation's rounding only costs an iteration or two.
 //
-// Band storage of simulation s (N = 6 n_s DOFs, half bandwidth b), two
+// Band storage of simulation s (N = 6 x its kept nodes, half bandwidth b), two
 // column-major parts so that each triangular sweep streams one contiguous
 // block of 32 columns:
 //   U part (i <= j): U[(b + i - j) + (b + 1) j]      starts at off[s]
@@ -17,7 +18,7 @@
 // Both parts are padded to multiples of 32 floats plus 32 spare floats, so
 // 16-byte-rounded bulk copies of a trailing block stay inside the allocation.
 #pragma once
-#include "eb_internal.cuh"
+#include "eb_cond.cuh"
 
 namespace eb {
 
@@ -25,8 +26,8 @@ struct BandDev {
   float* A;                 // concatenated band storage (FP32: filled and factorised in place)
   const int64_t* off;       // per sim: offset of its U part in A (L part follows)
   const int* bw;            // per sim: half bandwidth b in DOFs (0: no band, block-Jacobi)
-  const int* pos;           // per global node: position in its simulation's band order
-  const int* node_at;       // per (node_off[s] + position): global node id
+  CondDev cond;             // condensation: eliminated nodes, blocks, levels
+  const int* node_at;       // per (node_off[s] + position): global node id (eliminated nodes first, then band order)
   float* work;              // per DOF scratch (permuted vector)
   float* Linv;              // per panel: inverse of the unit-lower diagonal block (column-major)
   float* Uinv;              // per panel: inverse of the upper diagonal block (column-major)
@@ -45,10 +46,14 @@ __host__ __device__ __forceinline__ int64_t band_floats(int64_t n, int b) {
   return ustride(n, b) + pad32(n * (int64_t)b);
 }
 
-// Offset of simulation s's diagonal-block inverses: one kPanel x kPanel
-// block per panel, with kPanel spare rows per simulation for the last panel.
-__host__ __device__ __forceinline__ int64_t inv_base(int64_t n0, int s) {
-  return (6 * n0 + (int64_t)kPanel * s) * kPanel;
+// Offset of simulation s's diagonal-block inverses (r0: kept nodes before it): one kPanel x
+// kPanel block per panel, with kPanel spare rows per simulation for the last panel.
+__host__ __device__ __forceinline__ int64_t inv_base(int64_t r0, int s) {
+  return (6 * r0 + (int64_t)kPanel * s) * kPanel;
+}
+// DOFs of simulation s that the condensation keeps (the band's size)
+__device__ __forceinline__ int band_n(const BandDev& B, int s) {
+  return (int)(6 * (B.cond.roff[s + 1] - B.cond.roff[s]));
 }
 
 struct BandView {
@@ -151,8 +156,9 @@ __device__ __forceinline__ float row_dot32(const float* col, int stride, const f
   return a0 + a1;
 }
 
-// z = M⁻¹ v on the CTA owning simulation s: gather into band order, forward
-// substitution with unit L, backward substitution with U, scatter back.
+// z = M⁻¹ v on the CTA owning simulation s (ntot DOFs): gather into the plan's order, forward
+// condensation levels, forward substitution with unit L and backward substitution with U on the
+// kept DOFs, backward levels, scatter back.
 //
 // Each sweep is a look-ahead pipeline over 32-row blocks with one CTA barrier
 // per block.  At step s of the forward sweep warp 0 applies block s-1 to the
@@ -161,25 +167,36 @@ __device__ __forceinline__ float row_dot32(const float* col, int stride, const f
 // block s ("far" rows); every row receives its block contributions in
 // increasing block order, so the result does not depend on timing.  The
 // backward sweep is the mirror image.  `xs` (may be null) is shared-memory
-// room for the n permuted entries; without it the rows the sweeps touch live
+// room for the n kept entries; without it the rows the sweeps touch live
 // in a shared ring.  With `st` non-null, band columns and inverses are
 // streamed into shared memory by bulk async copies one step ahead; bit k of
 // `ph` is barrier k's next phase and is advanced here.  Everything the sweeps
 // keep per thread (stage pointers, phase bits) is selected without indexing,
 // so it stays in registers: no local-memory load sits on the block chain.
 template <typename TV, typename TZ>
-__device__ __forceinline__ void band_solve(const BandDev& B, int s, int64_t n0, int n, const TV* __restrict__ v,
+__device__ __forceinline__ void band_solve(const BandDev& B, int s, int64_t n0, int ntot, const TV* __restrict__ v,
                                            TZ* __restrict__ z, float* xs, const Stage* st, uint32_t& ph) {
+  const int n = band_n(B, s);
   const BandView V = band_view(B, s, n);
   const int b = V.b;
-  float* x = xs ? xs : B.work + 6 * n0;
-  const float* Li = B.Linv + inv_base(n0, s);
-  const float* Ui = B.Uinv + inv_base(n0, s);
+  const int ne = B.cond.ne[s];
+  float* xa = B.work + 6 * n0;                        // all entries: eliminated positions, then the kept ones
+  float* x = xs ? xs : xa + 6 * ne;                   // the kept entries during the sweeps
+  const float* Li = B.Linv + inv_base(B.cond.roff[s], s);
+  const float* Ui = B.Uinv + inv_base(B.cond.roff[s], s);
   __shared__ __align__(16) float yb[2][kPanel];  // y of the last two blocks
-  for (int r = threadIdx.x; r < n; r += blockDim.x) {
+  for (int r = threadIdx.x; r < ntot; r += blockDim.x) {
     const int node = B.node_at[n0 + r / 6];           // global id of the node at position r/6
-    x[r] = (float)v[6 * (node - n0) + r % 6];
+    xa[r] = (float)v[6 * (node - n0) + r % 6];
   }
+  __syncthreads();
+  const int* lev = B.cond.lev_ptr + B.cond.lev_off[s];
+  const int nlev = B.cond.lev_off[s + 1] - B.cond.lev_off[s] - 1;
+  for (int l = 1; l < nlev; ++l) {  // level 0 receives nothing
+    cond_rows<true>(B.cond, n0, lev[l], lev[l + 1], xa, nullptr, ne);
+    __syncthreads();
+  }
+  cond_rows<true>(B.cond, n0, ne, ne + n / 6, xa, x, ne);
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nblk = (n + kPanel - 1) / kPanel;
@@ -406,14 +423,22 @@ __device__ __forceinline__ void band_solve(const BandDev& B, int s, int64_t n0, 
     __syncthreads();
   }
   __syncthreads();
-  for (int r = threadIdx.x; r < n; r += blockDim.x) {
+  if (xs) {
+    for (int r = threadIdx.x; r < n; r += blockDim.x) xa[6 * ne + r] = xs[r];
+    __syncthreads();
+  }
+  for (int l = nlev - 1; l >= 0; --l) {
+    cond_rows<false>(B.cond, n0, lev[l], lev[l + 1], xa, nullptr, ne);
+    __syncthreads();
+  }
+  for (int r = threadIdx.x; r < ntot; r += blockDim.x) {
     const int node = B.node_at[n0 + r / 6];
-    z[6 * (node - n0) + r % 6] = (TZ)x[r];
+    z[6 * (node - n0) + r % 6] = (TZ)xa[r];
   }
   __syncthreads();
 }
 
-void launch_band_fill(const Dev& d, const BandDev& B, const int* blk_row, cudaStream_t s);
+void launch_band_fill(const Dev& d, const BandDev& B, const CondFactor& f, cudaStream_t s);
 cudaError_t launch_band_lu(const Dev& d, const BandDev& B, int max_b, cudaStream_t s);
 // The same factorisation with the trailing updates on the tensor cores (eb_band_tc.cu); its
 // shared memory for the widest band of the launch is band_lu_tc_smem(max_b).

@@ -81,11 +81,10 @@ __global__ void __launch_bounds__(kTcThreads) k_band_lu_tc(Dev d, BandDev B, int
   if (!d.active[s] || !B.refactor[s]) return;
   const int b = B.bw[s];
   if (b == 0) return;
-  const int64_t n0 = d.sim_node_off[s];
-  const int n = (int)(6 * (d.sim_node_off[s + 1] - n0));
+  const int n = band_n(B, s);
   const BandView V = band_view(B, s, n);
-  float* Li = B.Linv + inv_base(n0, s);
-  float* Ui = B.Uinv + inv_base(n0, s);
+  float* Li = B.Linv + inv_base(B.cond.roff[s], s);
+  float* Ui = B.Uinv + inv_base(B.cond.roff[s], s);
   extern __shared__ __align__(1024) char smc[];
   uint64_t* bar = reinterpret_cast<uint64_t*>(smc);          // two MMA-completion barriers
   uint32_t* tslot = reinterpret_cast<uint32_t*>(smc + 64);   // tensor-memory base address

@@ -34,7 +34,7 @@ struct SolverArgs {
   int* status;           // per sim, max over the step
   BandDev band;          // band-LU preconditioner (bw[s] == 0: block-Jacobi for that sim)
   int x_in_smem;         // 1: the permuted solve vector lives in shared memory
-  int max_n;             // largest simulation, in DOFs
+  int max_n;             // most kept DOFs of a simulation of this launch
   int stage_floats;      // > 0: band blocks staged in shared memory, floats per buffer (32 (b_max + 1))
   int stage_test_extra;  // > 0: the first forward block waits for bytes no copy delivers (tests the bounded wait)
   // inexact Newton: 0 fixed tolerance `tol`; 1 Eisenstat-Walker forcing term from this solve's
