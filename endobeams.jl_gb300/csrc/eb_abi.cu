@@ -999,7 +999,8 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
   d.node_cptr = p_nc; d.node_contrib = p_ncl;
   CK(A.alloc(&d.K1, NB * 36)); CK(A.alloc(&d.C1, NB * 36)); CK(A.alloc(&d.M1, NB * 36));
   CK(A.alloc(&d.Kn, NB * 36)); CK(A.alloc(&d.Cn, NB * 36)); CK(A.alloc(&d.Mn, NB * 36));
-  CK(A.alloc(&d.Kt, NB * 36)); CK(A.alloc(&d.Kt32, NB * 36));
+  CK(A.alloc(&d.Kt, NB * 36));
+  if (p->precision == EB_PREC_MIXED) CK(A.alloc(&d.Ktp, NB * 36));
   CK(A.alloc(&d.D, ND)); CK(A.alloc(&d.Dd, ND)); CK(A.alloc(&d.Ddd, ND)); CK(A.alloc(&d.dD, ND)); CK(A.alloc(&d.r, ND));
   CK(A.upload(&d.fext1, fext)); CK(A.upload(&d.fextn, fext));
   CK(A.alloc(&d.Ti1, ND)); CK(A.alloc(&d.Tin, ND)); CK(A.alloc(&d.Tk1, ND)); CK(A.alloc(&d.Tkn, ND));
@@ -1023,9 +1024,9 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
   sa.sim_node_off = d.sim_node_off;
   sa.active = d.active;
   sa.row_ptr = d.row_ptr;
-  sa.col = d.col;
   sa.Kt = d.Kt;
-  sa.Kt32 = d.Kt32;
+  sa.Ktp = d.Ktp;
+  sa.team = 1;
   sa.Dinv64 = h->d_Dinv64;
   sa.Dinv32 = h->d_Dinv32;
   sa.fixed = d.fixed;
@@ -1174,6 +1175,14 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
       cf.red_n = (int64_t)red.size();
       cf.red = p_red; cf.rpos = p_rpos;
       h->band.node_at = p_nat;
+      std::vector<int> pcol(NB);
+      for (int64_t b = 0; b < NB; ++b) {
+        const int s = blk_sim[b];
+        pcol[b] = plan[s].pos[col[b] - h->node_off[s]];
+      }
+      int* p_pc;
+      CK(A.upload(&p_pc, pcol));
+      sa.pcol = p_pc;
       h->band.cond = cf.c;
     }
     int64_t *p_boff;
@@ -1260,12 +1269,19 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
         SolverArgs cb = args_for(big, false), cs = args_for(small, true);
         cb.cta_sim = p_cta;
         cs.cta_sim = p_cta + big.size();
+        cb.team = cs.team = 1;  // both classes present: teams only where one launch has the GPU to itself
         h->gclass = {cb, cs};
         CK(cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking));
         CK(cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming));
         CK(cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming));
       }
     }
+  }
+
+  if (h->gclass.empty()) {
+    int64_t nmax = 0;
+    for (int s = 0; s < n_sims; ++s) nmax = std::max(nmax, 6 * (h->node_off[s + 1] - h->node_off[s]));
+    sa.team = gmres_team(sa, fp32, p->threads_per_sim > 0 ? p->threads_per_sim : 256, (int)nmax);
   }
 
   // ---- learned warm start: neighbour table and surface flags (buffers for features on first use)

@@ -156,9 +156,8 @@ __device__ __forceinline__ float row_dot32(const float* col, int stride, const f
   return a0 + a1;
 }
 
-// z = M⁻¹ v on the CTA owning simulation s (ntot DOFs): gather into the plan's order, forward
-// condensation levels, forward substitution with unit L and backward substitution with U on the
-// kept DOFs, backward levels, scatter back.
+// xk <- U⁻¹ L⁻¹ xk on one CTA: forward substitution with unit L and backward substitution with
+// U over simulation s's kept DOFs, in place.
 //
 // Each sweep is a look-ahead pipeline over 32-row blocks with one CTA barrier
 // per block.  At step s of the forward sweep warp 0 applies block s-1 to the
@@ -167,36 +166,23 @@ __device__ __forceinline__ float row_dot32(const float* col, int stride, const f
 // block s ("far" rows); every row receives its block contributions in
 // increasing block order, so the result does not depend on timing.  The
 // backward sweep is the mirror image.  `xs` (may be null) is shared-memory
-// room for the n kept entries; without it the rows the sweeps touch live
+// room for the kept entries; without it the rows the sweeps touch live
 // in a shared ring.  With `st` non-null, band columns and inverses are
 // streamed into shared memory by bulk async copies one step ahead; bit k of
 // `ph` is barrier k's next phase and is advanced here.  Everything the sweeps
 // keep per thread (stage pointers, phase bits) is selected without indexing,
 // so it stays in registers: no local-memory load sits on the block chain.
-template <typename TV, typename TZ>
-__device__ __forceinline__ void band_solve(const BandDev& B, int s, int64_t n0, int ntot, const TV* __restrict__ v,
-                                           TZ* __restrict__ z, float* xs, const Stage* st, uint32_t& ph) {
+__device__ __forceinline__ void band_sweeps(const BandDev& B, int s, float* xk, float* xs, const Stage* st,
+                                            uint32_t& ph) {
   const int n = band_n(B, s);
   const BandView V = band_view(B, s, n);
   const int b = V.b;
-  const int ne = B.cond.ne[s];
-  float* xa = B.work + 6 * n0;                        // all entries: eliminated positions, then the kept ones
-  float* x = xs ? xs : xa + 6 * ne;                   // the kept entries during the sweeps
+  float* x = xs ? xs : xk;
   const float* Li = B.Linv + inv_base(B.cond.roff[s], s);
   const float* Ui = B.Uinv + inv_base(B.cond.roff[s], s);
   __shared__ __align__(16) float yb[2][kPanel];  // y of the last two blocks
-  for (int r = threadIdx.x; r < ntot; r += blockDim.x) {
-    const int node = B.node_at[n0 + r / 6];           // global id of the node at position r/6
-    xa[r] = (float)v[6 * (node - n0) + r % 6];
-  }
-  __syncthreads();
-  const int* lev = B.cond.lev_ptr + B.cond.lev_off[s];
-  const int nlev = B.cond.lev_off[s + 1] - B.cond.lev_off[s] - 1;
-  for (int l = 1; l < nlev; ++l) {  // level 0 receives nothing
-    cond_rows<true>(B.cond, n0, lev[l], lev[l + 1], xa, nullptr, ne);
-    __syncthreads();
-  }
-  cond_rows<true>(B.cond, n0, ne, ne + n / 6, xa, x, ne);
+  if (xs)
+    for (int r = threadIdx.x; r < n; r += blockDim.x) xs[r] = xk[r];
   __syncthreads();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nblk = (n + kPanel - 1) / kPanel;
@@ -423,19 +409,8 @@ __device__ __forceinline__ void band_solve(const BandDev& B, int s, int64_t n0, 
     __syncthreads();
   }
   __syncthreads();
-  if (xs) {
-    for (int r = threadIdx.x; r < n; r += blockDim.x) xa[6 * ne + r] = xs[r];
-    __syncthreads();
-  }
-  for (int l = nlev - 1; l >= 0; --l) {
-    cond_rows<false>(B.cond, n0, lev[l], lev[l + 1], xa, nullptr, ne);
-    __syncthreads();
-  }
-  for (int r = threadIdx.x; r < ntot; r += blockDim.x) {
-    const int node = B.node_at[n0 + r / 6];
-    z[6 * (node - n0) + r % 6] = (TZ)xa[r];
-  }
-  __syncthreads();
+  if (xs)
+    for (int r = threadIdx.x; r < n; r += blockDim.x) xk[r] = xs[r];
 }
 
 void launch_band_fill(const Dev& d, const BandDev& B, const CondFactor& f, cudaStream_t s);

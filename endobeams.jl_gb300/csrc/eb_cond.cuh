@@ -49,14 +49,15 @@ struct CondFactor {
   const int* rpos;          // positions of their rows
 };
 
-// Rows r of positions [p0, p1): y_r = (first block's product if `diag`) + Σ blocks; five positions
-// per warp so that a position's six rows are read before any of them is written (in place).
-// `x` holds the simulation's permuted vector; kept rows (position >= ne) are written to `xr`.
-template <bool FWD>
-__device__ __forceinline__ void cond_rows(const CondDev& c, int64_t base, int p0, int p1, float* x, float* xr, int ne) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+// Rows of positions [p0, p1) of one sweep phase, five positions per warp (`warp` of `nwarps`
+// working together), a position's six rows read before any of them is written (x is updated
+// in place).  x: the simulation's permuted vector; z (backward sweep): the result in T besides.
+template <bool FWD, typename T>
+__device__ __forceinline__ void cond_rows(const CondDev& c, int64_t base, int p0, int p1, float* x, T* z, int warp,
+                                          int nwarps) {
+  const int lane = threadIdx.x & 31;
   const int sub = lane / 6, r = lane - 6 * sub;
-  for (int q = p0 + 5 * warp; q < p1; q += 5 * nw) {
+  for (int q = p0 + 5 * warp; q < p1; q += 5 * nwarps) {
     const int p = q + sub;
     const bool on = sub < 5 && p < p1;
     float a0 = 0.f, a1 = 0.f;
@@ -75,8 +76,9 @@ __device__ __forceinline__ void cond_rows(const CondDev& c, int64_t base, int p0
     }
     __syncwarp();
     if (on) {
-      if (FWD && p >= ne) xr[6 * (p - ne) + r] = a0 + a1;
-      else x[6 * p + r] = a0 + a1;
+      const float y = a0 + a1;
+      x[6 * p + r] = y;
+      if (!FWD) z[6 * p + r] = (T)y;
     }
   }
 }

@@ -5,11 +5,12 @@
 // GMRES; the preconditioner is the condensation with the band LU of the kept
 // nodes (eb_cond.cuh, eb_band.cuh) or 6x6 block-Jacobi (the LU of each node's
 // diagonal block, fixed DOFs replaced by identity rows/columns).  Each
-// simulation is owned by one CTA for the whole solve: its Krylov basis
-// lives in global memory (L2-resident for the sizes of a batched run), its
-// Hessenberg matrix and Givens rotations in shared memory, and every
-// reduction is a fixed-order block reduction, so results do not depend on
-// how many simulations share the launch.
+// simulation is owned by one team of CTAs (a cluster of 1 to 16, so that few
+// simulations use many SMs) for the whole solve: its Krylov basis lives in
+// global memory in the preconditioner's node order, its Hessenberg matrix and
+// Givens rotations in every CTA's shared memory, and every sum has an order
+// fixed by the simulation's size, so results do not depend on how many CTAs
+// work on a simulation or how many simulations share the launch.
 //
 // Precision: the outer loop always measures the true residual b - A x in
 // FP64.  Each pass runs one GMRES(m) cycle on that residual, in FP64
@@ -24,93 +25,178 @@
 
 namespace eb {
 
-template <int NV>
-__device__ __forceinline__ void block_sum(double (&v)[NV], double* red) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-#pragma unroll
-  for (int q = 0; q < NV; ++q)
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) v[q] += __shfl_down_sync(0xffffffffu, v[q], off);
-  if (lane == 0)
-#pragma unroll
-    for (int q = 0; q < NV; ++q) red[q * 32 + warp] = v[q];
-  __syncthreads();
-  if (warp == 0) {
-#pragma unroll
-    for (int q = 0; q < NV; ++q) {
-      double x = lane < nw ? red[q * 32 + lane] : 0.0;
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) x += __shfl_down_sync(0xffffffffu, x, off);
-      if (lane == 0) red[q * 32] = x;
+// The CTAs of one simulation: a cluster of `size` (1: a single CTA).
+struct Team {
+  int rank, size;
+  __device__ __forceinline__ void sync() const {
+    if (size == 1) {
+      __syncthreads();
+    } else {
+      // release / acquire at cluster scope: global and shared writes of the other CTAs are seen
+      asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
     }
   }
-  __syncthreads();
-#pragma unroll
-  for (int q = 0; q < NV; ++q) v[q] = red[q * 32];
-  __syncthreads();
-}
+};
 
-// y = P A x over the rows of one simulation (P zeroes fixed rows).
-template <typename TA, typename TX, typename TY, typename TACC>
-__device__ __forceinline__ void cta_spmv(const TA* __restrict__ A, const int* __restrict__ row_ptr,
-                                         const int* __restrict__ col, int64_t n0, int n, const TX* __restrict__ x,
-                                         TY* __restrict__ y, const uint8_t* __restrict__ fx) {
-  for (int r = threadIdx.x; r < n; r += blockDim.x) {
-    const int64_t node = n0 + r / 6;
-    const int k = r % 6;
-    TACC acc = 0;
-    for (int bb = row_ptr[node]; bb < row_ptr[node + 1]; ++bb) {
-      const int c = (int)(col[bb] - n0);
-      const TA* Ab = A + (int64_t)bb * 36 + k;
-      const TX* xc = x + 6 * c;
-#pragma unroll
-      for (int j = 0; j < 6; ++j) acc += (TACC)Ab[6 * j] * (TACC)xc[j];
+// Vectors are cut into chunks whose length depends on the simulation alone (at most
+// kMaxChunks of them); a warp owns whole chunks, and sums are formed chunk by chunk and then
+// over the chunks in one fixed order, so no result depends on the number of CTAs or threads.
+constexpr int kMaxChunks = 128;
+__device__ __forceinline__ int chunk_len(int n) { return ((n + kMaxChunks - 1) / kMaxChunks + 31) / 32 * 32; }
+
+struct Work {
+  Team t;
+  int n, ch, nchunk;     // DOFs, chunk length, chunks
+  int warp0, nwarps;     // this warp's first chunk, stride between its chunks
+  double* part[2];       // chunk sums of a reduction (kMaxChunks x 8), used in turn
+  double* sums;          // 8
+  int flip;
+  template <typename F>
+  __device__ __forceinline__ void each(F f) const {  // f(i) over this warp's chunks
+    const int lane = threadIdx.x & 31;
+    for (int c = warp0; c < nchunk; c += nwarps) {
+      const int i1 = min(n, (c + 1) * ch);
+      for (int i = c * ch + lane; i < i1; i += 32) f(i);
     }
-    y[r] = fx[r] ? (TY)0 : (TY)acc;
   }
+};
+
+// out[q] = Σ_i of what f(i, acc) adds to acc[q]: per lane in TA, over lanes and chunks in FP64.  Each
+// chunk's sums go to every CTA of the team; one team barrier; two buffers in turn, so that a CTA
+// that is ahead does not overwrite sums that another still reads.
+template <int NQ, typename TA, typename F>
+__device__ __forceinline__ void team_sum(Work& w, double (&out)[NQ], F f) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  double* part = w.flip ? w.part[1] : w.part[0];
+  w.flip ^= 1;
+  for (int c = w.warp0; c < w.nchunk; c += w.nwarps) {
+    TA acc[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) acc[q] = 0;
+    const int i1 = min(w.n, (c + 1) * w.ch);
+    for (int i = c * w.ch + lane; i < i1; i += 32) f(i, acc);
+    double v[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; ++q) {
+      v[q] = (double)acc[q];
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], off);
+    }
+    if (w.t.size == 1) {
+      if (lane == 0)
+#pragma unroll
+        for (int q = 0; q < NQ; ++q) part[q * kMaxChunks + c] = v[q];
+    } else if (lane < w.t.size) {  // lane r writes CTA r's copy
+#pragma unroll
+      for (int q = 0; q < NQ; ++q) {
+        uint32_t a;
+        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(part + q * kMaxChunks + c)), "r"(lane));
+        asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v[q]) : "memory");
+      }
+    }
+  }
+  w.t.sync();
+  for (int q = warp; q < NQ; q += nw) {
+    double s = 0.0;
+    for (int c = lane; c < w.nchunk; c += 32) s += part[q * kMaxChunks + c];
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+    if (lane == 0) w.sums[q] = s;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) out[q] = w.sums[q];
 }
 
-// z = M⁻¹ v with M the block diagonal
-template <typename TM, typename TV, typename TZ>
-__device__ __forceinline__ void cta_prec(const TM* __restrict__ Dinv, int64_t n0, int n, const TV* __restrict__ v,
-                                         TZ* __restrict__ z) {
-  for (int r = threadIdx.x; r < n; r += blockDim.x) {
-    const int nl = r / 6, k = r % 6;
-    const TM* Db = Dinv + (n0 + nl) * 36 + k;
-    const TV* vv = v + 6 * nl;
-    TM acc = 0;
+// Row i of P A x in FP64 (P zeroes fixed rows); vectors are in the solver's order.
+template <typename TX>
+__device__ __forceinline__ double row64(const SolverArgs& a, int64_t n0, int i, const TX* x) {
+  const int p = i / 6, k = i - 6 * p;
+  const int node = a.band.node_at[n0 + p];
+  if (a.fixed[6 * (int64_t)node + k]) return 0.0;
+  double acc = 0.0;
+  for (int bb = a.row_ptr[node]; bb < a.row_ptr[node + 1]; ++bb) {
+    const double* Ab = a.Kt + (int64_t)bb * 36 + k;
+    const TX* xc = x + 6 * a.pcol[bb];
 #pragma unroll
-    for (int j = 0; j < 6; ++j) acc += Db[6 * j] * (TM)vv[j];
-    z[r] = (TZ)acc;
+    for (int j = 0; j < 6; ++j) acc += Ab[6 * j] * (double)xc[j];
   }
+  return acc;
+}
+
+// The same row from the tangent as FP32 pairs (hi + lo carry 48 bits of it), summed as FP32
+// pairs (exact products by FMA, Knuth's two-sum): an FP64 sum's error in FP32 operations, of
+// which an SM does 64 times as many.  With plain FP32 products the Arnoldi relation was off by
+// 1e-4 of the residual and most solves to 1e-4 ended just above their target, one cycle more
+// each (24-wire stent: 12 cycles and 36 iterations a step, now 6 and 32).
+__device__ __forceinline__ float row_pairs(const SolverArgs& a, int64_t n0, int i, const float* x) {
+  const int p = i / 6, k = i - 6 * p;
+  const int node = a.band.node_at[n0 + p];
+  if (a.fixed[6 * (int64_t)node + k]) return 0.f;
+  float hi = 0.f, lo = 0.f;
+  for (int bb = a.row_ptr[node]; bb < a.row_ptr[node + 1]; ++bb) {
+    const float2* Ab = a.Ktp + (int64_t)bb * 36 + k;
+    const float* xc = x + 6 * a.pcol[bb];
+#pragma unroll
+    for (int j = 0; j < 6; ++j) {
+      const float2 e = Ab[6 * j];
+      const float xv = xc[j];
+      const float q = __fmul_rn(e.x, xv), qe = __fmaf_rn(e.x, xv, -q);
+      const float s = __fadd_rn(hi, q), t = __fsub_rn(s, hi);
+      const float err = __fadd_rn(__fsub_rn(hi, __fsub_rn(s, t)), __fsub_rn(q, t));
+      hi = s;
+      lo = __fadd_rn(lo, __fadd_rn(err, __fmaf_rn(e.y, xv, qe)));
+    }
+  }
+  return hi + lo;
 }
 
 template <typename T>
 __global__ void __launch_bounds__(512) k_gmres(SolverArgs a) {
-  const int s = a.cta_sim[blockIdx.x];
+  Work wk;
+  {
+    uint32_t r, c;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(c));
+    wk.t = Team{(int)r, (int)c};
+  }
+  const Team& team = wk.t;
+  const int s = a.cta_sim[blockIdx.x / team.size];
   if (!a.active[s]) return;
   const int m = a.m;
   const int64_t n0 = a.sim_node_off[s];
   const int64_t o = 6 * n0;
   const int n = (int)(6 * (a.sim_node_off[s + 1] - n0));
   extern __shared__ double sm[];
-  double* H = sm;                  // (m+1) x m, column j at H + (m+1) j
+  double* H = sm;                  // (m+1) x m, column j at H + (m+1) j; every CTA keeps its own copy
   double* cs = H + (m + 1) * m;
   double* sn = cs + m;
   double* g = sn + m;              // m+1
   double* y = g + m + 1;           // m
-  double* red = y + m;             // 8 x 32
+  wk.part[0] = y + m;
+  wk.part[1] = wk.part[0] + 8 * kMaxChunks;
+  wk.sums = wk.part[1] + 8 * kMaxChunks;
+  wk.flip = 0;
+  wk.n = n;
+  wk.ch = chunk_len(n);
+  wk.nchunk = (n + wk.ch - 1) / wk.ch;
+  wk.warp0 = team.rank * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  wk.nwarps = team.size * (blockDim.x >> 5);
   T* V = reinterpret_cast<T*>(a.V) + (int64_t)(m + 1) * o;
   T* Zb = reinterpret_cast<T*>(a.Z) + (int64_t)m * o;  // z_j = M⁻¹ v_j at Zb + j n
   double* X = a.X + o;
   double* R = a.R64 + o;
-  const double* b = a.b + o;
-  const uint8_t* fx = a.fixed + o;
+  float* xa = a.band.work + o;     // the vector the preconditioner works on
+  const int* node_at = a.band.node_at + n0;
+  auto dof = [&](int i) { return 6 * (int64_t)node_at[i / 6] + i % 6; };  // caller's DOF of entry i
   const T* Dm = std::is_same<T, double>::value ? reinterpret_cast<const T*>(a.Dinv64)
                                               : reinterpret_cast<const T*>(a.Dinv32);
-  using TACC = T;
   const bool use_band = a.band.bw != nullptr && a.band.bw[s] > 0;
-  float* xs = a.x_in_smem ? reinterpret_cast<float*>(red + 8 * 32) : nullptr;  // permuted solve vector
+  const CondDev& cd = a.band.cond;
+  const int ne = cd.ne[s];
+  const int* lev = cd.lev_ptr + cd.lev_off[s];
+  const int nlev = max(0, cd.lev_off[s + 1] - cd.lev_off[s] - 1);
+  float* xs = a.x_in_smem ? reinterpret_cast<float*>(wk.sums + 8) : nullptr;  // the kept entries during the sweeps
   // shared-memory staging of band blocks for the triangular solves (bulk async copies)
   __shared__ __align__(8) uint64_t bars[4];
   __shared__ int stage_fail;
@@ -118,8 +204,8 @@ __global__ void __launch_bounds__(512) k_gmres(SolverArgs a) {
   Stage stage;
   const Stage* stp = nullptr;
   uint32_t ph = 0u;  // bit k: next phase of staging barrier k
-  if (use_band && a.stage_floats > 0) {
-    char* base = reinterpret_cast<char*>(xs ? xs + a.max_n : reinterpret_cast<float*>(red + 8 * 32));
+  if (use_band && a.stage_floats > 0 && team.rank == 0) {
+    char* base = reinterpret_cast<char*>(xs ? xs + a.max_n : reinterpret_cast<float*>(wk.sums + 8));
     base = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(base) + 127) & ~uintptr_t(127));
     // two band-column buffers of stage_floats = 32 (b_max + 1) floats, then the inverses
     float* f = reinterpret_cast<float*>(base);
@@ -142,43 +228,39 @@ __global__ void __launch_bounds__(512) k_gmres(SolverArgs a) {
     __syncthreads();
     stp = &stage;
   }
+  team.sync();  // every CTA of the team runs before any writes another's shared memory
 
-  double v1[1] = {0.0};
   const bool use_x0 = a.x0_on != nullptr && a.x0_on[s] != 0;
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const double bi = fx[i] ? 0.0 : b[i];
-    X[i] = (use_x0 && !fx[i]) ? a.dD[o + i] : 0.0;
+  double v1[1];
+  team_sum<1, double>(wk, v1, [&](int i, double (&q)[1]) {
+    const int64_t d = dof(i);
+    const bool fx = a.fixed[d];
+    const double bi = fx ? 0.0 : a.b[d];
+    X[i] = (use_x0 && !fx) ? a.dD[d] : 0.0;
     R[i] = bi;
-    v1[0] += bi * bi;
-  }
-  block_sum<1>(v1, red);
+    q[0] += bi * bi;
+  });
   const double bnorm = sqrt(v1[0]);
   double rnorm = bnorm;
   if (use_x0 && isfinite(bnorm)) {
     // initial guess: X = α x0 with α = <A x0, b> / <A x0, A x0> clipped to [0, 1], so that
     // ‖b − A X‖ <= ‖b‖ (a guess that does not help costs one FP64 product)
-    cta_spmv<double, double, double, double>(a.Kt, a.row_ptr, a.col, n0, n, X, R, fx);
-    __syncthreads();
-    double yb[2] = {0.0, 0.0};
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      const double bi = fx[i] ? 0.0 : b[i];
-      yb[0] += R[i] * bi;
-      yb[1] += R[i] * R[i];
-    }
-    block_sum<2>(yb, red);
+    double yb[2];
+    team_sum<2, double>(wk, yb, [&](int i, double (&q)[2]) {
+      const double bi = R[i], ax = row64(a, n0, i, X);
+      q[0] += ax * bi;
+      q[1] += ax * ax;
+    });
     double alpha = yb[1] > 0.0 ? yb[0] / yb[1] : 0.0;
     if (!(alpha > 0.0)) alpha = 0.0;
     if (alpha > 1.0) alpha = 1.0;
-    double rr0[1] = {0.0};
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-      const double bi = fx[i] ? 0.0 : b[i];
-      X[i] *= alpha;
-      const double ri = bi - alpha * R[i];
+    team_sum<1, double>(wk, v1, [&](int i, double (&q)[1]) {
+      const double ri = R[i] - alpha * row64(a, n0, i, X);
       R[i] = ri;
-      rr0[0] += ri * ri;
-    }
-    block_sum<1>(rr0, red);
-    rnorm = sqrt(rr0[0]);
+      q[0] += ri * ri;
+    });
+    wk.each([&](int i) { X[i] *= alpha; });
+    rnorm = sqrt(v1[0]);
   }
   int its = 0, refs = 0, status = 0;
   if (!isfinite(bnorm)) status = 2;  // EB_SIM_NAN
@@ -197,8 +279,8 @@ __global__ void __launch_bounds__(512) k_gmres(SolverArgs a) {
       eta = fmin(fmax(eta, a.tol), a.forcing_max);
     }
     rtol = eta;
-    __syncthreads();  // every thread has read the previous values
-    if (threadIdx.x == 0) {
+    team.sync();  // every thread has read the previous values
+    if (threadIdx.x == 0 && team.rank == 0) {
       a.prev_bnorm[s] = bnorm;
       a.prev_eta[s] = eta;
     }
@@ -209,9 +291,13 @@ __global__ void __launch_bounds__(512) k_gmres(SolverArgs a) {
       // ---- one GMRES(m) cycle on the FP64 residual R
       const double beta = rnorm;
       const double ib = 1.0 / beta;
-      for (int i = threadIdx.x; i < n; i += blockDim.x) V[i] = (T)(R[i] * ib);
+      wk.each([&](int i) {
+        const T v = (T)(R[i] * ib);
+        V[i] = v;
+        xa[i] = (float)v;
+      });
       if (threadIdx.x == 0) g[0] = beta;
-      __syncthreads();
+      team.sync();
       // a cycle that can reach the target aims at half of it, from zero as from an initial guess: its
       // estimate differs from the true residual by rounding, and a residual left just above the
       // target costs another cycle
@@ -220,57 +306,80 @@ __global__ void __launch_bounds__(512) k_gmres(SolverArgs a) {
       int k = 0;  // dimension of the Krylov space built in this cycle
       const int jmax = min(m, a.max_iter - its);
       for (int j = 0; j < jmax; ++j) {
-        T* vj = V + (int64_t)j * n;
         T* w = V + (int64_t)(j + 1) * n;
         T* zj = Zb + (int64_t)j * n;
-        if (use_band) band_solve<T, T>(a.band, s, n0, n, vj, zj, xs, stp, ph);
-        else cta_prec<T, T, T>(Dm, n0, n, vj, zj);
-        __syncthreads();
-        // w = A z from the FP64 tangent also in FP32 cycles: with FP32 products the Arnoldi relation
-        // was off by 1e-4 of the residual and most solves to 1e-4 ended just above their target,
-        // one cycle more each (24-wire stent: 12 cycles and 36 iterations a step, now 6 and 32)
-        cta_spmv<double, T, T, double>(a.Kt, a.row_ptr, a.col, n0, n, zj, w, fx);
-        __syncthreads();
-        // classical Gram-Schmidt, twice
+        // ---- z_j = M⁻¹ v_j; v_j lies in xa (FP32) when the preconditioner starts
+        if (use_band) {
+          for (int l = 1; l < nlev; ++l) {  // level 0 receives nothing
+            cond_rows<true>(cd, n0, lev[l], lev[l + 1], xa, (T*)nullptr, wk.warp0, wk.nwarps);
+            team.sync();
+          }
+          if (ne > 0) {
+            cond_rows<true>(cd, n0, ne, n / 6, xa, (T*)nullptr, wk.warp0, wk.nwarps);
+            team.sync();
+          }
+          if (team.rank == 0) band_sweeps(a.band, s, xa + 6 * ne, xs, stp, ph);
+          team.sync();
+          for (int i = 6 * ne + wk.warp0 * 32 + (threadIdx.x & 31); i < n; i += 32 * wk.nwarps) zj[i] = (T)xa[i];
+          for (int l = nlev - 1; l >= 0; --l) {
+            cond_rows<false>(cd, n0, lev[l], lev[l + 1], xa, zj, wk.warp0, wk.nwarps);
+            team.sync();
+          }
+          if (nlev == 0) team.sync();
+        } else {
+          const T* vj = V + (int64_t)j * n;
+          wk.each([&](int i) {
+            const int p = i / 6, r = i - 6 * p;
+            const T* Db = Dm + (int64_t)node_at[p] * 36 + r;
+            T acc = 0;
+#pragma unroll
+            for (int q = 0; q < 6; ++q) acc += Db[6 * q] * vj[6 * p + q];
+            zj[i] = acc;
+          });
+          team.sync();
+        }
+        // ---- w = A z_j, orthogonalised by classical Gram-Schmidt, twice
+        wk.each([&](int i) {
+          if constexpr (std::is_same<T, double>::value) w[i] = row64(a, n0, i, zj);
+          else w[i] = row_pairs(a, n0, i, zj);
+        });
+        __syncwarp();
         for (int pass = 0; pass < 2; ++pass) {
           for (int i0 = 0; i0 <= j; i0 += 8) {
-            TACC hl[8];
-#pragma unroll
-            for (int q = 0; q < 8; ++q) hl[q] = 0;
             const int nq = min(8, j + 1 - i0);
-            for (int i = threadIdx.x; i < n; i += blockDim.x) {
-              const TACC wi = (TACC)w[i];
-#pragma unroll
-              for (int q = 0; q < 8; ++q)
-                if (q < nq) hl[q] += (TACC)V[(int64_t)(i0 + q) * n + i] * wi;
-            }
+            const T* Vq = V + (int64_t)i0 * n;
             double hp[8];
+            team_sum<8, T>(wk, hp, [&](int i, T (&q)[8]) {
+              const T wi = w[i];
 #pragma unroll
-            for (int q = 0; q < 8; ++q) hp[q] = (double)hl[q];
-            block_sum<8>(hp, red);
+              for (int u = 0; u < 8; ++u)
+                if (u < nq) q[u] += Vq[(int64_t)u * n + i] * wi;
+            });
             if (threadIdx.x == 0)
-              for (int q = 0; q < nq; ++q) H[(m + 1) * j + i0 + q] = (pass == 0 ? 0.0 : H[(m + 1) * j + i0 + q]) + hp[q];
-            // stash this chunk's coefficients in y (free until the back-substitution)
-#pragma unroll
-            for (int q = 0; q < 8; ++q)
-              if (threadIdx.x == q && q < nq) y[i0 + q] = hp[q];
-            __syncthreads();
-          }
-          for (int i = threadIdx.x; i < n; i += blockDim.x) {
-            TACC acc = (TACC)w[i];
-            for (int q = 0; q <= j; ++q) acc -= (TACC)y[q] * (TACC)V[(int64_t)q * n + i];
-            w[i] = (T)acc;
+              for (int q = 0; q < nq; ++q) {
+                double* h = H + (m + 1) * j + i0 + q;
+                *h = (pass == 0 ? 0.0 : *h) + hp[q];
+                y[i0 + q] = hp[q];  // this pass's coefficients (y is free until the back-substitution)
+              }
           }
           __syncthreads();
+          wk.each([&](int i) {
+            T acc = w[i];
+            for (int q = 0; q <= j; ++q) acc -= (T)y[q] * V[(int64_t)q * n + i];
+            w[i] = acc;
+          });
+          __syncthreads();  // y is read before the next pass rewrites it
         }
-        TACC nl = 0;
-        for (int i = threadIdx.x; i < n; i += blockDim.x) nl += (TACC)w[i] * (TACC)w[i];
-        double nn[1] = {(double)nl};
-        block_sum<1>(nn, red);
+        double nn[1];
+        team_sum<1, T>(wk, nn, [&](int i, T (&q)[1]) { q[0] += w[i] * w[i]; });
         const double hn = sqrt(nn[0]);
         if (hn > 0.0) {
           const T ihn = (T)(1.0 / hn);
-          for (int i = threadIdx.x; i < n; i += blockDim.x) w[i] = w[i] * ihn;
+          wk.each([&](int i) {
+            const T v = w[i] * ihn;
+            w[i] = v;
+            xa[i] = (float)v;
+          });
         }
         if (threadIdx.x == 0) {
           double* Hj = H + (m + 1) * j;
@@ -290,7 +399,7 @@ __global__ void __launch_bounds__(512) k_gmres(SolverArgs a) {
           g[j + 1] = -sv * g[j];
           g[j] = c * g[j];
         }
-        __syncthreads();
+        team.sync();
         ++its;
         k = j + 1;
         const double gres = fabs(g[j + 1]);
@@ -307,23 +416,20 @@ __global__ void __launch_bounds__(512) k_gmres(SolverArgs a) {
       __syncthreads();
       // X += M⁻¹ V y = Z y: the preconditioned basis was kept, so the update needs no further
       // preconditioner application (one band solve per cycle saved)
-      for (int i = threadIdx.x; i < n; i += blockDim.x) {
+      wk.each([&](int i) {
         double acc = 0.0;
         for (int q = 0; q < k; ++q) acc += y[q] * (double)Zb[(int64_t)q * n + i];
         X[i] += acc;
-      }
-      __syncthreads();
+      });
+      team.sync();
       // true FP64 residual R = b - Ktan X
-      cta_spmv<double, double, double, double>(a.Kt, a.row_ptr, a.col, n0, n, X, R, fx);
-      __syncthreads();
-      double rr[1] = {0.0};
-      for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const double ri = (fx[i] ? 0.0 : b[i]) - R[i];
+      team_sum<1, double>(wk, v1, [&](int i, double (&q)[1]) {
+        const int64_t d = dof(i);
+        const double ri = (a.fixed[d] ? 0.0 : a.b[d]) - row64(a, n0, i, X);
         R[i] = ri;
-        rr[0] += ri * ri;
-      }
-      block_sum<1>(rr, red);
-      rnorm = sqrt(rr[0]);
+        q[0] += ri * ri;
+      });
+      rnorm = sqrt(v1[0]);
       ++refs;
       if (!isfinite(rnorm)) { status = 2; break; }
     }
@@ -335,22 +441,24 @@ __global__ void __launch_bounds__(512) k_gmres(SolverArgs a) {
     stage_drain(stp);
   }
 
-  // ΔD[free] = x; Newton norms of compute_norms_corrector (utils_solver.jl:126-151)
-  double q[4] = {0.0, 0.0, 0.0, 0.0};
-  for (int i = threadIdx.x; i < n; i += blockDim.x) {
-    const double f = (a.fext1[o + i] + a.Tc1[o + i]) + a.Tk1[o + i];
-    if (fx[i]) {
-      q[3] += f * f;
+  // ΔD[free] = x; Newton norms of compute_norms_corrector (utils_solver.jl:126-151).  The
+  // increment is written whenever the solve was finite, also where a staging wait ran out (rank 0
+  // knows it and reports the step as not converged).
+  double q[4];
+  team_sum<4, double>(wk, q, [&](int i, double (&v)[4]) {
+    const int64_t d = dof(i);
+    const double f = (a.fext1[d] + a.Tc1[d]) + a.Tk1[d];
+    if (a.fixed[d]) {
+      v[3] += f * f;
     } else {
       const double x = (bnorm > 0.0 && status != 2) ? X[i] : 0.0;
-      a.dD[o + i] = x;
-      q[0] += x * x;
-      q[1] += b[i] * b[i];
-      q[2] += f * f;
+      a.dD[d] = x;
+      v[0] += x * x;
+      v[1] += a.b[d] * a.b[d];
+      v[2] += f * f;
     }
-  }
-  block_sum<4>(q, red);
-  if (threadIdx.x == 0) {
+  });
+  if (threadIdx.x == 0 && team.rank == 0) {
     a.norms[5 * s + 0] = q[0];
     a.norms[5 * s + 1] = q[1];
     a.norms[5 * s + 2] = q[2];
@@ -410,7 +518,9 @@ void launch_block_jacobi(const Dev& d, double* Dinv64, float* Dinv32, cudaStream
   if (d.n_nodes) k_block_jacobi<<<nblocks(d.n_nodes), kThreads, 0, s>>>(d, Dinv64, Dinv32);
 }
 
-size_t gmres_smem(int m) { return sizeof(double) * ((size_t)(m + 1) * m + 4 * (size_t)m + 1 + 8 * 32); }
+size_t gmres_smem(int m) {
+  return sizeof(double) * ((size_t)(m + 1) * m + 4 * (size_t)m + 1 + 16 * (size_t)kMaxChunks + 8);
+}
 
 size_t gmres_smem_total(const SolverArgs& a) {
   return gmres_smem(a.m) + (a.x_in_smem ? sizeof(float) * (size_t)a.max_n : 0) +
@@ -419,20 +529,58 @@ size_t gmres_smem_total(const SolverArgs& a) {
                              : 0);
 }
 
-cudaError_t launch_gmres(const SolverArgs& a, bool fp32, int threads, cudaStream_t s) {
-  const size_t smem = gmres_smem_total(a);
-  // shared memory is the occupancy limit: prefer the largest carveout so two CTAs fit when they can
-  cudaFuncSetAttribute(k_gmres<float>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-  cudaFuncSetAttribute(k_gmres<double>, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-  if (fp32) {
-    cudaError_t e = raise_smem_limit((const void*)k_gmres<float>, smem);
-    if (e != cudaSuccess) return e;
-    k_gmres<float><<<a.n_sims, threads, smem, s>>>(a);
-  } else {
-    cudaError_t e = raise_smem_limit((const void*)k_gmres<double>, smem);
-    if (e != cudaSuccess) return e;
-    k_gmres<double><<<a.n_sims, threads, smem, s>>>(a);
+namespace {
+const void* gmres_kernel(bool fp32) { return fp32 ? (const void*)k_gmres<float> : (const void*)k_gmres<double>; }
+
+cudaLaunchConfig_t gmres_config(const SolverArgs& a, int threads, cudaStream_t s, cudaLaunchAttribute* at) {
+  cudaLaunchConfig_t c{};
+  c.gridDim = dim3((unsigned)(a.n_sims * a.team));
+  c.blockDim = dim3((unsigned)threads);
+  c.dynamicSmemBytes = gmres_smem_total(a);
+  c.stream = s;
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)a.team;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  c.attrs = at;
+  c.numAttrs = 1;
+  return c;
+}
+}  // namespace
+
+// CTAs per simulation of a launch: the largest power of two up to 16 for which all teams are
+// resident at once and every CTA still has kTeamDofs entries of the largest simulation.
+int gmres_team(const SolverArgs& a, bool fp32, int threads, int max_dofs) {
+  const void* k = gmres_kernel(fp32);
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return 1;
+  if (raise_smem_limit(k, gmres_smem_total(a)) != cudaSuccess) return 1;
+  cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  for (int t = 16; t > 1; t /= 2) {
+    if (a.n_sims * t > sms || (t / 2) * kTeamDofs >= max_dofs) continue;
+    SolverArgs b = a;
+    b.team = t;
+    cudaLaunchAttribute at[1];
+    const cudaLaunchConfig_t c = gmres_config(b, threads, 0, at);
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, k, &c) == cudaSuccess && clusters >= a.n_sims) return t;
+    cudaGetLastError();
   }
+  return 1;
+}
+
+cudaError_t launch_gmres(const SolverArgs& a, bool fp32, int threads, cudaStream_t s) {
+  // shared memory is the occupancy limit: prefer the largest carveout so two CTAs fit when they can
+  const void* k = gmres_kernel(fp32);
+  cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 100);
+  cudaError_t e = raise_smem_limit(k, gmres_smem_total(a));
+  if (e != cudaSuccess) return e;
+  if (a.team > 8) cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  cudaLaunchAttribute at[1];
+  const cudaLaunchConfig_t c = gmres_config(a, threads, s, at);
+  void* args[1] = {const_cast<SolverArgs*>(&a)};
+  e = cudaLaunchKernelExC(&c, k, args);
+  if (e != cudaSuccess) return e;
   return cudaGetLastError();
 }
 

@@ -5,14 +5,15 @@
 namespace eb {
 
 struct SolverArgs {
-  int n_sims;            // CTAs of this launch (one simulation each)
-  const int* cta_sim;    // CTA -> simulation
+  int n_sims;            // simulations of this launch
+  int team;              // CTAs per simulation (cluster size)
+  const int* cta_sim;    // team -> simulation
   const int64_t* sim_node_off;
   const int* active;
   const int* row_ptr;
-  const int* col;
+  const int* pcol;       // per block of the tangent: position of its column node in the solver's order
   const double* Kt;
-  const float* Kt32;
+  const float2* Ktp;     // the tangent as FP32 pairs (mixed precision)
   const double* Dinv64;
   const float* Dinv32;
   const uint8_t* fixed;
@@ -48,6 +49,8 @@ struct SolverArgs {
 };
 
 void launch_block_jacobi(const Dev& d, double* Dinv64, float* Dinv32, cudaStream_t s);
+constexpr int kTeamDofs = 512;  // fewest DOFs per CTA of a team
+int gmres_team(const SolverArgs& a, bool fp32, int threads, int max_dofs);
 cudaError_t launch_gmres(const SolverArgs& a, bool fp32, int threads, cudaStream_t s);
 size_t gmres_smem(int m);
 size_t gmres_smem_total(const SolverArgs& a);  // dynamic shared memory of one launch

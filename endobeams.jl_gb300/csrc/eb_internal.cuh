@@ -76,7 +76,7 @@ struct Dev {
   const int* node_contrib;// 2 e + I
   double *K1, *C1, *M1, *Kn, *Cn, *Mn;  // nnzb * 36
   double* Kt;                           // tangent, FP64
-  float* Kt32;                          // tangent, FP32 copy
+  float2* Ktp;                          // tangent as FP32 pairs (mixed precision; null otherwise)
 
   // ---- launch shapes (threads per block), chosen by eb_autotune among shapes whose
   // results are bitwise identical

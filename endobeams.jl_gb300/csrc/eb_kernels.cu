@@ -90,6 +90,12 @@ void launch_contact(const Dev& d, const Gauss3& g, cudaStream_t s) {
   if (d.n_elem) k_contact<<<nblocks(d.n_elem, d.contact_threads), d.contact_threads, 0, s>>>(d, g);
 }
 
+// v as an unevaluated sum of two FP32 numbers (48 bits of it)
+__device__ __forceinline__ float2 fp32_pair(double v) {
+  const float hi = (float)v;
+  return make_float2(hi, (float)(v - (double)hi));
+}
+
 // ------------------------------------------------------------------ ordered block assembly
 // Thread per (block, entry): the reference's `nzval[global_sparsity_map] += vec(K)`
 // (assemble_beams.jl:64-66, compute&assemble…:496-497) as a fixed-order sum over
@@ -130,7 +136,7 @@ __global__ void k_gather_mat(Dev d, double alpha, int with_contact) {
   d.M1[t] = Ms;
   const double kt = (d.cK[s] * Ks + d.cC[s] * Cs) + d.cM[s] * Ms;
   d.Kt[t] = kt;
-  d.Kt32[t] = (float)kt;
+  if (d.Ktp) d.Ktp[t] = fp32_pair(kt);
 }
 
 // Thread per (node, dof): Tⁱⁿᵗ, Tᵏ, Tᶜ as ordered sums over incident elements
@@ -215,7 +221,7 @@ __global__ void k_predictor_rhs(Dev d, double alpha, double beta, double gamma) 
       mv += Mb[6 * j + k] * t2;
       const double kt = (cK * Kb[6 * j + k] + cC * Cb[6 * j + k]) + cM * Mb[6 * j + k];
       d.Kt[(int64_t)bb * 36 + 6 * j + k] = kt;
-      d.Kt32[(int64_t)bb * 36 + 6 * j + k] = (float)kt;
+      if (d.Ktp) d.Ktp[(int64_t)bb * 36 + 6 * j + k] = fp32_pair(kt);
     }
   }
   r = cv + r;
