@@ -340,13 +340,15 @@ struct eb_handle {
   std::vector<double> tol_res, tol_disp;  // per simulation Newton tolerances (params unless set)
   // band-LU preconditioner
   bool any_band = false, any_jacobi = false;
-  int max_b = 0;
+  int max_b = 0;            // widest band among the simulations with a band LU
   bool tc_lu = false;  // band LU trailing updates on the tensor cores
   size_t band_floats = 0;
   BandDev band{};
   CondFactor cond{};
+  DenseWork dense_work{};
   std::vector<int64_t> cond_elim_off, cond_tgt_off;  // per level (all simulations): offsets of its lists
-  std::vector<int> band_b;  // per sim half bandwidth (0: block-Jacobi)
+  std::vector<int> band_b;  // per sim half bandwidth of the kept nodes (0: block-Jacobi)
+  std::vector<int> dense_n; // per sim kept DOFs of its explicit inverse (0: band LU)
   // factorisation reuse
   int* d_refactor = nullptr;
   std::vector<int> need_refactor, refactor_mask;
@@ -439,10 +441,14 @@ int launch_solve(eb_handle* h, bool refactor, const int* refactor_src, PhaseTime
     CK(cudaMemcpyAsync(h->d_refactor, refactor_src, sizeof(int) * h->n_sims, cudaMemcpyHostToDevice, h->stream));
     const CondLevels lv{h->cond_elim_off.data(), h->cond_tgt_off.data(), (int)h->cond_elim_off.size() - 1};
     launch_cond_factor(h->d, h->cond, lv, h->d_refactor, h->stream);
-    launch_band_fill(h->d, h->band, h->cond, h->stream);
-    if (h->tc_lu) CK(launch_band_lu_tc(h->d, h->band, h->max_b, h->band.lu_fail, h->stream));
-    else CK(launch_band_lu(h->d, h->band, h->max_b, h->stream));
-    T.launches[EB_PHASE_PRECOND] += 3 + 2 + 2 * lv.n;
+    launch_dense_inverse(h->d, h->sa.dense, h->dense_work, h->cond, h->d_refactor, h->stream);
+    if (h->max_b > 0) {
+      launch_band_fill(h->d, h->band, h->cond, h->stream);
+      if (h->tc_lu) CK(launch_band_lu_tc(h->d, h->band, h->max_b, h->band.lu_fail, h->stream));
+      else CK(launch_band_lu(h->d, h->band, h->max_b, h->stream));
+    }
+    T.launches[EB_PHASE_PRECOND] += 2 + 2 * lv.n + (h->max_b > 0 ? 3 : 0) +
+                                    (h->dense_work.max_ld ? 3 + 2 * (h->dense_work.max_ld / kDenseTile) : 0);
   }
   CK(cudaGetLastError());
   T.mark(EB_PHASE_PRECOND, h->stream);
@@ -857,7 +863,9 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
 
   // ---- preconditioner plan per simulation: condensation levels, then the band of the kept nodes
   std::vector<int64_t> band_off(n_sims + 1, 0), roff(n_sims + 1, 0);
+  std::vector<int64_t> dense_off(n_sims + 1, 0), panel_off(n_sims + 1, 0);
   h->band_b.assign(n_sims, 0);
+  h->dense_n.assign(n_sims, 0);
   const int bmax = (((227 * 1024) / 4 - 8) / kPanel - kPanel) / 2;  // shared-memory limit of k_band_lu
   std::vector<CondPlan> plan(n_sims);
   {
@@ -867,7 +875,7 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
       for (int64_t i = 0; i < n; ++i)
         for (int g : adj[no + i])
           if (g != (int)(no + i)) la[i].push_back((int)(g - no));
-      cond_plan(la, (bmax - 5) / 6, plan[s]);
+      cond_plan(la, (bmax - 5) / 6, p->stage_band == 2 ? 0 : kDenseMax, plan[s]);
     };
     const int nthr = std::max(1, std::min<int>({16, (int)std::thread::hardware_concurrency(), (int)n_sims}));
     std::vector<std::thread> pool;
@@ -878,8 +886,16 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
   }
   for (int s = 0; s < n_sims; ++s) {
     const int b = 6 * plan[s].w + 5, nr = plan[s].n - plan[s].ne;
-    if (p->preconditioner != EB_PRECOND_BLOCK_JACOBI && b <= bmax) h->band_b[s] = b;
-    band_off[s + 1] = band_off[s] + (h->band_b[s] ? band_floats(6 * (int64_t)nr, b) : 0);
+    // few kept nodes: explicit inverse (the staging test asks for the staged band sweeps)
+    const bool dense = 6 * nr <= kDenseMax && p->stage_band != 2;
+    if (p->preconditioner != EB_PRECOND_BLOCK_JACOBI && (dense || b <= bmax)) {
+      h->band_b[s] = b;
+      h->dense_n[s] = dense ? 6 * nr : 0;
+    }
+    const int64_t ld = dense_ld(h->dense_n[s]);
+    band_off[s + 1] = band_off[s] + (h->band_b[s] && !ld ? band_floats(6 * (int64_t)nr, b) : 0);
+    dense_off[s + 1] = dense_off[s] + ld * ld;
+    panel_off[s + 1] = panel_off[s] + ld * kDenseTile;
     roff[s + 1] = roff[s] + nr;
   }
 
@@ -1080,16 +1096,20 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
     CK(cudaMemGetInfo(&fr, &tot));
     // the band, its diagonal-block inverses and the condensation's blocks must leave 2 GB free
     const size_t inv_bytes = 2 * sizeof(float) * (size_t)inv_base(roff[n_sims], n_sims);
-    size_t need = sizeof(float) * (size_t)band_off[n_sims];
+    size_t need = sizeof(float) * (size_t)(band_off[n_sims] + dense_off[n_sims] + 2 * panel_off[n_sims]);
     for (int s = 0; s < n_sims; ++s)
       if (h->band_b[s]) need += (size_t)plan[s].n_blocks * (36 * sizeof(float) + 10 * sizeof(int));
     const size_t margin = (size_t)2 << 30;
     if (need + inv_bytes + margin > fr) {
       std::fill(h->band_b.begin(), h->band_b.end(), 0);
+      std::fill(h->dense_n.begin(), h->dense_n.end(), 0);
       std::fill(band_off.begin(), band_off.end(), 0);
+      std::fill(dense_off.begin(), dense_off.end(), 0);
+      std::fill(panel_off.begin(), panel_off.end(), 0);
     }
     for (int s = 0; s < n_sims; ++s) {
-      h->max_b = std::max(h->max_b, h->band_b[s]);
+      if (!h->dense_n[s]) h->max_b = std::max(h->max_b, h->band_b[s]);
+      h->dense_work.max_ld = std::max(h->dense_work.max_ld, dense_ld(h->dense_n[s]));
       if (h->band_b[s]) h->any_band = true;
       else h->any_jacobi = true;
     }
@@ -1188,12 +1208,29 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
     int64_t *p_boff;
     int* p_bw;
     CK(A.upload(&p_boff, band_off));
-    CK(A.upload(&p_bw, h->band_b));
+    std::vector<int> bw(h->band_b);  // half bandwidths of the band LUs alone
+    for (int s = 0; s < n_sims; ++s)
+      if (h->dense_n[s]) bw[s] = 0;
+    CK(A.upload(&p_bw, bw));
+    int64_t *p_doff, *p_poff;
+    int* p_dn;
+    CK(A.upload(&p_doff, dense_off));
+    CK(A.upload(&p_poff, panel_off));
+    CK(A.upload(&p_dn, h->dense_n));
+    CK(A.alloc(&sa.dense.G, (size_t)dense_off[n_sims]));
+    sa.dense.off = p_doff;
+    sa.dense.n = p_dn;
+    sa.dense_ld = h->dense_work.max_ld;
+    CK(A.alloc(&h->dense_work.Ct, (size_t)panel_off[n_sims]));
+    CK(A.alloc(&h->dense_work.O, (size_t)panel_off[n_sims]));
+    CK(A.alloc(&h->dense_work.D, h->dense_work.max_ld ? (size_t)n_sims * 2 * kDenseTile * kDenseTile : 1));
+    h->dense_work.poff = p_poff;
+    CK(A.alloc(&sa.kin, 6 * (size_t)roff[n_sims]));
     h->band_floats = (size_t)band_off[n_sims];
     float *p_band, *p_work, *p_li, *p_ui;
     CK(A.alloc(&p_band, h->band_floats));
     CK(A.alloc(&p_work, ND));
-    const size_t inv = h->any_band ? (size_t)inv_base(roff[n_sims], n_sims) : 1;
+    const size_t inv = h->max_b > 0 ? (size_t)inv_base(roff[n_sims], n_sims) : 1;
     CK(A.alloc(&p_li, inv));
     CK(A.alloc(&p_ui, inv));
     CK(A.alloc(&h->d_refactor, n_sims));
@@ -1204,13 +1241,15 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
     std::vector<int> order(n_sims);
     for (int s = 0; s < n_sims; ++s) order[s] = s;
     auto kept = [&](int s) { return (int)(6 * (roff[s + 1] - roff[s])); };
-    auto cost = [&](int s) { return 6 * (h->node_off[s + 1] - h->node_off[s]) * (int64_t)64 + kept(s) * (int64_t)(h->band_b[s] + 6); };
+    auto cost = [&](int s) {
+      return 6 * (h->node_off[s + 1] - h->node_off[s]) * (int64_t)64 + kept(s) * (int64_t)(h->dense_n[s] ? kept(s) : h->band_b[s] + 6);
+    };
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost(x) > cost(y); });
     int* p_order;
     CK(A.upload(&p_order, order));
     h->band = BandDev{p_band, p_boff, p_bw, h->band.cond, h->band.node_at, p_work, p_li, p_ui, h->d_refactor, p_order, p_lu_fail};
     // the tensor-core factorisation where its shared memory fits the widest band
-    h->tc_lu = h->any_band && p->band_lu == EB_LU_TENSOR && band_lu_tc_smem(h->max_b) <= kLuTcSmemLimit;
+    h->tc_lu = h->max_b > 0 && p->band_lu == EB_LU_TENSOR && band_lu_tc_smem(h->max_b) <= kLuTcSmemLimit;
     sa.band = h->band;
     sa.cta_sim = p_order;
     h->need_refactor.assign(n_sims, 1);
@@ -1223,13 +1262,13 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
     h->cur_dt.assign(n_sims, 0.0);
     h->cur_active.assign(n_sims, 0);
     int max_n = 0;
-    for (int s = 0; s < n_sims; ++s) max_n = std::max(max_n, kept(s));
+    for (int s = 0; s < n_sims; ++s) if (bw[s]) max_n = std::max(max_n, kept(s));
     sa.max_n = max_n;
-    sa.x_in_smem = h->any_band && gmres_smem(m) + sizeof(float) * (size_t)max_n <= 200 * 1024;
+    sa.x_in_smem = h->max_b > 0 && gmres_smem(m) + sizeof(float) * (size_t)sa.dense_ld + sizeof(float) * (size_t)max_n <= 200 * 1024;
     // stage band blocks through shared memory when the two buffers fit beside the rest
     sa.stage_floats = 0;
     sa.stage_test_extra = p->stage_band == 2 ? 16 : 0;
-    if (h->any_band && p->stage_band) {
+    if (h->max_b > 0 && p->stage_band) {
       sa.stage_floats = kPanel * (h->max_b + 1);
       if (gmres_smem_total(sa) > kGmresSmemLimit) sa.stage_floats = 0;
     }
@@ -1243,8 +1282,8 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
         SolverArgs c = sa;
         int bmax = 0, nmax = 0;
         for (int s2 : sims) {
-          bmax = std::max(bmax, h->band_b[s2]);
-          nmax = std::max(nmax, kept(s2));
+          bmax = std::max(bmax, bw[s2]);
+          if (bw[s2]) nmax = std::max(nmax, kept(s2));
         }
         c.n_sims = (int)sims.size();
         c.max_n = nmax;
@@ -1258,8 +1297,8 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
       for (int s2 : order) {
         SolverArgs one = sa;
         one.x_in_smem = 0;
-        one.stage_floats = kPanel * (h->band_b[s2] + 1);
-        (h->band_b[s2] > 0 && gmres_smem_total(one) > kGmresTwoPerSm ? big : small).push_back(s2);
+        one.stage_floats = kPanel * (bw[s2] + 1);
+        (bw[s2] > 0 && gmres_smem_total(one) > kGmresTwoPerSm ? big : small).push_back(s2);
       }
       if (!big.empty() && !small.empty()) {
         std::vector<int> cta(big);

@@ -51,10 +51,11 @@ struct CondFactor {
 
 // Rows of positions [p0, p1) of one sweep phase, five positions per warp (`warp` of `nwarps`
 // working together), a position's six rows read before any of them is written (x is updated
-// in place).  x: the simulation's permuted vector; z (backward sweep): the result in T besides.
+// in place unless `out` is another vector).  x: the simulation's permuted vector; z (backward
+// sweep): the result in T besides.
 template <bool FWD, typename T>
-__device__ __forceinline__ void cond_rows(const CondDev& c, int64_t base, int p0, int p1, float* x, T* z, int warp,
-                                          int nwarps) {
+__device__ __forceinline__ void cond_rows(const CondDev& c, int64_t base, int p0, int p1, float* x, float* out, T* z,
+                                          int warp, int nwarps) {
   const int lane = threadIdx.x & 31;
   const int sub = lane / 6, r = lane - 6 * sub;
   for (int q = p0 + 5 * warp; q < p1; q += 5 * nwarps) {
@@ -77,7 +78,7 @@ __device__ __forceinline__ void cond_rows(const CondDev& c, int64_t base, int p0
     __syncwarp();
     if (on) {
       const float y = a0 + a1;
-      x[6 * p + r] = y;
+      out[6 * p + r] = y;
       if (!FWD) z[6 * p + r] = (T)y;
     }
   }

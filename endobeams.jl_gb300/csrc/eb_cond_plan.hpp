@@ -8,14 +8,17 @@
 // crossings at next to no fill.  The plan eliminates independent sets (levels)
 // of nodes: first all nodes of degree <= 2, level after level (a segment of
 // q nodes takes about log2 q levels), then, while it pays, independent sets
-// of nodes of degree <= 4, 8 and 12.  Every level is data-parallel; the
-// remaining nodes, a much smaller graph, go to the band LU in reverse
-// Cuthill-McKee order.  A 48-wire stent of 8,664 nodes keeps 297-480 nodes, and N b² (the
-// band LU's work) falls by two orders of magnitude.
+// of nodes of degree <= 4 and upwards.  Every level is data-parallel; the
+// remaining nodes, a much smaller graph, go to the explicit inverse
+// (eb_dense.cuh) or, where they are many, to the band LU in reverse
+// Cuthill-McKee order.  A 48-wire stent of 8,664 nodes keeps about 250 nodes,
+// and N b² (the band LU's work) falls by two orders of magnitude.
 //
-// When another level pays: the band sweeps walk N/32 blocks one after the other, and
-// one step takes about 0.9 us + 3.5 ns per DOF of half bandwidth on one SM, so a level
-// is kept when it lowers N (256 + b) by 5% or more.
+// When another level pays (cond_cost, in us of one application): a level costs 2 us (a barrier
+// of the team in each sweep, its launches in the factorisation) and its blocks' bytes; the
+// explicit inverse reads 4 N² bytes at about 1 TB/s and its 2 N³ operations at 20 TFLOP/s are
+// spread over some 30 applications; the band sweeps walk 2 N/32 blocks one after the other, a
+// step taking about 0.9 us + 3.5 ns per DOF of half bandwidth on one SM.
 #pragma once
 #include <algorithm>
 #include <cstdint>
@@ -126,9 +129,16 @@ struct CondPlan {
   std::vector<int> rptr;               // kept rows: blocks among the kept nodes
 };
 
+// The cheaper of the two (past max_dense the explicit inverse is still what the next levels aim at).
+inline double cond_cost(int nodes, int w, int max_dense) {
+  const double N = 6.0 * nodes, b = 6.0 * w + 5, band = N / 16 * (0.9 + 0.0035 * b);
+  return max_dense > 0 ? std::min(band, 4e-6 * N * N + 2.0 * N * N * N / (20e6 * 30)) : band;
+}
+
 // Symbolic elimination of one simulation's node graph (adj: sorted neighbour lists, self
-// excluded).  At least one node is kept.  max_w: the widest band (nodes) the band LU takes.
-inline void cond_plan(const std::vector<std::vector<int>>& adj0, int max_w, CondPlan& P) {
+// excluded).  At least one node is kept.  max_w: the widest band (nodes) the band LU takes;
+// max_dense: the most DOFs of an explicit inverse.
+inline void cond_plan(const std::vector<std::vector<int>>& adj0, int max_w, int max_dense, CondPlan& P) {
   const int n = (int)adj0.size();
   P = CondPlan();
   P.n = n;
@@ -187,14 +197,17 @@ inline void cond_plan(const std::vector<std::vector<int>>& adj0, int max_w, Cond
     left.erase(std::remove_if(left.begin(), left.end(), [&](int v) { return gone[v] != 0; }), left.end());
   };
 
-  while (left.size() > 1) {  // wire segments: degree <= 2, while a level removes at least 5% of the nodes
+  // wire segments: degree <= 2, while a level removes at least 5% of the nodes.  Also where the
+  // inverse would be small: on a 64-node ring it costs as much as the levels (45 us an iteration
+  // either way), and the levels round less (15 iterations a step against 17)
+  while (left.size() > 1) {
     std::vector<int> set = pick(2);
     if (set.empty() || set.size() * 20 < left.size()) break;
     commit(set);
   }
   std::vector<int> rpos;
   int w = band(adj, left, rpos);
-  for (int cap : {4, 8, 12}) {
+  for (int cap : {4, 8, 12, 16, 24, 32}) {
     while (left.size() > 1) {
       std::vector<int> set = pick(cap);
       if (set.empty() || set.size() * 20 < left.size()) break;
@@ -207,8 +220,10 @@ inline void cond_plan(const std::vector<std::vector<int>>& adj0, int max_w, Cond
       for (int v : set) eliminate(g, v);
       std::vector<int> rp;
       const int w2 = band(g, keep, rp);
-      const double c1 = (double)left.size() * (256 + 6 * w + 5), c2 = (double)keep.size() * (256 + 6 * w2 + 5);
-      if (c2 > 0.95 * c1 || (w2 > max_w && w <= max_w)) break;
+      double blocks = 0;
+      for (int v : set) blocks += 1.0 + 2.0 * adj[v].size();
+      if (cond_cost((int)keep.size(), w2, max_dense) + 2.0 + 144e-6 * blocks > cond_cost((int)left.size(), w, max_dense)) break;
+      if (w2 > max_w && w <= max_w && 6 * (int)keep.size() > max_dense) break;
       commit(set);
       w = w2;
       rpos = rp;

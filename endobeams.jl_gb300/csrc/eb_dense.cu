@@ -1,0 +1,243 @@
+// Blocked in-place Gauss-Jordan inversion of the condensed tangents (see eb_dense.cuh), without
+// pivoting (the dynamic tangent carries the positive mass term on its diagonal, as for the band
+// LU), FP32.  All marked simulations advance together, one 64-wide pivot block per step:
+//   k_dense_panel   C_i = A_ik D⁻¹ for every block row i and a copy O_j of the pivot block row;
+//   k_dense_update  A_ij -= C_i O_j; the pivot block row becomes D⁻¹ O_j, the pivot block column
+//                   -C_i, the pivot block D⁻¹; the CTA of the next diagonal block inverts it at once.
+// 2 N^3 operations; the chain is N / 64 steps of two launches.
+#include <algorithm>
+
+#include "eb_dense.cuh"
+
+namespace eb {
+
+namespace {
+
+constexpr int kT = kDenseTile;
+constexpr int kMm = 256;   // threads per CTA: 16 x 16, 4 x 4 outputs each
+constexpr int kLd = kT + 4;
+
+// acc (+)= Aᵀ-stored (k, m) times B (k, n), both kT x kT in shared memory with stride kLd
+__device__ __forceinline__ void mm64(const float* At, const float* B, float (&acc)[4][4]) {
+  const int tm = threadIdx.x >> 4, tn = threadIdx.x & 15;
+#pragma unroll 8
+  for (int k = 0; k < kT; ++k) {
+    const float4 a = *reinterpret_cast<const float4*>(At + k * kLd + 4 * tm);
+    const float4 b = *reinterpret_cast<const float4*>(B + k * kLd + 4 * tn);
+    const float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+  }
+}
+
+// 64 x 64 tile (row stride ld) into shared memory, as it is or transposed
+__device__ __forceinline__ void load_tile(float* sm, const float* g, int64_t ld) {
+  for (int e = threadIdx.x; e < kT * kT / 4; e += kMm) {
+    const int r = e >> 4, c = 4 * (e & 15);
+    *reinterpret_cast<float4*>(sm + r * kLd + c) = *reinterpret_cast<const float4*>(g + r * ld + c);
+  }
+}
+__device__ __forceinline__ void load_tile_t(float* sm, const float* g, int64_t ld) {
+  for (int e = threadIdx.x; e < kT * kT / 4; e += kMm) {
+    const int r = e & 63, c = 4 * (e >> 6);  // lanes along the rows: the transposed stores are conflict free
+    const float4 v = *reinterpret_cast<const float4*>(g + r * ld + c);
+    sm[c * kLd + r] = v.x; sm[(c + 1) * kLd + r] = v.y; sm[(c + 2) * kLd + r] = v.z; sm[(c + 3) * kLd + r] = v.w;
+  }
+}
+
+// In-place Gauss-Jordan of a 64 x 64 matrix held by the CTA: thread t has row t / 4, columns
+// 16 (t % 4) .. of it in v; row buffers in shared memory, one barrier per pivot.
+__device__ __forceinline__ void invert64(float (&v)[16], float* rows /* 2 x 64 */) {
+  const int r = threadIdx.x >> 2, q = threadIdx.x & 3, lane = threadIdx.x & 31;
+  for (int pb = 0; pb < 4; ++pb) {
+#pragma unroll
+    for (int pi = 0; pi < 16; ++pi) {
+      const int p = 16 * pb + pi;
+      float* row = rows + (pi & 1) * kT;
+      const float f = __shfl_sync(0xffffffffu, v[pi], (lane & ~3) | pb);  // a(r, p)
+      if (r == p) {
+        const float d = 1.f / f;
+#pragma unroll
+        for (int c = 0; c < 16; ++c) v[c] *= d;
+        if (q == pb) v[pi] = d;
+#pragma unroll
+        for (int c = 0; c < 16; c += 4)
+          *reinterpret_cast<float4*>(row + 16 * q + c) = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+      }
+      __syncthreads();
+      if (r != p) {
+        if (q == pb) v[pi] = 0.f;  // becomes -f d
+#pragma unroll
+        for (int c = 0; c < 16; c += 4) {
+          const float4 w = *reinterpret_cast<const float4*>(row + 16 * q + c);
+          v[c] = fmaf(-f, w.x, v[c]);
+          v[c + 1] = fmaf(-f, w.y, v[c + 1]);
+          v[c + 2] = fmaf(-f, w.z, v[c + 2]);
+          v[c + 3] = fmaf(-f, w.w, v[c + 3]);
+        }
+      }
+    }
+  }
+}
+
+__device__ __forceinline__ void store_inverse(const float (&v)[16], float* dst) {
+  const int r = threadIdx.x >> 2, q = threadIdx.x & 3;
+#pragma unroll
+  for (int c = 0; c < 16; c += 4)
+    *reinterpret_cast<float4*>(dst + r * kT + 16 * q + c) = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+}
+
+__device__ __forceinline__ bool marked(const Dev& d, const DenseDev& g, const int* refactor, int s) {
+  return g.n[s] > 0 && d.active[s] && refactor[s];
+}
+
+}  // namespace
+
+// Zeros, with ones on the diagonal beyond N; blockIdx.y = simulation.
+__global__ void k_dense_zero(Dev d, DenseDev g, const int* refactor) {
+  const int s = blockIdx.y;
+  if (!marked(d, g, refactor, s)) return;
+  const int n = g.n[s], ld = dense_ld(n);
+  float* G = g.G + g.off[s];
+  const int64_t len = (int64_t)ld * ld;
+  for (int64_t i = 4 * ((int64_t)blockIdx.x * blockDim.x + threadIdx.x); i < len; i += 4 * (int64_t)gridDim.x * blockDim.x) {
+    float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int r = (int)(i / ld), c = (int)(i - (int64_t)r * ld);
+    if (r >= n && r >= c && r < c + 4) (&z.x)[r - c] = 1.f;
+    *reinterpret_cast<float4*>(G + i) = z;
+  }
+}
+
+// Thread per (block among the kept nodes, entry).
+__global__ void k_dense_fill(Dev d, DenseDev g, CondFactor f, const int* refactor) {
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= f.red_n * 36) return;
+  const int blk = f.red[t / 36], k = (int)(t % 36);
+  const int s = d.node_sim[f.rnode[blk]];
+  if (!marked(d, g, refactor, s)) return;
+  const int ne = f.c.ne[s], ld = dense_ld(g.n[s]);
+  const int i = 6 * (f.rpos[t / 36] - ne) + k / 6, j = 6 * (f.c.scol[blk] - ne) + k % 6;
+  g.G[g.off[s] + (int64_t)i * ld + j] = f.c.S[(int64_t)blk * 36 + k];
+}
+
+// The first diagonal block's inverse.
+__global__ void __launch_bounds__(kMm) k_dense_first(Dev d, DenseDev g, DenseWork w, const int* refactor) {
+  const int s = blockIdx.x;
+  if (!marked(d, g, refactor, s)) return;
+  __shared__ __align__(16) float rows[2 * kT];
+  const int ld = dense_ld(g.n[s]);
+  const float* A = g.G + g.off[s];
+  const int r = threadIdx.x >> 2, q = threadIdx.x & 3;
+  float v[16];
+#pragma unroll
+  for (int c = 0; c < 16; ++c) v[c] = A[(int64_t)r * ld + 16 * q + c];
+  invert64(v, rows);
+  store_inverse(v, w.D + (int64_t)s * 2 * kT * kT);
+}
+
+// CTA (i, s): C_i = A_ik D⁻¹ (stored transposed) and O_i = A_ki, for i != k.
+__global__ void __launch_bounds__(kMm) k_dense_panel(Dev d, DenseDev g, DenseWork w, const int* refactor, int k) {
+  const int s = blockIdx.y, i = blockIdx.x;
+  if (!marked(d, g, refactor, s)) return;
+  const int ld = dense_ld(g.n[s]);
+  if (kT * k >= ld || kT * i >= ld || i == k) return;
+  __shared__ __align__(16) float At[kT * kLd], B[kT * kLd];
+  const float* A = g.G + g.off[s];
+  load_tile_t(At, A + (int64_t)kT * i * ld + kT * k, ld);
+  load_tile(B, w.D + ((int64_t)s * 2 + (k & 1)) * kT * kT, kT);
+  float* O = w.O + w.poff[s] + kT * i;
+  for (int e = threadIdx.x; e < kT * kT / 4; e += kMm) {
+    const int r = e >> 4, c = 4 * (e & 15);
+    *reinterpret_cast<float4*>(O + (int64_t)r * ld + c) =
+        *reinterpret_cast<const float4*>(A + (int64_t)(kT * k + r) * ld + kT * i + c);
+  }
+  __syncthreads();
+  float acc[4][4] = {};
+  mm64(At, B, acc);
+  const int tm = threadIdx.x >> 4, tn = threadIdx.x & 15;
+  float* Ct = w.Ct + w.poff[s] + kT * i;
+#pragma unroll
+  for (int c = 0; c < 4; ++c)
+    *reinterpret_cast<float4*>(Ct + (int64_t)(4 * tn + c) * ld + 4 * tm) =
+        make_float4(acc[0][c], acc[1][c], acc[2][c], acc[3][c]);
+}
+
+// CTA (tile, s) of step k; the next diagonal block's tile comes first, so that its inversion
+// runs beside the other tiles.
+__global__ void __launch_bounds__(kMm) k_dense_update(Dev d, DenseDev g, DenseWork w, const int* refactor, int k) {
+  const int s = blockIdx.y;
+  if (!marked(d, g, refactor, s)) return;
+  const int ld = dense_ld(g.n[s]), nb = ld / kT;
+  if (k >= nb || (int)blockIdx.x >= nb * nb) return;
+  const int first = k + 1 < nb ? (k + 1) * nb + k + 1 : 0;
+  const int tile = blockIdx.x == 0 ? first : ((int)blockIdx.x <= first ? (int)blockIdx.x - 1 : (int)blockIdx.x);
+  const int i = tile / nb, j = tile - i * nb;
+  __shared__ __align__(16) float At[kT * kLd], B[kT * kLd];
+  __shared__ __align__(16) float rows[2 * kT];
+  float* A = g.G + g.off[s] + (int64_t)kT * i * ld + kT * j;
+  const float* Dk = w.D + ((int64_t)s * 2 + (k & 1)) * kT * kT;
+  const float* Ct = w.Ct + w.poff[s] + kT * i;
+  const float* O = w.O + w.poff[s] + kT * j;
+  const int tm = threadIdx.x >> 4, tn = threadIdx.x & 15;
+  if (j == k) {  // pivot block column: -C_i, or D⁻¹ itself
+    for (int e = threadIdx.x; e < kT * kT; e += kMm) {
+      const int r = e & 63, c = e >> 6;
+      A[(int64_t)r * ld + c] = i == k ? Dk[r * kT + c] : -Ct[(int64_t)c * ld + r];
+    }
+    return;
+  }
+  if (i == k) load_tile_t(At, Dk, kT);  // D⁻¹ O_j
+  else load_tile(At, Ct, ld);
+  load_tile(B, O, ld);
+  float acc[4][4];
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) acc[a][c] = 0.f;
+  float4 old[4];
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+    old[a] = i == k ? make_float4(0.f, 0.f, 0.f, 0.f)
+                    : *reinterpret_cast<const float4*>(A + (int64_t)(4 * tm + a) * ld + 4 * tn);
+  __syncthreads();
+  mm64(At, B, acc);
+  const float sg = i == k ? 1.f : -1.f;
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    const float4 v = make_float4(fmaf(sg, acc[a][0], old[a].x), fmaf(sg, acc[a][1], old[a].y),
+                                 fmaf(sg, acc[a][2], old[a].z), fmaf(sg, acc[a][3], old[a].w));
+    *reinterpret_cast<float4*>(A + (int64_t)(4 * tm + a) * ld + 4 * tn) = v;
+    old[a] = v;
+  }
+  if (blockIdx.x != 0 || k + 1 >= nb) return;
+  // the next diagonal block: invert it from the updated values
+  __syncthreads();  // every thread is done with At
+#pragma unroll
+  for (int a = 0; a < 4; ++a) *reinterpret_cast<float4*>(At + (4 * tm + a) * kLd + 4 * tn) = old[a];
+  __syncthreads();
+  const int r = threadIdx.x >> 2, q = threadIdx.x & 3;
+  float v[16];
+#pragma unroll
+  for (int c = 0; c < 16; ++c) v[c] = At[r * kLd + 16 * q + c];
+  invert64(v, rows);
+  store_inverse(v, w.D + ((int64_t)s * 2 + ((k + 1) & 1)) * kT * kT);
+}
+
+void launch_dense_inverse(const Dev& d, const DenseDev& g, const DenseWork& w, const CondFactor& f, const int* refactor,
+                          cudaStream_t s) {
+  if (w.max_ld == 0) return;
+  const unsigned S = (unsigned)d.n_sims;
+  const int nb = w.max_ld / kT;
+  // float4 stores of the largest matrix over 256-thread CTAs, eight per thread
+  k_dense_zero<<<dim3((unsigned)std::max(1, nb * nb / 2), S), 256, 0, s>>>(d, g, refactor);
+  if (f.red_n) k_dense_fill<<<nblocks(f.red_n * 36, 256), 256, 0, s>>>(d, g, f, refactor);
+  k_dense_first<<<S, kMm, 0, s>>>(d, g, w, refactor);
+  for (int k = 0; k < nb; ++k) {
+    if (nb > 1) k_dense_panel<<<dim3((unsigned)nb, S), kMm, 0, s>>>(d, g, w, refactor, k);
+    k_dense_update<<<dim3((unsigned)(nb * nb), S), kMm, 0, s>>>(d, g, w, refactor, k);
+  }
+}
+
+}  // namespace eb

@@ -2,8 +2,8 @@
 // called from solve_free_dofs!, src/utils_solver.jl:107-120).
 //
 // Ktan_free ΔD_free = r_free is solved per simulation by right-preconditioned
-// GMRES; the preconditioner is the condensation with the band LU of the kept
-// nodes (eb_cond.cuh, eb_band.cuh) or 6x6 block-Jacobi (the LU of each node's
+// GMRES; the preconditioner is the condensation with the explicit inverse or the
+// band LU of the kept nodes (eb_cond.cuh, eb_dense.cuh, eb_band.cuh) or 6x6 block-Jacobi (the LU of each node's
 // diagonal block, fixed DOFs replaced by identity rows/columns).  Each
 // simulation is owned by one team of CTAs (a cluster of 1 to 16, so that few
 // simulations use many SMs) for the whole solve: its Krylov basis lives in
@@ -192,11 +192,14 @@ __global__ void __launch_bounds__(512) k_gmres(SolverArgs a) {
   const T* Dm = std::is_same<T, double>::value ? reinterpret_cast<const T*>(a.Dinv64)
                                               : reinterpret_cast<const T*>(a.Dinv32);
   const bool use_band = a.band.bw != nullptr && a.band.bw[s] > 0;
+  const int dn = a.dense.n[s];     // kept DOFs of the explicit inverse, 0 = none
   const CondDev& cd = a.band.cond;
   const int ne = cd.ne[s];
   const int* lev = cd.lev_ptr + cd.lev_off[s];
   const int nlev = max(0, cd.lev_off[s + 1] - cd.lev_off[s] - 1);
-  float* xs = a.x_in_smem ? reinterpret_cast<float*>(wk.sums + 8) : nullptr;  // the kept entries during the sweeps
+  // the dense product's input, dense_ld entries, read as float4
+  float* xd = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(wk.sums + 8) + 15) & ~uintptr_t(15));
+  float* xs = a.x_in_smem ? xd + a.dense_ld : nullptr;           // the kept entries during the band sweeps
   // shared-memory staging of band blocks for the triangular solves (bulk async copies)
   __shared__ __align__(8) uint64_t bars[4];
   __shared__ int stage_fail;
@@ -205,7 +208,7 @@ __global__ void __launch_bounds__(512) k_gmres(SolverArgs a) {
   const Stage* stp = nullptr;
   uint32_t ph = 0u;  // bit k: next phase of staging barrier k
   if (use_band && a.stage_floats > 0 && team.rank == 0) {
-    char* base = reinterpret_cast<char*>(xs ? xs + a.max_n : reinterpret_cast<float*>(wk.sums + 8));
+    char* base = reinterpret_cast<char*>(xd + a.dense_ld + (xs ? a.max_n : 0));
     base = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(base) + 127) & ~uintptr_t(127));
     // two band-column buffers of stage_floats = 32 (b_max + 1) floats, then the inverses
     float* f = reinterpret_cast<float*>(base);
@@ -309,23 +312,34 @@ __global__ void __launch_bounds__(512) k_gmres(SolverArgs a) {
         T* w = V + (int64_t)(j + 1) * n;
         T* zj = Zb + (int64_t)j * n;
         // ---- z_j = M⁻¹ v_j; v_j lies in xa (FP32) when the preconditioner starts
-        if (use_band) {
+        if (use_band || dn) {
           for (int l = 1; l < nlev; ++l) {  // level 0 receives nothing
-            cond_rows<true>(cd, n0, lev[l], lev[l + 1], xa, (T*)nullptr, wk.warp0, wk.nwarps);
+            cond_rows<true>(cd, n0, lev[l], lev[l + 1], xa, xa, (T*)nullptr, wk.warp0, wk.nwarps);
             team.sync();
           }
-          if (ne > 0) {
-            cond_rows<true>(cd, n0, ne, n / 6, xa, (T*)nullptr, wk.warp0, wk.nwarps);
+          if (dn) {
+            float* kin = a.kin + 6 * cd.roff[s];
+            cond_rows<true>(cd, n0, ne, n / 6, xa, kin - 6 * ne, (T*)nullptr, wk.warp0, wk.nwarps);
             team.sync();
+            const int ld = dense_ld(dn);
+            for (int i = threadIdx.x; i < ld; i += blockDim.x) xd[i] = i < dn ? kin[i] : 0.f;
+            __syncthreads();
+            dense_rows(a.dense.G + a.dense.off[s], dn, ld, xd, xa + 6 * ne, zj + 6 * ne, wk.warp0, wk.nwarps);
+            team.sync();
+          } else {
+            if (ne > 0) {
+              cond_rows<true>(cd, n0, ne, n / 6, xa, xa, (T*)nullptr, wk.warp0, wk.nwarps);
+              team.sync();
+            }
+            if (team.rank == 0) band_sweeps(a.band, s, xa + 6 * ne, xs, stp, ph);
+            team.sync();
+            for (int i = 6 * ne + wk.warp0 * 32 + (threadIdx.x & 31); i < n; i += 32 * wk.nwarps) zj[i] = (T)xa[i];
+            if (nlev == 0) team.sync();
           }
-          if (team.rank == 0) band_sweeps(a.band, s, xa + 6 * ne, xs, stp, ph);
-          team.sync();
-          for (int i = 6 * ne + wk.warp0 * 32 + (threadIdx.x & 31); i < n; i += 32 * wk.nwarps) zj[i] = (T)xa[i];
           for (int l = nlev - 1; l >= 0; --l) {
-            cond_rows<false>(cd, n0, lev[l], lev[l + 1], xa, zj, wk.warp0, wk.nwarps);
+            cond_rows<false>(cd, n0, lev[l], lev[l + 1], xa, xa, zj, wk.warp0, wk.nwarps);
             team.sync();
           }
-          if (nlev == 0) team.sync();
         } else {
           const T* vj = V + (int64_t)j * n;
           wk.each([&](int i) {
@@ -519,11 +533,11 @@ void launch_block_jacobi(const Dev& d, double* Dinv64, float* Dinv32, cudaStream
 }
 
 size_t gmres_smem(int m) {
-  return sizeof(double) * ((size_t)(m + 1) * m + 4 * (size_t)m + 1 + 16 * (size_t)kMaxChunks + 8);
+  return sizeof(double) * ((size_t)(m + 1) * m + 4 * (size_t)m + 1 + 16 * (size_t)kMaxChunks + 8 + 1);
 }
 
 size_t gmres_smem_total(const SolverArgs& a) {
-  return gmres_smem(a.m) + (a.x_in_smem ? sizeof(float) * (size_t)a.max_n : 0) +
+  return gmres_smem(a.m) + sizeof(float) * (size_t)a.dense_ld + (a.x_in_smem ? sizeof(float) * (size_t)a.max_n : 0) +
          (a.stage_floats > 0 ? 128 + sizeof(float) * 2 * (size_t)a.stage_floats +
                                    sizeof(float) * 2 * kPanel * kPanel
                              : 0);

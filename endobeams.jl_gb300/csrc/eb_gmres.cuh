@@ -1,6 +1,7 @@
 // Per-simulation GMRES solver interface (implementation in eb_gmres.cu).
 #pragma once
 #include "eb_band.cuh"
+#include "eb_dense.cuh"
 
 namespace eb {
 
@@ -34,6 +35,9 @@ struct SolverArgs {
   double* relres;        // per sim, max over the step
   int* status;           // per sim, max over the step
   BandDev band;          // band-LU preconditioner (bw[s] == 0: block-Jacobi for that sim)
+  DenseDev dense;        // explicit inverse of the kept system (dense.n[s] == 0: band sweeps)
+  float* kin;            // per kept DOF scratch: the dense product's input
+  int dense_ld;          // largest ld of a dense simulation of the handle, 0 = none
   int x_in_smem;         // 1: the permuted solve vector lives in shared memory
   int max_n;             // most kept DOFs of a simulation of this launch
   int stage_floats;      // > 0: band blocks staged in shared memory, floats per buffer (32 (b_max + 1))

@@ -49,7 +49,8 @@ Blk mul(double s, const Blk& a, const Blk& b) {
 
 // Relative residual |A z - v| / |v| of z = M^-1 v for a random block matrix on the graph with the
 // m edges (pairs of nodes); out: eliminated nodes, levels, half bandwidth of the kept graph.
-extern "C" double host_cond_residual(int n, int m, const int32_t* edges, int max_w, int seed, int32_t* out) {
+extern "C" double host_cond_residual(int n, int m, const int32_t* edges, int max_w, int max_dense, int seed,
+                                     int32_t* out) {
   std::vector<std::vector<int>> adj(n);
   for (int e = 0; e < m; ++e) {
     adj[edges[2 * e]].push_back(edges[2 * e + 1]);
@@ -60,7 +61,7 @@ extern "C" double host_cond_residual(int n, int m, const int32_t* edges, int max
     a.erase(std::unique(a.begin(), a.end()), a.end());
   }
   CondPlan P;
-  cond_plan(adj, max_w, P);
+  cond_plan(adj, max_w, max_dense, P);
   out[0] = P.ne; out[1] = (int)P.lev_ptr.size() - 1; out[2] = P.w;
   std::mt19937 rng(seed);
   std::uniform_real_distribution<double> U(-1, 1);

@@ -55,8 +55,8 @@ def _graphs():
 def test_plan_solves_like_the_whole_system(host, name, n, edges):
     e = np.ascontiguousarray([x for x in np.asarray(edges).reshape(-1, 2) if x[0] != x[1]], np.int32).reshape(-1, 2)
     out = np.zeros(3, np.int32)
-    for max_w in (148, 2):
-        r = host.host_cond_residual(n, len(e), e.ctypes.data_as(ctypes.c_void_p), max_w, 5,
+    for max_w, max_dense in ((148, 2048), (148, 0), (2, 0), (2, 36)):
+        r = host.host_cond_residual(n, len(e), e.ctypes.data_as(ctypes.c_void_p), max_w, max_dense, 5,
                                     out.ctypes.data_as(ctypes.c_void_p))
         assert r <= 1e-12, f"{name}: {r}"
         assert 0 <= out[0] < n
@@ -67,7 +67,7 @@ def test_stent_condenses_onto_its_crossings(host, scenes):
     conf, _, _ = scenes.braided_stent(wires=16, elems_per_wire=60, crossing_every=5)
     e = np.ascontiguousarray(conf.beams.conn, np.int32)
     out = np.zeros(3, np.int32)
-    r = host.host_cond_residual(len(conf.nodes), len(e), e.ctypes.data_as(ctypes.c_void_p), 148, 5,
+    r = host.host_cond_residual(len(conf.nodes), len(e), e.ctypes.data_as(ctypes.c_void_p), 148, 0, 5,
                                 out.ctypes.data_as(ctypes.c_void_p))
     crossings = int((np.bincount(e.ravel()) == 4).sum())
     assert r <= 1e-12 and len(conf.nodes) - out[0] <= crossings
