@@ -16,7 +16,7 @@
 #include <vector>
 
 #include "../../include/endobeams_gb300.h"
-#include "eb_contact.cuh"
+#include "eb_internal.cuh"
 
 using namespace ebd;
 
@@ -191,58 +191,125 @@ __global__ void k_sdf_interior(const double* __restrict__ vals, int nx, int ny, 
   c[(i + 1) + (int64_t)(nx + 2) * ((j + 1) + (int64_t)(ny + 2) * (k + 1))] = vals[t];
 }
 
-// One thread per grid line along `axis`: in-place solve of the quadratic
-// B-spline interpolation system ⅛c[i-1] + ¾c[i] + ⅛c[i+1] = y[i] with the
+// In-place solve of the quadratic B-spline interpolation system
+// ⅛c[i-1] + ¾c[i] + ⅛c[i+1] = y[i] along every grid line of `axis` with the
 // reflected ends (first/last diagonal 7/8), then the two pads c[0] = c[1],
 // c[n+1] = c[n].  Lines run over the padded range of axes already filtered.
-__global__ void k_sdf_prefilter_axis(double* c, int nx, int ny, int nz, int axis) {
+//
+// The elimination's factors do not depend on the samples and reach their fixed
+// point within 32 rows: they come as a table.  A CTA takes 32 lines into shared
+// memory (rows of consecutive lines, or whole lines along x, both coalesced) and
+// one warp runs the recurrences there, a chain of two FP64 operations per row;
+// with a thread per line in global memory every row waited for a load and a
+// division (61³ points: 76 us a pass, 147 us at 128³).
+struct LineFactors {
+  double cp[32], im[32];  // super-diagonal factor, inverse pivot of rows 0 .. 31 (row 31: all later ones)
+};
+LineFactors line_factors() {
+  LineFactors f;
+  double cp = 0.0;
+  for (int i = 0; i < 32; ++i) {
+    const double m = i == 0 ? 0.875 : 0.75 - 0.125 * cp;
+    cp = 0.125 / m;
+    f.cp[i] = cp;
+    f.im[i] = 1.0 / m;
+  }
+  return f;
+}
+
+constexpr int kLines = 32;       // lines per CTA, one per lane of the solving warp
+constexpr int kLineStride = 33;  // doubles between rows in shared memory
+constexpr int kLineThreads = 256;
+constexpr int kMaxLine = 800;    // longest line whose tile fits in shared memory (211 KB)
+
+__device__ __forceinline__ int64_t line_base(int64_t t, int nx, int ny, int nz, int axis, int64_t* stride) {
   const int64_t px = nx + 2, py = ny + 2;
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  int n;
-  int64_t base, stride;
   if (axis == 0) {  // lines (j, k), interior j and k
-    if (t >= (int64_t)ny * nz) return;
-    const int64_t j = 1 + t % ny, k = 1 + t / ny;
-    n = nx; stride = 1; base = px * (j + py * k);
-  } else if (axis == 1) {  // lines (i, k), all i, interior k
-    if (t >= px * nz) return;
-    const int64_t i = t % px, k = 1 + t / px;
-    n = ny; stride = px; base = i + px * py * k;
-  } else {  // lines (i, j), all i and j
-    if (t >= px * py) return;
-    const int64_t i = t % px, j = t / px;
-    n = nz; stride = px * py; base = i + px * j;
+    *stride = 1;
+    return px * ((1 + t % ny) + py * (1 + t / ny));
   }
-  double* y = c + base + stride;  // first interior point of the line
-  if (n > 1) {
-    double cpa[32];
-    double cp = 0.125 / 0.875;
-    cpa[0] = cp;
-    y[0] = y[0] / 0.875;
-    for (int i = 1; i < n; ++i) {
-      const bool last = i == n - 1;
-      const double m = (last ? 0.875 : 0.75) - 0.125 * cp;
-      y[i * stride] = (y[i * stride] - 0.125 * y[(i - 1) * stride]) / m;
-      cp = last ? 0.0 : 0.125 / m;
-      if (i < 32) cpa[i] = cp;
+  if (axis == 1) {  // lines (i, k), all i, interior k
+    *stride = px;
+    return t % px + px * py * (1 + t / px);
+  }
+  *stride = px * py;  // lines (i, j), all i and j
+  return t;
+}
+
+__global__ void __launch_bounds__(kLineThreads) k_sdf_prefilter_axis(double* c, int nx, int ny, int nz, int axis,
+                                                                     int64_t lines, LineFactors f) {
+  extern __shared__ double row[];
+  const int n = axis == 0 ? nx : (axis == 1 ? ny : nz);
+  const int64_t l0 = (int64_t)blockIdx.x * kLines;
+  const int nl = (int)(lines - l0 < kLines ? lines - l0 : kLines);
+  int64_t stride;
+  // element (row i, line l) of the tile: threads run along the contiguous direction
+  auto each = [&](auto op) {
+    for (int e = threadIdx.x; e < n * kLines; e += kLineThreads) {
+      const int i = axis == 0 ? e % n : e / kLines, l = axis == 0 ? e / n : e % kLines;
+      if (l < nl) op(i, l, c + line_base(l0 + l, nx, ny, nz, axis, &stride) + (int64_t)(i + 1) * stride);
     }
-    // beyond the first 32 rows the factor has converged to its fixed point
-    for (int i = n - 2; i >= 0; --i) y[i * stride] -= cpa[i < 32 ? i : 31] * y[(i + 1) * stride];
+  };
+  each([&](int i, int l, double* p) { row[i * kLineStride + l] = *p; });
+  __syncthreads();
+  if (threadIdx.x < nl && n > 1) {
+    double* y = row + threadIdx.x;
+    double v = y[0] * f.im[0];
+    y[0] = v;
+    for (int i = 1; i < n - 1; ++i) {
+      v = (y[i * kLineStride] - 0.125 * v) * f.im[i < 32 ? i : 31];
+      y[i * kLineStride] = v;
+    }
+    v = (y[(n - 1) * kLineStride] - 0.125 * v) / (0.875 - 0.125 * f.cp[n - 2 < 32 ? n - 2 : 31]);
+    y[(n - 1) * kLineStride] = v;
+    for (int i = n - 2; i >= 0; --i) {
+      v = y[i * kLineStride] - f.cp[i < 32 ? i : 31] * v;
+      y[i * kLineStride] = v;
+    }
   }
-  y[-stride] = y[0];
-  y[n * stride] = y[(n - 1) * stride];
+  __syncthreads();
+  each([&](int i, int l, double* p) {
+    const double v = row[i * kLineStride + l];
+    *p = v;
+    if (i == 0) p[-stride] = v;
+    if (i == n - 1) p[stride] = v;
+  });
+}
+
+// The same for lines longer than kMaxLine: one thread per line, in place in global memory.
+__global__ void k_sdf_prefilter_long(double* c, int nx, int ny, int nz, int axis, int64_t lines, LineFactors f) {
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= lines) return;
+  const int n = axis == 0 ? nx : (axis == 1 ? ny : nz);
+  int64_t stride;
+  double* y = c + line_base(t, nx, ny, nz, axis, &stride);
+  y += stride;
+  double v = y[0] * f.im[0];
+  y[0] = v;
+  for (int i = 1; i < n - 1; ++i) y[i * stride] = v = (y[i * stride] - 0.125 * v) * f.im[i < 32 ? i : 31];
+  v = (y[(n - 1) * stride] - 0.125 * v) / (0.875 - 0.125 * f.cp[31]);
+  y[(n - 1) * stride] = y[n * stride] = v;
+  for (int i = n - 2; i >= 0; --i) y[i * stride] = v = y[i * stride] - f.cp[i < 32 ? i : 31] * v;
+  y[-stride] = v;
 }
 
 }  // namespace
 
 // Prefilters a padded coefficient grid whose interior holds the SDF samples
-// (three passes, one thread per grid line).
+// (three passes over the grid lines of an axis).
 namespace eb {
 void launch_sdf_prefilter(double* coef, int nx, int ny, int nz, cudaStream_t st) {
-  const int64_t px = nx + 2, py = ny + 2;
-  k_sdf_prefilter_axis<<<(unsigned)(((int64_t)ny * nz + 127) / 128), 128, 0, st>>>(coef, nx, ny, nz, 0);
-  k_sdf_prefilter_axis<<<(unsigned)((px * nz + 127) / 128), 128, 0, st>>>(coef, nx, ny, nz, 1);
-  k_sdf_prefilter_axis<<<(unsigned)((px * py + 127) / 128), 128, 0, st>>>(coef, nx, ny, nz, 2);
+  static const LineFactors f = line_factors();
+  const int64_t px = nx + 2, py = ny + 2, lines[3] = {(int64_t)ny * nz, px * nz, px * py};
+  const int n[3] = {nx, ny, nz};
+  for (int a = 0; a < 3; ++a) {
+    const size_t smem = sizeof(double) * kLineStride * (size_t)n[a];
+    if (n[a] <= kMaxLine && (smem <= 48 * 1024 || raise_smem_limit((const void*)k_sdf_prefilter_axis, smem) == cudaSuccess))
+      k_sdf_prefilter_axis<<<(unsigned)((lines[a] + kLines - 1) / kLines), kLineThreads, smem, st>>>(coef, nx, ny, nz, a,
+                                                                                                    lines[a], f);
+    else
+      k_sdf_prefilter_long<<<(unsigned)((lines[a] + 127) / 128), 128, 0, st>>>(coef, nx, ny, nz, a, lines[a], f);
+  }
 }
 }  // namespace eb
 
@@ -307,9 +374,7 @@ extern "C" int eb_contact_eval_noalloc(int64_t n, const double* d_in, const doub
     const int NX = (int)nx, NY = (int)ny, NZ = (int)nz;
     const int64_t pts = nx * ny * nz;
     k_sdf_interior<<<(unsigned)((pts + 255) / 256), 256, 0, st>>>(d_sdf_values, NX, NY, NZ, coef);
-    k_sdf_prefilter_axis<<<(unsigned)((ny * nz + 127) / 128), 128, 0, st>>>(coef, NX, NY, NZ, 0);
-    k_sdf_prefilter_axis<<<(unsigned)(((nx + 2) * nz + 127) / 128), 128, 0, st>>>(coef, NX, NY, NZ, 1);
-    k_sdf_prefilter_axis<<<(unsigned)(((nx + 2) * (ny + 2) + 127) / 128), 128, 0, st>>>(coef, NX, NY, NZ, 2);
+    eb::launch_sdf_prefilter(coef, NX, NY, NZ, st);
     s.coef = coef;
     s.nx = NX; s.ny = NY; s.nz = NZ;
     s.x0 = surf[8]; s.y0 = surf[9]; s.z0 = surf[10];
