@@ -868,22 +868,23 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
   h->dense_n.assign(n_sims, 0);
   const int bmax = (((227 * 1024) / 4 - 8) / kPanel - kPanel) / 2;  // shared-memory limit of k_band_lu
   std::vector<CondPlan> plan(n_sims);
-  {
-    auto build = [&](int s) {
-      const int64_t no = h->node_off[s], n = h->node_off[s + 1] - no;
-      std::vector<std::vector<int>> la(n);
-      for (int64_t i = 0; i < n; ++i)
-        for (int g : adj[no + i])
-          if (g != (int)(no + i)) la[i].push_back((int)(g - no));
-      cond_plan(la, (bmax - 5) / 6, p->stage_band == 2 ? 0 : kDenseMax, plan[s]);
-    };
+  // f(s) for every simulation on up to 16 host threads
+  auto each_sim = [&](auto f) {
     const int nthr = std::max(1, std::min<int>({16, (int)std::thread::hardware_concurrency(), (int)n_sims}));
     std::vector<std::thread> pool;
     for (int k = 1; k < nthr; ++k)
-      pool.emplace_back([&, k] { for (int s = k; s < n_sims; s += nthr) build(s); });
-    for (int s = 0; s < n_sims; s += nthr) build(s);
+      pool.emplace_back([&, k] { for (int s = k; s < n_sims; s += nthr) f(s); });
+    for (int s = 0; s < n_sims; s += nthr) f(s);
     for (auto& th : pool) th.join();
-  }
+  };
+  each_sim([&](int s) {
+    const int64_t no = h->node_off[s], n = h->node_off[s + 1] - no;
+    std::vector<std::vector<int>> la(n);
+    for (int64_t i = 0; i < n; ++i)
+      for (int g : adj[no + i])
+        if (g != (int)(no + i)) la[i].push_back((int)(g - no));
+    cond_plan(la, (bmax - 5) / 6, p->stage_band == 2 ? 0 : kDenseMax, plan[s]);
+  });
   for (int s = 0; s < n_sims; ++s) {
     const int b = 6 * plan[s].w + 5, nr = plan[s].n - plan[s].ne;
     // few kept nodes: explicit inverse (the staging test asks for the staged band sweeps)
@@ -1117,67 +1118,81 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
     // elimination and update lists level by level
     CondFactor& cf = h->cond;
     {
-      std::vector<int> node_at(NN), scol, src, rnode, cnode, ldiag, elim, elim_node, tgt, tptr, cl, cw, red, rpos;
-      std::vector<int> ne(n_sims, 0), lev_off(n_sims + 1, 0), lev_ptr;
+      std::vector<int> node_at(NN), ne(n_sims, 0), lev_off(n_sims + 1, 0), lev_ptr;
       std::vector<CondRange> range(NN, CondRange{0, 0, 0, 0});
-      std::vector<int64_t> base(n_sims + 1, 0);
+      std::vector<int64_t> base(n_sims + 1, 0), red_off(n_sims + 1, 0);  // first block, first kept block of a simulation
       size_t nlev = 0;
       for (int s = 0; s < n_sims; ++s) {
         const CondPlan& P = plan[s];
-        const int64_t no = h->node_off[s];
-        base[s + 1] = base[s];
-        lev_off[s + 1] = lev_off[s];
-        for (int i = 0; i < P.n; ++i) node_at[no + P.pos[i]] = (int)(no + i);
-        if (!h->band_b[s]) continue;
-        const int o = (int)base[s];
-        base[s + 1] += P.n_blocks;
-        if (base[s + 1] >= (1LL << 31)) return fail(EB_ERR_ARG, "problem too large for 32-bit block indices");
+        const bool on = h->band_b[s] > 0;
+        base[s + 1] = base[s] + (on ? P.n_blocks : 0);
+        red_off[s + 1] = red_off[s] + (on ? P.n_blocks - P.red0 : 0);
+        lev_off[s + 1] = lev_off[s] + (on ? (int)P.lev_ptr.size() : 0);
+        if (!on) continue;
         ne[s] = P.ne;
         lev_ptr.insert(lev_ptr.end(), P.lev_ptr.begin(), P.lev_ptr.end());
-        lev_off[s + 1] += (int)P.lev_ptr.size();
         nlev = std::max(nlev, P.tgt.size());
-        for (int q = 0; q < P.n; ++q)
-          range[no + q] = CondRange{q < P.ne ? o + P.wptr[q] : 0, q < P.ne ? o + P.wptr[q + 1] : 0, o + P.lptr[q],
-                                    o + P.lptr[q + 1]};
-        const int l0 = P.lptr[0];
-        for (int k = 0; k < P.n_blocks; ++k) {
-          const int r = node_at[no + P.srow[k]], c = node_at[no + P.scol[k]];
-          auto it = std::lower_bound(col.begin() + row_ptr[r], col.begin() + row_ptr[r + 1], c);
-          src.push_back(it != col.begin() + row_ptr[r + 1] && *it == c ? (int)(it - col.begin()) : -1);
-          rnode.push_back(r);
-          cnode.push_back(c);
-          scol.push_back(P.scol[k]);
-          ldiag.push_back(k >= l0 && k < P.red0 ? o + P.wptr[P.scol[k]] : -1);
-          if (k >= P.red0) {
-            red.push_back(o + k);
-            rpos.push_back(P.srow[k]);
-          }
-        }
       }
-      h->cond_elim_off.assign(1, 0);
-      h->cond_tgt_off.assign(1, 0);
+      if (base[n_sims] >= (1LL << 31)) return fail(EB_ERR_ARG, "problem too large for 32-bit block indices");
+      // offsets of (level, simulation) in the level-ordered lists
+      std::vector<int64_t> eo(nlev * n_sims + 1, 0), to(eo), co(eo);
+      h->cond_elim_off.assign(nlev + 1, 0);
+      h->cond_tgt_off.assign(nlev + 1, 0);
       for (size_t l = 0; l < nlev; ++l) {
         for (int s = 0; s < n_sims; ++s) {
           const CondPlan& P = plan[s];
-          if (!h->band_b[s] || l >= P.tgt.size()) continue;
-          const int o = (int)base[s];
-          for (int q = P.lev_ptr[l]; q < P.lev_ptr[l + 1]; ++q) {
-            elim.push_back((int)(h->node_off[s] + q));
-            elim_node.push_back(node_at[h->node_off[s] + q]);
-          }
-          for (size_t k = 0; k < P.tgt[l].size(); ++k) {
-            tgt.push_back(o + P.tgt[l][k]);
-            tptr.push_back((int)cl.size());
-            for (int u = P.tptr[l][k]; u < P.tptr[l][k + 1]; ++u) {
-              cl.push_back(o + P.cl[l][u]);
-              cw.push_back(o + P.cw[l][u]);
-            }
+          const size_t k = l * n_sims + s;
+          const bool on = h->band_b[s] > 0 && l < P.tgt.size();
+          eo[k + 1] = eo[k] + (on ? P.lev_ptr[l + 1] - P.lev_ptr[l] : 0);
+          to[k + 1] = to[k] + (on ? (int64_t)P.tgt[l].size() : 0);
+          co[k + 1] = co[k] + (on ? (int64_t)P.cl[l].size() : 0);
+        }
+        h->cond_elim_off[l + 1] = eo[(l + 1) * n_sims];
+        h->cond_tgt_off[l + 1] = to[(l + 1) * n_sims];
+      }
+      if (co.back() >= (1LL << 31)) return fail(EB_ERR_ARG, "problem too large for 32-bit update indices");
+      std::vector<int> scol(base[n_sims]), src(base[n_sims]), rnode(base[n_sims]), cnode(base[n_sims]), ldiag(base[n_sims]);
+      std::vector<int> red(red_off[n_sims]), rpos(red_off[n_sims]);
+      std::vector<int> elim(eo.back()), elim_node(eo.back()), tgt(to.back()), tptr(to.back() + 1), cl(co.back()), cw(co.back());
+      tptr.back() = (int)co.back();
+      each_sim([&](int s) {
+        const CondPlan& P = plan[s];
+        const int64_t no = h->node_off[s];
+        for (int i = 0; i < P.n; ++i) node_at[no + P.pos[i]] = (int)(no + i);
+        if (!h->band_b[s]) return;
+        const int o = (int)base[s];
+        for (int q = 0; q < P.n; ++q)
+          range[no + q] = CondRange{q < P.ne ? o + P.wptr[q] : 0, q < P.ne ? o + P.wptr[q + 1] : 0, o + P.lptr[q],
+                                    o + P.lptr[q + 1]};
+        for (int k = 0; k < P.n_blocks; ++k) {
+          const int r = node_at[no + P.srow[k]], c = node_at[no + P.scol[k]];
+          auto it = std::lower_bound(col.begin() + row_ptr[r], col.begin() + row_ptr[r + 1], c);
+          src[o + k] = it != col.begin() + row_ptr[r + 1] && *it == c ? (int)(it - col.begin()) : -1;
+          rnode[o + k] = r;
+          cnode[o + k] = c;
+          scol[o + k] = P.scol[k];
+          ldiag[o + k] = k >= P.lptr[0] && k < P.red0 ? o + P.wptr[P.scol[k]] : -1;
+          if (k >= P.red0) {
+            red[red_off[s] + k - P.red0] = o + k;
+            rpos[red_off[s] + k - P.red0] = P.srow[k];
           }
         }
-        h->cond_elim_off.push_back((int64_t)elim.size());
-        h->cond_tgt_off.push_back((int64_t)tgt.size());
-      }
-      tptr.push_back((int)cl.size());
+        for (size_t l = 0; l < P.tgt.size(); ++l) {
+          const size_t i = l * n_sims + s;
+          for (int q = P.lev_ptr[l]; q < P.lev_ptr[l + 1]; ++q) {
+            elim[eo[i] + q - P.lev_ptr[l]] = (int)(no + q);
+            elim_node[eo[i] + q - P.lev_ptr[l]] = node_at[no + q];
+          }
+          for (size_t k = 0; k < P.tgt[l].size(); ++k) {
+            tgt[to[i] + k] = o + P.tgt[l][k];
+            tptr[to[i] + k] = (int)(co[i] + P.tptr[l][k]);
+          }
+          for (size_t u = 0; u < P.cl[l].size(); ++u) {
+            cl[co[i] + u] = o + P.cl[l][u];
+            cw[co[i] + u] = o + P.cw[l][u];
+          }
+        }
+      });
       int *p_scol, *p_ne, *p_lo, *p_lp, *p_src, *p_rn, *p_cn, *p_ld, *p_el, *p_en, *p_t, *p_tp, *p_cl, *p_cw, *p_red,
           *p_rpos, *p_nat;
       CondRange* p_range;

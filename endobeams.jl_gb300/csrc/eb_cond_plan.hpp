@@ -129,10 +129,12 @@ struct CondPlan {
   std::vector<int> rptr;               // kept rows: blocks among the kept nodes
 };
 
-// The cheaper of the two (past max_dense the explicit inverse is still what the next levels aim at).
+// The cheaper of the two (past max_dense the explicit inverse is still what the next levels aim
+// at); w < 0: the inverse.
 inline double cond_cost(int nodes, int w, int max_dense) {
   const double N = 6.0 * nodes, b = 6.0 * w + 5, band = N / 16 * (0.9 + 0.0035 * b);
-  return max_dense > 0 ? std::min(band, 4e-6 * N * N + 2.0 * N * N * N / (20e6 * 30)) : band;
+  const double dense = 4e-6 * N * N + 2.0 * N * N * N / (20e6 * 30);
+  return max_dense <= 0 ? band : w < 0 ? dense : std::min(band, dense);
 }
 
 // Symbolic elimination of one simulation's node graph (adj: sorted neighbour lists, self
@@ -205,30 +207,36 @@ inline void cond_plan(const std::vector<std::vector<int>>& adj0, int max_w, int 
     if (set.empty() || set.size() * 20 < left.size()) break;
     commit(set);
   }
+  // half bandwidths only where the explicit inverse does not cost less than the band sweeps of
+  // any bandwidth (w < 0: not needed)
+  auto needs_band = [&](int nodes) { return max_dense <= 0 || cond_cost(nodes, 0, max_dense) < cond_cost(nodes, n, max_dense); };
   std::vector<int> rpos;
-  int w = band(adj, left, rpos);
+  int w = needs_band((int)left.size()) ? band(adj, left, rpos) : -1;
   for (int cap : {4, 8, 12, 16, 24, 32}) {
     while (left.size() > 1) {
       std::vector<int> set = pick(cap);
       if (set.empty() || set.size() * 20 < left.size()) break;
-      std::vector<std::vector<int>> g(adj);
-      std::vector<char> out(n, 0);
-      for (int v : set) out[v] = 1;
-      std::vector<int> keep;
-      for (int v : left)
-        if (!out[v]) keep.push_back(v);
-      for (int v : set) eliminate(g, v);
-      std::vector<int> rp;
-      const int w2 = band(g, keep, rp);
       double blocks = 0;
       for (int v : set) blocks += 1.0 + 2.0 * adj[v].size();
-      if (cond_cost((int)keep.size(), w2, max_dense) + 2.0 + 144e-6 * blocks > cond_cost((int)left.size(), w, max_dense)) break;
-      if (w2 > max_w && w <= max_w && 6 * (int)keep.size() > max_dense) break;
+      const int m = (int)left.size(), m2 = m - (int)set.size();
+      int w2 = -1;
+      if (needs_band(m2)) {
+        std::vector<std::vector<int>> g(adj);
+        std::vector<char> out(n, 0);
+        for (int v : set) out[v] = 1;
+        std::vector<int> keep, rp;
+        for (int v : left)
+          if (!out[v]) keep.push_back(v);
+        for (int v : set) eliminate(g, v);
+        w2 = band(g, keep, rp);
+        if (w2 > max_w && w <= max_w && 6 * m2 > max_dense) break;
+      }
+      if (cond_cost(m2, w2, max_dense) + 2.0 + 144e-6 * blocks > cond_cost(m, w, max_dense)) break;
       commit(set);
       w = w2;
-      rpos = rp;
     }
   }
+  w = band(adj, left, rpos);
   P.w = w;
   P.ne = (int)order.size();
 
@@ -280,25 +288,37 @@ inline void cond_plan(const std::vector<std::vector<int>>& adj0, int max_w, int 
   P.tptr.resize(nlev);
   P.cl.resize(nlev);
   P.cw.resize(nlev);
-  struct Upd { int t, l, w; };
-  std::vector<Upd> up;
+  std::vector<int> ut, cnt(P.n_blocks + 1, 0), touched;
   for (int l = 0; l < nlev; ++l) {
-    up.clear();
+    ut.clear();
+    touched.clear();
+    for (int p = P.lev_ptr[l]; p < P.lev_ptr[l + 1]; ++p)
+      for (int a = P.wptr[p] + 1; a < P.wptr[p + 1]; ++a)
+        for (int b = P.wptr[p] + 1; b < P.wptr[p + 1]; ++b) {
+          const int t = P.find(P.scol[a], P.scol[b]);
+          if (cnt[t]++ == 0) touched.push_back(t);
+          ut.push_back(t);
+        }
+    std::sort(touched.begin(), touched.end());
+    P.tgt[l] = touched;
+    P.tptr[l].assign(1, 0);
+    for (int t : touched) {
+      P.tptr[l].push_back(P.tptr[l].back() + cnt[t]);
+      cnt[t] = P.tptr[l][P.tptr[l].size() - 2];  // next free entry of the target
+    }
+    P.cl[l].resize(ut.size());
+    P.cw[l].resize(ut.size());
+    size_t u = 0;
     for (int p = P.lev_ptr[l]; p < P.lev_ptr[l + 1]; ++p)
       for (int a = P.wptr[p] + 1; a < P.wptr[p + 1]; ++a) {
-        const int lb = P.find(P.scol[a], p);
-        for (int b = P.wptr[p] + 1; b < P.wptr[p + 1]; ++b) up.push_back(Upd{P.find(P.scol[a], P.scol[b]), lb, b});
+        const int left_block = P.find(P.scol[a], p);
+        for (int b = P.wptr[p] + 1; b < P.wptr[p + 1]; ++b) {
+          const int k = cnt[ut[u++]]++;
+          P.cl[l][k] = left_block;
+          P.cw[l][k] = b;
+        }
       }
-    std::stable_sort(up.begin(), up.end(), [](const Upd& x, const Upd& y) { return x.t < y.t; });
-    for (size_t i = 0; i < up.size(); ++i) {
-      if (i == 0 || up[i].t != up[i - 1].t) {
-        P.tgt[l].push_back(up[i].t);
-        P.tptr[l].push_back((int)i);
-      }
-      P.cl[l].push_back(up[i].l);
-      P.cw[l].push_back(up[i].w);
-    }
-    P.tptr[l].push_back((int)up.size());
+    for (int t : touched) cnt[t] = 0;
   }
 }
 
