@@ -908,8 +908,8 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
   d.n_elem = NE;
   d.nnzb = NB;
   d.n_dof = ND;
-  d.beam_threads = kThreads;
-  d.contact_threads = kThreads;
+  d.beam_threads = NE > kBeamWide ? 256 : kThreads;
+  d.contact_threads = NE > kBeamWide ? 256 : kThreads;
   d.gmat_threads = 256;
   d.gvec_threads = 256;
   int64_t *p_node_off, *p_blk_off;

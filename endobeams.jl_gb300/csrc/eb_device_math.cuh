@@ -215,6 +215,28 @@ EB_DEV M3 Gmul(Gt g, const M3& p) {
   return m;
 }
 
+// Gᵀ * p
+EB_DEV M3 GTmul(Gu g, const M3& p) {
+  M3 m;
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    m(0, j) = 0.0;
+    m(1, j) = g.g32 * p(2, j);
+    m(2, j) = g.g13 * p(0, j) + g.g23 * p(1, j);
+  }
+  return m;
+}
+EB_DEV M3 GTmul(Gt g, const M3& p) {
+  M3 m;
+#pragma unroll
+  for (int j = 0; j < 3; ++j) {
+    m(0, j) = g.a * p(0, j);
+    m(1, j) = g.b * p(0, j);
+    m(2, j) = 0.0;
+  }
+  return m;
+}
+
 constexpr double EPS64 = 2.220446049250313e-16;  // eps(Float64)
 
 // utils_beams.jl:11-32

@@ -26,68 +26,72 @@ __device__ __forceinline__ V3 elem3(const double* f, int64_t ne, int64_t e) {
 }
 
 // ------------------------------------------------------------------ assemble! element pass
-// One thread per element (compute_beams via assemble_beams.jl:21-48).
-__global__ void __launch_bounds__(kMaxElemThreads) k_beam(Dev d, Gauss3 g) {
-  int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= d.n_elem) return;
-  if (!d.active[d.elem_sim[e]]) return;
-  const int a = d.ea[e], b = d.eb[e];
-  const int64_t n = d.n_nodes, ne = d.n_elem;
-  BeamIn in;
-  in.X1 = node3(d.X0, n, a);   in.X2 = node3(d.X0, n, b);
-  in.u1 = node3(d.u, n, a);    in.u2 = node3(d.u, n, b);
-  in.ud1 = node3(d.ud, n, a);  in.ud2 = node3(d.ud, n, b);
-  in.wd1 = node3(d.wd, n, a);  in.wd2 = node3(d.wd, n, b);
-  in.udd1 = node3(d.udd, n, a); in.udd2 = node3(d.udd, n, b);
-  in.wdd1 = node3(d.wdd, n, a); in.wdd2 = node3(d.wdd, n, b);
-  in.R1 = node9(d.R, n, a);    in.R2 = node9(d.R, n, b);
-  in.dR1 = node9(d.dR, n, a);  in.dR2 = node9(d.dR, n, b);
+// compute_beams via assemble_beams.jl:21-48, ten or thirty elements per CTA (eb_beam.cuh).
+struct BeamElem {
+  const Dev& d;
+  int64_t e;
+  int nd[2];
+  __device__ __forceinline__ V3 x(int n) const { return node3(d.X0, d.n_nodes, nd[n]) + node3(d.u, d.n_nodes, nd[n]); }
+  __device__ __forceinline__ M3 R(int n) const { return node9(d.R, d.n_nodes, nd[n]); }
+  __device__ __forceinline__ M3 dR(int n) const { return node9(d.dR, d.n_nodes, nd[n]); }
+  __device__ __forceinline__ M3 Re0() const {
+    M3 m;
 #pragma unroll
-  for (int k = 0; k < 9; ++k) in.Re0.a[k] = d.Re0[k * ne + e];
-  in.l0 = d.l0[e];
-  in.Ku = d.Kbar[e];
-  in.KT = v3(d.Kbar[ne + e], d.Kbar[2 * ne + e], d.Kbar[3 * ne + e]);
-  in.KTT = v3(d.Kbar[4 * ne + e], d.Kbar[5 * ne + e], d.Kbar[6 * ne + e]);
-  in.Jr = elem3(d.Jr, ne, e);
-  in.Ar = d.Ar[e];
-  in.damping = d.damp[e];
-  BeamOut o{d.stK + e * 144, d.stM + e * 144, d.stC + e * 144, d.stTi + e * 12, d.stTk + e * 12, d.stE + e * 2};
-  beam_element(in, g, o);
+    for (int k = 0; k < 9; ++k) m.a[k] = d.Re0[k * d.n_elem + e];
+    return m;
+  }
+  __device__ __forceinline__ V3 ud(int n) const { return node3(d.ud, d.n_nodes, nd[n]); }
+  __device__ __forceinline__ V3 wd(int n) const { return node3(d.wd, d.n_nodes, nd[n]); }
+  __device__ __forceinline__ V3 udd(int n) const { return node3(d.udd, d.n_nodes, nd[n]); }
+  __device__ __forceinline__ V3 wdd(int n) const { return node3(d.wdd, d.n_nodes, nd[n]); }
+  __device__ __forceinline__ double l0() const { return d.l0[e]; }
+  __device__ __forceinline__ double Ku() const { return d.Kbar[e]; }
+  __device__ __forceinline__ V3 KT() const { return elem3(d.Kbar + d.n_elem, d.n_elem, e); }
+  __device__ __forceinline__ V3 KTT() const { return elem3(d.Kbar + 4 * d.n_elem, d.n_elem, e); }
+  __device__ __forceinline__ V3 Jr() const { return elem3(d.Jr, d.n_elem, e); }
+  __device__ __forceinline__ double Ar() const { return d.Ar[e]; }
+  __device__ __forceinline__ double damping() const { return d.damp[e]; }
+  __device__ __forceinline__ BeamOut out() const {
+    return BeamOut{d.stK + e * 144, d.stM + e * 144, d.stC + e * 144, d.stTi + e * 12, d.stTk + e * 12, d.stE + e * 2};
+  }
+};
+
+__global__ void __launch_bounds__(kBeamCta, 3) k_beam(const __grid_constant__ Dev d, Gauss3 g, int nb) {
+  extern __shared__ double beam_tab[];
+  beam_cta(d.n_elem, nb, g, beam_tab, [&](int64_t e) { return BeamElem{d, e, {d.ea[e], d.eb[e]}}; },
+           [&](int64_t e) { return d.active[d.elem_sim[e]] != 0; });
 }
 
-// One thread per contact element (compute_contact_beams via compute&assemble…:460-482).
-__global__ void __launch_bounds__(kMaxElemThreads) k_contact(Dev d, Gauss3 g) {
-  int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= d.n_elem) return;
-  if (!d.is_contact[e]) return;
-  const int s = d.elem_sim[e];
-  if (!d.active[s]) return;
-  const int a = d.ea[e], b = d.eb[e];
-  const int64_t n = d.n_nodes, ne = d.n_elem;
-  ContactIn in;
-  in.X1 = node3(d.X0, n, a);   in.X2 = node3(d.X0, n, b);
-  in.u1 = node3(d.u, n, a);    in.u2 = node3(d.u, n, b);
-  in.ud1 = node3(d.ud, n, a);  in.ud2 = node3(d.ud, n, b);
-  in.wd1 = node3(d.wd, n, a);  in.wd2 = node3(d.wd, n, b);
-  in.R1 = node9(d.R, n, a);    in.R2 = node9(d.R, n, b);
-  in.dR1 = node9(d.dR, n, a);  in.dR2 = node9(d.dR, n, b);
-#pragma unroll
-  for (int k = 0; k < 9; ++k) in.Re0.a[k] = d.Re0[k * ne + e];
-  in.l0 = d.l0[e];
-  in.radius = d.radius[e];
-  const SurfaceDev srf = d.surf[s];
-  const ContactProps cp = d.props[s];
-  ContactOut o{d.scK + e * 144, d.scC + e * 144, d.scT + e * 12, d.scE + e};
-  bool any = false;
-  contact_element(in, g, cp, srf, o, &any);
-  d.sc_on[e] = any ? 1 : 0;
+// compute_contact_beams via compute&assemble…:460-482, ten or thirty elements per CTA (eb_contact.cuh).
+struct ContactElem : BeamElem {
+  __device__ __forceinline__ double radius() const { return d.radius[e]; }
+  __device__ __forceinline__ const SurfaceDev& surf() const { return d.surf[d.elem_sim[e]]; }
+  __device__ __forceinline__ const ContactProps& props() const { return d.props[d.elem_sim[e]]; }
+  __device__ __forceinline__ ContactOut out() const {
+    return ContactOut{d.scK + e * 144, d.scC + e * 144, d.scT + e * 12, d.scE + e};
+  }
+  __device__ __forceinline__ void touched(bool any) const { d.sc_on[e] = any ? 1 : 0; }
+};
+
+__global__ void __launch_bounds__(kContactCta) k_contact(const __grid_constant__ Dev d, Gauss3 g, int nb) {
+  extern __shared__ double beam_tab[];
+  contact_cta(d.n_elem, nb, g, beam_tab, [&](int64_t e) { return ContactElem{{d, e, {d.ea[e], d.eb[e]}}}; },
+              [&](int64_t e) { return d.is_contact[e] && d.active[d.elem_sim[e]]; });
 }
 
 void launch_beam(const Dev& d, const Gauss3& g, cudaStream_t s) {
-  if (d.n_elem) k_beam<<<nblocks(d.n_elem, d.beam_threads), d.beam_threads, 0, s>>>(d, g);
+  if (!d.n_elem) return;
+  const int nb = beam_groups(d.beam_threads);
+  const size_t smem = beam_smem(nb);
+  if (smem > 48 * 1024) raise_smem_limit((const void*)k_beam, smem);
+  k_beam<<<nblocks(d.n_elem, kBeamGroup * nb), kBeamCta, smem, s>>>(d, g, nb);
 }
 void launch_contact(const Dev& d, const Gauss3& g, cudaStream_t s) {
-  if (d.n_elem) k_contact<<<nblocks(d.n_elem, d.contact_threads), d.contact_threads, 0, s>>>(d, g);
+  if (!d.n_elem) return;
+  const int nb = beam_groups(d.contact_threads);
+  const size_t smem = contact_smem(nb);
+  if (smem > 48 * 1024) raise_smem_limit((const void*)k_contact, smem);
+  k_contact<<<nblocks(d.n_elem, kBeamGroup * nb), kContactCta, smem, s>>>(d, g, nb);
 }
 
 // v as an unevaluated sum of two FP32 numbers (48 bits of it)

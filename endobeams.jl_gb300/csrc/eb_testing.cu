@@ -31,37 +31,62 @@ __device__ __forceinline__ M3 P9(const double* p) {
   return m;
 }
 
-__global__ void k_element_eval(int64_t n, const double* in, Gauss3 g, double* out) {
-  int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= n) return;
-  const double* p = in + 96 * e;
-  double* o = out + 458 * e;
-  BeamIn b;
-  b.X1 = P3(p + 0); b.X2 = P3(p + 3); b.u1 = P3(p + 6); b.u2 = P3(p + 9);
-  b.R1 = P9(p + 12); b.R2 = P9(p + 21); b.dR1 = P9(p + 30); b.dR2 = P9(p + 39);
-  b.ud1 = P3(p + 48); b.ud2 = P3(p + 51); b.wd1 = P3(p + 54); b.wd2 = P3(p + 57);
-  b.udd1 = P3(p + 60); b.udd2 = P3(p + 63); b.wdd1 = P3(p + 66); b.wdd2 = P3(p + 69);
-  b.l0 = p[72]; b.Re0 = P9(p + 73); b.Ku = p[82]; b.KT = P3(p + 83); b.KTT = P3(p + 86); b.Jr = P3(p + 89);
-  b.Ar = p[92]; b.damping = p[93];
-  BeamOut bo{o + 26, o + 170, o + 314, o + 2, o + 14, o + 0};
-  beam_element(b, g, bo);
+// Packed record p with outputs at o.
+struct PackedElem {
+  const double* p;
+  double* o;
+  __device__ __forceinline__ V3 x(int n) const { return P3(p + 3 * n) + P3(p + 6 + 3 * n); }
+  __device__ __forceinline__ M3 R(int n) const { return P9(p + 12 + 9 * n); }
+  __device__ __forceinline__ M3 dR(int n) const { return P9(p + 30 + 9 * n); }
+  __device__ __forceinline__ M3 Re0() const { return P9(p + 73); }
+  __device__ __forceinline__ V3 ud(int n) const { return P3(p + 48 + 3 * n); }
+  __device__ __forceinline__ V3 wd(int n) const { return P3(p + 54 + 3 * n); }
+  __device__ __forceinline__ V3 udd(int n) const { return P3(p + 60 + 3 * n); }
+  __device__ __forceinline__ V3 wdd(int n) const { return P3(p + 66 + 3 * n); }
+  __device__ __forceinline__ double l0() const { return p[72]; }
+  __device__ __forceinline__ double Ku() const { return p[82]; }
+  __device__ __forceinline__ V3 KT() const { return P3(p + 83); }
+  __device__ __forceinline__ V3 KTT() const { return P3(p + 86); }
+  __device__ __forceinline__ V3 Jr() const { return P3(p + 89); }
+  __device__ __forceinline__ double Ar() const { return p[92]; }
+  __device__ __forceinline__ double damping() const { return p[93]; }
+  __device__ __forceinline__ BeamOut out() const { return BeamOut{o + 26, o + 170, o + 314, o + 2, o + 14, o}; }
+};
+
+__global__ void __launch_bounds__(kBeamCta) k_element_eval(int64_t n, int nb, const double* in, Gauss3 g, double* out) {
+  extern __shared__ double beam_tab[];
+  beam_cta(n, nb, g, beam_tab, [&](int64_t e) { return PackedElem{in + 96 * e, out + 458 * e}; }, [](int64_t) { return true; });
 }
 
-__global__ void k_contact_eval(int64_t n, const double* in, Gauss3 g, ContactProps cp, SurfaceDev s, double* out,
-                               int32_t* flags) {
-  int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= n) return;
-  const double* p = in + 96 * e;
-  double* o = out + 301 * e;
-  ContactIn c;
-  c.X1 = P3(p + 0); c.X2 = P3(p + 3); c.u1 = P3(p + 6); c.u2 = P3(p + 9);
-  c.R1 = P9(p + 12); c.R2 = P9(p + 21); c.dR1 = P9(p + 30); c.dR2 = P9(p + 39);
-  c.ud1 = P3(p + 48); c.ud2 = P3(p + 51); c.wd1 = P3(p + 54); c.wd2 = P3(p + 57);
-  c.l0 = p[72]; c.Re0 = P9(p + 73); c.radius = p[94];
-  ContactOut co{o + 13, o + 157, o + 1, o + 0};
-  bool any = false;
-  contact_element(c, g, cp, s, co, &any);
-  flags[e] = any ? 1 : 0;
+struct PackedContact : PackedElem {
+  const SurfaceDev& s;
+  const ContactProps& cp;
+  int32_t* flag;
+  __device__ __forceinline__ PackedContact(const double* p_, double* o_, const SurfaceDev& s_, const ContactProps& c_, int32_t* f_)
+      : PackedElem{p_, o_}, s(s_), cp(c_), flag(f_) {}
+  __device__ __forceinline__ double radius() const { return p[94]; }
+  __device__ __forceinline__ const SurfaceDev& surf() const { return s; }
+  __device__ __forceinline__ const ContactProps& props() const { return cp; }
+  __device__ __forceinline__ ContactOut out() const { return ContactOut{o + 13, o + 157, o + 1, o}; }
+  __device__ __forceinline__ void touched(bool any) const { *flag = any ? 1 : 0; }
+};
+
+__global__ void __launch_bounds__(kContactCta) k_contact_eval(int64_t n, int nb, const double* in, Gauss3 g,
+                                                              const __grid_constant__ ContactProps cp,
+                                                              const __grid_constant__ SurfaceDev s, double* out,
+                                                              int32_t* flags) {
+  extern __shared__ double beam_tab[];
+  contact_cta(n, nb, g, beam_tab, [&](int64_t e) { return PackedContact(in + 96 * e, out + 301 * e, s, cp, flags + e); },
+              [](int64_t) { return true; });
+}
+
+cudaError_t launch_contact_eval(int64_t n, const double* in, const Gauss3& g, const ContactProps& cp, const SurfaceDev& s,
+                                double* out, int32_t* flags, cudaStream_t st) {
+  const int nb = beam_groups(n > eb::kBeamWide ? 256 : 128);
+  const cudaError_t e = eb::raise_smem_limit((const void*)k_contact_eval, contact_smem(nb));
+  if (e != cudaSuccess) return e;
+  k_contact_eval<<<eb::nblocks(n, kBeamGroup * nb), kContactCta, contact_smem(nb), st>>>(n, nb, in, g, cp, s, out, flags);
+  return cudaGetLastError();
 }
 
 struct DBuf {
@@ -93,7 +118,10 @@ extern "C" int eb_element_eval(int64_t n, const double* in, const double* gauss6
   if ((e = cudaMalloc(&dout.p, sizeof(double) * 458 * n)) != cudaSuccess) return err("cudaMalloc", e);
   cudaMemcpy(di.p, in, sizeof(double) * 96 * n, cudaMemcpyHostToDevice);
   cudaMemset(dout.p, 0, sizeof(double) * 458 * n);
-  k_element_eval<<<(unsigned)((n + 127) / 128), 128>>>(n, (const double*)di.p, g, (double*)dout.p);
+  const int nb = beam_groups(n > eb::kBeamWide ? 256 : 128);
+  if ((e = eb::raise_smem_limit((const void*)k_element_eval, beam_smem(nb))) != cudaSuccess) return err("k_element_eval", e);
+  k_element_eval<<<eb::nblocks(n, kBeamGroup * nb), kBeamCta, beam_smem(nb)>>>(n, nb, (const double*)di.p, g,
+                                                                                (double*)dout.p);
   if ((e = cudaGetLastError()) != cudaSuccess) return err("k_element_eval launch", e);
   if ((e = cudaMemcpy(out, dout.p, sizeof(double) * 458 * n, cudaMemcpyDeviceToHost)) != cudaSuccess)
     return err("k_element_eval", e);
@@ -140,9 +168,8 @@ extern "C" int eb_contact_eval(int64_t n, const double* in, const double* gauss6
   if ((e = cudaMalloc(&dfl.p, sizeof(int32_t) * n)) != cudaSuccess) return err("cudaMalloc", e);
   cudaMemcpy(di.p, in, sizeof(double) * 96 * n, cudaMemcpyHostToDevice);
   cudaMemset(dout.p, 0, sizeof(double) * 301 * n);
-  k_contact_eval<<<(unsigned)((n + 127) / 128), 128>>>(n, (const double*)di.p, g, cp, s, (double*)dout.p,
-                                                      (int32_t*)dfl.p);
-  if ((e = cudaGetLastError()) != cudaSuccess) return err("k_contact_eval launch", e);
+  if ((e = launch_contact_eval(n, (const double*)di.p, g, cp, s, (double*)dout.p, (int32_t*)dfl.p, 0)) != cudaSuccess)
+    return err("k_contact_eval launch", e);
   if ((e = cudaMemcpy(out, dout.p, sizeof(double) * 301 * n, cudaMemcpyDeviceToHost)) != cudaSuccess)
     return err("k_contact_eval", e);
   cudaMemcpy(flags, dfl.p, sizeof(int32_t) * n, cudaMemcpyDeviceToHost);
@@ -384,8 +411,7 @@ extern "C" int eb_contact_eval_noalloc(int64_t n, const double* d_in, const doub
   // untouched elements leave zero records, as in eb_contact_eval
   cudaError_t e = cudaMemsetAsync(d_out, 0, sizeof(double) * 301 * n, st);
   if (e != cudaSuccess) return err("cudaMemsetAsync", e);
-  k_contact_eval<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(n, d_in, g, cp, s, d_out, d_flags);
-  e = cudaGetLastError();
+  e = launch_contact_eval(n, d_in, g, cp, s, d_out, d_flags, st);
   if (e != cudaSuccess) return err("k_contact_eval (no-alloc) launch", e);
   return EB_OK;
 }

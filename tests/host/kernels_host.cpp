@@ -36,7 +36,7 @@ extern "C" void host_element_eval(int64_t n, const double* in, const double* gau
     b.l0 = p[72]; b.Re0 = P9(p + 73); b.Ku = p[82]; b.KT = P3(p + 83); b.KTT = P3(p + 86); b.Jr = P3(p + 89);
     b.Ar = p[92]; b.damping = p[93];
     BeamOut bo{o + 26, o + 170, o + 314, o + 2, o + 14, o + 0};
-    beam_element(b, g, bo);
+    beam_element(BeamRecord{b, bo}, g);
   }
 }
 
