@@ -657,6 +657,9 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
   h->n_sims = n_sims;
   for (int i = 0; i < 3; ++i) { h->gauss.w[i] = p->gauss_w[i]; h->gauss.z[i] = p->gauss_z[i]; }
   CK(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
+  CK(cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking));
+  CK(cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming));
+  CK(cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming));
   CK(cudaEventCreate(&h->t0));
   CK(cudaEventCreate(&h->t1));
   h->timer.init(p->timing != 0);
@@ -1044,6 +1047,7 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
   sa.Kt = d.Kt;
   sa.Ktp = d.Ktp;
   sa.team = 1;
+  sa.vec_smem = 0;
   sa.Dinv64 = h->d_Dinv64;
   sa.Dinv32 = h->d_Dinv32;
   sa.fixed = d.fixed;
@@ -1325,9 +1329,6 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
         cs.cta_sim = p_cta + big.size();
         cb.team = cs.team = 1;  // both classes present: teams only where one launch has the GPU to itself
         h->gclass = {cb, cs};
-        CK(cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking));
-        CK(cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming));
-        CK(cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming));
       }
     }
   }
@@ -1336,6 +1337,12 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
     int64_t nmax = 0;
     for (int s = 0; s < n_sims; ++s) nmax = std::max(nmax, 6 * (h->node_off[s + 1] - h->node_off[s]));
     sa.team = gmres_team(sa, fp32, p->threads_per_sim > 0 ? p->threads_per_sim : 256, (int)nmax);
+    // z_j, w (double or float) and the FP32 vector of the largest simulation
+    const int vec = (int)((nmax * (fp32 ? 3 : 5) + 3) / 4 * 4);
+    if (sa.team == 1 && sizeof(float) * (size_t)vec <= kGmresVecSmem) {
+      sa.vec_smem = vec;
+      if (gmres_smem_total(sa) > kGmresSmemLimit) sa.vec_smem = 0;
+    }
   }
 
   // ---- learned warm start: neighbour table and surface flags (buffers for features on first use)

@@ -61,12 +61,40 @@ struct Work {
   }
 };
 
+// Sums NQ values over the warp, NQ a power of two: while a lane holds several values it keeps half of
+// them and sends the others' partial sums to the lane that keeps those, so that eight values take 9
+// FP64 additions instead of 40 (each holds the SM's FP64 pipe for 16 cycles).  Afterwards the
+// lanes q (32 / NQ) .. hold the sum of value q.
+template <int NQ>
+__device__ __forceinline__ double warp_sums(const double (&in)[NQ]) {
+  const int lane = threadIdx.x & 31;
+  double v[NQ];
+#pragma unroll
+  for (int q = 0; q < NQ; ++q) v[q] = in[q];
+#pragma unroll
+  for (int off = 16, cnt = NQ; off > 0; off >>= 1) {
+    if (cnt > 1) {
+      const bool up = (lane & off) != 0;
+#pragma unroll
+      for (int q = 0; q < cnt / 2; ++q) {
+        const double keep = up ? v[q + cnt / 2] : v[q], send = up ? v[q] : v[q + cnt / 2];
+        v[q] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+      }
+      cnt /= 2;
+    } else {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], off);
+    }
+  }
+  return v[0];
+}
+
 // out[q] = Σ_i of what f(i, acc) adds to acc[q]: per lane in TA, over lanes and chunks in FP64.  Each
 // chunk's sums go to every CTA of the team; one team barrier; two buffers in turn, so that a CTA
 // that is ahead does not overwrite sums that another still reads.
 template <int NQ, typename TA, typename F>
 __device__ __forceinline__ void team_sum(Work& w, double (&out)[NQ], F f) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  constexpr int G = 32 / NQ;  // lanes that hold the same sum
   double* part = w.flip ? w.part[1] : w.part[0];
   w.flip ^= 1;
   for (int c = w.warp0; c < w.nchunk; c += w.nwarps) {
@@ -77,21 +105,16 @@ __device__ __forceinline__ void team_sum(Work& w, double (&out)[NQ], F f) {
     for (int i = c * w.ch + lane; i < i1; i += 32) f(i, acc);
     double v[NQ];
 #pragma unroll
-    for (int q = 0; q < NQ; ++q) {
-      v[q] = (double)acc[q];
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], off);
-    }
+    for (int q = 0; q < NQ; ++q) v[q] = (double)acc[q];
+    const double sum = warp_sums<NQ>(v);
+    double* mine = part + lane / G * kMaxChunks + c;
     if (w.t.size == 1) {
-      if (lane == 0)
-#pragma unroll
-        for (int q = 0; q < NQ; ++q) part[q * kMaxChunks + c] = v[q];
-    } else if (lane < w.t.size) {  // lane r writes CTA r's copy
-#pragma unroll
-      for (int q = 0; q < NQ; ++q) {
+      if (lane % G == 0) *mine = sum;
+    } else {  // the lanes of a sum write the CTAs' copies
+      for (int r = lane % G; r < w.t.size; r += G) {
         uint32_t a;
-        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(part + q * kMaxChunks + c)), "r"(lane));
-        asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v[q]) : "memory");
+        asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(mine)), "r"(r));
+        asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(sum) : "memory");
       }
     }
   }
@@ -114,14 +137,17 @@ __device__ __forceinline__ double row64(const SolverArgs& a, int64_t n0, int i, 
   const int p = i / 6, k = i - 6 * p;
   const int node = a.band.node_at[n0 + p];
   if (a.fixed[6 * (int64_t)node + k]) return 0.0;
-  double acc = 0.0;
+  double acc0 = 0.0, acc1 = 0.0;
   for (int bb = a.row_ptr[node]; bb < a.row_ptr[node + 1]; ++bb) {
     const double* Ab = a.Kt + (int64_t)bb * 36 + k;
     const TX* xc = x + 6 * a.pcol[bb];
 #pragma unroll
-    for (int j = 0; j < 6; ++j) acc += Ab[6 * j] * (double)xc[j];
+    for (int j = 0; j < 6; j += 2) {
+      acc0 += Ab[6 * j] * (double)xc[j];
+      acc1 += Ab[6 * j + 6] * (double)xc[j + 1];
+    }
   }
-  return acc;
+  return acc0 + acc1;
 }
 
 // The same row from the tangent as FP32 pairs (hi + lo carry 48 bits of it), summed as FP32
@@ -186,7 +212,10 @@ __global__ void __launch_bounds__(512) k_gmres(SolverArgs a) {
   T* Zb = reinterpret_cast<T*>(a.Z) + (int64_t)m * o;  // z_j = M⁻¹ v_j at Zb + j n
   double* X = a.X + o;
   double* R = a.R64 + o;
-  float* xa = a.band.work + o;     // the vector the preconditioner works on
+  // the vector the preconditioner works on, z_j and w: in shared memory where one CTA owns a small
+  // simulation (every phase reads what another thread has just written, an L2 round trip each)
+  const bool vs = a.vec_smem > 0 && team.size == 1;
+  float* xa = a.band.work + o;
   const int* node_at = a.band.node_at + n0;
   auto dof = [&](int i) { return 6 * (int64_t)node_at[i / 6] + i % 6; };  // caller's DOF of entry i
   const T* Dm = std::is_same<T, double>::value ? reinterpret_cast<const T*>(a.Dinv64)
@@ -199,7 +228,10 @@ __global__ void __launch_bounds__(512) k_gmres(SolverArgs a) {
   const int nlev = max(0, cd.lev_off[s + 1] - cd.lev_off[s] - 1);
   // the dense product's input, dense_ld entries, read as float4
   float* xd = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(wk.sums + 8) + 15) & ~uintptr_t(15));
-  float* xs = a.x_in_smem ? xd + a.dense_ld : nullptr;           // the kept entries during the band sweeps
+  float* xs = a.x_in_smem ? xd + a.dense_ld + a.vec_smem : nullptr;  // the kept entries during the band sweeps
+  T* zs = reinterpret_cast<T*>(xd + a.dense_ld);  // vec_smem floats: z_j, w, xa
+  T* ws = zs + n;
+  if (vs) xa = reinterpret_cast<float*>(ws + n);
   // shared-memory staging of band blocks for the triangular solves (bulk async copies)
   __shared__ __align__(8) uint64_t bars[4];
   __shared__ int stage_fail;
@@ -208,7 +240,7 @@ __global__ void __launch_bounds__(512) k_gmres(SolverArgs a) {
   const Stage* stp = nullptr;
   uint32_t ph = 0u;  // bit k: next phase of staging barrier k
   if (use_band && a.stage_floats > 0 && team.rank == 0) {
-    char* base = reinterpret_cast<char*>(xd + a.dense_ld + (xs ? a.max_n : 0));
+    char* base = reinterpret_cast<char*>(xd + a.dense_ld + a.vec_smem + (xs ? a.max_n : 0));
     base = reinterpret_cast<char*>((reinterpret_cast<uintptr_t>(base) + 127) & ~uintptr_t(127));
     // two band-column buffers of stage_floats = 32 (b_max + 1) floats, then the inverses
     float* f = reinterpret_cast<float*>(base);
@@ -309,8 +341,10 @@ __global__ void __launch_bounds__(512) k_gmres(SolverArgs a) {
       int k = 0;  // dimension of the Krylov space built in this cycle
       const int jmax = min(m, a.max_iter - its);
       for (int j = 0; j < jmax; ++j) {
-        T* w = V + (int64_t)(j + 1) * n;
-        T* zj = Zb + (int64_t)j * n;
+        T* vn = V + (int64_t)(j + 1) * n;
+        T* w = vs ? ws : vn;
+        T* zg = Zb + (int64_t)j * n;
+        T* zj = vs ? zs : zg;
         // ---- z_j = M⁻¹ v_j; v_j lies in xa (FP32) when the preconditioner starts
         if (use_band || dn) {
           for (int l = 1; l < nlev; ++l) {  // level 0 receives nothing
@@ -356,25 +390,38 @@ __global__ void __launch_bounds__(512) k_gmres(SolverArgs a) {
         wk.each([&](int i) {
           if constexpr (std::is_same<T, double>::value) w[i] = row64(a, n0, i, zj);
           else w[i] = row_pairs(a, n0, i, zj);
+          if (vs) zg[i] = zj[i];
         });
         __syncwarp();
         for (int pass = 0; pass < 2; ++pass) {
-          for (int i0 = 0; i0 <= j; i0 += 8) {
-            const int nq = min(8, j + 1 - i0);
-            const T* Vq = V + (int64_t)i0 * n;
-            double hp[8];
-            team_sum<8, T>(wk, hp, [&](int i, T (&q)[8]) {
-              const T wi = w[i];
+          for (int i0 = 0; i0 <= j;) {
+            // inner products with v_i0 .., as many at a time as are left (at most 8)
+            auto dots = [&](auto width) {
+              constexpr int NQ = decltype(width)::value;
+              const int nq = min(NQ, j + 1 - i0);
+              const T* Vq = V + (int64_t)i0 * n;
+              double hp[NQ];
+              team_sum<NQ, T>(wk, hp, [&](int i, T (&q)[NQ]) {
+                const T wi = w[i];
 #pragma unroll
-              for (int u = 0; u < 8; ++u)
-                if (u < nq) q[u] += Vq[(int64_t)u * n + i] * wi;
-            });
-            if (threadIdx.x == 0)
-              for (int q = 0; q < nq; ++q) {
-                double* h = H + (m + 1) * j + i0 + q;
-                *h = (pass == 0 ? 0.0 : *h) + hp[q];
-                y[i0 + q] = hp[q];  // this pass's coefficients (y is free until the back-substitution)
-              }
+                for (int u = 0; u < NQ; ++u)
+                  if (u < nq) q[u] += Vq[(int64_t)u * n + i] * wi;
+              });
+              if (threadIdx.x == 0)
+#pragma unroll
+                for (int q = 0; q < NQ; ++q)
+                  if (q < nq) {
+                    double* h = H + (m + 1) * j + i0 + q;
+                    *h = (pass == 0 ? 0.0 : *h) + hp[q];
+                    y[i0 + q] = hp[q];  // this pass's coefficients (y is free until the back-substitution)
+                  }
+              i0 += NQ;
+            };
+            const int left = j + 1 - i0;
+            if (left > 4) dots(std::integral_constant<int, 8>{});
+            else if (left > 2) dots(std::integral_constant<int, 4>{});
+            else if (left > 1) dots(std::integral_constant<int, 2>{});
+            else dots(std::integral_constant<int, 1>{});
           }
           __syncthreads();
           wk.each([&](int i) {
@@ -391,7 +438,7 @@ __global__ void __launch_bounds__(512) k_gmres(SolverArgs a) {
           const T ihn = (T)(1.0 / hn);
           wk.each([&](int i) {
             const T v = w[i] * ihn;
-            w[i] = v;
+            vn[i] = v;
             xa[i] = (float)v;
           });
         }
@@ -537,7 +584,7 @@ size_t gmres_smem(int m) {
 }
 
 size_t gmres_smem_total(const SolverArgs& a) {
-  return gmres_smem(a.m) + sizeof(float) * (size_t)a.dense_ld + (a.x_in_smem ? sizeof(float) * (size_t)a.max_n : 0) +
+  return gmres_smem(a.m) + sizeof(float) * ((size_t)a.dense_ld + (size_t)a.vec_smem) + (a.x_in_smem ? sizeof(float) * (size_t)a.max_n : 0) +
          (a.stage_floats > 0 ? 128 + sizeof(float) * 2 * (size_t)a.stage_floats +
                                    sizeof(float) * 2 * kPanel * kPanel
                              : 0);

@@ -38,6 +38,7 @@ struct SolverArgs {
   DenseDev dense;        // explicit inverse of the kept system (dense.n[s] == 0: band sweeps)
   float* kin;            // per kept DOF scratch: the dense product's input
   int dense_ld;          // largest ld of a dense simulation of the handle, 0 = none
+  int vec_smem;          // > 0: floats of shared memory for the working vectors of a simulation on one CTA
   int x_in_smem;         // 1: the permuted solve vector lives in shared memory
   int max_n;             // most kept DOFs of a simulation of this launch
   int stage_floats;      // > 0: band blocks staged in shared memory, floats per buffer (32 (b_max + 1))
@@ -53,6 +54,7 @@ struct SolverArgs {
 };
 
 void launch_block_jacobi(const Dev& d, double* Dinv64, float* Dinv32, cudaStream_t s);
+constexpr size_t kGmresVecSmem = 48 * 1024;  // most shared memory for a simulation's working vectors
 constexpr int kTeamDofs = 512;  // fewest DOFs per CTA of a team
 int gmres_team(const SolverArgs& a, bool fp32, int threads, int max_dofs);
 cudaError_t launch_gmres(const SolverArgs& a, bool fp32, int threads, cudaStream_t s);
