@@ -324,6 +324,7 @@ struct eb_handle {
   double *d_cK = nullptr, *d_cC = nullptr, *d_cM = nullptr, *d_dt = nullptr;
   // solver
   SolverArgs sa{};
+  int gmres_threads = 256;
   std::vector<SolverArgs> gclass;  // empty, or {wide-band class, two-CTAs-per-SM class}
   cudaStream_t side = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
@@ -453,7 +454,7 @@ int launch_solve(eb_handle* h, bool refactor, const int* refactor_src, PhaseTime
   CK(cudaGetLastError());
   T.mark(EB_PHASE_PRECOND, h->stream);
   const bool fp32 = h->P.precision == EB_PREC_MIXED;
-  int threads = h->P.threads_per_sim > 0 ? h->P.threads_per_sim : 256;
+  const int threads = h->gmres_threads;
   if (h->gclass.size() == 2) {
     // wide-band simulations on the handle's stream, the two-per-SM class beside them
     CK(cudaEventRecord(h->ev_fork, h->stream));
@@ -1043,6 +1044,7 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
   // ---- solver work
   const int m = p->krylov_restart;
   const bool fp32 = p->precision == EB_PREC_MIXED;
+  if (p->threads_per_sim > 0) h->gmres_threads = p->threads_per_sim;
   CK(A.alloc(&h->d_Dinv64, NN * 36));
   CK(A.alloc(&h->d_Dinv32, NN * 36));
   CK(A.alloc(&h->d_norms, 5 * (size_t)n_sims));
@@ -1052,7 +1054,6 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
   sa.n_sims = n_sims;
   sa.sim_node_off = d.sim_node_off;
   sa.active = d.active;
-  sa.row_ptr = d.row_ptr;
   sa.Kt = d.Kt;
   sa.Ktp = d.Ktp;
   sa.team = 1;
@@ -1131,7 +1132,7 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
     // elimination and update lists level by level
     CondFactor& cf = h->cond;
     {
-      std::vector<int> node_at(NN), ne(n_sims, 0), lev_off(n_sims + 1, 0), lev_ptr;
+      std::vector<int> node_at(NN), ne(n_sims, 0), solo(n_sims, 0), lev_off(n_sims + 1, 0), lev_ptr, lev_wide;
       std::vector<CondRange> range(NN, CondRange{0, 0, 0, 0});
       std::vector<int64_t> base(n_sims + 1, 0), red_off(n_sims + 1, 0);  // first block, first kept block of a simulation
       size_t nlev = 0;
@@ -1144,6 +1145,19 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
         if (!on) continue;
         ne[s] = P.ne;
         lev_ptr.insert(lev_ptr.end(), P.lev_ptr.begin(), P.lev_ptr.end());
+        for (size_t l = 0; l < P.lev_ptr.size(); ++l) {
+          const int p0 = P.lev_ptr[l], p1 = l + 1 < P.lev_ptr.size() ? P.lev_ptr[l + 1] : P.n;
+          const int fwd = P.lptr[p1] - P.lptr[p0], bwd = p1 <= P.ne ? P.wptr[p1] - P.wptr[p0] : 0;
+          lev_wide.push_back((fwd >= kWideBlocks * (p1 - p0) ? kWideFwd : 0) | (bwd >= kWideBlocks * (p1 - p0) ? kWideBwd : 0));
+        }
+        solo[s] = (int)P.tgt.size();
+        while (solo[s] > 1) {
+          const int l = solo[s] - 1;
+          const size_t at = lev_wide.size() - P.lev_ptr.size() + (size_t)l;
+          if (P.lev_ptr[l + 1] - P.lev_ptr[l] > (lev_wide[at] ? kSoloWide : kSoloNarrow)) break;
+          solo[s] = l;
+        }
+        if (solo[s] + 1 >= (int)P.tgt.size()) solo[s] = (int)P.tgt.size();  // a single level gains nothing
         nlev = std::max(nlev, P.tgt.size());
       }
       if (base[n_sims] >= (1LL << 31)) return fail(EB_ERR_ARG, "problem too large for 32-bit block indices");
@@ -1215,6 +1229,9 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
       CK(A.upload(&p_src, src)); CK(A.upload(&p_rn, rnode)); CK(A.upload(&p_cn, cnode)); CK(A.upload(&p_ld, ldiag));
       CK(A.upload(&p_el, elim)); CK(A.upload(&p_en, elim_node)); CK(A.upload(&p_t, tgt)); CK(A.upload(&p_tp, tptr));
       CK(A.upload(&p_cl, cl)); CK(A.upload(&p_cw, cw)); CK(A.upload(&p_red, red)); CK(A.upload(&p_rpos, rpos));
+      int *p_lw, *p_solo;
+      CK(A.upload(&p_lw, lev_wide)); CK(A.upload(&p_solo, solo));
+      cf.c.lev_wide = p_lw; cf.c.solo = p_solo;
       CK(A.upload(&p_range, range)); CK(A.upload(&p_roff, roff)); CK(A.upload(&p_nat, node_at));
       cf.c.scol = p_scol; cf.c.range = p_range; cf.c.ne = p_ne; cf.c.lev_off = p_lo; cf.c.lev_ptr = p_lp; cf.c.roff = p_roff;
       cf.n_blocks = base[n_sims];
@@ -1224,13 +1241,22 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
       cf.red = p_red; cf.rpos = p_rpos;
       h->band.node_at = p_nat;
       std::vector<int> pcol(NB);
-      for (int64_t b = 0; b < NB; ++b) {
-        const int s = blk_sim[b];
-        pcol[b] = plan[s].pos[col[b] - h->node_off[s]];
-      }
+      std::vector<int2> prow(NN);
+      std::vector<uint8_t> pfix(NN, 0);
+      each_sim([&](int s) {
+        const int64_t no = h->node_off[s];
+        for (int64_t b = h->blk_off[s]; b < h->blk_off[s + 1]; ++b) pcol[b] = plan[s].pos[col[b] - no];
+        for (int q = 0; q < plan[s].n; ++q) {
+          const int node = node_at[no + q];
+          prow[no + q] = make_int2(row_ptr[node], row_ptr[node + 1]);
+          for (int k = 0; k < 6; ++k) pfix[no + q] |= (uint8_t)(fixed[6 * (int64_t)node + k] << k);
+        }
+      });
       int* p_pc;
-      CK(A.upload(&p_pc, pcol));
-      sa.pcol = p_pc;
+      int2* p_pr;
+      uint8_t* p_pf;
+      CK(A.upload(&p_pc, pcol)); CK(A.upload(&p_pr, prow)); CK(A.upload(&p_pf, pfix));
+      sa.pcol = p_pc; sa.prow = p_pr; sa.pfix = p_pf;
       h->band.cond = cf.c;
     }
     int64_t *p_boff;
@@ -1345,7 +1371,12 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
   if (h->gclass.empty()) {
     int64_t nmax = 0;
     for (int s = 0; s < n_sims; ++s) nmax = std::max(nmax, 6 * (h->node_off[s + 1] - h->node_off[s]));
-    sa.team = gmres_team(sa, fp32, p->threads_per_sim > 0 ? p->threads_per_sim : 256, (int)nmax);
+    sa.team = gmres_team(sa, fp32, p->threads_per_sim > 0 ? p->threads_per_sim : 512, (int)nmax);
+    // sixteen warps where every CTA has an SM to itself: their phases wait for loads
+    int dev = 0, sms = 0;
+    CK(cudaGetDevice(&dev));
+    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    if (p->threads_per_sim <= 0 && n_sims * sa.team <= sms) h->gmres_threads = 512;
     // z_j, w (double or float) and the FP32 vector of the largest simulation
     const int vec = (int)((nmax * (fp32 ? 3 : 5) + 3) / 4 * 4);
     if (sa.team == 1 && sizeof(float) * (size_t)vec <= kGmresVecSmem) {

@@ -27,6 +27,8 @@ struct CondDev {
   const int* ne;            // per sim: eliminated nodes
   const int* lev_off;       // per sim (n_sims + 1): its range in lev_ptr
   const int* lev_ptr;       // per sim: first position of each level, then ne
+  const int* lev_wide;      // beside lev_ptr: rows of many blocks, kWideFwd | kWideBwd (last: the kept rows)
+  const int* solo;          // per sim: first of the last levels that one CTA walks alone
   const int64_t* roff;      // per sim (n_sims + 1): kept nodes before it (offsets of the diagonal-block inverses)
 };
 
@@ -49,35 +51,99 @@ struct CondFactor {
   const int* rpos;          // positions of their rows
 };
 
-// Rows of positions [p0, p1) of one sweep phase, five positions per warp (`warp` of `nwarps`
-// working together), a position's six rows read before any of them is written (x is updated
-// in place unless `out` is another vector).  x: the simulation's permuted vector; z (backward
-// sweep): the result in T besides.
+constexpr int kWideFwd = 1, kWideBwd = 2;
+// Rows of at least this many blocks (on average over a level) are summed by a warp each, five lanes
+// per row: the last levels of a net have a few dozen rows of 20 to 40 blocks, a serial chain of
+// loads for one lane per row (33 x 33 net, ten levels: a backward sweep 46 us with lanes per row
+// throughout, 29 us with this rule).
+constexpr int kWideBlocks = 6;
+
+// A level that one CTA of sixteen warps finishes in two rounds (positions of warps, of lanes).
+constexpr int kSoloWide = 32, kSoloNarrow = 160;
+
+// What a lane's first row of a sweep phase needs besides the vector: its blocks' range, and the
+// first kAhead blocks' columns and values.  Loaded between the halves of the barrier that ends the
+// previous phase (none of it changes during a solve), so that after it only the vector's loads are
+// left of a chain of three; a team's barrier drops the L1 contents, so each was an L2 round trip.
+// The columns of eight blocks ahead instead were no faster (48 x 200 stent: 28 and 29 us a sweep).
+constexpr int kAhead = 3;
+struct CondAhead {
+  int b, b1;             // first and past the last block of this lane
+  int col[kAhead];
+  float2 s[kAhead][3];
+};
+template <bool FWD>
+__device__ __forceinline__ void cond_ahead(const CondDev& c, int64_t base, int p0, int p1, bool wide, int warp, CondAhead& a) {
+  const int lane = threadIdx.x & 31, sub = lane / 6, r = lane - 6 * sub;
+  const int p = wide ? p0 + warp : p0 + 5 * warp + sub, step = wide ? 5 : 1;
+  a.b = a.b1 = 0;
+  if (sub >= 5 || p >= p1) return;
+  const CondRange g = c.range[base + p];
+  a.b = (FWD ? g.l0 : g.w0) + (wide ? sub : 0);
+  a.b1 = FWD ? g.l1 : g.w1;
+#pragma unroll
+  for (int k = 0; k < kAhead; ++k)
+    if (a.b + k * step < a.b1) {
+      const int64_t b = a.b + k * step;
+      const float2* s = reinterpret_cast<const float2*>(c.S + b * 36 + 6 * r);
+      a.col[k] = c.scol[b];
+      a.s[k][0] = s[0]; a.s[k][1] = s[1]; a.s[k][2] = s[2];
+    }
+}
+
+// Rows of positions [p0, p1) of one sweep phase (`warp` of `nwarps` working together): five
+// positions per warp, one lane per row, or with `wide` one position per warp, five lanes per row.  A
+// position's six rows are read before any of them is written (in place unless `out` is another
+// vector).  x: the simulation's permuted vector; z (backward sweep): the result in T besides;
+// ahead: this phase's cond_ahead.
 template <bool FWD, typename T>
-__device__ __forceinline__ void cond_rows(const CondDev& c, int64_t base, int p0, int p1, float* x, float* out, T* z,
-                                          int warp, int nwarps) {
+__device__ __forceinline__ void cond_rows(const CondDev& c, int64_t base, int p0, int p1, bool wide, float* x, float* out,
+                                          T* z, int warp, int nwarps, const CondAhead& ahead) {
   const int lane = threadIdx.x & 31;
   const int sub = lane / 6, r = lane - 6 * sub;
-  for (int q = p0 + 5 * warp; q < p1; q += 5 * nwarps) {
-    const int p = q + sub;
+  const int per = wide ? 1 : 5, step = wide ? 5 : 1, first = wide ? sub : 0;
+  for (int q = p0 + per * warp; q < p1; q += per * nwarps) {
+    const int p = wide ? q : q + sub;
     const bool on = sub < 5 && p < p1;
     float a0 = 0.f, a1 = 0.f;
+    auto add = [&](const float2 (&s)[3], int col) {
+      const float2* v = reinterpret_cast<const float2*>(x + 6 * col);
+      const float2 v0 = v[0], v1 = v[1], v2 = v[2];
+      a0 = fmaf(s[0].x, v0.x, a0); a1 = fmaf(s[0].y, v0.y, a1);
+      a0 = fmaf(s[1].x, v1.x, a0); a1 = fmaf(s[1].y, v1.y, a1);
+      a0 = fmaf(s[2].x, v2.x, a0); a1 = fmaf(s[2].y, v2.y, a1);
+    };
     if (on) {
-      const CondRange g = c.range[base + p];
-      if (FWD) a0 = x[6 * p + r];
-      const int b0 = FWD ? g.l0 : g.w0, b1 = FWD ? g.l1 : g.w1;
-      for (int b = b0; b < b1; ++b) {
+      if (FWD && first == 0) a0 = x[6 * p + r];
+      int b, b1;
+      if (q == p0 + per * warp) {
+        b = ahead.b;
+        b1 = ahead.b1;
+#pragma unroll
+        for (int k = 0; k < kAhead; ++k) {
+          if (b < b1) add(ahead.s[k], ahead.col[k]);
+          b += step;
+        }
+      } else {
+        const CondRange g = c.range[base + p];
+        b = (FWD ? g.l0 : g.w0) + first;
+        b1 = FWD ? g.l1 : g.w1;
+      }
+#pragma unroll 2
+      for (; b < b1; b += step) {
         const float2* s = reinterpret_cast<const float2*>(c.S + (int64_t)b * 36 + 6 * r);
-        const float2* v = reinterpret_cast<const float2*>(x + 6 * c.scol[b]);
-        const float2 s0 = s[0], s1 = s[1], s2 = s[2], v0 = v[0], v1 = v[1], v2 = v[2];
-        a0 = fmaf(s0.x, v0.x, a0); a1 = fmaf(s0.y, v0.y, a1);
-        a0 = fmaf(s1.x, v1.x, a0); a1 = fmaf(s1.y, v1.y, a1);
-        a0 = fmaf(s2.x, v2.x, a0); a1 = fmaf(s2.y, v2.y, a1);
+        const float2 sv[3] = {s[0], s[1], s[2]};
+        add(sv, c.scol[b]);
       }
     }
+    float y = a0 + a1;
+    if (wide) {  // lanes r, r + 6 .. r + 24
+      const float y1 = __shfl_sync(0xffffffffu, y, r + 6), y2 = __shfl_sync(0xffffffffu, y, r + 12),
+                  y3 = __shfl_sync(0xffffffffu, y, r + 18), y4 = __shfl_sync(0xffffffffu, y, r + 24);
+      y += (y1 + y2) + (y3 + y4);
+    }
     __syncwarp();
-    if (on) {
-      const float y = a0 + a1;
+    if (on && (!wide || sub == 0)) {
       out[6 * p + r] = y;
       if (!FWD) z[6 * p + r] = (T)y;
     }

@@ -28,20 +28,25 @@ namespace eb {
 // The CTAs of one simulation: a cluster of `size` (1: a single CTA).
 struct Team {
   int rank, size;
+  // Barrier in two halves: what needs no other CTA's results is loaded between them.  Release /
+  // acquire at cluster scope: global and shared writes of the other CTAs are seen after wait().
+  __device__ __forceinline__ void arrive() const {
+    if (size > 1) asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+  }
+  __device__ __forceinline__ void wait() const {
+    if (size > 1) asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    else __syncthreads();
+  }
   __device__ __forceinline__ void sync() const {
-    if (size == 1) {
-      __syncthreads();
-    } else {
-      // release / acquire at cluster scope: global and shared writes of the other CTAs are seen
-      asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
-    }
+    arrive();
+    wait();
   }
 };
 
 // Vectors are cut into chunks whose length depends on the simulation alone (at most
 // kMaxChunks of them); a warp owns whole chunks, and sums are formed chunk by chunk and then
 // over the chunks in one fixed order, so no result depends on the number of CTAs or threads.
-constexpr int kMaxChunks = 128;
+constexpr int kMaxChunks = 256;
 __device__ __forceinline__ int chunk_len(int n) { return ((n + kMaxChunks - 1) / kMaxChunks + 31) / 32 * 32; }
 
 struct Work {
@@ -90,9 +95,11 @@ __device__ __forceinline__ double warp_sums(const double (&in)[NQ]) {
 
 // out[q] = Σ_i of what f(i, acc) adds to acc[q]: per lane in TA, over lanes and chunks in FP64.  Each
 // chunk's sums go to every CTA of the team; one team barrier; two buffers in turn, so that a CTA
-// that is ahead does not overwrite sums that another still reads.
+// that is ahead does not overwrite sums that another still reads.  root: out is the sum's square
+// root, with its reciprocal left in w.sums[NQ + q] (one thread's work: a square root and a division
+// by every warp of a CTA hold the FP64 pipe for 2 us).
 template <int NQ, typename TA, typename F>
-__device__ __forceinline__ void team_sum(Work& w, double (&out)[NQ], F f) {
+__device__ __forceinline__ void team_sum(Work& w, double (&out)[NQ], F f, bool root = false) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   constexpr int G = 32 / NQ;  // lanes that hold the same sum
   double* part = w.flip ? w.part[1] : w.part[0];
@@ -102,6 +109,7 @@ __device__ __forceinline__ void team_sum(Work& w, double (&out)[NQ], F f) {
 #pragma unroll
     for (int q = 0; q < NQ; ++q) acc[q] = 0;
     const int i1 = min(w.n, (c + 1) * w.ch);
+#pragma unroll 4
     for (int i = c * w.ch + lane; i < i1; i += 32) f(i, acc);
     double v[NQ];
 #pragma unroll
@@ -124,7 +132,11 @@ __device__ __forceinline__ void team_sum(Work& w, double (&out)[NQ], F f) {
     for (int c = lane; c < w.nchunk; c += 32) s += part[q * kMaxChunks + c];
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-    if (lane == 0) w.sums[q] = s;
+    if (lane == 0) {
+      if (root) s = sqrt(s);
+      w.sums[q] = s;
+      if (root) w.sums[q + NQ] = 1.0 / s;
+    }
   }
   __syncthreads();
 #pragma unroll
@@ -135,10 +147,10 @@ __device__ __forceinline__ void team_sum(Work& w, double (&out)[NQ], F f) {
 template <typename TX>
 __device__ __forceinline__ double row64(const SolverArgs& a, int64_t n0, int i, const TX* x) {
   const int p = i / 6, k = i - 6 * p;
-  const int node = a.band.node_at[n0 + p];
-  if (a.fixed[6 * (int64_t)node + k]) return 0.0;
+  if ((a.pfix[n0 + p] >> k) & 1) return 0.0;
+  const int2 blocks = a.prow[n0 + p];
   double acc0 = 0.0, acc1 = 0.0;
-  for (int bb = a.row_ptr[node]; bb < a.row_ptr[node + 1]; ++bb) {
+  for (int bb = blocks.x; bb < blocks.y; ++bb) {
     const double* Ab = a.Kt + (int64_t)bb * 36 + k;
     const TX* xc = x + 6 * a.pcol[bb];
 #pragma unroll
@@ -157,10 +169,10 @@ __device__ __forceinline__ double row64(const SolverArgs& a, int64_t n0, int i, 
 // each (24-wire stent: 12 cycles and 36 iterations a step, now 6 and 32).
 __device__ __forceinline__ float row_pairs(const SolverArgs& a, int64_t n0, int i, const float* x) {
   const int p = i / 6, k = i - 6 * p;
-  const int node = a.band.node_at[n0 + p];
-  if (a.fixed[6 * (int64_t)node + k]) return 0.f;
+  if ((a.pfix[n0 + p] >> k) & 1) return 0.f;
+  const int2 blocks = a.prow[n0 + p];
   float hi = 0.f, lo = 0.f;
-  for (int bb = a.row_ptr[node]; bb < a.row_ptr[node + 1]; ++bb) {
+  for (int bb = blocks.x; bb < blocks.y; ++bb) {
     const float2* Ab = a.Ktp + (int64_t)bb * 36 + k;
     const float* xc = x + 6 * a.pcol[bb];
 #pragma unroll
@@ -187,6 +199,7 @@ __global__ void __launch_bounds__(512) k_gmres(SolverArgs a) {
     wk.t = Team{(int)r, (int)c};
   }
   const Team& team = wk.t;
+  const int warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
   const int s = a.cta_sim[blockIdx.x / team.size];
   if (!a.active[s]) return;
   const int m = a.m;
@@ -198,15 +211,16 @@ __global__ void __launch_bounds__(512) k_gmres(SolverArgs a) {
   double* cs = H + (m + 1) * m;
   double* sn = cs + m;
   double* g = sn + m;              // m+1
-  double* y = g + m + 1;           // m
-  wk.part[0] = y + m;
+  double* y = g + m + 1;           // m + 1
+  T* yt = reinterpret_cast<T*>(y + m + 1);  // y in the cycle's precision
+  wk.part[0] = y + 2 * m + 2;
   wk.part[1] = wk.part[0] + 8 * kMaxChunks;
-  wk.sums = wk.part[1] + 8 * kMaxChunks;
+  wk.sums = wk.part[1] + 8 * kMaxChunks;  // 16
   wk.flip = 0;
   wk.n = n;
   wk.ch = chunk_len(n);
   wk.nchunk = (n + wk.ch - 1) / wk.ch;
-  wk.warp0 = team.rank * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  wk.warp0 = team.rank + team.size * (threadIdx.x >> 5);  // neighbouring work on different CTAs
   wk.nwarps = team.size * (blockDim.x >> 5);
   T* V = reinterpret_cast<T*>(a.V) + (int64_t)(m + 1) * o;
   T* Zb = reinterpret_cast<T*>(a.Z) + (int64_t)m * o;  // z_j = M⁻¹ v_j at Zb + j n
@@ -225,9 +239,10 @@ __global__ void __launch_bounds__(512) k_gmres(SolverArgs a) {
   const CondDev& cd = a.band.cond;
   const int ne = cd.ne[s];
   const int* lev = cd.lev_ptr + cd.lev_off[s];
+  const int* wide = cd.lev_wide + cd.lev_off[s];
   const int nlev = max(0, cd.lev_off[s + 1] - cd.lev_off[s] - 1);
   // the dense product's input, dense_ld entries, read as float4
-  float* xd = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(wk.sums + 8) + 15) & ~uintptr_t(15));
+  float* xd = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(wk.sums + 16) + 15) & ~uintptr_t(15));
   float* xs = a.x_in_smem ? xd + a.dense_ld + a.vec_smem : nullptr;  // the kept entries during the band sweeps
   T* zs = reinterpret_cast<T*>(xd + a.dense_ld);  // vec_smem floats: z_j, w, xa
   T* ws = zs + n;
@@ -274,8 +289,8 @@ __global__ void __launch_bounds__(512) k_gmres(SolverArgs a) {
     X[i] = (use_x0 && !fx) ? a.dD[d] : 0.0;
     R[i] = bi;
     q[0] += bi * bi;
-  });
-  const double bnorm = sqrt(v1[0]);
+  }, true);
+  const double bnorm = v1[0];
   double rnorm = bnorm;
   if (use_x0 && isfinite(bnorm)) {
     // initial guess: X = α x0 with α = <A x0, b> / <A x0, A x0> clipped to [0, 1], so that
@@ -293,9 +308,9 @@ __global__ void __launch_bounds__(512) k_gmres(SolverArgs a) {
       const double ri = R[i] - alpha * row64(a, n0, i, X);
       R[i] = ri;
       q[0] += ri * ri;
-    });
+    }, true);
     wk.each([&](int i) { X[i] *= alpha; });
-    rnorm = sqrt(v1[0]);
+    rnorm = v1[0];
   }
   int its = 0, refs = 0, status = 0;
   if (!isfinite(bnorm)) status = 2;  // EB_SIM_NAN
@@ -325,14 +340,22 @@ __global__ void __launch_bounds__(512) k_gmres(SolverArgs a) {
     for (int ref = 0; ref < a.max_ref && rnorm > target && its < a.max_iter; ++ref) {
       // ---- one GMRES(m) cycle on the FP64 residual R
       const double beta = rnorm;
-      const double ib = 1.0 / beta;
+      const double ib = wk.sums[1];  // 1 / beta: beta is the last sum's root
       wk.each([&](int i) {
         const T v = (T)(R[i] * ib);
         V[i] = v;
         xa[i] = (float)v;
       });
       if (threadIdx.x == 0) g[0] = beta;
-      team.sync();
+      CondAhead ahead;
+      auto first_ahead = [&] {
+        const int l = min(1, nlev);
+        if (use_band || dn)
+          cond_ahead<true>(cd, n0, l < nlev ? lev[l] : ne, l < nlev ? lev[l + 1] : n / 6, wide[l] & kWideFwd, wk.warp0, ahead);
+      };
+      team.arrive();
+      first_ahead();
+      team.wait();
       // a cycle that can reach the target aims at half of it, from zero as from an initial guess: its
       // estimate differs from the true residual by rounding, and a residual left just above the
       // target costs another cycle
@@ -347,32 +370,66 @@ __global__ void __launch_bounds__(512) k_gmres(SolverArgs a) {
         T* zj = vs ? zs : zg;
         // ---- z_j = M⁻¹ v_j; v_j lies in xa (FP32) when the preconditioner starts
         if (use_band || dn) {
-          for (int l = 1; l < nlev; ++l) {  // level 0 receives nothing
-            cond_rows<true>(cd, n0, lev[l], lev[l + 1], xa, xa, (T*)nullptr, wk.warp0, wk.nwarps);
-            team.sync();
+          // phases: forward levels 1 .. (level 0 receives nothing), the kept rows (phase nlev), the kept
+          // system, backward levels; `ahead` always holds the next phase's first blocks
+          auto fwd_ahead = [&](int l) {
+            cond_ahead<true>(cd, n0, l < nlev ? lev[l] : ne, l < nlev ? lev[l + 1] : n / 6, wide[l] & kWideFwd, wk.warp0, ahead);
+          };
+          auto bwd_ahead = [&](int l) {
+            if (l >= 0) cond_ahead<false>(cd, n0, lev[l], lev[l + 1], wide[l] & kWideBwd, wk.warp0, ahead);
+          };
+          float* kin = dn ? a.kin + 6 * cd.roff[s] - 6 * ne : xa;
+          // levels from `solo` on are so small that one CTA walks them faster by its own barriers (1.1
+          // us a phase on a ring, whose levels are all that small) than the team by its own (2.4 us)
+          const int solo = team.size > 1 ? max(1, cd.solo[s]) : nlev;
+          for (int l = 1; l < min(solo, nlev); ++l) {
+            cond_rows<true>(cd, n0, lev[l], lev[l + 1], wide[l] & kWideFwd, xa, xa, (T*)nullptr, wk.warp0, wk.nwarps, ahead);
+            team.arrive();
+            if (l + 1 < solo || solo >= nlev) fwd_ahead(l + 1);
+            team.wait();
           }
+          if (solo < nlev) {
+            if (team.rank == 0)
+              for (int l = solo; l < nlev; ++l) {
+                cond_ahead<true>(cd, n0, lev[l], lev[l + 1], wide[l] & kWideFwd, warp, ahead);
+                if (l > solo) __syncthreads();
+                cond_rows<true>(cd, n0, lev[l], lev[l + 1], wide[l] & kWideFwd, xa, xa, (T*)nullptr, warp, nwarp, ahead);
+              }
+            team.arrive();
+            fwd_ahead(nlev);
+            team.wait();
+          }
+          cond_rows<true>(cd, n0, ne, n / 6, wide[nlev] & kWideFwd, xa, kin, (T*)nullptr, wk.warp0, wk.nwarps, ahead);
+          team.sync();
           if (dn) {
-            float* kin = a.kin + 6 * cd.roff[s];
-            cond_rows<true>(cd, n0, ne, n / 6, xa, kin - 6 * ne, (T*)nullptr, wk.warp0, wk.nwarps);
-            team.sync();
             const int ld = dense_ld(dn);
-            for (int i = threadIdx.x; i < ld; i += blockDim.x) xd[i] = i < dn ? kin[i] : 0.f;
+            for (int i = threadIdx.x; i < ld; i += blockDim.x) xd[i] = i < dn ? kin[6 * ne + i] : 0.f;
             __syncthreads();
             dense_rows(a.dense.G + a.dense.off[s], dn, ld, xd, xa + 6 * ne, zj + 6 * ne, wk.warp0, wk.nwarps);
-            team.sync();
           } else {
-            if (ne > 0) {
-              cond_rows<true>(cd, n0, ne, n / 6, xa, xa, (T*)nullptr, wk.warp0, wk.nwarps);
-              team.sync();
-            }
             if (team.rank == 0) band_sweeps(a.band, s, xa + 6 * ne, xs, stp, ph);
             team.sync();
             for (int i = 6 * ne + wk.warp0 * 32 + (threadIdx.x & 31); i < n; i += 32 * wk.nwarps) zj[i] = (T)xa[i];
-            if (nlev == 0) team.sync();
           }
-          for (int l = nlev - 1; l >= 0; --l) {
-            cond_rows<false>(cd, n0, lev[l], lev[l + 1], xa, xa, zj, wk.warp0, wk.nwarps);
-            team.sync();
+          team.arrive();
+          if (solo >= nlev) bwd_ahead(nlev - 1);
+          team.wait();
+          if (solo < nlev) {
+            if (team.rank == 0)
+              for (int l = nlev - 1; l >= solo; --l) {
+                cond_ahead<false>(cd, n0, lev[l], lev[l + 1], wide[l] & kWideBwd, warp, ahead);
+                if (l < nlev - 1) __syncthreads();
+                cond_rows<false>(cd, n0, lev[l], lev[l + 1], wide[l] & kWideBwd, xa, xa, zj, warp, nwarp, ahead);
+              }
+            team.arrive();
+            bwd_ahead(solo - 1);
+            team.wait();
+          }
+          for (int l = min(solo, nlev) - 1; l >= 0; --l) {
+            cond_rows<false>(cd, n0, lev[l], lev[l + 1], wide[l] & kWideBwd, xa, xa, zj, wk.warp0, wk.nwarps, ahead);
+            team.arrive();
+            bwd_ahead(l - 1);
+            team.wait();
           }
         } else {
           const T* vj = V + (int64_t)j * n;
@@ -393,54 +450,87 @@ __global__ void __launch_bounds__(512) k_gmres(SolverArgs a) {
           if (vs) zg[i] = zj[i];
         });
         __syncwarp();
+        // The second pass also forms w·w: ‖w - Σ y v‖² = w·w - Σ y², of which the first pass has left next
+        // to nothing to subtract, so that its update can normalise w at once.
         for (int pass = 0; pass < 2; ++pass) {
-          for (int i0 = 0; i0 <= j;) {
+          const int last = j + pass;  // in the second pass, "v_(j+1)" is w itself
+          for (int i0 = 0; i0 <= last;) {
             // inner products with v_i0 .., as many at a time as are left (at most 8)
             auto dots = [&](auto width) {
               constexpr int NQ = decltype(width)::value;
-              const int nq = min(NQ, j + 1 - i0);
+              const int nq = min(NQ, last + 1 - i0);
               const T* Vq = V + (int64_t)i0 * n;
               double hp[NQ];
               team_sum<NQ, T>(wk, hp, [&](int i, T (&q)[NQ]) {
                 const T wi = w[i];
 #pragma unroll
                 for (int u = 0; u < NQ; ++u)
-                  if (u < nq) q[u] += Vq[(int64_t)u * n + i] * wi;
+                  if (u < nq) q[u] += (i0 + u > j ? wi : Vq[(int64_t)u * n + i]) * wi;
               });
               if (threadIdx.x == 0)
 #pragma unroll
                 for (int q = 0; q < NQ; ++q)
                   if (q < nq) {
-                    double* h = H + (m + 1) * j + i0 + q;
-                    *h = (pass == 0 ? 0.0 : *h) + hp[q];
-                    y[i0 + q] = hp[q];  // this pass's coefficients (y is free until the back-substitution)
+                    y[i0 + q] = hp[q];
+                    if (i0 + q <= j) {
+                      double* h = H + (m + 1) * j + i0 + q;
+                      *h = (pass == 0 ? 0.0 : *h) + hp[q];
+                      yt[i0 + q] = (T)hp[q];  // this pass's coefficients
+                    }
                   }
               i0 += NQ;
             };
-            const int left = j + 1 - i0;
+            const int left = last + 1 - i0;
             if (left > 4) dots(std::integral_constant<int, 8>{});
             else if (left > 2) dots(std::integral_constant<int, 4>{});
             else if (left > 1) dots(std::integral_constant<int, 2>{});
             else dots(std::integral_constant<int, 1>{});
           }
-          __syncthreads();
-          wk.each([&](int i) {
-            T acc = w[i];
-            for (int q = 0; q <= j; ++q) acc -= (T)y[q] * V[(int64_t)q * n + i];
-            w[i] = acc;
-          });
-          __syncthreads();  // y is read before the next pass rewrites it
+          if (pass == 0) {
+            __syncthreads();
+            wk.each([&](int i) {
+              T acc = w[i];
+#pragma unroll 4
+              for (int q = 0; q <= j; ++q) acc -= yt[q] * V[(int64_t)q * n + i];
+              w[i] = acc;
+            });
+            __syncthreads();  // yt is read before the next pass rewrites it
+          }
         }
-        double nn[1];
-        team_sum<1, T>(wk, nn, [&](int i, T (&q)[1]) { q[0] += w[i] * w[i]; });
-        const double hn = sqrt(nn[0]);
-        if (hn > 0.0) {
-          const T ihn = (T)(1.0 / hn);
-          wk.each([&](int i) {
-            const T v = w[i] * ihn;
-            vn[i] = v;
-            xa[i] = (float)v;
-          });
+        if (threadIdx.x == 0) {
+          double ww = y[j + 1], yy = 0.0;
+          for (int q = 0; q <= j; ++q) yy += y[q] * y[q];
+          const double h2 = ww - yy;
+          const double hn = h2 > 0.25 * ww ? sqrt(h2) : -1.0;  // else too much was subtracted (or NaN)
+          wk.sums[8] = hn;
+          wk.sums[9] = hn > 0.0 ? 1.0 / hn : 0.0;
+        }
+        __syncthreads();
+        double hn = wk.sums[8];
+        const bool direct = !(hn >= 0.0);  // the same in every CTA: the sums are
+        T ihn = (T)wk.sums[9];
+        if (direct) ihn = (T)1;
+        wk.each([&](int i) {
+          T acc = w[i];
+#pragma unroll 4
+          for (int q = 0; q <= j; ++q) acc -= yt[q] * V[(int64_t)q * n + i];
+          const T v = acc * ihn;
+          if (direct) w[i] = v;
+          vn[i] = v;
+          xa[i] = (float)v;
+        });
+        if (direct) {
+          double nn[1];
+          team_sum<1, T>(wk, nn, [&](int i, T (&q)[1]) { q[0] += w[i] * w[i]; }, true);
+          hn = nn[0];
+          if (hn > 0.0) {
+            ihn = (T)wk.sums[1];
+            wk.each([&](int i) {
+              const T v = w[i] * ihn;
+              vn[i] = v;
+              xa[i] = (float)v;
+            });
+          }
         }
         if (threadIdx.x == 0) {
           double* Hj = H + (m + 1) * j;
@@ -450,9 +540,10 @@ __global__ void __launch_bounds__(512) k_gmres(SolverArgs a) {
             Hj[i + 1] = -sn[i] * Hj[i] + cs[i] * Hj[i + 1];
             Hj[i] = t;
           }
-          const double den = hypot(Hj[j], Hj[j + 1]);
-          const double c = den > 0.0 ? Hj[j] / den : 1.0;
-          const double sv = den > 0.0 ? Hj[j + 1] / den : 0.0;
+          const double den = sqrt(Hj[j] * Hj[j] + hn * hn);
+          const double rden = den > 0.0 ? 1.0 / den : 0.0;
+          const double c = den > 0.0 ? Hj[j] * rden : 1.0;
+          const double sv = hn * rden;
           cs[j] = c;
           sn[j] = sv;
           Hj[j] = den;
@@ -460,18 +551,35 @@ __global__ void __launch_bounds__(512) k_gmres(SolverArgs a) {
           g[j + 1] = -sv * g[j];
           g[j] = c * g[j];
         }
-        team.sync();
+        team.arrive();
+        first_ahead();
+        team.wait();
         ++its;
         k = j + 1;
         const double gres = fabs(g[j + 1]);
         if (!(gres > inner_target) || hn <= DBL_MIN || !isfinite(gres)) break;
       }
       // back-substitution H y = g (k x k upper triangular)
-      if (threadIdx.x == 0) {
+      if (threadIdx.x < 32) {  // a lane per row (four beyond 32), column by column
+        const int lane = threadIdx.x;
+        double t[4], inv[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int q = lane + 32 * u;
+          t[u] = q < k ? g[q] : 0.0;
+          inv[u] = q < k ? 1.0 / H[(m + 1) * q + q] : 0.0;
+        }
         for (int i = k - 1; i >= 0; --i) {
-          double t = g[i];
-          for (int q = i + 1; q < k; ++q) t -= H[(m + 1) * q + i] * y[q];
-          y[i] = t / H[(m + 1) * i + i];
+          double yi = 0.0;
+#pragma unroll
+          for (int u = 0; u < 4; ++u)
+            if ((i >> 5) == u) yi = __shfl_sync(0xffffffffu, t[u] * inv[u], i & 31);
+          if (lane == 0) y[i] = yi;
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int q = lane + 32 * u;
+            if (q < i) t[u] -= H[(m + 1) * i + q] * yi;
+          }
         }
       }
       __syncthreads();
@@ -489,8 +597,8 @@ __global__ void __launch_bounds__(512) k_gmres(SolverArgs a) {
         const double ri = (a.fixed[d] ? 0.0 : a.b[d]) - row64(a, n0, i, X);
         R[i] = ri;
         q[0] += ri * ri;
-      });
-      rnorm = sqrt(v1[0]);
+      }, true);
+      rnorm = v1[0];
       ++refs;
       if (!isfinite(rnorm)) { status = 2; break; }
     }
@@ -580,7 +688,7 @@ void launch_block_jacobi(const Dev& d, double* Dinv64, float* Dinv32, cudaStream
 }
 
 size_t gmres_smem(int m) {
-  return sizeof(double) * ((size_t)(m + 1) * m + 4 * (size_t)m + 1 + 16 * (size_t)kMaxChunks + 8 + 1);
+  return sizeof(double) * ((size_t)(m + 1) * m + 5 * (size_t)m + 3 + 16 * (size_t)kMaxChunks + 16 + 1);
 }
 
 size_t gmres_smem_total(const SolverArgs& a) {

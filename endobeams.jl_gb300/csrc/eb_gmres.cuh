@@ -11,7 +11,8 @@ struct SolverArgs {
   const int* cta_sim;    // team -> simulation
   const int64_t* sim_node_off;
   const int* active;
-  const int* row_ptr;
+  const int2* prow;      // per position: the tangent's blocks of its row
+  const uint8_t* pfix;   // per position: bit d = its DOF d is fixed
   const int* pcol;       // per block of the tangent: position of its column node in the solver's order
   const double* Kt;
   const float2* Ktp;     // the tangent as FP32 pairs (mixed precision)
