@@ -48,14 +48,37 @@ struct MlpTrainer {
   int64_t step = 0;
 };
 
-cudaError_t mlp_trainer_init(MlpTrainer& t, const float* params_host, cudaStream_t s);
-void mlp_trainer_free(MlpTrainer& t);
+// Device arrays of one call in one allocation, each aligned to 256 bytes (an allocation and its
+// release cost 30 to 40 us; a gradient call made nine).
+struct MlpSlab {
+  void* base = nullptr;
+  size_t bytes = 0;
+  struct Part {
+    void** to;
+    size_t off;
+  } parts[16];
+  int n_parts = 0;
+  template <typename T>
+  void want(T** p, size_t n) {
+    parts[n_parts++] = {reinterpret_cast<void**>(p), bytes};
+    bytes += (sizeof(T) * n + 255) / 256 * 256;
+  }
+  cudaError_t make();
+  MlpSlab() = default;
+  MlpSlab(const MlpSlab&) = delete;
+  MlpSlab& operator=(const MlpSlab&) = delete;
+  ~MlpSlab() { cudaFree(base); }
+};
+
+// Adds the trainer's arrays to the slab, allocates it and sets the first state.
+cudaError_t mlp_trainer_init(MlpTrainer& t, MlpSlab& slab, const float* params_host, cudaStream_t s);
 // Loss (mean squared error over rows[0..n) and outputs) and its gradient in t.G;
 // rows == nullptr: rows 0..n-1.  *loss_dev (device) receives the loss.
 cudaError_t mlp_loss_grad(MlpTrainer& t, const float* X, const float* T, const int* rows, int64_t n, double* loss_dev,
                           cudaStream_t s);
-// One Adam step on t.P from t.G; refreshes the BF16 copy.
-cudaError_t mlp_adam(MlpTrainer& t, float lr, cudaStream_t s);
+// One Adam step on t.P from the same gradient (t.G is not written); refreshes the BF16 copy.
+cudaError_t mlp_train_step(MlpTrainer& t, const float* X, const float* T, const int* rows, int64_t n, float lr,
+                           double* loss_dev, cudaStream_t s);
 // BF16 copy of an FP32 parameter vector.
 cudaError_t mlp_to_bf16(const float* P, __nv_bfloat16* W, cudaStream_t s);
 
