@@ -8,6 +8,7 @@
 #include <cstdio>
 #include <cstring>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <thread>
 #include <vector>
@@ -264,6 +265,11 @@ struct IterGraph {
   PhaseTimer timer;  // events recorded by the graph; launch counts per replay
 };
 
+// Doubles of a step's inputs (four per simulation, a mask) and of its statistics (one, four ints).
+constexpr size_t in_doubles(size_t sims) { return 4 * sims + (sims + 1) / 2; }
+constexpr size_t out_doubles(size_t sims) { return 3 * sims; }
+constexpr int64_t kStateChunk = 4096;  // nodes of a simulation's state per launch (1.2 MB pinned)
+
 struct eb_handle {
   // Releases the streams, events, graphs, pinned mirrors and output writer; the arena and
   // the warm-start buffers free their device memory in their own destructors.
@@ -281,9 +287,7 @@ struct eb_handle {
       if (G.exec) cudaGraphExecDestroy(G.exec);
       G.timer.destroy();
     }
-    if (pin_active) cudaFreeHost(pin_active);
-    if (pin_refactor) cudaFreeHost(pin_refactor);
-    if (pin_norms) cudaFreeHost(pin_norms);
+    if (pin) cudaFreeHost(pin);
     if (side) cudaStreamDestroy(side);
     if (ev_fork) cudaEventDestroy(ev_fork);
     if (ev_join) cudaEventDestroy(ev_join);
@@ -294,8 +298,14 @@ struct eb_handle {
   PhaseTimer timer;
   WsHost ws;
   // pinned host mirrors used by the captured iterations, and the graphs
-  int *pin_active = nullptr, *pin_refactor = nullptr;
-  double* pin_norms = nullptr;
+  // (one allocation: Newton norms; a step's inputs as in d_in; its statistics as in d_out; masks;
+  // node state of up to state_chunk nodes)
+  char* pin = nullptr;
+  double *pin_norms = nullptr, *pin_in = nullptr, *pin_out = nullptr, *pin_state = nullptr;
+  int *pin_active = nullptr, *pin_refactor = nullptr, *pin_mask = nullptr;
+  int state_chunk = 0;
+  std::mutex state_mu;  // pin_state
+  bool any_fixed = false;  // some simulation has boundary conditions
   IterGraph graph[2];      // without / with band refactorisation
   uint64_t graph_gen = 1;  // bumped when launch parameters captured in the graphs change
   cudaEvent_t t0 = nullptr, t1 = nullptr;
@@ -321,7 +331,8 @@ struct eb_handle {
   // per-sim device arrays
   int* d_mask = nullptr;
   int* d_active = nullptr;
-  double *d_cK = nullptr, *d_cC = nullptr, *d_cM = nullptr, *d_dt = nullptr;
+  double* d_in = nullptr;   // cK, cC, cM, Δt of every simulation, then the activity mask (one copy per step)
+  double* d_out = nullptr;  // relres of every simulation, then its, refs, status, pred_its (one copy per step)
   // solver
   SolverArgs sa{};
   int gmres_threads = 256;
@@ -375,11 +386,9 @@ __global__ void k_interleave3(const double* __restrict__ u, int64_t n, double* _
 }
 
 int upload_mask(eb_handle* h, int* dst, const int32_t* mask) {
-  std::vector<int> m(h->n_sims, 1);
-  if (mask)
-    for (int s = 0; s < h->n_sims; ++s) m[s] = mask[s] != 0;
-  CK(cudaMemcpyAsync(dst, m.data(), sizeof(int) * h->n_sims, cudaMemcpyHostToDevice, h->stream));
-  CK(cudaStreamSynchronize(h->stream));
+  CK(cudaStreamSynchronize(h->stream));  // an earlier copy from the mirror has ended
+  for (int s = 0; s < h->n_sims; ++s) h->pin_mask[s] = mask ? mask[s] != 0 : 1;
+  CK(cudaMemcpyAsync(dst, h->pin_mask, sizeof(int) * h->n_sims, cudaMemcpyHostToDevice, h->stream));
   return EB_OK;
 }
 
@@ -532,6 +541,13 @@ void resolve_graph_times(eb_handle* h, bool refactor) {
   }
 }
 
+// r -= Ktan[:, fixed] ΔD[fixed]
+void lift_bc(eb_handle* h, PhaseTimer& T) {
+  if (!h->any_fixed) return;
+  launch_bc_lift(h->d, h->stream);
+  T.launches[EB_PHASE_RESIDUAL] += 1;
+}
+
 // One corrector iteration after the first (assembly, residual, solve, Newmark
 // and rotation updates, norms) as stream operations; eb_step replays it from
 // a CUDA graph, one per refactorisation variant.  Its host inputs and outputs
@@ -563,16 +579,13 @@ int record_iteration(eb_handle* h, bool refactor, PhaseTimer& T) {
     CK(cudaEventRecord(h->ev_join, h->side));
     CK(cudaStreamWaitEvent(st, h->ev_join, 0));
   }
-  launch_gather(d, a, h->any_contact, st);
+  launch_gather(d, a, h->any_contact, true, st);
   T.launches[EB_PHASE_ASSEMBLY] += 2;
-  launch_corrector_rhs(d, a, st);
-  launch_apply_bc(d, st);
-  T.launches[EB_PHASE_RESIDUAL] += 3;
+  lift_bc(h, T);
   int rc = launch_solve(h, refactor, h->pin_refactor, T, true);
   if (rc) return rc;
-  launch_global_corrector(d, st);
-  launch_local_corrector(d, b, g, st);
-  T.launches[EB_PHASE_UPDATE] += 2;
+  launch_corrector_update(d, b, g, st);
+  T.launches[EB_PHASE_UPDATE] += 1;
   CK(cudaMemcpyAsync(h->pin_norms, h->d_norms, sizeof(double) * 5 * S, cudaMemcpyDeviceToHost, st));
   T.mark(EB_PHASE_UPDATE, st);
   return EB_OK;
@@ -673,9 +686,6 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
   CK(cudaEventCreate(&h->t0));
   CK(cudaEventCreate(&h->t1));
   h->timer.init(p->timing != 0);
-  CK(cudaMallocHost(&h->pin_active, sizeof(int) * (size_t)n_sims));
-  CK(cudaMallocHost(&h->pin_refactor, sizeof(int) * (size_t)n_sims));
-  CK(cudaMallocHost(&h->pin_norms, sizeof(double) * 5 * (size_t)n_sims));
 
   // ---- sizes and offsets
   h->node_off.assign(n_sims + 1, 0);
@@ -817,6 +827,7 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
       h->fix_dof.push_back(6 * no + S.fixed_dofs[k]);
     }
     has_fixed[s] = S.n_fixed > 0;
+    h->any_fixed |= S.n_fixed > 0;
     for (int64_t k = 0; k < S.n_loaded; ++k) {
       h->load_dof.push_back(6 * no + S.loaded_dofs[k]);
       fext[6 * no + S.loaded_dofs[k]] = S.fext0 ? S.fext0[k] : 0.0;  // Forces(conf), def_structures.jl:10-31
@@ -930,13 +941,26 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
   CK(A.upload(&p_blk_off, h->blk_off));
   d.sim_node_off = p_node_off;
   d.sim_blk_off = p_blk_off;
-  CK(A.alloc(&h->d_active, n_sims));
+  CK(A.alloc(&h->d_in, in_doubles(n_sims)));
+  h->d_active = reinterpret_cast<int*>(h->d_in + 4 * (size_t)n_sims);
   CK(A.alloc(&h->d_mask, n_sims));
-  CK(A.alloc(&h->d_cK, n_sims));
-  CK(A.alloc(&h->d_cC, n_sims));
-  CK(A.alloc(&h->d_cM, n_sims));
-  CK(A.alloc(&h->d_dt, n_sims));
-  d.active = h->d_active; d.cK = h->d_cK; d.cC = h->d_cC; d.cM = h->d_cM; d.dt = h->d_dt;
+  d.active = h->d_active;
+  d.cK = h->d_in; d.cC = d.cK + n_sims; d.cM = d.cC + n_sims; d.dt = d.cM + n_sims;
+  // pinned mirrors
+  {
+    int64_t nmax = 0;
+    for (int s = 0; s < n_sims; ++s) nmax = std::max(nmax, h->node_off[s + 1] - h->node_off[s]);
+    h->state_chunk = (int)std::min<int64_t>(nmax, kStateChunk);
+    const size_t S = n_sims, doubles = 5 * S + in_doubles(S) + out_doubles(S) + (3 * S + 1) / 2 + 36 * (size_t)h->state_chunk;
+    CK(cudaMallocHost(&h->pin, sizeof(double) * doubles));
+    h->pin_norms = reinterpret_cast<double*>(h->pin);
+    h->pin_in = h->pin_norms + 5 * S;
+    h->pin_out = h->pin_in + in_doubles(S);
+    h->pin_state = h->pin_out + out_doubles(S);
+    h->pin_active = reinterpret_cast<int*>(h->pin_state + 36 * (size_t)h->state_chunk);
+    h->pin_refactor = h->pin_active + S;
+    h->pin_mask = h->pin_refactor + S;
+  }
   // SDF coefficient grids: simulations that pass the same grid (same values pointer,
   // dims, spacing, origin and inside flag) share one device copy; distinct grids are
   // prefiltered on host threads in chunks and uploaded as each chunk completes.
@@ -1048,8 +1072,12 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
   CK(A.alloc(&h->d_Dinv64, NN * 36));
   CK(A.alloc(&h->d_Dinv32, NN * 36));
   CK(A.alloc(&h->d_norms, 5 * (size_t)n_sims));
-  CK(A.alloc(&h->d_its, n_sims)); CK(A.alloc(&h->d_refs, n_sims)); CK(A.alloc(&h->d_status, n_sims));
-  CK(A.alloc(&h->d_relres, n_sims));
+  CK(A.alloc(&h->d_out, out_doubles(n_sims)));
+  h->d_relres = h->d_out;
+  h->d_its = reinterpret_cast<int*>(h->d_out + n_sims);
+  h->d_refs = h->d_its + n_sims;
+  h->d_status = h->d_refs + n_sims;
+  h->d_pred_its = h->d_status + n_sims;
   SolverArgs& sa = h->sa;
   sa.n_sims = n_sims;
   sa.sim_node_off = d.sim_node_off;
@@ -1095,7 +1123,6 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
   sa.forcing_max = p->forcing_max;
   CK(A.alloc(&sa.prev_bnorm, n_sims));
   CK(A.alloc(&sa.prev_eta, n_sims));
-  CK(A.alloc(&h->d_pred_its, n_sims));
   CK(A.alloc(&h->d_x0_on, n_sims));
   CK(cudaMemset(h->d_x0_on, 0, sizeof(int) * n_sims));
   sa.x0_on = h->d_x0_on;
@@ -1410,7 +1437,7 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
   int rc = upload_mask(h.get(), h->d_active, nullptr);
   if (rc) return rc;
   launch_beam(d, h->gauss, h->stream);
-  launch_gather(d, p->alpha, false, h->stream);
+  launch_gather(d, p->alpha, false, false, h->stream);
   CK(cudaGetLastError());
   CK(cudaMemcpyAsync(d.Kn, d.K1, sizeof(double) * NB * 36, cudaMemcpyDeviceToDevice, h->stream));
   CK(cudaMemcpyAsync(d.Cn, d.C1, sizeof(double) * NB * 36, cudaMemcpyDeviceToDevice, h->stream));
@@ -1597,9 +1624,9 @@ int eb_autotune(eb_handle* h, int32_t* chosen) {
   if (err == cudaSuccess && h->any_contact)
     err = time_it(&d.contact_threads, kElem, 3, [&] { launch_contact(d, h->gauss, st); });
   if (err == cudaSuccess)
-    err = time_it(&d.gmat_threads, kGather, 3, [&] { launch_gather(d, alpha, h->any_contact, st); });
+    err = time_it(&d.gmat_threads, kGather, 3, [&] { launch_gather(d, alpha, h->any_contact, true, st); });
   if (err == cudaSuccess)
-    err = time_it(&d.gvec_threads, kGather, 3, [&] { launch_gather(d, alpha, h->any_contact, st); });
+    err = time_it(&d.gvec_threads, kGather, 3, [&] { launch_gather(d, alpha, h->any_contact, true, st); });
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   CK(err);
@@ -1719,19 +1746,16 @@ static int learned_start_check(eb_handle* h, const std::vector<int>& running, do
   launch_restore_nodes(d, h->d_mask, st);
   launch_init_predictor(d, st);
   launch_predictor_rhs(d, a, b, g, st);
-  launch_apply_bc(d, st);
-  T.launches[EB_PHASE_PREDICTOR] += 4;
+  lift_bc(h, T);
+  T.launches[EB_PHASE_PREDICTOR] += 3;
   int rc = solve(h, fb.data(), false);
   if (rc) return rc;
-  launch_global_predictor(d, b, g, st);
-  launch_local_predictor(d, b, g, st);
-  launch_init_corrector(d, st);
+  launch_predictor_update(d, b, g, st);
   launch_beam(d, h->gauss, st);
   if (h->any_contact) launch_contact(d, h->gauss, st);
-  launch_gather(d, a, h->any_contact, st);
-  launch_corrector_rhs(d, a, st);
-  launch_apply_bc(d, st);
-  T.launches[EB_PHASE_PREDICTOR] += 9;
+  launch_gather(d, a, h->any_contact, true, st);
+  lift_bc(h, T);
+  T.launches[EB_PHASE_PREDICTOR] += 5;
   CK(cudaMemcpyAsync(h->d_active, running.data(), sizeof(int) * S, cudaMemcpyHostToDevice, st));
   CK(cudaGetLastError());
   return EB_OK;
@@ -1746,8 +1770,8 @@ int eb_step(eb_handle* h, const double* dt, const int32_t* active, int32_t* k_ou
   if ((learned || learned_x0) && !h->ws.model)
     return fail(EB_ERR_STATE, "eb_step: a learned warm start is selected but no model is set");
   const double a = P.alpha, b = P.beta, g = P.gamma;
-  std::vector<double> cK(S), cC(S), cM(S), dts(S);
   std::vector<int> act(S), iter(S, 0), k(S, 1);
+  double *cK = h->pin_in, *cC = cK + S, *cM = cC + S, *dts = cM + S;
   for (int s = 0; s < S; ++s) {
     act[s] = active ? (active[s] != 0) : 1;
     if (act[s] && !(dt[s] > 0)) return fail(EB_ERR_ARG, "eb_step: dt[%d] must be positive", s);
@@ -1759,15 +1783,9 @@ int eb_step(eb_handle* h, const double* dt, const int32_t* active, int32_t* k_ou
     cM[s] = 1 / (b * (dt[s] * dt[s]));
   }
   cudaStream_t st = h->stream;
-  CK(cudaMemcpyAsync(h->d_cK, cK.data(), sizeof(double) * S, cudaMemcpyHostToDevice, st));
-  CK(cudaMemcpyAsync(h->d_cC, cC.data(), sizeof(double) * S, cudaMemcpyHostToDevice, st));
-  CK(cudaMemcpyAsync(h->d_cM, cM.data(), sizeof(double) * S, cudaMemcpyHostToDevice, st));
-  CK(cudaMemcpyAsync(h->d_dt, dts.data(), sizeof(double) * S, cudaMemcpyHostToDevice, st));
-  CK(cudaMemcpyAsync(h->d_active, act.data(), sizeof(int) * S, cudaMemcpyHostToDevice, st));
-  CK(cudaMemsetAsync(h->d_its, 0, sizeof(int) * S, st));
-  CK(cudaMemsetAsync(h->d_refs, 0, sizeof(int) * S, st));
-  CK(cudaMemsetAsync(h->d_status, 0, sizeof(int) * S, st));
-  CK(cudaMemsetAsync(h->d_relres, 0, sizeof(double) * S, st));
+  std::memcpy(dts + S, act.data(), sizeof(int) * S);
+  CK(cudaMemcpyAsync(h->d_in, h->pin_in, sizeof(double) * in_doubles(S), cudaMemcpyHostToDevice, st));
+  CK(cudaMemsetAsync(h->d_out, 0, sizeof(double) * out_doubles(S), st));
   const Dev& d = h->d;
   PhaseTimer& T = h->timer;
   h->mid_step = true;
@@ -1783,9 +1801,9 @@ int eb_step(eb_handle* h, const double* dt, const int32_t* active, int32_t* k_ou
   // ---- predictor! (predictor.jl:1-27)
   launch_init_predictor(d, st);
   launch_predictor_rhs(d, a, b, g, st);
-  launch_apply_bc(d, st);
+  lift_bc(h, T);
   T.mark(EB_PHASE_PREDICTOR, st);
-  T.launches[EB_PHASE_PREDICTOR] += 4;
+  T.launches[EB_PHASE_PREDICTOR] += 2;
   int rc = 0;
   if (learned) {
     // Simulations whose learned starts were rejected recently back off (1, 2, 4 .. 64 steps)
@@ -1827,12 +1845,10 @@ int eb_step(eb_handle* h, const double* dt, const int32_t* active, int32_t* k_ou
     if (rc) return rc;
   }
   CK(cudaMemcpyAsync(h->d_pred_its, h->d_its, sizeof(int) * S, cudaMemcpyDeviceToDevice, st));
-  launch_global_predictor(d, b, g, st);
-  launch_local_predictor(d, b, g, st);
-  // ---- corrector! (corrector.jl:1-59)
-  launch_init_corrector(d, st);
+  // ---- end of the predictor, start of corrector! (corrector.jl:1-59)
+  launch_predictor_update(d, b, g, st);
   T.mark(EB_PHASE_PREDICTOR, st);
-  T.launches[EB_PHASE_PREDICTOR] += 3;
+  T.launches[EB_PHASE_PREDICTOR] += 1;
   CK(cudaGetLastError());
   if (T.on) {
     CK(cudaStreamSynchronize(st));
@@ -1873,13 +1889,11 @@ int eb_step(eb_handle* h, const double* dt, const int32_t* active, int32_t* k_ou
       T.mark(EB_PHASE_CONTACT, st);
       T.launches[EB_PHASE_CONTACT] += 1;
     }
-    launch_gather(d, a, h->any_contact, st);
+    launch_gather(d, a, h->any_contact, true, st);
     T.mark(EB_PHASE_ASSEMBLY, st);
     T.launches[EB_PHASE_ASSEMBLY] += 2;
-    launch_corrector_rhs(d, a, st);
-    launch_apply_bc(d, st);
+    lift_bc(h, T);
     T.mark(EB_PHASE_RESIDUAL, st);
-    T.launches[EB_PHASE_RESIDUAL] += 3;
     if (learned && first) {
       rc = learned_start_check(h, running, a, b, g);
       if (rc) return rc;
@@ -1887,9 +1901,8 @@ int eb_step(eb_handle* h, const double* dt, const int32_t* active, int32_t* k_ou
     first = false;
     rc = solve(h, running.data(), true);
     if (rc) return rc;
-    launch_global_corrector(d, st);
-    launch_local_corrector(d, b, g, st);
-    T.launches[EB_PHASE_UPDATE] += 2;
+    launch_corrector_update(d, b, g, st);
+    T.launches[EB_PHASE_UPDATE] += 1;
     CK(cudaMemcpyAsync(h->h_norms.data(), h->d_norms, sizeof(double) * 5 * S, cudaMemcpyDeviceToHost, st));
     T.mark(EB_PHASE_UPDATE, st);
     CK(cudaStreamSynchronize(st));
@@ -1936,14 +1949,10 @@ int eb_step(eb_handle* h, const double* dt, const int32_t* active, int32_t* k_ou
     }
   }
   // ---- statistics
-  std::vector<int> its(S), refs(S), status(S), pred_its(S);
-  std::vector<double> rel(S);
-  CK(cudaMemcpyAsync(pred_its.data(), h->d_pred_its, sizeof(int) * S, cudaMemcpyDeviceToHost, st));
-  CK(cudaMemcpyAsync(its.data(), h->d_its, sizeof(int) * S, cudaMemcpyDeviceToHost, st));
-  CK(cudaMemcpyAsync(refs.data(), h->d_refs, sizeof(int) * S, cudaMemcpyDeviceToHost, st));
-  CK(cudaMemcpyAsync(status.data(), h->d_status, sizeof(int) * S, cudaMemcpyDeviceToHost, st));
-  CK(cudaMemcpyAsync(rel.data(), h->d_relres, sizeof(double) * S, cudaMemcpyDeviceToHost, st));
+  CK(cudaMemcpyAsync(h->pin_out, h->d_out, sizeof(double) * out_doubles(S), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
+  const double* rel = h->pin_out;
+  const int *its = reinterpret_cast<const int*>(rel + S), *refs = its + S, *status = refs + S, *pred_its = status + S;
   for (int s = 0; s < S; ++s) {
     eb_sim_stats& q = h->stats[s];
     if (!act[s]) continue;
@@ -1989,7 +1998,7 @@ static int commit_impl(eb_handle* h, const int32_t* mask, bool commit) {
   }
   ws.features_valid = false;
   launch_commit(h->d, h->d_mask, commit, h->stream);
-  h->timer.launches[EB_PHASE_UPDATE] += 3;
+  h->timer.launches[EB_PHASE_UPDATE] += 1;
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(h->stream));
   return EB_OK;
@@ -2001,18 +2010,22 @@ int eb_rollback(eb_handle* h, const int32_t* mask) { return commit_impl(h, mask,
 static int get_state_impl(eb_handle* h, int32_t sim, bool at_n, double* u, double* ud, double* udd, double* w,
                           double* wd, double* wdd, double* R, double* dR) {
   if (!h || sim < 0 || sim >= h->n_sims) return fail(EB_ERR_ARG, "bad handle or sim index");
-  const int64_t NN = h->d.n_nodes, o = h->node_off[sim], n = h->node_off[sim + 1] - o;
-  const Dev& d = h->d;
-  double* src[8] = {at_n ? d.un : d.u,   at_n ? d.udn : d.ud, at_n ? d.uddn : d.udd, at_n ? d.wn : d.w,
-                    at_n ? d.wdn : d.wd, at_n ? d.wddn : d.wdd, at_n ? d.Rn : d.R,   at_n ? d.dRn : d.dR};
+  const int64_t o = h->node_off[sim], n = h->node_off[sim + 1] - o;
   double* dst[8] = {u, ud, udd, w, wd, wdd, R, dR};
-  const int nc[8] = {3, 3, 3, 3, 3, 3, 9, 9};
-  std::vector<double> tmp((size_t)n);
-  for (int f = 0; f < 8; ++f) {
-    if (!dst[f]) continue;
-    for (int k = 0; k < nc[f]; ++k) {
-      CK(cudaMemcpy(tmp.data(), src[f] + k * NN + o, sizeof(double) * n, cudaMemcpyDeviceToHost));
-      for (int64_t i = 0; i < n; ++i) dst[f][nc[f] * i + k] = tmp[i];
+  unsigned fields = 0;
+  for (int f = 0; f < 8; ++f) fields |= (dst[f] ? 1u : 0u) << f;
+  if (!fields) return EB_OK;
+  std::lock_guard<std::mutex> lock(h->state_mu);
+  for (int64_t i0 = 0; i0 < n; i0 += h->state_chunk) {
+    const int m = (int)std::min<int64_t>(h->state_chunk, n - i0);
+    launch_state(h->d, at_n, fields, o + i0, m, h->pin_state, h->stream);
+    CK(cudaGetLastError());
+    CK(cudaStreamSynchronize(h->stream));
+    const double* src = h->pin_state;
+    for (int f = 0; f < 8; ++f) {
+      const int nc = f < 6 ? 3 : 9;
+      if (dst[f]) std::memcpy(dst[f] + nc * i0, src, sizeof(double) * nc * m);
+      src += (int64_t)nc * m;
     }
   }
   return EB_OK;
@@ -2049,6 +2062,7 @@ int eb_set_state(eb_handle* h, int32_t sim, const double* u, const double* ud, c
         CK(cudaMemcpy(dst[f][t] + k * NN + o, tmp.data(), sizeof(double) * n, cudaMemcpyHostToDevice));
     }
   }
+  CK(cudaStreamSynchronize(nullptr));  // the handle's stream does not wait for the default stream
   return EB_OK;
 }
 

@@ -102,19 +102,18 @@ cudaError_t raise_smem_limit(const void* func, size_t bytes);
 
 void launch_beam(const Dev& d, const Gauss3& g, cudaStream_t s);
 void launch_contact(const Dev& d, const Gauss3& g, cudaStream_t s);
-void launch_gather(const Dev& d, double alpha, bool with_contact, cudaStream_t s);
+// rhs: also the corrector's residual and the imposed increments.
+void launch_gather(const Dev& d, double alpha, bool with_contact, bool rhs, cudaStream_t s);
 void launch_init_predictor(const Dev& d, cudaStream_t s);
 void launch_predictor_rhs(const Dev& d, double alpha, double beta, double gamma, cudaStream_t s);
-void launch_corrector_rhs(const Dev& d, double alpha, cudaStream_t s);
-void launch_apply_bc(const Dev& d, cudaStream_t s);
-void launch_global_predictor(const Dev& d, double beta, double gamma, cudaStream_t s);
-void launch_local_predictor(const Dev& d, double beta, double gamma, cudaStream_t s);
-void launch_init_corrector(const Dev& d, cudaStream_t s);
-void launch_global_corrector(const Dev& d, cudaStream_t s);
-void launch_local_corrector(const Dev& d, double beta, double gamma, cudaStream_t s);
+void launch_bc_lift(const Dev& d, cudaStream_t s);
+void launch_predictor_update(const Dev& d, double beta, double gamma, cudaStream_t s);
+void launch_corrector_update(const Dev& d, double beta, double gamma, cudaStream_t s);
 void launch_commit(const Dev& d, const int* mask, bool commit, cudaStream_t s);
 // node state at n+1 <- node state at n (the node part of update_not_converged!)
 void launch_restore_nodes(const Dev& d, const int* mask, cudaStream_t s);
+// The fields set in `fields` (bit order u, ud, udd, w, wd, wdd, R, dR) of m nodes, 36 m values.
+void launch_state(const Dev& d, bool at_n, unsigned fields, int64_t first, int m, double* out, cudaStream_t s);
 // quadratic B-spline prefilter of a padded SDF coefficient grid (interior = samples), eb_testing.cu
 void launch_sdf_prefilter(double* coef, int nx, int ny, int nz, cudaStream_t s);
 

@@ -143,9 +143,17 @@ __global__ void k_gather_mat(Dev d, double alpha, int with_contact) {
   if (d.Ktp) d.Ktp[t] = fp32_pair(kt);
 }
 
+// ΔD[fixed] = imposed - D[fixed] (apply_boundary_conditions!, utils_bcs_and_loads.jl:5-29); the
+// other part, r -= Ktan[:, fixed] ΔD[fixed], is k_bc_lift.
+__device__ __forceinline__ void bc_delta(const Dev& d, int64_t t) {
+  if (d.fixed[t]) d.dD[t] = d.imposed[t] - d.D[t];
+}
+
 // Thread per (node, dof): Tⁱⁿᵗ, Tᵏ, Tᶜ as ordered sums over incident elements
-// (assemble_beams.jl:60-61, compute&assemble…:493).
-__global__ void k_gather_vec(Dev d, int with_contact) {
+// (assemble_beams.jl:60-61, compute&assemble…:493); with `rhs` also the residual
+// (compute_tangent_and_residuals_corrector!, utils_solver.jl:87) and the imposed increments: as
+// launches of their own these two cost 4.3 and 2.7 us of a 64-element ring's iteration.
+__global__ void k_gather_vec(Dev d, double alpha, int with_contact, int rhs) {
   int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= d.n_dof) return;
   const int i = (int)(t / 6), k = (int)(t % 6);
@@ -167,14 +175,18 @@ __global__ void k_gather_vec(Dev d, int with_contact) {
       Tc += d.scT[e * 12 + 6 * (v & 1) + k];
     }
   }
+  if (rhs) {
+    d.r[t] = ((1 + alpha) * ((d.fext1[t] + Tc) - Ti) - alpha * ((d.fextn[t] + d.Tcn[t]) - d.Tin[t])) - Tk;
+    bc_delta(d, t);
+  }
   d.Ti1[t] = Ti;
   d.Tk1[t] = Tk;
   d.Tc1[t] = Tc;
 }
 
-void launch_gather(const Dev& d, double alpha, bool with_contact, cudaStream_t s) {
+void launch_gather(const Dev& d, double alpha, bool with_contact, bool rhs, cudaStream_t s) {
   if (d.nnzb) k_gather_mat<<<nblocks(d.nnzb * 36, d.gmat_threads), d.gmat_threads, 0, s>>>(d, alpha, with_contact ? 1 : 0);
-  if (d.n_dof) k_gather_vec<<<nblocks(d.n_dof, d.gvec_threads), d.gvec_threads, 0, s>>>(d, with_contact ? 1 : 0);
+  if (d.n_dof) k_gather_vec<<<nblocks(d.n_dof, d.gvec_threads), d.gvec_threads, 0, s>>>(d, alpha, with_contact ? 1 : 0, rhs ? 1 : 0);
 }
 
 // ------------------------------------------------------------------ predictor
@@ -198,7 +210,9 @@ __global__ void k_init_predictor(Dev d) {
 }
 
 // compute_tangent_and_residuals_predictor! (utils_solver.jl:54-74), thread per (node, dof):
-// Ktan from the matrices at n, r = (1+α)fⁿ⁺¹ - Tⁱⁿᵗⁿ - Tᵏⁿ - αfⁿ + Cⁿ t₁ + Mⁿ t₂ /(βΔt²).
+// Ktan from the matrices at n, r = (1+α)fⁿ⁺¹ - Tⁱⁿᵗⁿ - Tᵏⁿ - αfⁿ + Cⁿ t₁ + Mⁿ t₂ /(βΔt²); the
+// imposed increments.  A block's 30 values are loaded before any is stored: with loads and stores
+// in turn a thread waited for L2 six times per block (64-element ring: 19.7 us).
 __global__ void k_predictor_rhs(Dev d, double alpha, double beta, double gamma) {
   int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= d.n_dof) return;
@@ -216,14 +230,22 @@ __global__ void k_predictor_rhs(Dev d, double alpha, double beta, double gamma) 
     const double* Cb = d.Cn + (int64_t)bb * 36;
     const double* Mb = d.Mn + (int64_t)bb * 36;
     const double* Kb = d.Kn + (int64_t)bb * 36;
+    double vd[6], va[6], kv[6], cw[6], mw[6];
 #pragma unroll
     for (int j = 0; j < 6; ++j) {
-      const double vd = d.Dd[6 * c + j], va = d.Ddd[6 * c + j];
-      const double t1 = a1 * vd - a2 * va;
-      const double t2 = dt * vd + b2 * va;
-      cv += Cb[6 * j + k] * t1;
-      mv += Mb[6 * j + k] * t2;
-      const double kt = (cK * Kb[6 * j + k] + cC * Cb[6 * j + k]) + cM * Mb[6 * j + k];
+      kv[j] = Kb[6 * j + k];
+      cw[j] = Cb[6 * j + k];
+      mw[j] = Mb[6 * j + k];
+      vd[j] = d.Dd[6 * c + j];
+      va[j] = d.Ddd[6 * c + j];
+    }
+#pragma unroll
+    for (int j = 0; j < 6; ++j) {
+      const double t1 = a1 * vd[j] - a2 * va[j];
+      const double t2 = dt * vd[j] + b2 * va[j];
+      cv += cw[j] * t1;
+      mv += mw[j] * t2;
+      const double kt = (cK * kv[j] + cC * cw[j]) + cM * mw[j];
       d.Kt[(int64_t)bb * 36 + 6 * j + k] = kt;
       if (d.Ktp) d.Ktp[(int64_t)bb * 36 + 6 * j + k] = fp32_pair(kt);
     }
@@ -231,6 +253,7 @@ __global__ void k_predictor_rhs(Dev d, double alpha, double beta, double gamma) 
   r = cv + r;
   r = cM * mv + r;
   d.r[t] = r;
+  bc_delta(d, t);
 }
 
 void launch_init_predictor(const Dev& d, cudaStream_t s) {
@@ -240,27 +263,6 @@ void launch_predictor_rhs(const Dev& d, double alpha, double beta, double gamma,
   if (d.n_dof) k_predictor_rhs<<<nblocks(d.n_dof, 256), 256, 0, s>>>(d, alpha, beta, gamma);
 }
 
-// compute_tangent_and_residuals_corrector! residual (utils_solver.jl:87)
-__global__ void k_corrector_rhs(Dev d, double alpha) {
-  int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= d.n_dof) return;
-  if (!d.active[d.node_sim[t / 6]]) return;
-  d.r[t] = ((1 + alpha) * ((d.fext1[t] + d.Tc1[t]) - d.Ti1[t]) - alpha * ((d.fextn[t] + d.Tcn[t]) - d.Tin[t])) -
-           d.Tk1[t];
-}
-void launch_corrector_rhs(const Dev& d, double alpha, cudaStream_t s) {
-  if (d.n_dof) k_corrector_rhs<<<nblocks(d.n_dof, 256), 256, 0, s>>>(d, alpha);
-}
-
-// apply_boundary_conditions! (utils_bcs_and_loads.jl:5-29):
-// ΔD[fixed] = imposed - D[fixed]; r -= Ktan[:, fixed] ΔD[fixed].
-__global__ void k_bc_delta(Dev d) {
-  int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= d.n_dof) return;
-  if (!d.fixed[t]) return;
-  if (!d.active[d.node_sim[t / 6]]) return;
-  d.dD[t] = d.imposed[t] - d.D[t];
-}
 __global__ void k_bc_lift(Dev d) {
   int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= d.n_dof) return;
@@ -276,28 +278,22 @@ __global__ void k_bc_lift(Dev d) {
   }
   d.r[t] -= acc;
 }
-void launch_apply_bc(const Dev& d, cudaStream_t s) {
+void launch_bc_lift(const Dev& d, cudaStream_t s) {
   if (!d.n_dof) return;
-  k_bc_delta<<<nblocks(d.n_dof, 256), 256, 0, s>>>(d);
   k_bc_lift<<<nblocks(d.n_dof, 256), 256, 0, s>>>(d);
 }
 
-// compute_global_predictor! (utils_solver.jl:157-172)
-__global__ void k_global_predictor(Dev d, double beta, double gamma) {
-  int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= d.n_dof) return;
-  const int s = d.node_sim[t / 6];
-  if (!d.active[s]) return;
-  const double dt = d.dt[s];
-  const double g_bdt = gamma / (beta * dt), g_b = gamma / beta, inv = 1 / (beta * (dt * dt));
-  const double dt2b = (dt * (2 * beta - gamma)) / (2 * beta);
-  const double Ddn = d.Dd[t], dD = d.dD[t], Ddd = d.Ddd[t];
-  d.D[t] += dD;
-  d.Dd[t] += (g_bdt * dD - g_b * Ddn) + dt2b * Ddd;
-  d.Ddd[t] += inv * ((dD - dt * Ddn) - ((dt * dt) / 2) * Ddd);
+// A node's six values of a vector in DOF order (48 bytes, 16-byte aligned).
+__device__ __forceinline__ void load6(const double* p, int64_t i, double* v) {
+  const double2* q = reinterpret_cast<const double2*>(p + 6 * i);
+  const double2 a = q[0], b = q[1], c = q[2];
+  v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y; v[4] = c.x; v[5] = c.y;
 }
-void launch_global_predictor(const Dev& d, double beta, double gamma, cudaStream_t s) {
-  if (d.n_dof) k_global_predictor<<<nblocks(d.n_dof, 256), 256, 0, s>>>(d, beta, gamma);
+__device__ __forceinline__ void store6(double* p, int64_t i, V3 a, V3 b) {
+  double2* q = reinterpret_cast<double2*>(p + 6 * i);
+  q[0] = make_double2(a.x, a.y);
+  q[1] = make_double2(a.z, b.x);
+  q[2] = make_double2(b.y, b.z);
 }
 
 // angular rates of utils_solver.jl:214-215 / :239-240
@@ -309,144 +305,178 @@ __device__ __forceinline__ void rates(const M3& dR, V3 w, V3 wdn, V3 wddn, doubl
   *wdd = dR * b;
 }
 
-// compute_local_predictor! (utils_solver.jl:197-217)
-__global__ void k_local_predictor(Dev d, double beta, double gamma) {
+// End of the predictor, thread per node: compute_global_predictor! (utils_solver.jl:157-172),
+// compute_local_predictor! (:197-217) and initialize_global_corrector! (:6-24).  Everything a node
+// needs is loaded before the first store, one round trip to L2 instead of one per field (64-element
+// ring: 7.4 + 13.5 + 5 us as three launches with loads and stores in turn).
+__global__ void k_predictor_update(Dev d, double beta, double gamma) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= d.n_nodes) return;
   const int s = d.node_sim[i];
   if (!d.active[s]) return;
   const int64_t n = d.n_nodes;
   const double dt = d.dt[s];
-  const double* D = d.D + 6 * i;
-  const double* Dd = d.Dd + 6 * i;
-  const double* Ddd = d.Ddd + 6 * i;
-  store3(d.u, n, i, v3(D[0], D[1], D[2]));
-  store3(d.ud, n, i, v3(Dd[0], Dd[1], Dd[2]));
-  store3(d.udd, n, i, v3(Ddd[0], Ddd[1], Ddd[2]));
-  V3 th = v3(D[3], D[4], D[5]);
-  store3(d.w, n, i, th);
-  M3 dR = rotation_matrix(th);
-  store9(d.dR, n, i, dR);
-  store9(d.R, n, i, dR * node9(d.Rn, n, i));
-  V3 wd, wdd;
-  rates(dR, th, node3(d.wdn, n, i), node3(d.wddn, n, i), beta, gamma, dt, &wd, &wdd);
-  store3(d.wd, n, i, wd);
-  store3(d.wdd, n, i, wdd);
-}
-void launch_local_predictor(const Dev& d, double beta, double gamma, cudaStream_t s) {
-  if (d.n_nodes) k_local_predictor<<<nblocks(d.n_nodes), kThreads, 0, s>>>(d, beta, gamma);
-}
-
-// initialize_global_corrector! (utils_solver.jl:6-24)
-__global__ void k_init_corrector(Dev d) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= d.n_nodes) return;
-  if (!d.active[d.node_sim[i]]) return;
-  const int64_t n = d.n_nodes;
-  V3 u = node3(d.u, n, i), ud = node3(d.ud, n, i), udd = node3(d.udd, n, i);
-  V3 w = node3(d.w, n, i), wd = node3(d.wd, n, i), wdd = node3(d.wdd, n, i);
-  double* D = d.D + 6 * i;
-  double* Dd = d.Dd + 6 * i;
-  double* Ddd = d.Ddd + 6 * i;
-  double* dD = d.dD + 6 * i;
-  D[0] = u.x; D[1] = u.y; D[2] = u.z; D[3] = w.x; D[4] = w.y; D[5] = w.z;
-  Dd[0] = ud.x; Dd[1] = ud.y; Dd[2] = ud.z; Dd[3] = wd.x; Dd[4] = wd.y; Dd[5] = wd.z;
-  Ddd[0] = udd.x; Ddd[1] = udd.y; Ddd[2] = udd.z; Ddd[3] = wdd.x; Ddd[4] = wdd.y; Ddd[5] = wdd.z;
+  double D[6], Dd[6], Ddd[6], dD[6];
+  load6(d.D, i, D);
+  load6(d.Dd, i, Dd);
+  load6(d.Ddd, i, Ddd);
+  load6(d.dD, i, dD);
+  const V3 wdn = node3(d.wdn, n, i), wddn = node3(d.wddn, n, i);
+  const M3 Rn = node9(d.Rn, n, i);
+  const double g_bdt = gamma / (beta * dt), g_b = gamma / beta, inv = 1 / (beta * (dt * dt));
+  const double dt2b = (dt * (2 * beta - gamma)) / (2 * beta);
 #pragma unroll
-  for (int k = 0; k < 6; ++k) dD[k] = 0.0;
+  for (int k = 0; k < 6; ++k) {
+    const double v = Dd[k], a = Ddd[k];
+    D[k] += dD[k];
+    Dd[k] += (g_bdt * dD[k] - g_b * v) + dt2b * a;
+    Ddd[k] += inv * ((dD[k] - dt * v) - ((dt * dt) / 2) * a);
+  }
+  const V3 u = v3(D[0], D[1], D[2]), ud = v3(Dd[0], Dd[1], Dd[2]), udd = v3(Ddd[0], Ddd[1], Ddd[2]);
+  const V3 th = v3(D[3], D[4], D[5]);
+  const M3 dR = rotation_matrix(th);
+  V3 wd, wdd;
+  rates(dR, th, wdn, wddn, beta, gamma, dt, &wd, &wdd);
+  store3(d.u, n, i, u);
+  store3(d.ud, n, i, ud);
+  store3(d.udd, n, i, udd);
+  store3(d.w, n, i, th);
+  store9(d.dR, n, i, dR);
+  store9(d.R, n, i, dR * Rn);
+  store3(d.wd, n, i, wd);
+  store3(d.wdd, n, i, wdd);
+  store6(d.D, i, u, th);
+  store6(d.Dd, i, ud, wd);
+  store6(d.Ddd, i, udd, wdd);
+  store6(d.dD, i, v3(0.0, 0.0, 0.0), v3(0.0, 0.0, 0.0));
 }
-void launch_init_corrector(const Dev& d, cudaStream_t s) {
-  if (d.n_nodes) k_init_corrector<<<nblocks(d.n_nodes), kThreads, 0, s>>>(d);
+void launch_predictor_update(const Dev& d, double beta, double gamma, cudaStream_t s) {
+  if (d.n_nodes) k_predictor_update<<<nblocks(d.n_nodes), kThreads, 0, s>>>(d, beta, gamma);
 }
 
-// compute_global_corrector! (utils_solver.jl:178-190)
-__global__ void k_global_corrector(Dev d) {
-  int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= d.n_dof) return;
-  const int s = d.node_sim[t / 6];
-  if (!d.active[s]) return;
-  const double dD = d.dD[t];
-  d.D[t] += dD;
-  d.Dd[t] += d.cC[s] * dD;
-  d.Ddd[t] += d.cM[s] * dD;
-}
-void launch_global_corrector(const Dev& d, cudaStream_t s) {
-  if (d.n_dof) k_global_corrector<<<nblocks(d.n_dof, 256), 256, 0, s>>>(d);
-}
-
-// compute_local_corrector! (utils_solver.jl:224-245); node w is not written, as in the reference.
-__global__ void k_local_corrector(Dev d, double beta, double gamma) {
+// End of a corrector iteration, thread per node: compute_global_corrector! (utils_solver.jl:178-190)
+// and compute_local_corrector! (:224-245); node w is not written, as in the reference.  Loads first,
+// as above (64-element ring: 4.5 + 16.3 us as two launches with loads and stores in turn).
+__global__ void k_corrector_update(Dev d, double beta, double gamma) {
   int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= d.n_nodes) return;
   const int s = d.node_sim[i];
   if (!d.active[s]) return;
   const int64_t n = d.n_nodes;
-  const double dt = d.dt[s];
-  const double* D = d.D + 6 * i;
-  const double* Dd = d.Dd + 6 * i;
-  const double* Ddd = d.Ddd + 6 * i;
-  const double* dD = d.dD + 6 * i;
-  store3(d.u, n, i, v3(D[0], D[1], D[2]));
-  store3(d.ud, n, i, v3(Dd[0], Dd[1], Dd[2]));
-  store3(d.udd, n, i, v3(Ddd[0], Ddd[1], Ddd[2]));
-  M3 dR = rotation_matrix(v3(dD[3], dD[4], dD[5])) * node9(d.dR, n, i);
-  V3 w1 = toangle(dR);
+  const double dt = d.dt[s], cC = d.cC[s], cM = d.cM[s];
+  double D[6], Dd[6], Ddd[6], dD[6];
+  load6(d.D, i, D);
+  load6(d.Dd, i, Dd);
+  load6(d.Ddd, i, Ddd);
+  load6(d.dD, i, dD);
+  const V3 wdn = node3(d.wdn, n, i), wddn = node3(d.wddn, n, i);
+  const M3 dR0 = node9(d.dR, n, i), Rn = node9(d.Rn, n, i);
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+    D[k] += dD[k];
+    Dd[k] += cC * dD[k];
+    Ddd[k] += cM * dD[k];
+  }
+  const V3 u = v3(D[0], D[1], D[2]), ud = v3(Dd[0], Dd[1], Dd[2]), udd = v3(Ddd[0], Ddd[1], Ddd[2]);
+  const M3 dR = rotation_matrix(v3(dD[3], dD[4], dD[5])) * dR0;
+  const V3 w1 = toangle(dR);
   V3 wd, wdd;
-  rates(dR, w1, node3(d.wdn, n, i), node3(d.wddn, n, i), beta, gamma, dt, &wd, &wdd);
+  rates(dR, w1, wdn, wddn, beta, gamma, dt, &wd, &wdd);
+  store6(d.D, i, u, v3(D[3], D[4], D[5]));
+  store6(d.Dd, i, ud, v3(Dd[3], Dd[4], Dd[5]));
+  store6(d.Ddd, i, udd, v3(Ddd[3], Ddd[4], Ddd[5]));
+  store3(d.u, n, i, u);
+  store3(d.ud, n, i, ud);
+  store3(d.udd, n, i, udd);
   store9(d.dR, n, i, dR);
   store3(d.wd, n, i, wd);
   store3(d.wdd, n, i, wdd);
-  store9(d.R, n, i, dR * node9(d.Rn, n, i));
+  store9(d.R, n, i, dR * Rn);
 }
-void launch_local_corrector(const Dev& d, double beta, double gamma, cudaStream_t s) {
-  if (d.n_nodes) k_local_corrector<<<nblocks(d.n_nodes), kThreads, 0, s>>>(d, beta, gamma);
+void launch_corrector_update(const Dev& d, double beta, double gamma, cudaStream_t s) {
+  if (d.n_nodes) k_corrector_update<<<nblocks(d.n_nodes), kThreads, 0, s>>>(d, beta, gamma);
 }
 
 // ------------------------------------------------------------------ commit / rollback
 // update_converged! (utils_solver.jl:252-275) when commit, else update_not_converged! (:282-305).
-__global__ void k_commit_nodes(Dev d, const int* mask, int commit) {
-  int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= d.n_nodes) return;
-  if (!mask[d.node_sim[i]]) return;
+// One launch: a thread per value of the node fields (component-major, 36 per node), then one per
+// DOF, then one per block entry.  A thread's loads precede its stores; a thread per node went through
+// 36 of them in turn (19 us for 64 nodes, and two more launches).
+struct NodeFields {
+  double* p[8];
+};
+constexpr int kNodeValues = 36;
+__global__ void k_commit(const __grid_constant__ Dev d, const __grid_constant__ NodeFields work,
+                         const __grid_constant__ NodeFields kept, const int* mask, int commit, int64_t total) {
+  int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= total) return;
   const int64_t n = d.n_nodes;
-  double* a[8] = {d.u, d.ud, d.udd, d.w, d.wd, d.wdd, d.R, d.dR};
-  double* b[8] = {d.un, d.udn, d.uddn, d.wn, d.wdn, d.wddn, d.Rn, d.dRn};
-  const int nc[8] = {3, 3, 3, 3, 3, 3, 9, 9};
-#pragma unroll
-  for (int f = 0; f < 8; ++f)
-    for (int k = 0; k < nc[f]; ++k) {
-      if (commit) b[f][k * n + i] = a[f][k * n + i];
-      else a[f][k * n + i] = b[f][k * n + i];
-    }
-}
-__global__ void k_commit_dofs(Dev d, const int* mask, int commit) {
-  int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= d.n_dof) return;
-  if (!mask[d.node_sim[t / 6]]) return;
-  if (commit) {
-    d.Tin[t] = d.Ti1[t]; d.Tkn[t] = d.Tk1[t]; d.Tcn[t] = d.Tc1[t]; d.fextn[t] = d.fext1[t];
-  } else {
-    d.Ti1[t] = d.Tin[t]; d.Tk1[t] = d.Tkn[t]; d.Tc1[t] = d.Tcn[t]; d.fext1[t] = d.fextn[t];
+  if (t < kNodeValues * n) {
+    const int c = (int)(t / n);
+    const int64_t i = t - c * n;
+    if (!mask[d.node_sim[i]]) return;
+    const int f = c < 18 ? c / 3 : 6 + (c - 18) / 9;
+    const int64_t at = (c < 18 ? c % 3 : (c - 18) % 9) * n + i;
+    if (commit) kept.p[f][at] = work.p[f][at];
+    else work.p[f][at] = kept.p[f][at];
+    return;
   }
-}
-__global__ void k_commit_blocks(Dev d, const int* mask, int commit) {
-  int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= d.nnzb * 36) return;
+  t -= kNodeValues * n;
+  if (t < d.n_dof) {
+    if (!mask[d.node_sim[t / 6]]) return;
+    if (commit) {
+      const double a = d.Ti1[t], b = d.Tk1[t], c = d.Tc1[t], e = d.fext1[t];
+      d.Tin[t] = a; d.Tkn[t] = b; d.Tcn[t] = c; d.fextn[t] = e;
+    } else {
+      const double a = d.Tin[t], b = d.Tkn[t], c = d.Tcn[t], e = d.fextn[t];
+      d.Ti1[t] = a; d.Tk1[t] = b; d.Tc1[t] = c; d.fext1[t] = e;
+    }
+    return;
+  }
+  t -= d.n_dof;
   if (!mask[d.blk_sim[t / 36]]) return;
   if (commit) {
-    d.Kn[t] = d.K1[t]; d.Cn[t] = d.C1[t]; d.Mn[t] = d.M1[t];
+    const double a = d.K1[t], b = d.C1[t], c = d.M1[t];
+    d.Kn[t] = a; d.Cn[t] = b; d.Mn[t] = c;
   } else {
-    d.K1[t] = d.Kn[t]; d.C1[t] = d.Cn[t]; d.M1[t] = d.Mn[t];
+    const double a = d.Kn[t], b = d.Cn[t], c = d.Mn[t];
+    d.K1[t] = a; d.C1[t] = b; d.M1[t] = c;
   }
 }
+
+static NodeFields node_fields(const Dev& d, bool at_n) {
+  return at_n ? NodeFields{{d.un, d.udn, d.uddn, d.wn, d.wdn, d.wddn, d.Rn, d.dRn}}
+              : NodeFields{{d.u, d.ud, d.udd, d.w, d.wd, d.wdd, d.R, d.dR}};
+}
+static void commit_values(const Dev& d, const int* mask, bool commit, int64_t total, cudaStream_t s) {
+  if (total) k_commit<<<nblocks(total, 256), 256, 0, s>>>(d, node_fields(d, false), node_fields(d, true), mask, commit ? 1 : 0, total);
+}
 void launch_commit(const Dev& d, const int* mask, bool commit, cudaStream_t s) {
-  if (d.n_nodes) k_commit_nodes<<<nblocks(d.n_nodes), kThreads, 0, s>>>(d, mask, commit ? 1 : 0);
-  if (d.n_dof) k_commit_dofs<<<nblocks(d.n_dof, 256), 256, 0, s>>>(d, mask, commit ? 1 : 0);
-  if (d.nnzb) k_commit_blocks<<<nblocks(d.nnzb * 36, 256), 256, 0, s>>>(d, mask, commit ? 1 : 0);
+  commit_values(d, mask, commit, kNodeValues * d.n_nodes + d.n_dof + 36 * d.nnzb, s);
 }
 
 void launch_restore_nodes(const Dev& d, const int* mask, cudaStream_t s) {
-  if (d.n_nodes) k_commit_nodes<<<nblocks(d.n_nodes), kThreads, 0, s>>>(d, mask, 0);
+  commit_values(d, mask, false, kNodeValues * d.n_nodes, s);
+}
+
+// Node fields of m nodes from `first` as arrays of structures, field by field, into `out` (pinned
+// host memory: the values go straight there, one launch instead of a copy per component).
+__global__ void k_state(const __grid_constant__ NodeFields f, int64_t n, int64_t first, int m, double* out) {
+  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= (int64_t)kNodeValues * m) return;
+  const bool vec = t < 18 * (int64_t)m;
+  const int nc = vec ? 3 : 9;
+  const int64_t u = vec ? t : t - 18 * (int64_t)m;
+  const int k = (int)(u / ((int64_t)nc * m));
+  const int64_t e = u - (int64_t)k * nc * m;
+  const double* src = f.p[vec ? k : 6 + k];
+  if (src) out[t] = src[(e % nc) * n + first + e / nc];
+}
+void launch_state(const Dev& d, bool at_n, unsigned fields, int64_t first, int m, double* out, cudaStream_t s) {
+  NodeFields f = node_fields(d, at_n);
+  for (int k = 0; k < 8; ++k)
+    if (!(fields >> k & 1)) f.p[k] = nullptr;
+  if (m) k_state<<<nblocks((int64_t)kNodeValues * m, 256), 256, 0, s>>>(f, d.n_nodes, first, m, out);
 }
 
 }  // namespace eb
