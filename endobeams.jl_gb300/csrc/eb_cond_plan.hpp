@@ -14,9 +14,10 @@
 // Cuthill-McKee order.  A 48-wire stent of 8,664 nodes keeps about 250 nodes,
 // and N b² (the band LU's work) falls by two orders of magnitude.
 //
-// When another level pays (cond_cost, in us of one application): a level costs 2 us (a barrier
-// of the team in each sweep, its launches in the factorisation) and its blocks' bytes; the
-// explicit inverse reads 4 N² bytes at about 1 TB/s and its 2 N³ operations at 20 TFLOP/s are
+// When another level pays (cond_cost, in us of one application): a level costs 5 us (about 2.5 in
+// each sweep: a barrier of the team and its instructions' latency) and its blocks' bytes (with 2 us
+// a 33 x 33 net took 2.10 ms a step, with 5 us 1.94, a 48 x 200 stent 11.4 and 10.8; from 6 us on a
+// stent that refactorises twice a step loses 4% to the larger inverse); the explicit inverse reads 4 N² bytes at about 1 TB/s and its 2 N³ operations at 20 TFLOP/s are
 // spread over some 30 applications; the band sweeps walk 2 N/32 blocks one after the other, a
 // step taking about 0.9 us + 3.5 ns per DOF of half bandwidth on one SM.
 #pragma once
@@ -129,6 +130,8 @@ struct CondPlan {
   std::vector<int> rptr;               // kept rows: blocks among the kept nodes
 };
 
+constexpr int kWholeDofs = 200;  // at most this many DOFs: nothing is eliminated
+
 // The cheaper of the two (past max_dense the explicit inverse is still what the next levels aim
 // at); w < 0: the inverse.
 inline double cond_cost(int nodes, int w, int max_dense) {
@@ -199,10 +202,12 @@ inline void cond_plan(const std::vector<std::vector<int>>& adj0, int max_w, int 
     left.erase(std::remove_if(left.begin(), left.end(), [&](int v) { return gone[v] != 0; }), left.end());
   };
 
-  // wire segments: degree <= 2, while a level removes at least 5% of the nodes.  Also where the
-  // inverse would be small: on a 64-node ring it costs as much as the levels (45 us an iteration
-  // either way), and the levels round less (15 iterations a step against 17)
-  while (left.size() > 1) {
+  // Very small systems go to the explicit inverse as they are (cantilever of 20 nodes, ten steps: 19.1
+  // ms with levels, 17.8 without; 31 nodes 18.2 and 17.1; 45 nodes 18.4 and 18.8; a 64-node ring's
+  // step 0.94 and 0.98).
+  const bool whole = 6 * n <= kWholeDofs && 6 * n <= max_dense;
+  // wire segments: degree <= 2, while a level removes at least 5% of the nodes
+  while (left.size() > 1 && !whole) {
     std::vector<int> set = pick(2);
     if (set.empty() || set.size() * 20 < left.size()) break;
     commit(set);
@@ -213,7 +218,7 @@ inline void cond_plan(const std::vector<std::vector<int>>& adj0, int max_w, int 
   std::vector<int> rpos;
   int w = needs_band((int)left.size()) ? band(adj, left, rpos) : -1;
   for (int cap : {4, 8, 12, 16, 24, 32}) {
-    while (left.size() > 1) {
+    while (left.size() > 1 && !whole) {
       std::vector<int> set = pick(cap);
       if (set.empty() || set.size() * 20 < left.size()) break;
       double blocks = 0;
@@ -231,7 +236,10 @@ inline void cond_plan(const std::vector<std::vector<int>>& adj0, int max_w, int 
         w2 = band(g, keep, rp);
         if (w2 > max_w && w <= max_w && 6 * m2 > max_dense) break;
       }
-      if (cond_cost(m2, w2, max_dense) + 2.0 + 144e-6 * blocks > cond_cost(m, w, max_dense)) break;
+      // past max_dense there is no inverse yet: go on towards it
+      if ((max_dense <= 0 || 6 * m <= max_dense) &&
+          cond_cost(m2, w2, max_dense) + 5.0 + 144e-6 * blocks > cond_cost(m, w, max_dense))
+        break;
       commit(set);
       w = w2;
     }
