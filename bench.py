@@ -64,12 +64,6 @@ F_ELEM_ALGORITHMIC = 12153.0 + 14362.0 + 164.0 + 8.0
 # Elements in contact also write their 2.4 KB of tangents; those writes are not counted.
 B_CONTACT_ELEM = 480.0 + 88.0 + 13.0 + 648.0
 
-# DRAM bytes k_gmres moves per algorithmic byte (band, inverses, tangent): 158.2 GB read + written
-# against 151.9 GB algorithmic over the 24 k_gmres launches of 2 steps of 16 stents (ncu
-# dram__bytes_read.sum + dram__bytes_write.sum); the full workload's launches are too large to
-# capture, so the line scales its algorithmic bytes per launch by this ratio.
-KRYLOV_TRAFFIC_RATIO = 158.2 / 151.9
-
 METRIC = "HHT steps/s & Newton iters/step, batched+learned vs plain"
 MODEL = os.path.join(ROOT, "endobeams.jl_gb300", "models", "warm_start_stents.npz")
 # Newton tolerances of the stents.  The configurations ask for 1e-8.  The normalised residual of
@@ -574,14 +568,14 @@ def output_leg(eb, wl, args):
 
 
 def gmres_bytes_per_iter(wl, idx):
-    """Algorithmic bytes one GMRES iteration reads per simulation (FP32 band L and U, the
-    32x32 diagonal-block inverses, the FP32 tangent and its block index), summed over idx."""
+    """Bytes one GMRES iteration cannot do without per simulation, summed over idx: the tangent as
+    FP32 pairs with its block index, and the condensation's five FP32 blocks per node (its inverse,
+    two couplings in each sweep).  The explicit inverse of the kept nodes (1 to 10 MB, known to the
+    library only) is left out."""
     tot = 0
     for i in idx:
-        n, ne, w, _, _ = wl.stats(i)
-        b = 6 * w + 5
-        N = 6 * n
-        tot += 4 * N * (2 * b + 1) + 2 * 4 * 32 * N + (n + 2 * ne) * (36 * 4 + 4)
+        n, ne, _, _, _ = wl.stats(i)
+        tot += (n + 2 * ne) * (36 * 8 + 4) + 5 * n * (36 * 4 + 4)
     return tot
 
 
@@ -670,13 +664,11 @@ def gpu_arm(args, rank, world):
         ach = bytes_total / (dev_ms["krylov"] * 1e-3) / 1e9
         hbm = peaks.get("hbm_gbs")
         per_launch = bytes_total / max(launches["krylov"], 1)
-        rooflines["krylov"] = {"kernel": "k_gmres (per-simulation restarted GMRES, band-LU preconditioned)",
+        rooflines["krylov"] = {"kernel": "k_gmres (per-simulation restarted GMRES, condensation and explicit inverse)",
                                "bound": "hbm", "achieved": ach, "peak": hbm,
                                "peak_source": "MEASURED_PEAKS.json hbm_gbs" if hbm else None, "unit": "GB/s",
                                "frac": (ach / hbm) if hbm else None,
-                               "traffic": KRYLOV_TRAFFIC_RATIO * per_launch,
-                               "traffic_note": "bytes per launch: the algorithmic bytes per launch x the DRAM/"
-                                               "algorithmic ratio ncu measured on 16 stents (1.04)",
+                               "traffic": None,
                                "algorithmic_bytes_per_launch": per_launch,
                                "avg_launch_ms": phase_ms["krylov"] / max(launches["krylov"], 1),
                                "time_basis": "union over the lanes of their Krylov intervals (lanes overlap: "

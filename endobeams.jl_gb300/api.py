@@ -354,10 +354,10 @@ class SimulationParams:
     max_refinements: int = 60
     threads_per_sim: int = 0
     timing: bool = False             # per-phase CUDA-event timing inside each step
-    preconditioner: str = "band"     # "band" (FP32 band LU, RCM order) | "block_jacobi"
-    refactor_its: int = 16           # reuse the band LU until a solve needs more GMRES iterations (0: always refactor)
+    preconditioner: str = "band"     # "band" (FP32 condensation + inverse or band LU) | "block_jacobi"
+    refactor_its: int = 16           # reuse the factors until a solve needs more GMRES iterations (0: always refactor)
     refactor_policy: str = "threshold"  # "threshold" (refactor_its only) | "cost" (excess iterations vs LU cost)
-    refactor_cost: float = 0.2       # "cost": GMRES iterations one band LU is worth per DOF of half bandwidth
+    refactor_cost: float = 0.2       # "cost": GMRES iterations a factorisation is worth per DOF of the kept system's half bandwidth
     band_lu: str = "fp32"            # "fp32" (CUDA cores) | "tensor" (trailing updates on the tensor cores)
     stage_band: int = 1              # 1: stream band blocks into shared memory with bulk async copies; 0: off;
                                      # 2: test of the bounded wait (the first block's wait runs out)

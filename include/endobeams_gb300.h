@@ -76,9 +76,9 @@ typedef struct {
   int32_t threads_per_sim;                /* CTA size of the per-simulation solver, 0 = auto */
   int32_t timing;                         /* 1: record per-phase CUDA-event times in eb_step */
   int32_t preconditioner;                 /* EB_PRECOND_* */
-  int32_t refactor_its;                   /* band LU is reused until a solve needs more GMRES
+  int32_t refactor_its;                   /* the preconditioner's factors are reused until a solve needs more GMRES
                                              iterations than this or Δt changes (0: refactorise every solve) */
-  int32_t stage_band;                     /* 1: the triangular solves stream band blocks into shared memory
+  int32_t stage_band;                     /* 1: a band LU's triangular solves stream band blocks into shared memory
                                              with bulk asynchronous copies (same arithmetic, same results);
                                              2: as 1, but the first block's wait expects 16 bytes that no copy
                                              delivers, so it runs out (tests EB_SIM_WAIT_TIMEOUT) */
@@ -127,7 +127,9 @@ typedef struct {
                             before trying the network again */
 
 /* GMRES preconditioner */
-#define EB_PRECOND_BAND 0          /* FP32 band LU in reverse Cuthill-McKee order (block-Jacobi where it does not fit) */
+#define EB_PRECOND_BAND 0          /* FP32 condensation of low-degree nodes, then the explicit inverse of the kept system
+                                      (up to 2,048 DOFs) or its band LU in reverse Cuthill-McKee order (block-Jacobi where
+                                      that does not fit) */
 #define EB_PRECOND_BLOCK_JACOBI 1  /* LU of each node's 6x6 diagonal block */
 
 /* Interpolation of a voxel SDF */
@@ -244,8 +246,9 @@ int eb_get_memory(eb_handle *h, int64_t *device_bytes, int32_t *band_sims);
 int eb_get_forces(eb_handle *h, int32_t sim, double *Tint, double *Tk, double *Tc);
 
 /* Launch-shape autotuner (no counterpart in the reference): times the element, contact and
- * assembly kernels on the current state at candidate block sizes (64/128/256 threads for the
- * element and contact kernels, 128/256/512 for the two assembly kernels) and keeps the fastest.
+ * assembly kernels on the current state at candidate shapes (64/128/256 for the element and
+ * contact kernels: ten elements per CTA below 256, thirty from there; 128/256/512 threads for the
+ * two assembly kernels) and keeps the fastest.
  * All candidates compute every value with the same operations in the same order, so results do
  * not depend on the choice.  Call between steps (after eb_commit / eb_rollback; EB_ERR_STATE
  * otherwise).  chosen (may be NULL) receives the four block sizes: element, contact, matrix
