@@ -3,12 +3,14 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
 #include <memory>
 #include <mutex>
+#include <new>
 #include <string>
 #include <thread>
 #include <vector>
@@ -892,23 +894,37 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
   h->dense_n.assign(n_sims, 0);
   const int bmax = (((227 * 1024) / 4 - 8) / kPanel - kPanel) / 2;  // shared-memory limit of k_band_lu
   std::vector<CondPlan> plan(n_sims);
-  // f(s) for every simulation on up to 16 host threads
+  // f(s) for every simulation on up to 16 host threads, fewer where no more can be started; false when
+  // memory ran out (an exception must leave neither a thread nor the C interface)
   auto each_sim = [&](auto f) {
     const int nthr = std::max(1, std::min<int>({16, (int)std::thread::hardware_concurrency(), (int)n_sims}));
+    std::atomic<int> next{0};
+    std::atomic<bool> failed{false};
+    auto work = [&] {
+      try {
+        for (int s = next++; s < n_sims; s = next++) f(s);
+      } catch (const std::bad_alloc&) {
+        failed = true;
+      }
+    };
     std::vector<std::thread> pool;
-    for (int k = 1; k < nthr; ++k)
-      pool.emplace_back([&, k] { for (int s = k; s < n_sims; s += nthr) f(s); });
-    for (int s = 0; s < n_sims; s += nthr) f(s);
+    try {
+      for (int k = 1; k < nthr; ++k) pool.emplace_back(work);
+    } catch (const std::exception&) {
+    }
+    work();
     for (auto& th : pool) th.join();
+    return !failed;
   };
-  each_sim([&](int s) {
+  if (!each_sim([&](int s) {
     const int64_t no = h->node_off[s], n = h->node_off[s + 1] - no;
     std::vector<std::vector<int>> la(n);
     for (int64_t i = 0; i < n; ++i)
       for (int g : adj[no + i])
         if (g != (int)(no + i)) la[i].push_back((int)(g - no));
     cond_plan(la, (bmax - 5) / 6, p->stage_band == 2 ? 0 : kDenseMax, plan[s]);
-  });
+  }))
+    return fail(EB_ERR_STATE, "out of host memory");
   for (int s = 0; s < n_sims; ++s) {
     const int b = 6 * plan[s].w + 5, nr = plan[s].n - plan[s].ne;
     // few kept nodes: explicit inverse (the staging test asks for the staged band sweeps)
@@ -1209,7 +1225,7 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
       std::vector<int> red(red_off[n_sims]), rpos(red_off[n_sims]);
       std::vector<int> elim(eo.back()), elim_node(eo.back()), tgt(to.back()), tptr(to.back() + 1), cl(co.back()), cw(co.back());
       tptr.back() = (int)co.back();
-      each_sim([&](int s) {
+      if (!each_sim([&](int s) {
         const CondPlan& P = plan[s];
         const int64_t no = h->node_off[s];
         for (int i = 0; i < P.n; ++i) node_at[no + P.pos[i]] = (int)(no + i);
@@ -1246,7 +1262,8 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
             cw[co[i] + u] = o + P.cw[l][u];
           }
         }
-      });
+      }))
+        return fail(EB_ERR_STATE, "out of host memory");
       int *p_scol, *p_ne, *p_lo, *p_lp, *p_src, *p_rn, *p_cn, *p_ld, *p_el, *p_en, *p_t, *p_tp, *p_cl, *p_cw, *p_red,
           *p_rpos, *p_nat;
       CondRange* p_range;
@@ -1270,7 +1287,7 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
       std::vector<int> pcol(NB);
       std::vector<int2> prow(NN);
       std::vector<uint8_t> pfix(NN, 0);
-      each_sim([&](int s) {
+      if (!each_sim([&](int s) {
         const int64_t no = h->node_off[s];
         for (int64_t b = h->blk_off[s]; b < h->blk_off[s + 1]; ++b) pcol[b] = plan[s].pos[col[b] - no];
         for (int q = 0; q < plan[s].n; ++q) {
@@ -1278,7 +1295,8 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
           prow[no + q] = make_int2(row_ptr[node], row_ptr[node + 1]);
           for (int k = 0; k < 6; ++k) pfix[no + q] |= (uint8_t)(fixed[6 * (int64_t)node + k] << k);
         }
-      });
+      }))
+        return fail(EB_ERR_STATE, "out of host memory");
       int* p_pc;
       int2* p_pr;
       uint8_t* p_pf;
