@@ -6,6 +6,7 @@
 #include <cstdio>
 #include <cstring>
 #include <random>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/endobeams_gb300.h"
@@ -18,30 +19,29 @@ namespace eb {
 namespace {
 
 constexpr int kThr = 256;      // threads per CTA
-constexpr int kLdX = 52;       // shared row stride of the input tile (floats)
-constexpr int kLdH = 132;      // shared row stride of hidden activations (floats)
-constexpr int kLdW1 = 52;      // shared row stride of W1 transposed (BF16 values)
-constexpr int kLdW2 = 132;     // shared row stride of W2, W2 and W3 transposed
-constexpr int kOutP = 8;       // padded output width
 constexpr int kWarps = kThr / 32;
+constexpr int kOutP = 8;       // padded output width
+constexpr int kRows = 32;      // rows of a tile: a gradient partial's unit, whatever the launch
+// Shared arrays of rows hold pairs of consecutive rows: entry k of pair p is the float2 at p ld + k.
+constexpr int kLdX = 52, kLdH = 132;   // ld of the inputs and of the hidden activations (float2)
+constexpr int kLdW2 = 132;             // row stride of W2 and of W3 transposed (BF16 values)
 
 static_assert(kMlpIn == 48 && kMlpHidden == 128 && kMlpOut == 6, "kernel tiling assumes 48-128-128-6");
 
-// A CTA's tile has RW rows per warp.  FP32 arithmetic on CUDA cores bounds a tile (63,700 FMAs per
-// row forward and backward: 14.6 us for 56 rows on one SM), so the products are packed two to an
-// instruction and every shared-memory operand feeds at least four of them.
-template <int RW>
+// A warp owns NP row pairs: 1 (16 rows a CTA), 2 (a tile) or 4 (two tiles).  FP32 arithmetic on CUDA
+// cores bounds a tile (63,700 FMAs per row forward and backward), so the products are packed two to
+// an instruction, both halves the same product of two rows, and every shared-memory operand feeds at
+// least four of them.
+template <int NP>
 struct Smem {
-  __nv_bfloat16 W1T[kMlpHidden * kLdW1];
-  __nv_bfloat16 W2T[kMlpHidden * kLdW2];
-  __nv_bfloat16 W2[kMlpHidden * kLdW2];  // as stored (backward only)
+  __nv_bfloat16 W1[kMlpIn * kMlpHidden];
+  __nv_bfloat16 W2[kMlpHidden * kLdW2];
   __nv_bfloat16 W3T[kOutP * kLdW2];
   float b1[kMlpHidden], b2[kMlpHidden], b3[kOutP];
-  float x[kWarps * RW * kLdX];
+  float2 x[kWarps * NP * kLdX];
   // hidden activations and the derivatives of silu there, later the gradients by z (in place)
-  float h1[kWarps * RW * kLdH], d1[kWarps * RW * kLdH], h2[kWarps * RW * kLdH], d2[kWarps * RW * kLdH];
-  float dy[kWarps * RW * kOutP];  // targets, then the gradient by y
-  float gb[kWarps * (2 * kMlpHidden + kOutP)];
+  float2 h1[kWarps * NP * kLdH], d1[kWarps * NP * kLdH], h2[kWarps * NP * kLdH], d2[kWarps * NP * kLdH];
+  float2 dy[kWarps * NP * kOutP];  // targets, then the gradient by y
   double red[kWarps];
 };
 
@@ -53,170 +53,210 @@ __device__ __forceinline__ void fma2(float2& d, float2 a, float2 b) {
       : "+l"(reinterpret_cast<unsigned long long&>(d))
       : "l"(reinterpret_cast<unsigned long long&>(a)), "l"(reinterpret_cast<unsigned long long&>(b)));
 }
+__device__ __forceinline__ float2 both(float v) { return make_float2(v, v); }
+__device__ __forceinline__ float2 both_lo(unsigned w) { return both(__uint_as_float(w << 16)); }
+__device__ __forceinline__ float2 both_hi(unsigned w) { return both(__uint_as_float(w & 0xffff0000u)); }
 
-__device__ __forceinline__ float2 unpack(unsigned w) {
-  return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+// Row pair q of this warp (NP of them); pairs 16 .. are the second tile's.
+template <int NP>
+__device__ __forceinline__ int pair_of(int q) {
+  const int warp = threadIdx.x >> 5;
+  return NP == 1 ? warp : 2 * warp + (q & 1) + kRows / 2 * (q >> 1);
 }
 
-// acc[a][c] = Σ_k in[row][k] W[col][k] for this warp's RW rows and columns lane + 32 c, even and
-// odd k in the two halves: both operands then are read along k, the inputs as one address per
-// warp, the weights without bank conflicts (row strides of 26 and 66 words).
-template <int K, int LDI, int LDW, int RW>
-__device__ __forceinline__ void tile_dot(const float* in, const __nv_bfloat16* W, float2 (&acc)[RW][4]) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-#pragma unroll
-  for (int a = 0; a < RW; ++a)
-#pragma unroll
-    for (int c = 0; c < 4; ++c) acc[a][c] = make_float2(0.f, 0.f);
-  const float* ip = in + warp * RW * LDI;
-  const __nv_bfloat16* wp = W + lane * LDW;
+// acc[q][c] += Σ_k in[row][k] W[k][4 lane + c] for the warp's first CNT row pairs, k in increasing
+// order in one chain per output.
+template <int NP, int CNT, int K, int LDI, int LDW>
+__device__ __forceinline__ void dot_rows(const float2* in, const __nv_bfloat16* W, float2 (&acc)[CNT][4]) {
+  const int lane = threadIdx.x & 31;
 #pragma unroll 2
-  for (int k = 0; k < K; k += 4) {
-    float4 v[RW];
+  for (int k = 0; k < K; k += 2) {
+    const uint2 w0 = *reinterpret_cast<const uint2*>(W + k * LDW + 4 * lane);
+    const uint2 w1 = *reinterpret_cast<const uint2*>(W + (k + 1) * LDW + 4 * lane);
+    const float2 a[4] = {both_lo(w0.x), both_hi(w0.x), both_lo(w0.y), both_hi(w0.y)};
+    const float2 b[4] = {both_lo(w1.x), both_hi(w1.x), both_lo(w1.y), both_hi(w1.y)};
 #pragma unroll
-    for (int a = 0; a < RW; ++a) v[a] = *reinterpret_cast<const float4*>(ip + a * LDI + k);
+    for (int q = 0; q < CNT; ++q) {
+      const float4 v = *reinterpret_cast<const float4*>(in + pair_of<NP>(q) * LDI + k);
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const uint2 w = *reinterpret_cast<const uint2*>(wp + 32 * c * LDW + k);
-      const float2 w0 = unpack(w.x), w1 = unpack(w.y);
+      for (int c = 0; c < 4; ++c) fma2(acc[q][c], make_float2(v.x, v.y), a[c]);
 #pragma unroll
-      for (int a = 0; a < RW; ++a) {
-        fma2(acc[a][c], make_float2(v[a].x, v[a].y), w0);
-        fma2(acc[a][c], make_float2(v[a].z, v[a].w), w1);
+      for (int c = 0; c < 4; ++c) fma2(acc[q][c], make_float2(v.z, v.w), b[c]);
+    }
+  }
+}
+
+// acc[q][c] += Σ_j in[row][j] W2[lane + 32 c][j], j in increasing order.
+template <int NP, int CNT>
+__device__ __forceinline__ void dot_cols(const float2* in, const __nv_bfloat16* W, float2 (&acc)[CNT][4]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll 1
+  for (int j = 0; j < kMlpHidden; j += 4) {
+    uint2 w[4];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) w[c] = *reinterpret_cast<const uint2*>(W + (lane + 32 * c) * kLdW2 + j);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float2 a[4], b[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const unsigned u = h ? w[c].y : w[c].x;
+        a[c] = both_lo(u);
+        b[c] = both_hi(u);
+      }
+#pragma unroll
+      for (int q = 0; q < CNT; ++q) {
+        const float4 v = *reinterpret_cast<const float4*>(in + pair_of<NP>(q) * kLdH + j + 2 * h);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) fma2(acc[q][c], make_float2(v.x, v.y), a[c]);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) fma2(acc[q][c], make_float2(v.z, v.w), b[c]);
       }
     }
   }
 }
 
-// h = silu(in W + b) of this warp's rows, and silu' (TRAIN).
-template <int K, int LDI, int LDW, int RW, bool TRAIN>
-__device__ __forceinline__ void dense_silu(const float* in, const __nv_bfloat16* W, const float* b, float* h, float* d) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float2 acc[RW][4];
-  tile_dot<K, LDI, LDW, RW>(in, W, acc);
+// h = silu(in W + b) of the warp's first CNT row pairs, and silu' (TRAIN).
+template <bool TRAIN, int NP, int CNT, int K, int LDI, int LDW>
+__device__ __forceinline__ void dense_silu(const float2* in, const __nv_bfloat16* W, const float* b, float2* h, float2* d) {
+  const int lane = threadIdx.x & 31;
+  float2 acc[CNT][4];
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    const float bc = b[lane + 32 * c];
+  for (int c = 0; c < 4; ++c)
 #pragma unroll
-    for (int a = 0; a < RW; ++a) {
-      const float z = (acc[a][c].x + acc[a][c].y) + bc, s = sigm(z);
-      const int at = (warp * RW + a) * kLdH + lane + 32 * c;
-      h[at] = z * s;
-      if (TRAIN) d[at] = s + z * s * (1.f - s);
+    for (int q = 0; q < CNT; ++q) acc[q][c] = both(b[4 * lane + c]);
+  dot_rows<NP, CNT, K, LDI, LDW>(in, W, acc);
+#pragma unroll
+  for (int q = 0; q < CNT; ++q) {
+    float hv[8], dv[8];
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const float z = r ? acc[q][c].y : acc[q][c].x, s = sigm(z);
+        hv[2 * c + r] = z * s;
+        if (TRAIN) dv[2 * c + r] = s + z * s * (1.f - s);
+      }
+    const int at = pair_of<NP>(q) * kLdH + 4 * lane;
+    float4* hp = reinterpret_cast<float4*>(h + at);
+    hp[0] = make_float4(hv[0], hv[1], hv[2], hv[3]);
+    hp[1] = make_float4(hv[4], hv[5], hv[6], hv[7]);
+    if (TRAIN) {
+      float4* dp = reinterpret_cast<float4*>(d + at);
+      dp[0] = make_float4(dv[0], dv[1], dv[2], dv[3]);
+      dp[1] = make_float4(dv[4], dv[5], dv[6], dv[7]);
     }
   }
 }
 
-// g += Σ_rows inᵀ dz over the tile: rows 4 tk .. +3 and K/2 + 4 tk .. +3 of the gradient (K = 48:
-// 3 tk .. +2), columns 4 tj .. +3 and 64 + 4 tj .. +3; 16-byte reads without bank conflicts.
-template <int K, int LDI, int ROWS, int NR>
-__device__ __forceinline__ void weight_grad(const float* in, const float* dz, float2 (&g)[NR][4]) {
+// g += Σ_rows inᵀ dz over `pairs` row pairs in row order: rows NR tk .. of the gradient, columns
+// 2 tj, 2 tj + 1 of each quarter of 32.
+template <int LDI, int NR>
+__device__ __forceinline__ void weight_grad(const float2* in, const float2* dz, int pairs, float2 (&g)[NR][4]) {
   const int tk = threadIdx.x >> 4, tj = threadIdx.x & 15;
-#pragma unroll 2
-  for (int i = 0; i < ROWS; ++i) {
-    float v[NR];
+#pragma unroll 1
+  for (int p = 0; p < pairs; ++p) {
+    float2 v[NR];
     if (NR == 8) {
-      const float4 p = *reinterpret_cast<const float4*>(in + i * LDI + 4 * tk);
-      const float4 q = *reinterpret_cast<const float4*>(in + i * LDI + K / 2 + 4 * tk);
-      v[0] = p.x; v[1] = p.y; v[2] = p.z; v[3 % NR] = p.w;
-      v[4 % NR] = q.x; v[5 % NR] = q.y; v[6 % NR] = q.z; v[7 % NR] = q.w;
+#pragma unroll
+      for (int a = 0; a < NR; a += 2) {
+        const float4 q = *reinterpret_cast<const float4*>(in + p * LDI + NR * tk + a);
+        v[a] = make_float2(q.x, q.y);
+        v[(a + 1) % NR] = make_float2(q.z, q.w);
+      }
     } else {
 #pragma unroll
-      for (int a = 0; a < NR; ++a) v[a] = in[i * LDI + NR * tk + a];
+      for (int a = 0; a < NR; ++a) v[a] = in[p * LDI + NR * tk + a];
     }
-    const float4 da = *reinterpret_cast<const float4*>(dz + i * kLdH + 4 * tj);
-    const float4 db = *reinterpret_cast<const float4*>(dz + i * kLdH + kMlpHidden / 2 + 4 * tj);
+    float2 d0[4], d1[4];
 #pragma unroll
-    for (int a = 0; a < NR; ++a) {
-      const float2 vv = make_float2(v[a], v[a]);
-      fma2(g[a][0], vv, make_float2(da.x, da.y));
-      fma2(g[a][1], vv, make_float2(da.z, da.w));
-      fma2(g[a][2], vv, make_float2(db.x, db.y));
-      fma2(g[a][3], vv, make_float2(db.z, db.w));
+    for (int c = 0; c < 4; ++c) {
+      const float4 q = *reinterpret_cast<const float4*>(dz + p * kLdH + 2 * tj + 32 * c);
+      d0[c] = make_float2(q.x, q.z);
+      d1[c] = make_float2(q.y, q.w);
     }
+#pragma unroll
+    for (int a = 0; a < NR; ++a)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) fma2(g[a][c], both(v[a].x), d0[c]);
+#pragma unroll
+    for (int a = 0; a < NR; ++a)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) fma2(g[a][c], both(v[a].y), d1[c]);
   }
 }
 
 __device__ __forceinline__ void put_grad(float* G, int row, const float2 (&g)[4]) {
   const int tj = threadIdx.x & 15;
-  float2* p = reinterpret_cast<float2*>(G + row * kMlpHidden + 4 * tj);
-  p[0] = g[0];
-  p[1] = g[1];
-  float2* q = reinterpret_cast<float2*>(G + row * kMlpHidden + kMlpHidden / 2 + 4 * tj);
-  q[0] = g[2];
-  q[1] = g[3];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) *reinterpret_cast<float2*>(G + row * kMlpHidden + 2 * tj + 32 * c) = g[c];
 }
 
-// One CTA processes tiles blockIdx.x, blockIdx.x + gridDim.x, ... of 8 RW rows; X is 16-byte
-// aligned.  TRAIN: targets T, gradient partials per CTA in gpart, loss partial in lpart.  A batch
-// of 8192 rows on 147 SMs: 84 us with a 4 x 4 tile per thread, scalar operands and two rounds of
-// 32 rows, 40 us now (10 of them weights in and gradients out).
-template <bool TRAIN, int RW>
+// One CTA processes tiles blockIdx.x, blockIdx.x + gridDim.x, ... (two at a time where NP = 4) of 32
+// rows, 16 where NP = 1; X is 16-byte aligned.  TRAIN: targets T, gradient partials per CTA in gpart,
+// loss partial in lpart.  Every sum has one order: over k in increasing order from the bias, over
+// rows tile by tile, over CTAs in order (k_mlp_reduce), so outputs and gradients depend neither on
+// NP nor on how the products are packed.  A batch of 8192 rows: 84 us with a 4 x 4 tile per thread and
+// scalar operands, 40 us with sums split over even and odd k and 56-row tiles (another order: a loss
+// after one epoch moved by 8e-8), 42 us now.
+template <bool TRAIN, int NP>
 __global__ void __launch_bounds__(kThr, 1)
     k_mlp(MlpDev m, const float* __restrict__ X, const int* __restrict__ rows, int64_t n,
           const float* __restrict__ T, float* __restrict__ Y, float* __restrict__ gpart, double* __restrict__ lpart,
           float gscale) {
-  constexpr int kTile = kWarps * RW;
+  constexpr int kTile = NP == 1 ? 16 : kRows, kParts = NP == 4 ? 2 : 1, kPairs = kWarps * NP;
   extern __shared__ __align__(16) unsigned char smraw[];
-  Smem<RW>& S = *reinterpret_cast<Smem<RW>*>(smraw);
+  Smem<NP>& S = *reinterpret_cast<Smem<NP>*>(smraw);
   const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
   const int64_t ntiles = (n + kTile - 1) / kTile;
-  // ---- a tile's input rows and targets, first into registers so that they arrive while other
+  // ---- a round's input rows and targets, first into registers so that they arrive while other
   // work goes on; a row past the end is zero and carries no sample
-  constexpr int kVecs = kTile * (kMlpIn / 4), kNx = (kVecs + kThr - 1) / kThr;
-  constexpr int kOuts = kTile * kOutP, kNt = (kOuts + kThr - 1) / kThr;
-  float4 xin[kNx];
-  float tin[kNt];
+  constexpr int kVecs = kPairs * (kMlpIn / 4), kNx = (kVecs + kThr - 1) / kThr;
+  static_assert(kPairs * kOutP <= kThr, "one target pair per thread");
+  float4 xin[kNx][2];
+  float2 tin;
+  auto row0 = [&](int64_t tile, int pair) { return (tile + pair / (kTile / 2) * (int64_t)gridDim.x) * kTile + 2 * (pair % (kTile / 2)); };
   auto load_tile = [&](int64_t tile) {
-    const int64_t r0 = tile * kTile;
 #pragma unroll
     for (int q = 0; q < kNx; ++q) {
-      const int e = t + q * kThr, i = e / (kMlpIn / 4), k = e % (kMlpIn / 4);
-      const int64_t r = r0 + i;
-      xin[q] = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (e < kVecs && r < n) xin[q] = reinterpret_cast<const float4*>(X + (rows ? (int64_t)rows[r] : r) * kMlpIn)[k];
-    }
-    if (TRAIN)
+      const int e = t + q * kThr, p = e / (kMlpIn / 4), k = e % (kMlpIn / 4);
 #pragma unroll
-      for (int q = 0; q < kNt; ++q) {
-        const int e = t + q * kThr, o = e % kOutP;
-        const int64_t r = r0 + e / kOutP;
-        tin[q] = e < kOuts && r < n && o < kMlpOut ? T[(rows ? (int64_t)rows[r] : r) * kMlpOut + o] : nanf("");
+      for (int u = 0; u < 2; ++u) {
+        const int64_t r = row0(tile, p) + u;
+        xin[q][u] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (e < kVecs && r < n) xin[q][u] = reinterpret_cast<const float4*>(X + (rows ? (int64_t)rows[r] : r) * kMlpIn)[k];
       }
+    }
+    if (TRAIN) {
+      const int p = t / kOutP, o = t % kOutP;
+      const bool on = t < kPairs * kOutP && o < kMlpOut;
+      const int64_t r = row0(tile, p);
+      tin = both(nanf(""));
+      if (on && r < n) tin.x = T[(rows ? (int64_t)rows[r] : r) * kMlpOut + o];
+      if (on && r + 1 < n) tin.y = T[(rows ? (int64_t)rows[r + 1] : r + 1) * kMlpOut + o];
+    }
   };
   auto store_tile = [&]() {
 #pragma unroll
     for (int q = 0; q < kNx; ++q) {
       const int e = t + q * kThr;
-      if (e < kVecs) *reinterpret_cast<float4*>(S.x + e / (kMlpIn / 4) * kLdX + 4 * (e % (kMlpIn / 4))) = xin[q];
+      if (e >= kVecs) continue;
+      const float4 a = xin[q][0], b = xin[q][1];
+      float4* dst = reinterpret_cast<float4*>(S.x + e / (kMlpIn / 4) * kLdX + 4 * (e % (kMlpIn / 4)));
+      dst[0] = make_float4(a.x, b.x, a.y, b.y);
+      dst[1] = make_float4(a.z, b.z, a.w, b.w);
     }
-    if (TRAIN)
-#pragma unroll
-      for (int q = 0; q < kNt; ++q)
-        if (t + q * kThr < kOuts) S.dy[t + q * kThr] = tin[q];
+    if (TRAIN && t < kPairs * kOutP) S.dy[t] = tin;
   };
-  // ---- weights: a thread takes eight columns of two rows k, k + 1 and stores the pairs along k
-  // (lanes along k: no bank conflicts); all loads are in flight before the first store waits
-  constexpr int kIt1 = (kMlpIn / 2 * 16 + kThr - 1) / kThr, kIt2 = kMlpHidden / 2 * 16 / kThr;
-  uint4 w1[kIt1][2], w2[kIt2][2];
+  // ---- weights: all loads are in flight before the first store waits
+  constexpr int kIt1 = kMlpIn * kMlpHidden / 8 / kThr, kIt2 = kMlpHidden * kMlpHidden / 8 / kThr;
+  static_assert(kIt1 * kThr * 8 == kMlpIn * kMlpHidden, "whole rounds");
+  uint4 w1[kIt1], w2[kIt2];
   load_tile(blockIdx.x);
-  auto load2 = [&](const __nv_bfloat16* W, int pairs, int e, uint4 (&v)[2]) {
-    const uint4* src = reinterpret_cast<const uint4*>(W + (2 * (e % pairs)) * kMlpHidden + 8 * (e / pairs));
-    v[0] = src[0];
-    v[1] = src[kMlpHidden / 8];
-  };
-  auto store2 = [&](const uint4 (&v)[2], int pairs, int e, __nv_bfloat16* WT, int ld) {
-    const unsigned a[4] = {v[0].x, v[0].y, v[0].z, v[0].w}, b[4] = {v[1].x, v[1].y, v[1].z, v[1].w};
-    unsigned* dst = reinterpret_cast<unsigned*>(WT + 8 * (e / pairs) * ld) + e % pairs;
 #pragma unroll
-    for (int c = 0; c < 8; ++c)
-      dst[c * ld / 2] = __byte_perm(a[c / 2], b[c / 2], c % 2 ? 0x7632 : 0x5410);
-  };
+  for (int q = 0; q < kIt1; ++q) w1[q] = reinterpret_cast<const uint4*>(m.W + kOffW1)[t + q * kThr];
 #pragma unroll
-  for (int q = 0; q < kIt1; ++q)
-    if (t + q * kThr < kMlpIn / 2 * 16) load2(m.W + kOffW1, kMlpIn / 2, t + q * kThr, w1[q]);
-#pragma unroll
-  for (int q = 0; q < kIt2; ++q) load2(m.W + kOffW2, kMlpHidden / 2, t + q * kThr, w2[q]);
+  for (int q = 0; q < kIt2; ++q) w2[q] = reinterpret_cast<const uint4*>(m.W + kOffW2)[t + q * kThr];
   for (int i = t; i < kMlpHidden * kOutP; i += kThr) {
     const int k = i / kOutP, o = i % kOutP;
     S.W3T[o * kLdW2 + k] = o < kMlpOut ? m.W[kOffW3 + k * kMlpOut + o] : __float2bfloat16_rn(0.f);
@@ -227,24 +267,18 @@ __global__ void __launch_bounds__(kThr, 1)
   }
   if (t < kOutP) S.b3[t] = t < kMlpOut ? m.P[kOffB3 + t] : 0.f;
 #pragma unroll
-  for (int q = 0; q < kIt1; ++q)
-    if (t + q * kThr < kMlpIn / 2 * 16) store2(w1[q], kMlpIn / 2, t + q * kThr, S.W1T, kLdW1);
+  for (int q = 0; q < kIt1; ++q) reinterpret_cast<uint4*>(S.W1)[t + q * kThr] = w1[q];
 #pragma unroll
   for (int q = 0; q < kIt2; ++q) {
-    const int e = t + q * kThr, k = 2 * (e % (kMlpHidden / 2)), j = 8 * (e / (kMlpHidden / 2));
-    store2(w2[q], kMlpHidden / 2, e, S.W2T, kLdW2);
-    if (TRAIN)
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        uint2* dst = reinterpret_cast<uint2*>(S.W2 + (k + h) * kLdW2 + j);  // rows are 8-byte aligned
-        dst[0] = make_uint2(w2[q][h].x, w2[q][h].y);
-        dst[1] = make_uint2(w2[q][h].z, w2[q][h].w);
-      }
+    const int e = t + q * kThr;
+    uint2* dst = reinterpret_cast<uint2*>(S.W2 + e / (kMlpHidden / 8) * kLdW2 + 8 * (e % (kMlpHidden / 8)));
+    dst[0] = make_uint2(w2[q].x, w2[q].y);  // rows are 8-byte aligned
+    dst[1] = make_uint2(w2[q].z, w2[q].w);
   }
 
-  // gradient accumulators (TRAIN): weights as in weight_grad, biases of this warp's rows
+  // gradient accumulators (TRAIN): weights as in weight_grad, biases: thread t < 128 of b2, t >= 128 of b1
   float2 g2[8][4], g1[3][4];
-  float g3[4], gb1[4], gb2[4], gb3 = 0.f;
+  float g3[4], gb = 0.f, gb3 = 0.f;
   double loss = 0.0;
   if (TRAIN) {
 #pragma unroll
@@ -253,142 +287,133 @@ __global__ void __launch_bounds__(kThr, 1)
       for (int a = 0; a < 8; ++a) g2[a][c] = make_float2(0.f, 0.f);
 #pragma unroll
       for (int a = 0; a < 3; ++a) g1[a][c] = make_float2(0.f, 0.f);
-      g3[c] = gb1[c] = gb2[c] = 0.f;
+      g3[c] = 0.f;
     }
   }
 
-  for (int64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-    const int64_t r0 = tile * kTile;
-    store_tile();
-    __syncthreads();
-    if (tile + gridDim.x < ntiles) load_tile(tile + gridDim.x);
-    // a warp reads only its own rows up to y
-    dense_silu<kMlpIn, kLdX, kLdW1, RW, TRAIN>(S.x, S.W1T, S.b1, S.h1, S.d1);
+  // a warp's row pairs through the network and back: a warp reads only its own rows
+  auto through = [&](auto count, int64_t tile) {
+    constexpr int CNT = decltype(count)::value;
+    dense_silu<TRAIN, NP, CNT, kMlpIn, kLdX, kMlpHidden>(S.x, S.W1, S.b1, S.h1, S.d1);
     __syncwarp();
-    dense_silu<kMlpHidden, kLdH, kLdW2, RW, TRAIN>(S.h1, S.W2T, S.b2, S.h2, S.d2);
+    dense_silu<TRAIN, NP, CNT, kMlpHidden, kLdH, kLdW2>(S.h1, S.W2, S.b2, S.h2, S.d2);
     __syncwarp();
-    // ---- output layer: lane (o, q) sums the k of quarter q, interleaved by four
-    {
-      const int o = lane & 7, q = lane >> 3;
-      float2 acc[RW];
-#pragma unroll
-      for (int a = 0; a < RW; ++a) acc[a] = make_float2(0.f, 0.f);
-#pragma unroll 2
-      for (int k = 4 * q; k < kMlpHidden; k += 16) {
+    // ---- output layer: lane (pair, output)
+    const int q = lane >> 3, o = lane & 7;
+    if (q < CNT) {
+      const int p = pair_of<NP>(q);
+      float2 acc = both(S.b3[o]);
+#pragma unroll 4
+      for (int k = 0; k < kMlpHidden; k += 4) {
         const uint2 w = *reinterpret_cast<const uint2*>(S.W3T + o * kLdW2 + k);
-        const float2 w0 = unpack(w.x), w1 = unpack(w.y);
-#pragma unroll
-        for (int a = 0; a < RW; ++a) {
-          const float4 v = *reinterpret_cast<const float4*>(S.h2 + (warp * RW + a) * kLdH + k);
-          fma2(acc[a], make_float2(v.x, v.y), w0);
-          fma2(acc[a], make_float2(v.z, v.w), w1);
-        }
+        const float4 u = *reinterpret_cast<const float4*>(S.h2 + p * kLdH + k);
+        const float4 v = *reinterpret_cast<const float4*>(S.h2 + p * kLdH + k + 2);
+        fma2(acc, make_float2(u.x, u.y), both_lo(w.x));
+        fma2(acc, make_float2(u.z, u.w), both_hi(w.x));
+        fma2(acc, make_float2(v.x, v.y), both_lo(w.y));
+        fma2(acc, make_float2(v.z, v.w), both_hi(w.y));
       }
-#pragma unroll
-      for (int a = 0; a < RW; ++a) {
-        float y = acc[a].x + acc[a].y;
-        y += __shfl_xor_sync(0xffffffffu, y, 8);
-        y += __shfl_xor_sync(0xffffffffu, y, 16);
-        y += S.b3[o];
-        const int i = warp * RW + a;
-        const int64_t r = r0 + i;
-        if (q != 0) continue;
-        if (!TRAIN) {
-          if (r < n && o < kMlpOut) Y[r * kMlpOut + o] = y;
-        } else {
-          const float tv = S.dy[i * kOutP + o];
-          const float d = tv == tv ? y - tv : 0.f;  // NaN target: row carries no sample
-          loss += (double)d * (double)d;
-          gb3 += d * gscale;
-          S.dy[i * kOutP + o] = d * gscale;
-        }
+      if (!TRAIN) {
+        const int64_t r = row0(tile, p);
+        if (o < kMlpOut && r < n) Y[r * kMlpOut + o] = acc.x;
+        if (o < kMlpOut && r + 1 < n) Y[(r + 1) * kMlpOut + o] = acc.y;
+      } else {
+        const float2 tv = S.dy[p * kOutP + o];
+        // NaN target: row carries no sample
+        const float da = tv.x == tv.x ? acc.x - tv.x : 0.f, db = tv.y == tv.y ? acc.y - tv.y : 0.f;
+        loss += (double)da * (double)da;
+        loss += (double)db * (double)db;
+        S.dy[p * kOutP + o] = make_float2(da * gscale, db * gscale);
       }
     }
+    if (!TRAIN) return;
+    __syncwarp();
+    // ---- dz2 = (dy W3ᵀ) ⊙ silu'(z2), in place in d2
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      float w[kMlpOut];
+#pragma unroll
+      for (int k = 0; k < kMlpOut; ++k) w[k] = __bfloat162float(S.W3T[k * kLdW2 + lane + 32 * c]);
+#pragma unroll
+      for (int a = 0; a < CNT; ++a) {
+        const int p = pair_of<NP>(a);
+        float2 s = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int k = 0; k < kMlpOut; ++k) fma2(s, S.dy[p * kOutP + k], both(w[k]));
+        const float2 d = S.d2[p * kLdH + lane + 32 * c];
+        S.d2[p * kLdH + lane + 32 * c] = make_float2(s.x * d.x, s.y * d.y);
+      }
+    }
+    __syncwarp();
+    // ---- dz1 = (dz2 W2ᵀ) ⊙ silu'(z1), in place in d1
+    float2 acc[CNT][4];
+#pragma unroll
+    for (int a = 0; a < CNT; ++a)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) acc[a][c] = make_float2(0.f, 0.f);
+    dot_cols<NP, CNT>(S.d2, S.W2, acc);
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+#pragma unroll
+      for (int a = 0; a < CNT; ++a) {
+        float2& d = S.d1[pair_of<NP>(a) * kLdH + lane + 32 * c];
+        d = make_float2(acc[a][c].x * d.x, acc[a][c].y * d.y);
+      }
+  };
+
+  for (int64_t tile = blockIdx.x; tile < ntiles; tile += kParts * (int64_t)gridDim.x) {
+    store_tile();
+    __syncthreads();
+    if (tile + kParts * (int64_t)gridDim.x < ntiles) load_tile(tile + kParts * (int64_t)gridDim.x);
+    const bool all = kParts == 1 || tile + gridDim.x < ntiles;  // else the second tile does not exist
+    if (all) through(std::integral_constant<int, NP>{}, tile);
+    else through(std::integral_constant<int, NP == 4 ? 2 : NP>{}, tile);
     if (TRAIN) {
-      __syncwarp();
-      // ---- dz2 = (dy W3ᵀ) ⊙ silu'(z2) of this warp's rows, in place in d2
-#pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        float w[kMlpOut];
-#pragma unroll
-        for (int o = 0; o < kMlpOut; ++o) w[o] = __bfloat162float(S.W3T[o * kLdW2 + lane + 32 * c]);
-#pragma unroll
-        for (int a = 0; a < RW; ++a) {
-          const int i = warp * RW + a;
-          float s = 0.f;
-#pragma unroll
-          for (int o = 0; o < kMlpOut; ++o) s = fmaf(S.dy[i * kOutP + o], w[o], s);
-          s *= S.d2[i * kLdH + lane + 32 * c];
-          S.d2[i * kLdH + lane + 32 * c] = s;
-          gb2[c] += s;
-        }
-      }
-      __syncwarp();
-      // ---- dz1 = (dz2 W2ᵀ) ⊙ silu'(z1) of this warp's rows, in place in d1
-      {
-        float2 acc[RW][4];
-        tile_dot<kMlpHidden, kLdH, kLdW2, RW>(S.d2, S.W2, acc);
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-#pragma unroll
-          for (int a = 0; a < RW; ++a) {
-            const int at = (warp * RW + a) * kLdH + lane + 32 * c;
-            const float s = (acc[a][c].x + acc[a][c].y) * S.d1[at];
-            S.d1[at] = s;
-            gb1[c] += s;
-          }
-      }
       __syncthreads();
-      // ---- weight gradients over all rows of the tile
-      weight_grad<kMlpHidden, kLdH, kTile, 8>(S.h1, S.d2, g2);
-      weight_grad<kMlpIn, kLdX, kTile, 3>(S.x, S.d1, g1);
-      {
-        const int k = t >> 1, o0 = (t & 1) * 4;
+      // ---- weight gradients over all rows of the round
+      const int pairs = all ? kPairs : kRows / 2;
+      weight_grad<kLdH, 8>(S.h1, S.d2, pairs, g2);
+      weight_grad<kLdX, 3>(S.x, S.d1, pairs, g1);
+      const int k = t >> 1, o0 = (t & 1) * 4;
+      const float2* db = (t < kMlpHidden ? S.d2 : S.d1) + (t & (kMlpHidden - 1));
 #pragma unroll 4
-        for (int i = 0; i < kTile; ++i) {
-          const float hv = S.h2[i * kLdH + k];
-          const float4 dv = *reinterpret_cast<const float4*>(S.dy + i * kOutP + o0);
-          g3[0] = fmaf(hv, dv.x, g3[0]);
-          g3[1] = fmaf(hv, dv.y, g3[1]);
-          g3[2] = fmaf(hv, dv.z, g3[2]);
-          g3[3] = fmaf(hv, dv.w, g3[3]);
-        }
+      for (int p = 0; p < pairs; ++p) {
+        const float2 hv = S.h2[p * kLdH + k], bv = db[p * kLdH];
+        const float4 u = *reinterpret_cast<const float4*>(S.dy + p * kOutP + o0);
+        const float4 v = *reinterpret_cast<const float4*>(S.dy + p * kOutP + o0 + 2);
+        g3[0] = fmaf(hv.x, u.x, g3[0]); g3[1] = fmaf(hv.x, u.z, g3[1]);
+        g3[2] = fmaf(hv.x, v.x, g3[2]); g3[3] = fmaf(hv.x, v.z, g3[3]);
+        g3[0] = fmaf(hv.y, u.y, g3[0]); g3[1] = fmaf(hv.y, u.w, g3[1]);
+        g3[2] = fmaf(hv.y, v.y, g3[2]); g3[3] = fmaf(hv.y, v.w, g3[3]);
+        gb += bv.x;
+        gb += bv.y;
       }
+      if (t < kOutP)
+        for (int p = 0; p < pairs; ++p) {
+          const float2 v = S.dy[p * kOutP + t];
+          gb3 += v.x;
+          gb3 += v.y;
+        }
     }
     __syncthreads();
   }
 
   if (TRAIN) {
     float* G = gpart + (int64_t)blockIdx.x * kMlpParams;  // kMlpParams and every offset are even
-    {
-      const int tk = t >> 4;
+    const int tk = t >> 4;
 #pragma unroll
-      for (int a = 0; a < 8; ++a) put_grad(G + kOffW2, (a < 4 ? 0 : kMlpHidden / 2) + 4 * tk + (a & 3), g2[a]);
+    for (int a = 0; a < 8; ++a) put_grad(G + kOffW2, 8 * tk + a, g2[a]);
 #pragma unroll
-      for (int a = 0; a < 3; ++a) put_grad(G + kOffW1, 3 * tk + a, g1[a]);
-    }
-    {
-      const int k = t >> 1, o0 = (t & 1) * 4;
+    for (int a = 0; a < 3; ++a) put_grad(G + kOffW1, 3 * tk + a, g1[a]);
+    const int k = t >> 1, o0 = (t & 1) * 4;
 #pragma unroll
-      for (int c = 0; c < 4; ++c)
-        if (o0 + c < kMlpOut) G[kOffW3 + k * kMlpOut + o0 + c] = g3[c];
-    }
-    // biases and loss: the warps' sums in warp order
-    float* gb = S.gb + warp * (2 * kMlpHidden + kOutP);
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      gb[lane + 32 * c] = gb1[c];
-      gb[kMlpHidden + lane + 32 * c] = gb2[c];
-    }
-    if (lane < kOutP) gb[2 * kMlpHidden + lane] = gb3;
+    for (int c = 0; c < 4; ++c)
+      if (o0 + c < kMlpOut) G[kOffW3 + k * kMlpOut + o0 + c] = g3[c];
+    G[t < kMlpHidden ? kOffB2 + t : kOffB1 + t - kMlpHidden] = gb;
+    if (t < kMlpOut) G[kOffB3 + t] = gb3;
     for (int off = 16; off > 0; off >>= 1) loss += __shfl_down_sync(0xffffffffu, loss, off);
     if (lane == 0) S.red[warp] = loss;
     __syncthreads();
-    for (int e = t; e < 2 * kMlpHidden + kMlpOut; e += kThr) {
-      float sum = 0.f;
-      for (int w = 0; w < kWarps; ++w) sum += S.gb[w * (2 * kMlpHidden + kOutP) + e];
-      G[e < kMlpHidden ? kOffB1 + e : e < 2 * kMlpHidden ? kOffB2 + e - kMlpHidden : kOffB3 + e - 2 * kMlpHidden] = sum;
-    }
     if (t == 0) {
       double sum = 0.0;
       for (int w = 0; w < kWarps; ++w) sum += S.red[w];
@@ -397,18 +422,18 @@ __global__ void __launch_bounds__(kThr, 1)
   }
 }
 
-// g[p] = Σ_c gpart[c][p]; loss = Σ_c lpart[c] · lscale.  A CTA owns 32 parameters: warp w sums the
-// partials w, w + 8, ... and the eight sums are added in warp order.  With ADAM the parameter is
-// updated at once, and its BF16 copy.  147 partials are 13.9 MB, read from L2: 17 us with a thread
-// per parameter plus 3.6 us for Adam's own launch, 7.4 us now.
-constexpr int kRedParams = 32, kRedWarps = 8;
+// g[p] = Σ_c gpart[c][p] in CTA order; loss = Σ_c lpart[c] · lscale.  A CTA owns 32 parameters: its
+// warps bring the partials into shared memory, one warp adds them.  With ADAM the parameter is
+// updated at once, and its BF16 copy.  152 partials are 14.3 MB, read from L2: 17 us with a thread
+// per parameter plus 3.6 us for Adam's own launch, 12 us now.
+constexpr int kRedParams = 32, kRedWarps = 8, kRedChunk = 160;
 constexpr int kRedCtas = (kMlpParams + kRedParams - 1) / kRedParams;
 
 template <bool ADAM>
 __global__ void __launch_bounds__(kRedParams * kRedWarps)
     k_mlp_reduce(const float* __restrict__ gpart, int grid, MlpTrainer t, const double* __restrict__ lpart,
                  double* __restrict__ loss, double lscale, float lr, float c1, float c2) {
-  __shared__ float part[kRedWarps][kRedParams];
+  __shared__ float part[kRedChunk][kRedParams];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   if (blockIdx.x == kRedCtas) {
     if (warp == 0 && loss) {
@@ -420,17 +445,19 @@ __global__ void __launch_bounds__(kRedParams * kRedWarps)
     return;
   }
   const int p = blockIdx.x * kRedParams + lane;
-  float s = 0.f;
-  if (p < kMlpParams) {
+  float gp = 0.f;
+  for (int c0 = 0; c0 < grid; c0 += kRedChunk) {
+    const int cnt = min(kRedChunk, grid - c0);
+    if (p < kMlpParams)
+#pragma unroll 20
+      for (int c = warp; c < cnt; c += kRedWarps) part[c][lane] = gpart[(int64_t)(c0 + c) * kMlpParams + p];
+    __syncthreads();
+    if (warp == 0)
 #pragma unroll 8
-    for (int c = warp; c < grid; c += kRedWarps) s += gpart[(int64_t)c * kMlpParams + p];
+      for (int c = 0; c < cnt; ++c) gp += part[c][lane];
+    __syncthreads();
   }
-  part[warp][lane] = s;
-  __syncthreads();
   if (warp != 0 || p >= kMlpParams) return;
-  float gp = part[0][lane];
-#pragma unroll
-  for (int w = 1; w < kRedWarps; ++w) gp += part[w][lane];
   if (!ADAM) {
     t.G[p] = gp;
     return;
@@ -450,31 +477,31 @@ __global__ void k_mlp_bf16(const float* __restrict__ P, __nv_bfloat16* __restric
   if (p < kMlpParams) W[p] = __float2bfloat16_rn(P[p]);
 }
 
-template <bool TRAIN, int RW>
+template <bool TRAIN, int NP>
 cudaError_t launch_mlp(int sms, const MlpDev& m, const float* X, const int* rows, int64_t n, const float* T, float* Y,
                        float* gpart, double* lpart, float gscale, int* grid_out, cudaStream_t s) {
-  const void* k = (const void*)k_mlp<TRAIN, RW>;
-  cudaError_t e = raise_smem_limit(k, sizeof(Smem<RW>));
+  constexpr int kTile = NP == 1 ? 16 : kRows;
+  const void* k = (const void*)k_mlp<TRAIN, NP>;
+  cudaError_t e = raise_smem_limit(k, sizeof(Smem<NP>));
   if (e != cudaSuccess) return e;
-  const int grid = (int)std::min<int64_t>((n + kWarps * RW - 1) / (kWarps * RW), sms);
-  k_mlp<TRAIN, RW><<<grid, kThr, sizeof(Smem<RW>), s>>>(m, X, rows, n, T, Y, gpart, lpart, gscale);
+  const int grid = (int)std::min<int64_t>((n + kTile - 1) / kTile, sms);
+  k_mlp<TRAIN, NP><<<grid, kThr, sizeof(Smem<NP>), s>>>(m, X, rows, n, T, Y, gpart, lpart, gscale);
   *grid_out = grid;
   return cudaGetLastError();
 }
 
-// Rows per tile: the smallest of 16, 32 and 56 for which every tile has an SM to itself (forward
-// and gradient: 11 and 20 us at 16 rows, 14 and 27 at 32; 27 and 54 with the 32-row tile of four by
-// four per thread), else 56, whose weights and gradients are loaded and stored least often.  A
-// row's outputs do not depend on the choice.
+// Rows per round of a CTA: one tile where every tile has an SM to itself, else two tiles, whose weights
+// are read half as often; without gradients also half a tile, where as many have an SM each
+// (2000 rows forward: 10.4 us in sixteens, 13.2 in tiles).  A gradient partial is whole tiles, so that its sums keep one order.
 template <bool TRAIN>
 cudaError_t run_mlp(const MlpDev& m, const float* X, const int* rows, int64_t n, const float* T, float* Y, float* gpart,
                     double* lpart, float gscale, int* grid, cudaStream_t s) {
   int dev = 0, sms = 152;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  auto go = n <= (int64_t)sms * kWarps * 2   ? launch_mlp<TRAIN, 2>
-            : n <= (int64_t)sms * kWarps * 4 ? launch_mlp<TRAIN, 4>
-                                             : launch_mlp<TRAIN, 7>;
+  auto go = n > (int64_t)sms * kRows            ? launch_mlp<TRAIN, 4>
+            : TRAIN || n > (int64_t)sms * 16    ? launch_mlp<TRAIN, 2>
+                                                : launch_mlp<TRAIN, TRAIN ? 2 : 1>;
   return go(sms, m, X, rows, n, T, Y, gpart, lpart, gscale, grid, s);
 }
 
