@@ -88,6 +88,7 @@ SIGNATURES = {
     "eb_set_tolerances": (C.c_int, [C.c_void_p, P_d, P_d]),
     "eb_get_stats": (C.c_int, [C.c_void_p, C.POINTER(EbSimStats)]),
     "eb_get_memory": (C.c_int, [C.c_void_p, P_i64, P_i32]),
+    "eb_get_solver": (C.c_int, [C.c_void_p, C.c_int32, P_i32]),
     "eb_get_forces": (C.c_int, [C.c_void_p, C.c_int32, P_d, P_d, P_d]),
     "eb_element_eval": (C.c_int, [C.c_int64, P_d, P_d, P_d]),
     "eb_contact_eval": (C.c_int, [C.c_int64, P_d, P_d, P_d, P_d, P_d, P_d, P_i32]),

@@ -683,6 +683,15 @@ class GpuSimulations:
         check(self.L.eb_get_memory(self.h, C.byref(b), C.byref(n)), "eb_get_memory")
         return int(b.value), int(n.value)
 
+    def solver(self, sim: int):
+        """How simulation ``sim`` is preconditioned: kept DOFs, half bandwidth of their band LU and DOFs of
+        their explicit inverse (0: none), whether the band is staged and factorised on the tensor cores,
+        whether the solves are two launches."""
+        i = np.zeros(4, np.int32)
+        check(self.L.eb_get_solver(self.h, int(sim), ptr(i, C.c_int32)), "eb_get_solver")
+        return dict(kept=int(i[0]), band=int(i[1]), inverse=int(i[2]), staged=bool(i[3] & 1), tensor_lu=bool(i[3] & 2),
+                    two_classes=bool(i[3] & 4))
+
     def stats(self):
         check(self.L.eb_get_stats(self.h, self._stats), "eb_get_stats")
         return [{f: getattr(x, f) for f, _ in _lib.EbSimStats._fields_} for x in self._stats]

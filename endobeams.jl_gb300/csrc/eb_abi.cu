@@ -363,6 +363,8 @@ struct eb_handle {
   std::vector<int64_t> cond_elim_off, cond_tgt_off;  // per level (all simulations): offsets of its lists
   std::vector<int> band_b;  // per sim half bandwidth of the kept nodes (0: block-Jacobi)
   std::vector<int> dense_n; // per sim kept DOFs of its explicit inverse (0: band LU)
+  std::vector<int> kept_n;  // per sim DOFs that the condensation keeps
+  std::vector<int> sim_class;  // per sim its launch in gclass
   // factorisation reuse
   int* d_refactor = nullptr;
   std::vector<int> need_refactor, refactor_mask;
@@ -892,6 +894,8 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
   std::vector<int64_t> dense_off(n_sims + 1, 0), panel_off(n_sims + 1, 0);
   h->band_b.assign(n_sims, 0);
   h->dense_n.assign(n_sims, 0);
+  h->kept_n.assign(n_sims, 0);
+  h->sim_class.assign(n_sims, 0);
   const int bmax = (((227 * 1024) / 4 - 8) / kPanel - kPanel) / 2;  // shared-memory limit of k_band_lu
   std::vector<CondPlan> plan(n_sims);
   // f(s) for every simulation on up to 16 host threads, fewer where no more can be started; false when
@@ -938,6 +942,7 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
     dense_off[s + 1] = dense_off[s] + ld * ld;
     panel_off[s + 1] = panel_off[s] + ld * kDenseTile;
     roff[s + 1] = roff[s] + nr;
+    h->kept_n[s] = 6 * nr;
   }
 
   // ---- device arenas
@@ -1404,6 +1409,7 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
         cta.insert(cta.end(), small.begin(), small.end());
         int* p_cta;
         CK(A.upload(&p_cta, cta));
+        for (int s2 : small) h->sim_class[s2] = 1;
         SolverArgs cb = args_for(big, false), cs = args_for(small, true);
         cb.cta_sim = p_cta;
         cs.cta_sim = p_cta + big.size();
@@ -2212,6 +2218,17 @@ int eb_get_memory(eb_handle* h, int64_t* device_bytes, int32_t* band_sims) {
     for (int b : h->band_b) c += b > 0;
     *band_sims = c;
   }
+  return EB_OK;
+}
+
+int eb_get_solver(eb_handle* h, int32_t sim, int32_t info[4]) {
+  if (!h || sim < 0 || sim >= h->n_sims || !info) return fail(EB_ERR_ARG, "bad handle or sim index");
+  const bool band = h->band_b[sim] > 0 && !h->dense_n[sim], two = h->gclass.size() == 2;
+  const bool staged = band && (two ? h->gclass[h->sim_class[sim]] : h->sa).stage_floats > 0;
+  info[0] = h->kept_n[sim];
+  info[1] = band ? h->band_b[sim] : 0;
+  info[2] = h->dense_n[sim];
+  info[3] = (staged ? EB_SOLVER_STAGED : 0) | (band && h->tc_lu ? EB_SOLVER_TENSOR_LU : 0) | (two ? EB_SOLVER_TWO_CLASSES : 0);
   return EB_OK;
 }
 

@@ -15,7 +15,8 @@ __global__ void k_band_fill(Dev d, BandDev B, CondFactor f) {
   const int blk = f.red[t / 36], k = (int)(t % 36);
   const int rn = f.rnode[blk];
   const int s = d.node_sim[rn];
-  if (!d.active[s] || !B.refactor[s]) return;
+  // the lists hold the kept blocks of every condensed simulation, also of those with an inverse
+  if (!d.active[s] || !B.refactor[s] || B.bw[s] == 0) return;
   const int ne = B.cond.ne[s];
   const int i = 6 * (f.rpos[t / 36] - ne) + k / 6, j = 6 * (B.cond.scol[blk] - ne) + k % 6;
   band_view(B, s, band_n(B, s)).at(i, j) = B.cond.S[(int64_t)blk * 36 + k];

@@ -242,6 +242,13 @@ int eb_set_tolerances(eb_handle *h, const double *tolerance_residual, const doub
 int eb_get_stats(eb_handle *h, eb_sim_stats *stats /* n_sims */);
 /* Device memory the handle holds (bytes), and how many simulations use the band-LU preconditioner. */
 int eb_get_memory(eb_handle *h, int64_t *device_bytes, int32_t *band_sims);
+/* How the handle solves simulation `sim`: info[0] DOFs the condensation keeps, [1] half bandwidth of
+ * their band LU (0: none), [2] DOFs of their explicit inverse (0: none), both 0 with block-Jacobi,
+ * [3] EB_SOLVER_* flags. */
+#define EB_SOLVER_STAGED 1      /* the band's triangular solves are staged through shared memory */
+#define EB_SOLVER_TENSOR_LU 2   /* the band LU runs on the tensor cores */
+#define EB_SOLVER_TWO_CLASSES 4 /* the handle's solves are two launches by shared-memory need */
+int eb_get_solver(eb_handle *h, int32_t sim, int32_t info[4]);
 /* Assembled global vectors of one simulation at n+1 (6 n_nodes each; NULL to skip). */
 int eb_get_forces(eb_handle *h, int32_t sim, double *Tint, double *Tk, double *Tc);
 
