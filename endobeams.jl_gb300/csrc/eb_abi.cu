@@ -19,6 +19,7 @@
 #include "eb_cond_plan.hpp"
 #include "eb_gmres.cuh"
 #include "eb_internal.cuh"
+#include "eb_launch_rules.hpp"
 #include "eb_output.cuh"
 #include "eb_warm.cuh"
 
@@ -678,6 +679,8 @@ int eb_device_info(int32_t* count, char* name, int32_t name_len) {
 int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_handle** out) {
   if (!p || !sims || !out || n_sims <= 0) return fail(EB_ERR_ARG, "eb_create: bad arguments");
   *out = nullptr;
+  const int asked_threads = gmres_cta_threads(p->threads_per_sim);
+  if (asked_threads < 0) return fail(EB_ERR_ARG, "threads_per_sim must be at most %d", kGmresMaxThreads);
   if (p->krylov_restart < 1 || p->krylov_restart > 128) return fail(EB_ERR_ARG, "krylov_restart must be in [1,128]");
   std::unique_ptr<eb_handle> h(new eb_handle());
   h->P = *p;
@@ -1089,7 +1092,7 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
   // ---- solver work
   const int m = p->krylov_restart;
   const bool fp32 = p->precision == EB_PREC_MIXED;
-  if (p->threads_per_sim > 0) h->gmres_threads = p->threads_per_sim;
+  if (asked_threads) h->gmres_threads = asked_threads;
   CK(A.alloc(&h->d_Dinv64, NN * 36));
   CK(A.alloc(&h->d_Dinv32, NN * 36));
   CK(A.alloc(&h->d_norms, 5 * (size_t)n_sims));
@@ -1422,12 +1425,12 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
   if (h->gclass.empty()) {
     int64_t nmax = 0;
     for (int s = 0; s < n_sims; ++s) nmax = std::max(nmax, 6 * (h->node_off[s + 1] - h->node_off[s]));
-    sa.team = gmres_team(sa, fp32, p->threads_per_sim > 0 ? p->threads_per_sim : 512, (int)nmax);
+    sa.team = gmres_team(sa, fp32, asked_threads ? asked_threads : kGmresMaxThreads, (int)nmax);
     // sixteen warps where every CTA has an SM to itself: their phases wait for loads
     int dev = 0, sms = 0;
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    if (p->threads_per_sim <= 0 && n_sims * sa.team <= sms) h->gmres_threads = 512;
+    if (!asked_threads && n_sims * sa.team <= sms) h->gmres_threads = kGmresMaxThreads;
     // z_j, w (double or float) and the FP32 vector of the largest simulation
     const int vec = (int)((nmax * (fp32 ? 3 : 5) + 3) / 4 * 4);
     if (sa.team == 1 && sizeof(float) * (size_t)vec <= kGmresVecSmem) {

@@ -22,6 +22,7 @@
 
 #include "eb_band.cuh"
 #include "eb_gmres.cuh"
+#include "eb_launch_rules.hpp"
 
 namespace eb {
 
@@ -190,7 +191,7 @@ __device__ __forceinline__ float row_pairs(const SolverArgs& a, int64_t n0, int 
 }
 
 template <typename T>
-__global__ void __launch_bounds__(512) k_gmres(SolverArgs a) {
+__global__ void __launch_bounds__(kGmresMaxThreads) k_gmres(SolverArgs a) {
   Work wk;
   {
     uint32_t r, c;

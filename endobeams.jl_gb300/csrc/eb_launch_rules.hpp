@@ -1,0 +1,19 @@
+// Rules of the launches that need no CUDA (host only).
+#pragma once
+
+namespace eb {
+
+constexpr int kGmresMaxThreads = 512;
+
+// CTA size of k_gmres for the caller's threads_per_sim: whole warps, because a warp owns whole chunks of
+// the vectors (fewer than 32 threads would own none and never finish, a partial warp would share
+// chunks with another), and at least two of them (the band sweeps' near and far rows).  The results
+// do not depend on it.  0: the library's choice; -1: refused.
+inline int gmres_cta_threads(int asked) {
+  if (asked <= 0) return 0;
+  if (asked > kGmresMaxThreads) return -1;
+  const int whole = (asked + 31) / 32 * 32;
+  return whole < 64 ? 64 : whole;
+}
+
+}  // namespace eb

@@ -73,7 +73,8 @@ typedef struct {
   double linear_tol;                      /* relative residual of each linear solve */
   double inner_tol;                       /* relative tolerance of the FP32 inner solve (mixed) */
   int32_t max_refinements;                /* FP64 refinement sweeps (mixed) */
-  int32_t threads_per_sim;                /* CTA size of the per-simulation solver, 0 = auto */
+  int32_t threads_per_sim;                /* CTA size of the per-simulation solver, 0 = auto; rounded up to
+                                             whole warps, at least two; more than 512: EB_ERR_ARG */
   int32_t timing;                         /* 1: record per-phase CUDA-event times in eb_step */
   int32_t preconditioner;                 /* EB_PRECOND_* */
   int32_t refactor_its;                   /* the preconditioner's factors are reused until a solve needs more GMRES

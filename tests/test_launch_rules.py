@@ -1,0 +1,30 @@
+"""Launch rules that need no GPU (csrc/eb_launch_rules.hpp)."""
+import ctypes
+import os
+import shutil
+import subprocess
+
+import pytest
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+
+@pytest.fixture(scope="module")
+def rules(tmp_path_factory):
+    cxx = shutil.which("g++")
+    if cxx is None:
+        pytest.skip("g++ not found")
+    so = str(tmp_path_factory.mktemp("rules") / "rules_host.so")
+    subprocess.run([cxx, "-O2", "-std=c++17", "-fPIC", "-shared", os.path.join(HERE, "host", "rules_host.cpp"), "-o", so],
+                   check=True)
+    return ctypes.CDLL(so)
+
+
+def test_solver_cta_is_whole_warps(rules):
+    """A warp owns whole chunks of the vectors: with no whole warp the solver's loops would not advance,
+    with a partial one two warps would own the same chunk."""
+    f = rules.host_gmres_cta_threads
+    assert [f(t) for t in (-7, 0)] == [0, 0]
+    for t in range(1, 513):
+        assert f(t) % 32 == 0 and max(64, t) <= f(t) <= max(64, t + 31)
+    assert f(513) < 0 and f(1024) < 0
