@@ -129,21 +129,28 @@ __device__ __forceinline__ P3 tri_vertex(const double* tri, int64_t t, int k) {
   return P3{v[0], v[1], v[2]};
 }
 
-// FP32 copy of the triangles relative to the grid's centre, scaled.  A needle (height below 1e-3 of its
-// longest edge) gets a NaN: no FP32 test ever discards it.
+// FP32 copy of the triangles relative to the grid's centre, scaled.  The FP32 distance divides by the
+// squared area: its error grows as the square of longest edge over height.  Host comparison with
+// FP64, 1e8 triangles of 1e-9 to 1 of the extent: 13 times the margin below a height of 1.1e-3 of the longest
+// edge, 0.6 of it at 5e-3, 0.04 at 2e-2.  A thinner triangle (a needle), also one that rounding to FP32 makes so,
+// gets a NaN: no FP32 test ever discards it.  The same below 1e-8 of the extent, where products of four
+// lengths come near FP32's smallest.
 __global__ void k_mesh_prep(const double* __restrict__ tri, int64_t nt, Grid g, float* __restrict__ tf) {
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= nt) return;
   const P3 c{g.cx, g.cy, g.cz};
-  const P3 v[3] = {sub(tri_vertex(tri, t, 0), c), sub(tri_vertex(tri, t, 1), c), sub(tri_vertex(tri, t, 2), c)};
-  const P3 e0 = sub(v[1], v[0]), e1 = sub(v[2], v[0]), e2 = sub(v[2], v[1]), n = cross(e0, e1);
-  const double L2 = fmax(dot(e0, e0), fmax(dot(e1, e1), dot(e2, e2)));
-  const bool needle = !(dot(n, n) > 1e-6 * L2 * L2);
+  float f[9];
   for (int k = 0; k < 3; ++k) {
-    tf[9 * t + 3 * k] = needle ? nanf("") : (float)(v[k].x * g.scale);
-    tf[9 * t + 3 * k + 1] = (float)(v[k].y * g.scale);
-    tf[9 * t + 3 * k + 2] = (float)(v[k].z * g.scale);
+    const P3 v = sub(tri_vertex(tri, t, k), c);
+    f[3 * k] = (float)(v.x * g.scale);
+    f[3 * k + 1] = (float)(v.y * g.scale);
+    f[3 * k + 2] = (float)(v.z * g.scale);
   }
+  const P3 a{f[0], f[1], f[2]}, b{f[3], f[4], f[5]}, q{f[6], f[7], f[8]};
+  const P3 e0 = sub(b, a), e1 = sub(q, a), e2 = sub(q, b), n = cross(e0, e1);
+  const double L2 = fmax(dot(e0, e0), fmax(dot(e1, e1), dot(e2, e2)));
+  const bool needle = !(dot(n, n) > 4e-4 * L2 * L2) || L2 < 1e-16;
+  for (int k = 0; k < 9; ++k) tf[9 * t + k] = needle && k % 3 == 0 ? nanf("") : f[k];
 }
 
 constexpr int kBx = 8, kBy = 4, kBz = 4;  // points of a brick
@@ -268,8 +275,8 @@ extern "C" int eb_sdf_from_mesh(int64_t n_vert, const double* verts, int64_t n_t
   g.cy = origin[1] + 0.5 * (double)(dims[1] - 1) * spacing[1];
   g.cz = origin[2] + 0.5 * (double)(dims[2] - 1) * spacing[2];
   // largest coordinate and longest edge; an FP32 coordinate is off by 2^-24 of the former, a
-  // distance by that and, through the face region's quotient (needles are kept out), by 1e-4 of
-  // the latter: ten times the sum is a safe bound
+  // distance by that and, through the face region's quotient (needles are kept out), by 8e-5 of
+  // the latter: the margin is 25 times the sum
   double ext = std::max(std::max(0.5 * (double)dims[0] * spacing[0], 0.5 * (double)dims[1] * spacing[1]),
                         0.5 * (double)dims[2] * spacing[2]);
   double L2 = 0.0;
@@ -287,7 +294,8 @@ extern "C" int eb_sdf_from_mesh(int64_t n_vert, const double* verts, int64_t n_t
   g.scale = 1.0 / ext;
   g.margin = (float)(2e-3 * std::sqrt(L2) * g.scale + 2e-5);
   // a vertex at 2e-3 of the extent is off by 3e-5 of its distance, a solid angle with den > |a||b||c| / 4
-  // then by 1e-3 at most, and 4e-6 for any triangle
+  // then by 3e-4 (the same for all triangles at a vertex: over a closed mesh it cancels), and by 1.8e-6
+  // through rounding (1e8 triangles compared on the host): 4e-6 for each
   g.lmin2 = 4e-6f;
   g.slack = 0.2 + 4e-6 * (double)n_tri;
   Buf dt, df, dout;
