@@ -89,20 +89,29 @@ __device__ __forceinline__ void store_inverse(const float (&v)[16], float* dst) 
     *reinterpret_cast<float4*>(dst + r * kT + 16 * q + c) = make_float4(v[c], v[c + 1], v[c + 2], v[c + 3]);
 }
 
+// Simulation of this CTA and its index among the simulation's `per` CTAs: everything on the grid's x
+// axis, whose limit no handle reaches (y ends at 65,535).
+__device__ __forceinline__ int sim_of(int per, int* i) {
+  const int s = (int)(blockIdx.x / (unsigned)per);
+  *i = (int)(blockIdx.x - (unsigned)s * (unsigned)per);
+  return s;
+}
+
 __device__ __forceinline__ bool marked(const Dev& d, const DenseDev& g, const int* refactor, int s) {
   return g.n[s] > 0 && d.active[s] && refactor[s];
 }
 
 }  // namespace
 
-// Zeros, with ones on the diagonal beyond N; blockIdx.y = simulation.
-__global__ void k_dense_zero(Dev d, DenseDev g, const int* refactor) {
-  const int s = blockIdx.y;
+// Zeros, with ones on the diagonal beyond N; `per` CTAs per simulation.
+__global__ void k_dense_zero(Dev d, DenseDev g, const int* refactor, int per) {
+  int part;
+  const int s = sim_of(per, &part);
   if (!marked(d, g, refactor, s)) return;
   const int n = g.n[s], ld = dense_ld(n);
   float* G = g.G + g.off[s];
   const int64_t len = (int64_t)ld * ld;
-  for (int64_t i = 4 * ((int64_t)blockIdx.x * blockDim.x + threadIdx.x); i < len; i += 4 * (int64_t)gridDim.x * blockDim.x) {
+  for (int64_t i = 4 * ((int64_t)part * blockDim.x + threadIdx.x); i < len; i += 4 * (int64_t)per * blockDim.x) {
     float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
     const int r = (int)(i / ld), c = (int)(i - (int64_t)r * ld);
     if (r >= n && r >= c && r < c + 4) (&z.x)[r - c] = 1.f;
@@ -138,8 +147,9 @@ __global__ void __launch_bounds__(kMm) k_dense_first(Dev d, DenseDev g, DenseWor
 }
 
 // CTA (i, s): C_i = A_ik D⁻¹ (stored transposed) and O_i = A_ki, for i != k.
-__global__ void __launch_bounds__(kMm) k_dense_panel(Dev d, DenseDev g, DenseWork w, const int* refactor, int k) {
-  const int s = blockIdx.y, i = blockIdx.x;
+__global__ void __launch_bounds__(kMm) k_dense_panel(Dev d, DenseDev g, DenseWork w, const int* refactor, int k, int per) {
+  int i;
+  const int s = sim_of(per, &i);
   if (!marked(d, g, refactor, s)) return;
   const int ld = dense_ld(g.n[s]);
   if (kT * k >= ld || kT * i >= ld || i == k) return;
@@ -166,13 +176,14 @@ __global__ void __launch_bounds__(kMm) k_dense_panel(Dev d, DenseDev g, DenseWor
 
 // CTA (tile, s) of step k; the next diagonal block's tile comes first, so that its inversion
 // runs beside the other tiles.
-__global__ void __launch_bounds__(kMm) k_dense_update(Dev d, DenseDev g, DenseWork w, const int* refactor, int k) {
-  const int s = blockIdx.y;
+__global__ void __launch_bounds__(kMm) k_dense_update(Dev d, DenseDev g, DenseWork w, const int* refactor, int k, int per) {
+  int at;
+  const int s = sim_of(per, &at);
   if (!marked(d, g, refactor, s)) return;
   const int ld = dense_ld(g.n[s]), nb = ld / kT;
-  if (k >= nb || (int)blockIdx.x >= nb * nb) return;
+  if (k >= nb || at >= nb * nb) return;
   const int first = k + 1 < nb ? (k + 1) * nb + k + 1 : 0;
-  const int tile = blockIdx.x == 0 ? first : ((int)blockIdx.x <= first ? (int)blockIdx.x - 1 : (int)blockIdx.x);
+  const int tile = at == 0 ? first : (at <= first ? at - 1 : at);
   const int i = tile / nb, j = tile - i * nb;
   __shared__ __align__(16) float At[kT * kLd], B[kT * kLd];
   __shared__ __align__(16) float rows[2 * kT];
@@ -211,7 +222,7 @@ __global__ void __launch_bounds__(kMm) k_dense_update(Dev d, DenseDev g, DenseWo
     *reinterpret_cast<float4*>(A + (int64_t)(4 * tm + a) * ld + 4 * tn) = v;
     old[a] = v;
   }
-  if (blockIdx.x != 0 || k + 1 >= nb) return;
+  if (at != 0 || k + 1 >= nb) return;
   // the next diagonal block: invert it from the updated values
   __syncthreads();  // every thread is done with At
 #pragma unroll
@@ -229,14 +240,14 @@ void launch_dense_inverse(const Dev& d, const DenseDev& g, const DenseWork& w, c
                           cudaStream_t s) {
   if (w.max_ld == 0) return;
   const unsigned S = (unsigned)d.n_sims;
-  const int nb = w.max_ld / kT;
+  const int nb = w.max_ld / kT, zero = std::max(1, nb * nb / 2);
   // float4 stores of the largest matrix over 256-thread CTAs, eight per thread
-  k_dense_zero<<<dim3((unsigned)std::max(1, nb * nb / 2), S), 256, 0, s>>>(d, g, refactor);
+  k_dense_zero<<<zero * S, 256, 0, s>>>(d, g, refactor, zero);
   if (f.red_n) k_dense_fill<<<nblocks(f.red_n * 36, 256), 256, 0, s>>>(d, g, f, refactor);
   k_dense_first<<<S, kMm, 0, s>>>(d, g, w, refactor);
   for (int k = 0; k < nb; ++k) {
-    if (nb > 1) k_dense_panel<<<dim3((unsigned)nb, S), kMm, 0, s>>>(d, g, w, refactor, k);
-    k_dense_update<<<dim3((unsigned)(nb * nb), S), kMm, 0, s>>>(d, g, w, refactor, k);
+    if (nb > 1) k_dense_panel<<<nb * S, kMm, 0, s>>>(d, g, w, refactor, k, nb);
+    k_dense_update<<<nb * nb * S, kMm, 0, s>>>(d, g, w, refactor, k, nb * nb);
   }
 }
 
