@@ -308,6 +308,7 @@ struct eb_handle {
   int *pin_active = nullptr, *pin_refactor = nullptr, *pin_mask = nullptr;
   int state_chunk = 0;
   std::mutex state_mu;  // pin_state
+  int device = 0;       // current at creation
   bool any_fixed = false;  // some simulation has boundary conditions
   IterGraph graph[2];      // without / with band refactorisation
   uint64_t graph_gen = 1;  // bumped when launch parameters captured in the graphs change
@@ -686,6 +687,7 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
   h->P = *p;
   h->n_sims = n_sims;
   for (int i = 0; i < 3; ++i) { h->gauss.w[i] = p->gauss_w[i]; h->gauss.z[i] = p->gauss_z[i]; }
+  CK(cudaGetDevice(&h->device));
   CK(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
   CK(cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking));
   CK(cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming));
@@ -2034,6 +2036,17 @@ static int commit_impl(eb_handle* h, const int32_t* mask, bool commit) {
 int eb_commit(eb_handle* h, const int32_t* mask) { return commit_impl(h, mask, true); }
 int eb_rollback(eb_handle* h, const int32_t* mask) { return commit_impl(h, mask, false); }
 
+namespace {
+struct CudaDevice {
+  static int get() {
+    int d = 0;
+    cudaGetDevice(&d);
+    return d;
+  }
+  static void set(int d) { cudaSetDevice(d); }
+};
+}  // namespace
+
 static int get_state_impl(eb_handle* h, int32_t sim, bool at_n, double* u, double* ud, double* udd, double* w,
                           double* wd, double* wdd, double* R, double* dR) {
   if (!h || sim < 0 || sim >= h->n_sims) return fail(EB_ERR_ARG, "bad handle or sim index");
@@ -2042,6 +2055,7 @@ static int get_state_impl(eb_handle* h, int32_t sim, bool at_n, double* u, doubl
   unsigned fields = 0;
   for (int f = 0; f < 8; ++f) fields |= (dst[f] ? 1u : 0u) << f;
   if (!fields) return EB_OK;
+  OnDevice<CudaDevice> on(h->device);  // the state comes by a launch, whatever device the caller works on
   std::lock_guard<std::mutex> lock(h->state_mu);
   for (int64_t i0 = 0; i0 < n; i0 += h->state_chunk) {
     const int m = (int)std::min<int64_t>(h->state_chunk, n - i0);

@@ -16,4 +16,23 @@ inline int gmres_cta_threads(int asked) {
   return whole < 64 ? 64 : whole;
 }
 
+// Makes `device` the thread's current one for a scope, for entry points that launch on a handle's
+// stream where the caller may have another device current (copies need no such thing).
+template <typename Api>
+class OnDevice {
+ public:
+  explicit OnDevice(int device) : back_(Api::get()), changed_(back_ != device) {
+    if (changed_) Api::set(device);
+  }
+  ~OnDevice() {
+    if (changed_) Api::set(back_);
+  }
+  OnDevice(const OnDevice&) = delete;
+  OnDevice& operator=(const OnDevice&) = delete;
+
+ private:
+  int back_;
+  bool changed_;
+};
+
 }  // namespace eb

@@ -2,3 +2,26 @@
 #include "../../endobeams.jl_gb300/csrc/eb_launch_rules.hpp"
 
 extern "C" int host_gmres_cta_threads(int asked) { return eb::gmres_cta_threads(asked); }
+
+// A fake of the two device calls: the current device and how often it was set.
+namespace {
+int current = 0, sets = 0;
+struct FakeDevice {
+  static int get() { return current; }
+  static void set(int d) { current = d; ++sets; }
+};
+}  // namespace
+
+// The device during a scope for `device` entered with `caller` current; out: the device after it, set calls.
+extern "C" int host_on_device(int caller, int device, int* out) {
+  current = caller;
+  sets = 0;
+  int inside;
+  {
+    eb::OnDevice<FakeDevice> on(device);
+    inside = current;
+  }
+  out[0] = current;
+  out[1] = sets;
+  return inside;
+}

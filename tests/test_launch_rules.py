@@ -28,3 +28,14 @@ def test_solver_cta_is_whole_warps(rules):
     for t in range(1, 513):
         assert f(t) % 32 == 0 and max(64, t) <= f(t) <= max(64, t + 31)
     assert f(513) < 0 and f(1024) < 0
+
+
+def test_state_is_read_on_the_handles_device(rules):
+    """eb_get_state launches: the handle's device is current during the call, the caller's afterwards."""
+    out = (ctypes.c_int * 2)()
+    for caller, device, sets in ((0, 0, 0), (1, 0, 2), (0, 3, 2)):
+        assert rules.host_on_device(caller, device, out) == device
+        assert list(out) == [caller, sets]
+    csrc = os.path.join(HERE, "..", "endobeams.jl_gb300", "csrc", "eb_abi.cu")
+    body = open(csrc).read().split("static int get_state_impl(", 1)[1].split("launch_state(", 1)[0]
+    assert "OnDevice<CudaDevice> on(h->device)" in body
