@@ -1372,15 +1372,26 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
     h->cur_active.assign(n_sims, 0);
     int max_n = 0;
     for (int s = 0; s < n_sims; ++s) if (bw[s]) max_n = std::max(max_n, kept(s));
-    sa.max_n = max_n;
-    sa.x_in_smem = h->max_b > 0 && gmres_smem(m) + sizeof(float) * (size_t)sa.dense_ld + sizeof(float) * (size_t)max_n <= 200 * 1024;
-    // stage band blocks through shared memory when the two buffers fit beside the rest
-    sa.stage_floats = 0;
     sa.stage_test_extra = p->stage_band == 2 ? 16 : 0;
-    if (h->max_b > 0 && p->stage_band) {
-      sa.stage_floats = kPanel * (h->max_b + 1);
-      if (gmres_smem_total(sa) > kGmresSmemLimit) sa.stage_floats = 0;
-    }
+    // Shared memory of a launch whose widest band is bmax and whose largest kept system is nmax, up to
+    // `limit` bytes: band blocks staged if at all possible (a 100 x 100 net, b = 605: 5.2 times the step
+    // without), then eight inner products a reduction, then the solve vector.
+    auto fit = [&](SolverArgs& c, int bmax, int nmax, size_t limit) {
+      c.max_n = nmax;
+      for (int dots : {8, 4})
+        for (int x : {1, 0}) {
+          c.dots = dots;
+          c.x_in_smem = x;
+          c.stage_floats = kPanel * (bmax + 1);
+          if (bmax > 0 && p->stage_band && gmres_smem_total(c) <= limit) return true;
+        }
+      c.stage_floats = 0;
+      c.dots = 8;
+      c.x_in_smem = 1;
+      if (bmax <= 0 || gmres_smem_total(c) > std::min(limit, (size_t)200 * 1024)) c.x_in_smem = 0;
+      return false;
+    };
+    fit(sa, h->max_b, max_n, kGmresSmemLimit);
     // Occupancy classes: the staging buffers are sized for the widest band of a launch, so
     // one launch runs every CTA at the occupancy of the largest simulation.  Simulations
     // whose own staged solve fits two CTAs per SM form a second launch with its own
@@ -1395,19 +1406,13 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
           if (bw[s2]) nmax = std::max(nmax, kept(s2));
         }
         c.n_sims = (int)sims.size();
-        c.max_n = nmax;
-        c.stage_floats = kPanel * (bmax + 1);
-        c.x_in_smem = 1;
-        if (gmres_smem_total(c) > (two ? kGmresTwoPerSm : (size_t)200 * 1024)) c.x_in_smem = 0;
-        if (gmres_smem_total(c) > (two ? kGmresTwoPerSm : kGmresSmemLimit)) c.stage_floats = 0;
+        fit(c, bmax, nmax, two ? kGmresTwoPerSm : kGmresSmemLimit);
         return c;
       };
       std::vector<int> big, small;
       for (int s2 : order) {
         SolverArgs one = sa;
-        one.x_in_smem = 0;
-        one.stage_floats = kPanel * (bw[s2] + 1);
-        (bw[s2] > 0 && gmres_smem_total(one) > kGmresTwoPerSm ? big : small).push_back(s2);
+        (bw[s2] > 0 && !fit(one, bw[s2], kept(s2), kGmresTwoPerSm) ? big : small).push_back(s2);
       }
       if (!big.empty() && !small.empty()) {
         std::vector<int> cta(big);

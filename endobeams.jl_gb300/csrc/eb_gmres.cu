@@ -54,7 +54,7 @@ struct Work {
   Team t;
   int n, ch, nchunk;     // DOFs, chunk length, chunks
   int warp0, nwarps;     // this warp's first chunk, stride between its chunks
-  double* part[2];       // chunk sums of a reduction (kMaxChunks x 8), used in turn
+  double* part[2];       // chunk sums of a reduction (kMaxChunks x SolverArgs::dots), used in turn
   double* sums;          // 8
   int flip;
   template <typename F>
@@ -215,8 +215,8 @@ __global__ void __launch_bounds__(kGmresMaxThreads) k_gmres(SolverArgs a) {
   double* y = g + m + 1;           // m + 1
   T* yt = reinterpret_cast<T*>(y + m + 1);  // y in the cycle's precision
   wk.part[0] = y + 2 * m + 2;
-  wk.part[1] = wk.part[0] + 8 * kMaxChunks;
-  wk.sums = wk.part[1] + 8 * kMaxChunks;  // 16
+  wk.part[1] = wk.part[0] + a.dots * kMaxChunks;
+  wk.sums = wk.part[1] + a.dots * kMaxChunks;  // 16
   wk.flip = 0;
   wk.n = n;
   wk.ch = chunk_len(n);
@@ -456,7 +456,8 @@ __global__ void __launch_bounds__(kGmresMaxThreads) k_gmres(SolverArgs a) {
         for (int pass = 0; pass < 2; ++pass) {
           const int last = j + pass;  // in the second pass, "v_(j+1)" is w itself
           for (int i0 = 0; i0 <= last;) {
-            // inner products with v_i0 .., as many at a time as are left (at most 8)
+            // inner products with v_i0 .., as many at a time as are left (at most a.dots; a sum's order
+            // does not depend on how many there are)
             auto dots = [&](auto width) {
               constexpr int NQ = decltype(width)::value;
               const int nq = min(NQ, last + 1 - i0);
@@ -482,7 +483,7 @@ __global__ void __launch_bounds__(kGmresMaxThreads) k_gmres(SolverArgs a) {
               i0 += NQ;
             };
             const int left = last + 1 - i0;
-            if (left > 4) dots(std::integral_constant<int, 8>{});
+            if (left > 4 && a.dots > 4) dots(std::integral_constant<int, 8>{});
             else if (left > 2) dots(std::integral_constant<int, 4>{});
             else if (left > 1) dots(std::integral_constant<int, 2>{});
             else dots(std::integral_constant<int, 1>{});
@@ -688,12 +689,12 @@ void launch_block_jacobi(const Dev& d, double* Dinv64, float* Dinv32, cudaStream
   if (d.n_nodes) k_block_jacobi<<<nblocks(d.n_nodes), kThreads, 0, s>>>(d, Dinv64, Dinv32);
 }
 
-size_t gmres_smem(int m) {
-  return sizeof(double) * ((size_t)(m + 1) * m + 5 * (size_t)m + 3 + 16 * (size_t)kMaxChunks + 16 + 1);
+size_t gmres_smem(int m, int dots) {
+  return sizeof(double) * ((size_t)(m + 1) * m + 5 * (size_t)m + 3 + 2 * (size_t)dots * kMaxChunks + 16 + 1);
 }
 
 size_t gmres_smem_total(const SolverArgs& a) {
-  return gmres_smem(a.m) + sizeof(float) * ((size_t)a.dense_ld + (size_t)a.vec_smem) + (a.x_in_smem ? sizeof(float) * (size_t)a.max_n : 0) +
+  return gmres_smem(a.m, a.dots) + sizeof(float) * ((size_t)a.dense_ld + (size_t)a.vec_smem) + (a.x_in_smem ? sizeof(float) * (size_t)a.max_n : 0) +
          (a.stage_floats > 0 ? 128 + sizeof(float) * 2 * (size_t)a.stage_floats +
                                    sizeof(float) * 2 * kPanel * kPanel
                              : 0);

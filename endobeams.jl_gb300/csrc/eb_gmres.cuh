@@ -41,6 +41,7 @@ struct SolverArgs {
   int dense_ld;          // largest ld of a dense simulation of the handle, 0 = none
   int vec_smem;          // > 0: floats of shared memory for the working vectors of a simulation on one CTA
   int x_in_smem;         // 1: the permuted solve vector lives in shared memory
+  int dots;              // inner products of a reduction: 8, or 4 where their partial sums' room lets band blocks be staged
   int max_n;             // most kept DOFs of a simulation of this launch
   int stage_floats;      // > 0: band blocks staged in shared memory, floats per buffer (32 (b_max + 1))
   int stage_test_extra;  // > 0: the first forward block waits for bytes no copy delivers (tests the bounded wait)
@@ -59,7 +60,7 @@ constexpr size_t kGmresVecSmem = 48 * 1024;  // most shared memory for a simulat
 constexpr int kTeamDofs = 512;  // fewest DOFs per CTA of a team
 int gmres_team(const SolverArgs& a, bool fp32, int threads, int max_dofs);
 cudaError_t launch_gmres(const SolverArgs& a, bool fp32, int threads, cudaStream_t s);
-size_t gmres_smem(int m);
+size_t gmres_smem(int m, int dots);
 size_t gmres_smem_total(const SolverArgs& a);  // dynamic shared memory of one launch
 constexpr size_t kGmresSmemLimit = 216 * 1024;  // leaves room for the kernel's static shared memory (ring, barriers)
 // Dynamic shared memory up to which two CTAs share an SM (228 KB per SM, minus the kernel's
