@@ -902,6 +902,7 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
   h->kept_n.assign(n_sims, 0);
   h->sim_class.assign(n_sims, 0);
   const int bmax = (((227 * 1024) / 4 - 8) / kPanel - kPanel) / 2;  // shared-memory limit of k_band_lu
+  const int stage_b = gmres_stage_b(p->krylov_restart);  // also with stage_band off: the plan is a result's bits
   std::vector<CondPlan> plan(n_sims);
   // f(s) for every simulation on up to 16 host threads, fewer where no more can be started; false when
   // memory ran out (an exception must leave neither a thread nor the C interface)
@@ -931,7 +932,7 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
     for (int64_t i = 0; i < n; ++i)
       for (int g : adj[no + i])
         if (g != (int)(no + i)) la[i].push_back((int)(g - no));
-    cond_plan(la, (bmax - 5) / 6, p->stage_band == 2 ? 0 : kDenseMax, plan[s]);
+    cond_plan(la, (bmax - 5) / 6, p->stage_band == 2 ? 0 : kDenseMax, plan[s], stage_b);
   }))
     return fail(EB_ERR_STATE, "out of host memory");
   for (int s = 0; s < n_sims; ++s) {

@@ -18,8 +18,16 @@
 // each sweep: a barrier of the team and its instructions' latency) and its blocks' bytes (with 2 us
 // a 33 x 33 net took 2.10 ms a step, with 5 us 1.94, a 48 x 200 stent 11.4 and 10.8; from 6 us on a
 // stent that refactorises twice a step loses 4% to the larger inverse); the explicit inverse reads 4 N² bytes at about 1 TB/s and its 2 N³ operations at 20 TFLOP/s are
-// spread over some 30 applications; the band sweeps walk 2 N/32 blocks one after the other, a
-// step taking about 0.9 us + 3.5 ns per DOF of half bandwidth on one SM.
+// spread over some 30 applications; the band sweeps walk 2 N/32 blocks one after the other on one
+// SM, a step taking about 0.9 us + 3.5 ns per DOF of half bandwidth where two blocks fit in shared
+// memory, else 6 us + 6 ns (42 x 42 net, b = 593: 3.0 and 10 us); the band LU's N/32 panels, again on
+// one SM, take 20 us + 0.3 b + 0.00046 b² each (75 us at b = 125, 337 at 593, 638 at 875), also
+// spread over 30 applications.
+//
+// Towards the inverse the levels are not priced one by one, because only the last one brings it
+// within reach.  Where it stays out of reach, a second plan is made for the band alone, every
+// level priced, and the cheaper of the two is taken: 50 x 50 net, kept 4,530 at b = 875 by the first
+// plan, 49 ms a step; 7,788 at b = 311 by the second, 12.7 (the band of the whole net: 26).
 #pragma once
 #include <algorithm>
 #include <cstdint>
@@ -128,14 +136,16 @@ struct CondPlan {
     return it != scol.begin() + hi && *it == c ? (int)(it - scol.begin()) : -1;
   }
   std::vector<int> rptr;               // kept rows: blocks among the kept nodes
+  double cost = 0;                     // us of one application, with its share of the factorisation
 };
 
 constexpr int kWholeDofs = 200;  // at most this many DOFs: nothing is eliminated
 
 // The cheaper of the two (past max_dense the explicit inverse is still what the next levels aim
-// at); w < 0: the inverse.
-inline double cond_cost(int nodes, int w, int max_dense) {
-  const double N = 6.0 * nodes, b = 6.0 * w + 5, band = N / 16 * (0.9 + 0.0035 * b);
+// at); w < 0: the inverse.  stage_b: the widest half bandwidth whose blocks fit in shared memory.
+inline double cond_cost(int nodes, int w, int max_dense, int stage_b) {
+  const double N = 6.0 * nodes, b = 6.0 * w + 5, step = b <= stage_b ? 0.9 + 0.0035 * b : 6.0 + 0.006 * b;
+  const double band = N / 16 * step + N / 960 * (20 + 0.3 * b + 0.00046 * b * b);
   const double dense = 4e-6 * N * N + 2.0 * N * N * N / (20e6 * 30);
   return max_dense <= 0 ? band : w < 0 ? dense : std::min(band, dense);
 }
@@ -143,7 +153,7 @@ inline double cond_cost(int nodes, int w, int max_dense) {
 // Symbolic elimination of one simulation's node graph (adj: sorted neighbour lists, self
 // excluded).  At least one node is kept.  max_w: the widest band (nodes) the band LU takes;
 // max_dense: the most DOFs of an explicit inverse.
-inline void cond_plan(const std::vector<std::vector<int>>& adj0, int max_w, int max_dense, CondPlan& P) {
+inline void cond_plan_for(const std::vector<std::vector<int>>& adj0, int max_w, int max_dense, int stage_b, CondPlan& P) {
   const int n = (int)adj0.size();
   P = CondPlan();
   P.n = n;
@@ -191,7 +201,9 @@ inline void cond_plan(const std::vector<std::vector<int>>& adj0, int max_w, int 
   };
   auto commit = [&](std::vector<int>& set) {
     std::sort(set.begin(), set.end());
+    P.cost += 5.0;
     for (int v : set) {
+      P.cost += 144e-6 * (1.0 + 2.0 * adj[v].size());
       nb[v] = adj[v];
       eliminate(adj, v);
       adj[v].clear();
@@ -214,7 +226,9 @@ inline void cond_plan(const std::vector<std::vector<int>>& adj0, int max_w, int 
   }
   // half bandwidths only where the explicit inverse does not cost less than the band sweeps of
   // any bandwidth (w < 0: not needed)
-  auto needs_band = [&](int nodes) { return max_dense <= 0 || cond_cost(nodes, 0, max_dense) < cond_cost(nodes, n, max_dense); };
+  auto needs_band = [&](int nodes) {
+    return max_dense <= 0 || cond_cost(nodes, 0, max_dense, stage_b) < cond_cost(nodes, n, max_dense, stage_b);
+  };
   std::vector<int> rpos;
   int w = needs_band((int)left.size()) ? band(adj, left, rpos) : -1;
   for (int cap : {4, 8, 12, 16, 24, 32}) {
@@ -238,7 +252,7 @@ inline void cond_plan(const std::vector<std::vector<int>>& adj0, int max_w, int 
       }
       // past max_dense there is no inverse yet: go on towards it
       if ((max_dense <= 0 || 6 * m <= max_dense) &&
-          cond_cost(m2, w2, max_dense) + 5.0 + 144e-6 * blocks > cond_cost(m, w, max_dense))
+          cond_cost(m2, w2, max_dense, stage_b) + 5.0 + 144e-6 * blocks > cond_cost(m, w, max_dense, stage_b))
         break;
       commit(set);
       w = w2;
@@ -247,6 +261,7 @@ inline void cond_plan(const std::vector<std::vector<int>>& adj0, int max_w, int 
   w = band(adj, left, rpos);
   P.w = w;
   P.ne = (int)order.size();
+  P.cost += cond_cost((int)left.size(), w, 6 * (int)left.size() <= max_dense ? max_dense : 0, stage_b);
 
   // ---- positions and block numbers
   const int ne = P.ne;
@@ -328,6 +343,15 @@ inline void cond_plan(const std::vector<std::vector<int>>& adj0, int max_w, int 
       }
     for (int t : touched) cnt[t] = 0;
   }
+}
+
+// The plan of one simulation (arguments as above).
+inline void cond_plan(const std::vector<std::vector<int>>& adj, int max_w, int max_dense, CondPlan& P, int stage_b = 1 << 30) {
+  cond_plan_for(adj, max_w, max_dense, stage_b, P);
+  if (max_dense <= 0 || 6 * (P.n - P.ne) <= max_dense) return;
+  CondPlan B;
+  cond_plan_for(adj, max_w, 0, stage_b, B);
+  if (B.w <= max_w && (P.w > max_w || B.cost < P.cost)) P = std::move(B);
 }
 
 }  // namespace eb

@@ -700,6 +700,11 @@ size_t gmres_smem_total(const SolverArgs& a) {
                              : 0);
 }
 
+int gmres_stage_b(int m) {
+  const size_t rest = gmres_smem(m, 4) + sizeof(float) * (kDenseMax + 2 * kPanel * kPanel) + 128;
+  return rest >= kGmresSmemLimit ? 0 : (int)((kGmresSmemLimit - rest) / (2 * sizeof(float) * kPanel)) - 1;
+}
+
 namespace {
 const void* gmres_kernel(bool fp32) { return fp32 ? (const void*)k_gmres<float> : (const void*)k_gmres<double>; }
 

@@ -62,6 +62,8 @@ int gmres_team(const SolverArgs& a, bool fp32, int threads, int max_dofs);
 cudaError_t launch_gmres(const SolverArgs& a, bool fp32, int threads, cudaStream_t s);
 size_t gmres_smem(int m, int dots);
 size_t gmres_smem_total(const SolverArgs& a);  // dynamic shared memory of one launch
+// The widest half bandwidth whose blocks can be staged, whatever other simulations share the launch.
+int gmres_stage_b(int m);
 constexpr size_t kGmresSmemLimit = 216 * 1024;  // leaves room for the kernel's static shared memory (ring, barriers)
 // Dynamic shared memory up to which two CTAs share an SM (228 KB per SM, minus the kernel's
 // static 4.4 KB and the 1 KB the hardware reserves, per CTA; 256 threads x 128 registers
