@@ -309,6 +309,7 @@ struct eb_handle {
   int state_chunk = 0;
   std::mutex state_mu;  // pin_state
   int device = 0;       // current at creation
+  int sms = 0;          // its multiprocessors
   bool any_fixed = false;  // some simulation has boundary conditions
   IterGraph graph[2];      // without / with band refactorisation
   uint64_t graph_gen = 1;  // bumped when launch parameters captured in the graphs change
@@ -566,11 +567,8 @@ int record_iteration(eb_handle* h, bool refactor, PhaseTimer& T) {
   T.begin(st);
   CK(cudaMemcpyAsync(h->d_active, h->pin_active, sizeof(int) * S, cudaMemcpyHostToDevice, st));
   T.mark(EB_PHASE_UPDATE, st);
-  // The element and the contact pass do not depend on each other and run side by side (64-element
-  // ring: a step 1.66 -> 1.43 ms, 9,600 elements 16.6 -> 15.8 ms).  Not where each has between one and
-  // two thirty-element CTAs per SM: two such CTAs on an SM compete for its L1, through which the
-  // elements' temporaries go, while other SMs idle (3,600 elements: 5.14 -> 5.93 ms).
-  const bool fork = h->any_contact && !(ebd::beam_groups(d.beam_threads) == 3 && d.n_elem < 2 * 30 * 152);
+  const bool fork = h->any_contact && side_by_side(ebd::beam_groups(d.beam_threads), ebd::beam_groups(d.contact_threads),
+                                                   d.n_elem, h->sms);
   if (fork) {
     CK(cudaEventRecord(h->ev_fork, st));
     CK(cudaStreamWaitEvent(h->side, h->ev_fork, 0));
@@ -688,6 +686,7 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
   h->n_sims = n_sims;
   for (int i = 0; i < 3; ++i) { h->gauss.w[i] = p->gauss_w[i]; h->gauss.z[i] = p->gauss_z[i]; }
   CK(cudaGetDevice(&h->device));
+  CK(cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, h->device));
   CK(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
   CK(cudaStreamCreateWithFlags(&h->side, cudaStreamNonBlocking));
   CK(cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming));
@@ -959,8 +958,7 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
   d.n_elem = NE;
   d.nnzb = NB;
   d.n_dof = ND;
-  d.beam_threads = NE > kBeamWide ? 256 : kThreads;
-  d.contact_threads = NE > kBeamWide ? 256 : kThreads;
+  d.beam_threads = d.contact_threads = wide_elements(NE, h->sms) ? 256 : kThreads;
   d.gmat_threads = 256;
   d.gvec_threads = 256;
   int64_t *p_node_off, *p_blk_off;
@@ -1435,10 +1433,7 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
     for (int s = 0; s < n_sims; ++s) nmax = std::max(nmax, 6 * (h->node_off[s + 1] - h->node_off[s]));
     sa.team = gmres_team(sa, fp32, asked_threads ? asked_threads : kGmresMaxThreads, (int)nmax);
     // sixteen warps where every CTA has an SM to itself: their phases wait for loads
-    int dev = 0, sms = 0;
-    CK(cudaGetDevice(&dev));
-    CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    if (!asked_threads && n_sims * sa.team <= sms) h->gmres_threads = kGmresMaxThreads;
+    if (!asked_threads && n_sims * sa.team <= h->sms) h->gmres_threads = kGmresMaxThreads;
     // z_j, w (double or float) and the FP32 vector of the largest simulation
     const int vec = (int)((nmax * (fp32 ? 3 : 5) + 3) / 4 * 4);
     if (sa.team == 1 && sizeof(float) * (size_t)vec <= kGmresVecSmem) {

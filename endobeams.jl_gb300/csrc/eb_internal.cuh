@@ -90,7 +90,6 @@ struct Dev {
 
 constexpr int kThreads = 128;
 constexpr int kMaxElemThreads = 256;  // largest block of the element and contact kernels
-constexpr int kBeamWide = 3040;       // element launches beyond twenty elements per SM start with 30 elements a CTA
 
 inline unsigned nblocks(int64_t n, int t = kThreads) { return (unsigned)((n + t - 1) / t); }
 

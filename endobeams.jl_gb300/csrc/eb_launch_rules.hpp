@@ -1,5 +1,6 @@
 // Rules of the launches that need no CUDA (host only).
 #pragma once
+#include <cstdint>
 
 namespace eb {
 
@@ -14,6 +15,18 @@ inline int gmres_cta_threads(int asked) {
   if (asked > kGmresMaxThreads) return -1;
   const int whole = (asked + 31) / 32 * 32;
   return whole < 64 ? 64 : whole;
+}
+
+// Element launches of more than twenty elements per SM start with thirty elements a CTA, others with ten.
+inline bool wide_elements(int64_t n_elem, int sms) { return n_elem > 20 * (int64_t)sms; }
+
+// Whether the element and the contact pass, which do not depend on each other, run side by side (152 SMs, 64-element
+// ring: a step 1.66 -> 1.43 ms, 9,600 elements 16.6 -> 15.8 ms).  Not where both have thirty elements a CTA (three
+// groups) and fewer than two CTAs per SM: two such CTAs on an SM compete for its L1, through which the elements'
+// temporaries go, while other SMs idle (3,600 elements: 5.14 -> 5.93 ms).  The limit was not measured more closely
+// than between these two sizes.
+inline bool side_by_side(int beam_groups, int contact_groups, int64_t n_elem, int sms) {
+  return !(beam_groups == 3 && contact_groups == 3 && n_elem < 2 * 30 * (int64_t)sms);
 }
 
 // Makes `device` the thread's current one for a scope, for entry points that launch on a handle's

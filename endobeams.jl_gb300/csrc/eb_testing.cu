@@ -17,6 +17,7 @@
 
 #include "../../include/endobeams_gb300.h"
 #include "eb_internal.cuh"
+#include "eb_launch_rules.hpp"
 
 using namespace ebd;
 
@@ -80,9 +81,17 @@ __global__ void __launch_bounds__(kContactCta) k_contact_eval(int64_t n, int nb,
               [](int64_t) { return true; });
 }
 
+// Launch shape of n elements on the current device (as eb_create's).
+int eval_groups(int64_t n) {
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return beam_groups(eb::wide_elements(n, sms) ? 256 : 128);
+}
+
 cudaError_t launch_contact_eval(int64_t n, const double* in, const Gauss3& g, const ContactProps& cp, const SurfaceDev& s,
                                 double* out, int32_t* flags, cudaStream_t st) {
-  const int nb = beam_groups(n > eb::kBeamWide ? 256 : 128);
+  const int nb = eval_groups(n);
   const cudaError_t e = eb::raise_smem_limit((const void*)k_contact_eval, contact_smem(nb));
   if (e != cudaSuccess) return e;
   k_contact_eval<<<eb::nblocks(n, kBeamGroup * nb), kContactCta, contact_smem(nb), st>>>(n, nb, in, g, cp, s, out, flags);
@@ -118,7 +127,7 @@ extern "C" int eb_element_eval(int64_t n, const double* in, const double* gauss6
   if ((e = cudaMalloc(&dout.p, sizeof(double) * 458 * n)) != cudaSuccess) return err("cudaMalloc", e);
   cudaMemcpy(di.p, in, sizeof(double) * 96 * n, cudaMemcpyHostToDevice);
   cudaMemset(dout.p, 0, sizeof(double) * 458 * n);
-  const int nb = beam_groups(n > eb::kBeamWide ? 256 : 128);
+  const int nb = eval_groups(n);
   if ((e = eb::raise_smem_limit((const void*)k_element_eval, beam_smem(nb))) != cudaSuccess) return err("k_element_eval", e);
   k_element_eval<<<eb::nblocks(n, kBeamGroup * nb), kBeamCta, beam_smem(nb)>>>(n, nb, (const double*)di.p, g,
                                                                                 (double*)dout.p);

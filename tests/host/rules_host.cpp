@@ -2,6 +2,10 @@
 #include "../../endobeams.jl_gb300/csrc/eb_launch_rules.hpp"
 
 extern "C" int host_gmres_cta_threads(int asked) { return eb::gmres_cta_threads(asked); }
+extern "C" int host_wide_elements(int64_t n_elem, int sms) { return eb::wide_elements(n_elem, sms); }
+extern "C" int host_side_by_side(int beam_groups, int contact_groups, int64_t n_elem, int sms) {
+  return eb::side_by_side(beam_groups, contact_groups, n_elem, sms);
+}
 
 // A fake of the two device calls: the current device and how often it was set.
 namespace {

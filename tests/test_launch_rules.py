@@ -39,3 +39,14 @@ def test_state_is_read_on_the_handles_device(rules):
     csrc = os.path.join(HERE, "..", "endobeams.jl_gb300", "csrc", "eb_abi.cu")
     body = open(csrc).read().split("static int get_state_impl(", 1)[1].split("launch_state(", 1)[0]
     assert "OnDevice<CudaDevice> on(h->device)" in body
+
+
+def test_element_launches_follow_the_devices_size(rules):
+    """Thirty elements a CTA beyond twenty per SM; the two passes side by side unless both have thirty elements a
+    CTA and fewer than two CTAs per SM."""
+    wide = lambda n, sms: bool(rules.host_wide_elements(ctypes.c_int64(n), sms))
+    beside = lambda b, c, n, sms: bool(rules.host_side_by_side(b, c, ctypes.c_int64(n), sms))
+    for sms in (152, 148, 76):
+        assert [wide(n, sms) for n in (0, 20 * sms, 20 * sms + 1)] == [False, False, True]
+        assert [beside(3, 3, n, sms) for n in (60 * sms - 1, 60 * sms)] == [False, True]
+        assert beside(3, 1, 60 * sms - 1, sms) and beside(1, 3, 60 * sms - 1, sms) and beside(1, 1, 1, sms)
