@@ -934,20 +934,23 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
     cond_plan(la, (bmax - 5) / 6, p->stage_band == 2 ? 0 : kDenseMax, plan[s], stage_b);
   }))
     return fail(EB_ERR_STATE, "out of host memory");
+  std::vector<int> kind(n_sims, kPrecondJacobi);
+  std::vector<PrecondBytes> precond_bytes(n_sims);
   for (int s = 0; s < n_sims; ++s) {
-    const int b = 6 * plan[s].w + 5, nr = plan[s].n - plan[s].ne;
+    const CondPlan& P = plan[s];
+    const int b = 6 * P.w + 5, nr = P.n - P.ne;
+    const int64_t N = 6 * (int64_t)nr, ld = dense_ld(6 * nr);
     // few kept nodes: explicit inverse (the staging test asks for the staged band sweeps)
-    const bool dense = 6 * nr <= kDenseMax && p->stage_band != 2;
-    if (p->preconditioner != EB_PRECOND_BLOCK_JACOBI && (dense || b <= bmax)) {
-      h->band_b[s] = b;
-      h->dense_n[s] = dense ? 6 * nr : 0;
-    }
-    const int64_t ld = dense_ld(h->dense_n[s]);
-    band_off[s + 1] = band_off[s] + (h->band_b[s] && !ld ? band_floats(6 * (int64_t)nr, b) : 0);
-    dense_off[s + 1] = dense_off[s] + ld * ld;
-    panel_off[s + 1] = panel_off[s] + ld * kDenseTile;
+    if (p->preconditioner != EB_PRECOND_BLOCK_JACOBI)
+      kind[s] = N <= kDenseMax && p->stage_band != 2 ? kPrecondInverse : (b <= bmax ? kPrecondBand : kPrecondJacobi);
     roff[s + 1] = roff[s] + nr;
     h->kept_n[s] = 6 * nr;
+    PrecondBytes& q = precond_bytes[s];
+    int64_t ints = 5 * (int64_t)P.n_blocks + 2 * (int64_t)(P.n_blocks - P.red0) + 2 * (int64_t)P.ne;
+    for (size_t l = 0; l < P.tgt.size(); ++l) ints += 2 * (int64_t)P.tgt[l].size() + 2 * (int64_t)P.cl[l].size();
+    q.shared = 4 * (36 * (int64_t)P.n_blocks + ints) + 2 * 4 * kPanel * (N + kPanel);  // and the diagonal blocks' inverses
+    q.inverse = 4 * (ld * ld + 2 * ld * kDenseTile + 2 * kDenseTile * kDenseTile);
+    q.band = b <= bmax ? 4 * band_floats(N, b) : 0;
   }
 
   // ---- device arenas
@@ -1157,24 +1160,18 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
   h->tol_res.assign(n_sims, p->tolerance_residual);
   h->tol_disp.assign(n_sims, p->tolerance_displacement);
 
-  // ---- band storage (falls back to block-Jacobi when it would not fit in half the free memory)
+  // ---- inverses, bands and condensation lists, as far as they fit into the free memory (fit_precond)
   {
     size_t fr = 0, tot = 0;
     CK(cudaMemGetInfo(&fr, &tot));
-    // the band, its diagonal-block inverses and the condensation's blocks must leave 2 GB free
-    const size_t inv_bytes = 2 * sizeof(float) * (size_t)inv_base(roff[n_sims], n_sims);
-    size_t need = sizeof(float) * (size_t)(band_off[n_sims] + dense_off[n_sims] + 2 * panel_off[n_sims]);
-    for (int s = 0; s < n_sims; ++s)
-      if (h->band_b[s]) need += (size_t)plan[s].n_blocks * (36 * sizeof(float) + 10 * sizeof(int));
-    const size_t margin = (size_t)2 << 30;
-    if (need + inv_bytes + margin > fr) {
-      std::fill(h->band_b.begin(), h->band_b.end(), 0);
-      std::fill(h->dense_n.begin(), h->dense_n.end(), 0);
-      std::fill(band_off.begin(), band_off.end(), 0);
-      std::fill(dense_off.begin(), dense_off.end(), 0);
-      std::fill(panel_off.begin(), panel_off.end(), 0);
-    }
+    fit_precond(precond_bytes, (int64_t)fr - ((int64_t)2 << 30), kind);  // 2 GB stay free
     for (int s = 0; s < n_sims; ++s) {
+      const int64_t ld = kind[s] == kPrecondInverse ? dense_ld(h->kept_n[s]) : 0;
+      h->band_b[s] = kind[s] == kPrecondJacobi ? 0 : 6 * plan[s].w + 5;
+      h->dense_n[s] = ld ? h->kept_n[s] : 0;
+      band_off[s + 1] = band_off[s] + (kind[s] == kPrecondBand ? band_floats(h->kept_n[s], h->band_b[s]) : 0);
+      dense_off[s + 1] = dense_off[s] + ld * ld;
+      panel_off[s + 1] = panel_off[s] + ld * kDenseTile;
       if (!h->dense_n[s]) h->max_b = std::max(h->max_b, h->band_b[s]);
       h->dense_work.max_ld = std::max(h->dense_work.max_ld, dense_ld(h->dense_n[s]));
       if (h->band_b[s]) h->any_band = true;

@@ -1,6 +1,9 @@
 // Rules of the launches that need no CUDA (host only).
 #pragma once
+#include <algorithm>
 #include <cstdint>
+#include <numeric>
+#include <vector>
 
 namespace eb {
 
@@ -27,6 +30,33 @@ inline bool wide_elements(int64_t n_elem, int sms) { return n_elem > 20 * (int64
 // than between these two sizes.
 inline bool side_by_side(int beam_groups, int contact_groups, int64_t n_elem, int sms) {
   return !(beam_groups == 3 && contact_groups == 3 && n_elem < 2 * 30 * (int64_t)sms);
+}
+
+// What a simulation's preconditioner is, and the device bytes each choice takes.
+enum PrecondKind { kPrecondJacobi = 0, kPrecondBand = 1, kPrecondInverse = 2 };
+struct PrecondBytes {
+  int64_t shared = 0;   // condensation: blocks and lists, whichever of the two follows
+  int64_t band = 0;     // 0: too wide for the band LU
+  int64_t inverse = 0;
+};
+
+// Fits the simulations' choices into `room` bytes: inverses that take more than the band of the same kept
+// nodes become bands, the largest gain first; where that is not enough, all become block-Jacobi.
+inline void fit_precond(const std::vector<PrecondBytes>& b, int64_t room, std::vector<int>& kind) {
+  int64_t need = 0;
+  std::vector<int> swap;
+  for (size_t s = 0; s < b.size(); ++s) {
+    if (kind[s] == kPrecondJacobi) continue;
+    need += b[s].shared + (kind[s] == kPrecondInverse ? b[s].inverse : b[s].band);
+    if (kind[s] == kPrecondInverse && b[s].band > 0 && b[s].band < b[s].inverse) swap.push_back((int)s);
+  }
+  std::stable_sort(swap.begin(), swap.end(), [&](int x, int y) { return b[x].inverse - b[x].band > b[y].inverse - b[y].band; });
+  for (int s : swap) {
+    if (need <= room) return;
+    kind[s] = kPrecondBand;
+    need -= b[s].inverse - b[s].band;
+  }
+  if (need > room) std::fill(kind.begin(), kind.end(), (int)kPrecondJacobi);
 }
 
 // Makes `device` the thread's current one for a scope, for entry points that launch on a handle's

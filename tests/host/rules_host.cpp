@@ -7,6 +7,15 @@ extern "C" int host_side_by_side(int beam_groups, int contact_groups, int64_t n_
   return eb::side_by_side(beam_groups, contact_groups, n_elem, sms);
 }
 
+// n simulations of (shared, band, inverse) bytes each; kind: wanted in, fitted out.
+extern "C" void host_fit_precond(int n, const int64_t* bytes, int64_t room, int32_t* kind) {
+  std::vector<eb::PrecondBytes> b(n);
+  for (int s = 0; s < n; ++s) b[s] = {bytes[3 * s], bytes[3 * s + 1], bytes[3 * s + 2]};
+  std::vector<int> k(kind, kind + n);
+  eb::fit_precond(b, room, k);
+  std::copy(k.begin(), k.end(), kind);
+}
+
 // A fake of the two device calls: the current device and how often it was set.
 namespace {
 int current = 0, sets = 0;

@@ -50,3 +50,26 @@ def test_element_launches_follow_the_devices_size(rules):
         assert [wide(n, sms) for n in (0, 20 * sms, 20 * sms + 1)] == [False, False, True]
         assert [beside(3, 3, n, sms) for n in (60 * sms - 1, 60 * sms)] == [False, True]
         assert beside(3, 1, 60 * sms - 1, sms) and beside(1, 3, 60 * sms - 1, sms) and beside(1, 1, 1, sms)
+
+
+def test_preconditioners_that_do_not_fit(rules):
+    """Inverses give way to the bands of the same kept nodes, the largest saving first; only where the bands do
+    not fit either does everything become block-Jacobi."""
+    jacobi, band, inverse = 0, 1, 2
+
+    def fit(sims, kinds, room):
+        n = len(sims)
+        b = (ctypes.c_int64 * (3 * n))(*[x for s in sims for x in s])
+        k = (ctypes.c_int32 * n)(*kinds)
+        rules.host_fit_precond(n, b, ctypes.c_int64(room), k)
+        return list(k)
+
+    sims = [(10, 20, 100), (10, 30, 200), (10, 0, 50), (10, 90, 80), (5, 40, 0), (1000, 1000, 1000)]
+    want = [inverse, inverse, inverse, inverse, band, jacobi]
+    full = 4 * 10 + 100 + 200 + 50 + 80 + 45
+    assert fit(sims, want, full) == want
+    assert fit(sims, want, full - 1) == [inverse, band, inverse, inverse, band, jacobi]
+    assert fit(sims, want, full - 170) == [inverse, band, inverse, inverse, band, jacobi]
+    assert fit(sims, want, full - 171) == [band, band, inverse, inverse, band, jacobi]
+    assert fit(sims, want, full - 250) == [band, band, inverse, inverse, band, jacobi]
+    assert fit(sims, want, full - 251) == [jacobi] * 6
