@@ -25,7 +25,7 @@ namespace eb {
 struct BandDev {
   float* A;                 // concatenated band storage (FP32: filled and factorised in place)
   const int64_t* off;       // per sim: offset of its U part in A (L part follows)
-  const int* bw;            // per sim: half bandwidth b in DOFs (0: no band, block-Jacobi)
+  const int* bw;            // per sim: half bandwidth b in DOFs (0: no band: explicit inverse or block-Jacobi)
   CondDev cond;             // condensation: eliminated nodes, blocks, levels
   const int* node_at;       // per (node_off[s] + position): global node id (eliminated nodes first, then band order)
   float* work;              // per DOF scratch (permuted vector)

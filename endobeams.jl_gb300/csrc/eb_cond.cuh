@@ -1,6 +1,6 @@
-// Condensation in front of the band LU: level-by-level block elimination of
-// low-degree nodes (plan in eb_cond_plan.hpp) and its part of the
-// preconditioner application.
+// Condensation in front of the kept nodes' explicit inverse or band LU:
+// level-by-level block elimination of low-degree nodes (plan in
+// eb_cond_plan.hpp) and its part of the preconditioner application.
 //
 // Blocks are 6x6 FP32, row-major (entry (r, c) at 6 r + c), so the thread that
 // owns a row reads its 24 bytes as three 8-byte words and six neighbouring

@@ -1,5 +1,5 @@
 // Symbolic part of the preconditioner (host only, no CUDA): which nodes of a
-// simulation are eliminated before the band LU, in which order, and the block
+// simulation are eliminated before the inverse or band LU of the others, in which order, and the block
 // lists that the numeric kernels and the solves walk.
 //
 // A beam structure is mostly wire: the interior nodes of a wire segment have

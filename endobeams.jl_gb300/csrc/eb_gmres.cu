@@ -3,8 +3,9 @@
 //
 // Ktan_free ΔD_free = r_free is solved per simulation by right-preconditioned
 // GMRES; the preconditioner is the condensation with the explicit inverse or the
-// band LU of the kept nodes (eb_cond.cuh, eb_dense.cuh, eb_band.cuh) or 6x6 block-Jacobi (the LU of each node's
-// diagonal block, fixed DOFs replaced by identity rows/columns).  Each
+// band LU of the kept nodes (eb_cond.cuh, eb_dense.cuh, eb_band.cuh) or 6x6
+// block-Jacobi (the LU of each node's diagonal block, fixed DOFs replaced by
+// identity rows/columns).  Each
 // simulation is owned by one team of CTAs (a cluster of 1 to 16, so that few
 // simulations use many SMs) for the whole solve: its Krylov basis lives in
 // global memory in the preconditioner's node order, its Hessenberg matrix and
@@ -14,9 +15,9 @@
 //
 // Precision: the outer loop always measures the true residual b - A x in
 // FP64.  Each pass runs one GMRES(m) cycle on that residual, in FP64
-// (EB_PREC_FP64) or in FP32 (basis and preconditioner; products with the FP64 tangent)
-// (EB_PREC_MIXED: iterative refinement).  A pass is therefore both the
-// GMRES restart and the refinement sweep.
+// (EB_PREC_FP64) or with an FP32 basis and preconditioner, the products with the
+// tangent in FP32 pairs (EB_PREC_MIXED: iterative refinement).  A pass is therefore
+// both the GMRES restart and the refinement sweep.
 #include <cfloat>
 #include <type_traits>
 

@@ -35,8 +35,8 @@ struct SolverArgs {
   int* refs;             // per sim, accumulated
   double* relres;        // per sim, max over the step
   int* status;           // per sim, max over the step
-  BandDev band;          // band-LU preconditioner (bw[s] == 0: block-Jacobi for that sim)
-  DenseDev dense;        // explicit inverse of the kept system (dense.n[s] == 0: band sweeps)
+  BandDev band;          // band LU of the kept nodes (bw[s] == 0: explicit inverse or block-Jacobi)
+  DenseDev dense;        // explicit inverse of the kept system (dense.n[s] == 0: band LU or block-Jacobi)
   float* kin;            // per kept DOF scratch: the dense product's input
   int dense_ld;          // largest ld of a dense simulation of the handle, 0 = none
   int vec_smem;          // > 0: floats of shared memory for the working vectors of a simulation on one CTA

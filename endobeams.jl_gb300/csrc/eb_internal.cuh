@@ -89,7 +89,7 @@ struct Dev {
 };
 
 constexpr int kThreads = 128;
-constexpr int kMaxElemThreads = 256;  // largest block of the element and contact kernels
+constexpr int kMaxElemThreads = 256;  // largest launch shape of the element and contact kernels (their blocks are fixed)
 
 inline unsigned nblocks(int64_t n, int t = kThreads) { return (unsigned)((n + t - 1) / t); }
 
