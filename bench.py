@@ -94,13 +94,13 @@ def parse():
     ap.add_argument("--warm-start", default=None, choices=[None, "off", "learned", "learned_x0"])
     ap.add_argument("--count", type=int, default=None, help="population size override (stents)")
     ap.add_argument("--band-lu", default="tensor", choices=["fp32", "tensor"],
-                    help="band LU engine of the stents' preconditioner")
+                    help="band LU engine of the stents' preconditioner (kept systems over 2,048 DOFs only)")
     ap.add_argument("--refactor", default="cost", choices=["threshold", "cost", "always"],
-                    help="stents: when a band LU is refactorised")
+                    help="stents: when the preconditioner is refactorised")
     ap.add_argument("--refactor-cost", type=float, default=0.12,
-                    help="--refactor cost: GMRES iterations one LU is worth per DOF of half bandwidth "
-                         "(256 stents with four lanes, 15 steps: 0.05 112.7, 0.08 115.5, 0.12 124.1, "
-                         "0.16 125.8, 0.24 115.4 HHT steps/s)")
+                    help="--refactor cost: GMRES iterations a factorisation is worth per DOF of the kept system's half "
+                         "bandwidth (chosen with the band LU of the whole tangent: 256 stents with four lanes, 15 "
+                         "steps: 0.05 112.7, 0.08 115.5, 0.12 124.1, 0.16 125.8, 0.24 115.4 HHT steps/s)")
     ap.add_argument("--mem-frac", type=float, default=0.75, help="device memory fraction per resident group")
     ap.add_argument("--lanes", type=int, default=4,
                     help="concurrent lanes per resident group (one engine, host thread and stream each)")
@@ -140,9 +140,9 @@ def stent_params(p, precision="mixed", warm="off"):
     p.tolerance_residual = STENT_TOL_RES
     p.tolerance_displacement = STENT_TOL_DISP
     p.krylov_restart = 32
-    # a stent's band LU costs ~0.1-1.5 s on one SM: it is reused, and refactorised by the cost rule
-    # when the GMRES iterations lost to its ageing reach its cost (64 stents, 20 steps: 15.2 HHT
-    # steps/s refactorising only past 200 iterations, 26-29 by the cost rule); 200 stays a cap
+    # the factors are reused, and remade by the cost rule when the GMRES iterations lost to their
+    # ageing reach its price (chosen when a factorisation was a band LU of 0.1-1.5 s on one SM: 64 stents,
+    # 20 steps: 15.2 HHT steps/s refactorising only past 200 iterations, 26-29 by the cost rule); 200 stays a cap
     p.refactor_its = 0 if SOLVER["refactor"] == "always" else 200
     p.refactor_policy = "cost" if SOLVER["refactor"] == "cost" else "threshold"
     p.refactor_cost = SOLVER["refactor_cost"]
@@ -266,15 +266,17 @@ class Workload:
 
 
 def est_bytes(stats):
-    """Device bytes eb_create will hold for one simulation (layout of eb_internal.cuh):
-    element staging, six FP64 BSR matrices plus the FP32 tangent, node state, DOF vectors,
-    Krylov basis, FP32 band and its diagonal-block inverses, SDF coefficients."""
-    n, ne, w, pts, m = stats
-    b = 6 * w + 5
+    """Device bytes eb_create will hold for one simulation, at most (layout of eb_internal.cuh and
+    eb_cond.cuh): element staging, six FP64 BSR matrices plus the FP64 and paired FP32 tangent, node state,
+    DOF vectors, Krylov basis, condensation blocks and lists, the kept system's inverse (up to 2,048 DOFs)
+    with its panels, SDF coefficients.  A few long stents keep more and have a band: less than an inverse
+    of that size beside the other terms."""
+    n, ne, _, pts, m = stats
     blocks = n + 2 * ne
-    band = 4 * (6 * n) * (2 * b + 1) if b <= 891 else 0
-    per_dof = 14 * 8 + 1 + 16 + (2 * m + 1) * 8 + 8 + 4 + 256  # ... Krylov basis V and its preconditioned Z
-    return 6300 * ne + 2200 * blocks + 1100 * n + per_dof * 6 * n + band + 8 * pts
+    ld = -(-min(6 * n, 2048) // 64) * 64
+    inverse = 4 * (ld * ld + 128 * ld) + 32768
+    per_dof = 14 * 8 + 1 + 16 + (2 * m + 1) * 8 + 8 + 4  # ... Krylov basis V and its preconditioned Z
+    return 6300 * ne + 2350 * blocks + (1100 + 900) * n + per_dof * 6 * n + inverse + 8 * pts
 
 
 def plan_groups(wl, budget):

@@ -241,7 +241,8 @@ int eb_set_max_iterations(eb_handle *h, const int32_t *max_iterations);
  * (src/def_params.jl:1-35), tested as in corrector.jl:15. */
 int eb_set_tolerances(eb_handle *h, const double *tolerance_residual, const double *tolerance_displacement);
 int eb_get_stats(eb_handle *h, eb_sim_stats *stats /* n_sims */);
-/* Device memory the handle holds (bytes), and how many simulations use the band-LU preconditioner. */
+/* Device memory the handle holds (bytes), and how many simulations use the EB_PRECOND_BAND preconditioner (an explicit
+ * inverse or a band LU, eb_get_solver tells which; the others have block-Jacobi). */
 int eb_get_memory(eb_handle *h, int64_t *device_bytes, int32_t *band_sims);
 /* How the handle solves simulation `sim`: info[0] DOFs the condensation keeps, [1] half bandwidth of
  * their band LU (0: none), [2] DOFs of their explicit inverse (0: none), both 0 with block-Jacobi,
