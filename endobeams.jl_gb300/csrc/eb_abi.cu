@@ -961,6 +961,7 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
   d.n_elem = NE;
   d.nnzb = NB;
   d.n_dof = ND;
+  d.many_elements = many_elements(NE, h->sms);
   d.beam_threads = d.contact_threads = wide_elements(NE, h->sms) ? 256 : kThreads;
   d.gmat_threads = 256;
   d.gvec_threads = 256;

@@ -7,9 +7,9 @@
 // (sparse Gᵀ/P/H₂ matrices, skew commutators, reuse of Bᵀ·K̄ₕ products) to
 // cut FP64 instructions, which bound this kernel on GB300.
 //
-// An element is about 16,400 FP64 operations.  One thread per element ran them
-// as one dependent chain (0.40 ms a launch even for 20 elements, 255 registers
-// and a quarter of the FP64 pipe busy); here the element is cut into pieces that
+// An element is about 16,400 FP64 operations.  One thread per element runs them
+// as one dependent chain (0.40 ms a launch even for 20 elements), which is best for
+// tens of thousands of elements only; here the element is cut into pieces that
 // share a table (shared memory on the device): its frame, angles and velocities
 // (beam_frame, beam_exact, beam_velocity, one lane per end node), the static
 // stiffness in two halves (beam_static), the mass and the gyroscopic blocks per
@@ -664,6 +664,49 @@ __device__ __forceinline__ void beam_cta(int64_t n, int nb, const Gauss3& gs, do
     const Tab t = table(e);
     for (int b = warp * per + sub; b < kBeamBlocks; b += nw * per) beam_block(io, t, b);
   }
+}
+
+// Adds Gauss-point values into the table, point after point: EmitSum's order (an addition of its own, never
+// part of a multiply-add).
+struct EmitAdd {
+  Tab t;
+  bool first;
+  __device__ __forceinline__ void operator()(int i, double x) const { t.at(i) = first ? x : __dadd_rn(t.at(i), x); }
+  __device__ __forceinline__ void operator()(int i, V3 x) const {
+    (*this)(i, x.x);
+    (*this)(i + 1, x.y);
+    (*this)(i + 2, x.z);
+  }
+  __device__ __forceinline__ void operator()(int i, const M3& x) const {
+#pragma unroll
+    for (int k = 0; k < 9; ++k) (*this)(i + k, x.a[k]);
+  }
+};
+
+// The same pieces by one thread, its table in local memory.
+template <typename IO>
+__device__ __forceinline__ void beam_thread(const IO& io, const Gauss3& gs) {
+  double tab[kTabSize];
+  const Tab t{tab, 1};
+  beam_frame(io, t);
+  for (int n = 0; n < 2; ++n) {
+    beam_exact(io, n, t);
+    beam_angle(io, n, t);
+    beam_velocity(io, n, t);
+  }
+  {
+    BeamStatic q;
+    beam_static_common(io, t, q);
+    for (int half = 0; half < 2; ++half) beam_static(io, t, q, half);
+  }
+  for (int g = 0; g < 3; ++g) {
+    GaussPoint q;
+    gauss_point(t, io.l0(), io.Jr(), gs.z[g], gs.w[g], q);
+    const EmitAdd emit{t, g == 0};
+    beam_mass(t, q, io.Ar(), io.damping(), emit);
+    beam_gyro(t, q, io.Ar(), emit);
+  }
+  for (int b = 0; b < kBeamBlocks; ++b) beam_block(io, t, b);
 }
 #endif
 

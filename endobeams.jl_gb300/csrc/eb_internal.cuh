@@ -78,6 +78,7 @@ struct Dev {
   double* Kt;                           // tangent, FP64
   float2* Ktp;                          // tangent as FP32 pairs (mixed precision; null otherwise)
 
+  int many_elements;                    // a thread per element (many_elements) instead of thirty elements a CTA
   // ---- launch shapes (threads per block), chosen by eb_autotune among shapes whose
   // results are bitwise identical
   int beam_threads, contact_threads, gmat_threads, gvec_threads;

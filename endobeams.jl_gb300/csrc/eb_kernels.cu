@@ -62,6 +62,13 @@ __global__ void __launch_bounds__(kBeamCta, 3) k_beam(const __grid_constant__ De
            [&](int64_t e) { return d.active[d.elem_sim[e]] != 0; });
 }
 
+// The same with a thread per element, for launches of many waves (many_elements).
+__global__ void __launch_bounds__(kBeamCta, 3) k_beam_thread(const __grid_constant__ Dev d, Gauss3 g) {
+  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= d.n_elem || !d.active[d.elem_sim[e]]) return;
+  beam_thread(BeamElem{d, e, {d.ea[e], d.eb[e]}}, g);
+}
+
 // compute_contact_beams via compute&assemble…:460-482, ten or thirty elements per CTA (eb_contact.cuh).
 struct ContactElem : BeamElem {
   __device__ __forceinline__ double radius() const { return d.radius[e]; }
@@ -82,6 +89,10 @@ __global__ void __launch_bounds__(kContactCta) k_contact(const __grid_constant__
 void launch_beam(const Dev& d, const Gauss3& g, cudaStream_t s) {
   if (!d.n_elem) return;
   const int nb = beam_groups(d.beam_threads);
+  if (nb == 3 && d.many_elements) {
+    k_beam_thread<<<nblocks(d.n_elem, kBeamCta), kBeamCta, 0, s>>>(d, g);
+    return;
+  }
   const size_t smem = beam_smem(nb);
   if (smem > 48 * 1024) raise_smem_limit((const void*)k_beam, smem);
   k_beam<<<nblocks(d.n_elem, kBeamGroup * nb), kBeamCta, smem, s>>>(d, g, nb);

@@ -23,6 +23,13 @@ inline int gmres_cta_threads(int asked) {
 // Element launches of more than twenty elements per SM start with thirty elements a CTA, others with ten.
 inline bool wide_elements(int64_t n_elem, int sms) { return n_elem > 20 * (int64_t)sms; }
 
+// Element launches that run a thread per element instead of thirty elements a CTA: 168 registers let an SM hold
+// 384 threads, whose dependent chains then fill the FP64 pipe better than a CTA's phases with their barriers and
+// unequal warps (element passes of a step, ms: 76,000 elements 5.8 -> 5.2, 389,000 31.8 -> 25.4, 642,000 53.2 ->
+// 40.8).  A second wave must be worth its chain: 60,800 elements, just over one wave, took 5.1, where thirty a CTA
+// at 76 ns an element would take 4.6; hence the line at one wave and a sixth.
+inline bool many_elements(int64_t n_elem, int sms) { return n_elem > 448 * (int64_t)sms; }
+
 // Whether the element and the contact pass, which do not depend on each other, run side by side (152 SMs, 64-element
 // ring: a step 1.66 -> 1.43 ms, 9,600 elements 16.6 -> 15.8 ms).  Not where both have thirty elements a CTA (three
 // groups) and fewer than two CTAs per SM: two such CTAs on an SM compete for its L1, through which the elements'

@@ -47,6 +47,7 @@ def test_element_launches_follow_the_devices_size(rules):
     wide = lambda n, sms: bool(rules.host_wide_elements(ctypes.c_int64(n), sms))
     beside = lambda b, c, n, sms: bool(rules.host_side_by_side(b, c, ctypes.c_int64(n), sms))
     for sms in (152, 148, 76):
+        assert [bool(rules.host_many_elements(ctypes.c_int64(n), sms)) for n in (448 * sms, 448 * sms + 1)] == [False, True]
         assert [wide(n, sms) for n in (0, 20 * sms, 20 * sms + 1)] == [False, False, True]
         assert [beside(3, 3, n, sms) for n in (60 * sms - 1, 60 * sms)] == [False, True]
         assert beside(3, 1, 60 * sms - 1, sms) and beside(1, 3, 60 * sms - 1, sms) and beside(1, 1, 1, sms)
