@@ -1326,6 +1326,9 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
     CK(A.alloc(&sa.dense.G, (size_t)dense_off[n_sims]));
     sa.dense.off = p_doff;
     sa.dense.n = p_dn;
+    int* p_db;
+    CK(A.upload(&p_db, h->band_b));
+    sa.dense.b = p_db;
     sa.dense_ld = h->dense_work.max_ld;
     CK(A.alloc(&h->dense_work.Ct, (size_t)panel_off[n_sims]));
     CK(A.alloc(&h->dense_work.O, (size_t)panel_off[n_sims]));

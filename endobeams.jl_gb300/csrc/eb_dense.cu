@@ -4,10 +4,16 @@
 //   k_dense_panel   C_i = A_ik D⁻¹ for every block row i and a copy O_j of the pivot block row;
 //   k_dense_update  A_ij -= C_i O_j; the pivot block row becomes D⁻¹ O_j, the pivot block column
 //                   -C_i, the pivot block D⁻¹; the CTA of the next diagonal block inverts it at once.
-// 2 N^3 operations; the chain is N / 64 steps of two launches.
+// The kept system is a band in its order (half bandwidth b); a step leaves out the blocks past what the
+// pivots so far have filled (dense_reach), whose C_i and O_j are zero: 2 (N^3 - b^3) / 3 + 2 b N^2
+// operations instead of 2 N^3, the same values (304 nets of 33 x 33, N = 1,578 and b = 479: 90.9 -> 65.4 ms a
+// factorisation; 512 of 20 x 20: 33.3 -> 23.6; 1,024 of 12 x 12, N = 864 and b = 77: 50.6 -> 30.4).  The
+// chain is N / 64 steps of two launches.  Tiles of 128 x 128 and 128 x 64 outputs (eight by eight and eight by four a
+// thread) were no faster than 64 x 64: shared memory's 16-byte reads bound both (ncu: L1 72%, FP32 41% busy).
 #include <algorithm>
 
 #include "eb_dense.cuh"
+#include "eb_launch_rules.hpp"
 
 namespace eb {
 
@@ -152,7 +158,7 @@ __global__ void __launch_bounds__(kMm) k_dense_panel(Dev d, DenseDev g, DenseWor
   const int s = sim_of(per, &i);
   if (!marked(d, g, refactor, s)) return;
   const int ld = dense_ld(g.n[s]);
-  if (kT * k >= ld || kT * i >= ld || i == k) return;
+  if (kT * k >= ld || kT * i >= ld || i == k || i >= dense_reach(k, g.b[s])) return;
   __shared__ __align__(16) float At[kT * kLd], B[kT * kLd];
   const float* A = g.G + g.off[s];
   load_tile_t(At, A + (int64_t)kT * i * ld + kT * k, ld);
@@ -184,7 +190,8 @@ __global__ void __launch_bounds__(kMm) k_dense_update(Dev d, DenseDev g, DenseWo
   if (k >= nb || at >= nb * nb) return;
   const int first = k + 1 < nb ? (k + 1) * nb + k + 1 : 0;
   const int tile = at == 0 ? first : (at <= first ? at - 1 : at);
-  const int i = tile / nb, j = tile - i * nb;
+  const int i = tile / nb, j = tile - i * nb, reach = dense_reach(k, g.b[s]);
+  if (i >= reach || j >= reach) return;  // C_i or O_j is zero
   __shared__ __align__(16) float At[kT * kLd], B[kT * kLd];
   __shared__ __align__(16) float rows[2 * kT];
   float* A = g.G + g.off[s] + (int64_t)kT * i * ld + kT * j;

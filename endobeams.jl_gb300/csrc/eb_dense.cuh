@@ -20,6 +20,7 @@ struct DenseDev {
   float* G;             // row-major ld x ld matrices, ld = N rounded up to 64 (identity beyond N)
   const int64_t* off;   // per sim: offset of its matrix in G
   const int* n;         // per sim: N, 0 = not dense
+  const int* b;         // per sim: half bandwidth of the kept system before its inversion
 };
 
 __host__ __device__ __forceinline__ int dense_ld(int n) { return (n + kDenseTile - 1) / kDenseTile * kDenseTile; }

@@ -66,6 +66,14 @@ inline void fit_precond(const std::vector<PrecondBytes>& b, int64_t room, std::v
   if (need > room) std::fill(kind.begin(), kind.end(), (int)kPrecondJacobi);
 }
 
+// Blocks [0, dense_reach) of 64 rows and columns that pivot block k of an in-place Gauss-Jordan can change, for a
+// matrix of half bandwidth b: what the pivots before it have filled ends b entries past them, and beyond
+// the reach the pivot block's column and row are still zero.
+#if defined(__CUDACC__)
+__host__ __device__
+#endif
+inline int dense_reach(int k, int b) { return k + 1 + (63 + b) / 64; }
+
 // Makes `device` the thread's current one for a scope, for entry points that launch on a handle's
 // stream where the caller may have another device current (copies need no such thing).
 template <typename Api>

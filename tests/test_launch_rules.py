@@ -4,6 +4,7 @@ import os
 import shutil
 import subprocess
 
+import numpy as np
 import pytest
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -74,3 +75,33 @@ def test_preconditioners_that_do_not_fit(rules):
     assert fit(sims, want, full - 171) == [band, band, inverse, inverse, band, jacobi]
     assert fit(sims, want, full - 250) == [band, band, inverse, inverse, band, jacobi]
     assert fit(sims, want, full - 251) == [jacobi] * 6
+
+
+@pytest.mark.parametrize("n,b", [(64, 11), (192, 5), (198, 11), (320, 64), (320, 65), (334, 129), (600, 200), (600, 599)])
+def test_inversion_leaves_out_zero_blocks_only(rules, n, b):
+    """Blocked in-place Gauss-Jordan (64-wide pivots) of a band matrix: with the blocks past dense_reach left
+    out every value is that of the full steps."""
+    rng = np.random.default_rng(n + b)
+    i, j = np.indices((n, n))
+    ld = -(-n // 64) * 64
+    full = np.eye(ld)
+    full[:n, :n] = np.where(abs(i - j) <= b, rng.standard_normal((n, n)), 0.0) + 3.0 * np.sqrt(2 * b + 1) * np.eye(n)
+    cut, nb = full.copy(), ld // 64
+    blk = lambda M, r, c: M[64 * r:64 * r + 64, 64 * c:64 * c + 64]
+    want = np.linalg.inv(full)
+    for M, reach in ((full, lambda k: nb), (cut, lambda k: min(nb, rules.host_dense_reach(k, b)))):
+        for k in range(nb):
+            D, m = np.linalg.inv(blk(M, k, k)), reach(k)
+            assert m > k + 1 or k + 1 == nb  # the next pivot block is updated
+            C = {r: blk(M, r, k) @ D for r in range(m) if r != k}
+            O = {c: blk(M, k, c).copy() for c in range(m) if c != k}
+            for r in range(m):
+                for c in range(m):
+                    if r == k:
+                        blk(M, r, c)[:] = D if c == k else D @ O[c]
+                    elif c == k:
+                        blk(M, r, c)[:] = -C[r]
+                    else:
+                        blk(M, r, c)[:] -= C[r] @ O[c]
+    assert np.array_equal(full, cut)
+    assert np.abs(cut - want).max() <= 1e-12 * np.abs(want).max() * n
