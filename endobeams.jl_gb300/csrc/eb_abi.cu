@@ -1435,11 +1435,19 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
     sa.team = gmres_team(sa, fp32, asked_threads ? asked_threads : kGmresMaxThreads, (int)nmax);
     // sixteen warps where every CTA has an SM to itself: their phases wait for loads
     if (!asked_threads && n_sims * sa.team <= h->sms) h->gmres_threads = kGmresMaxThreads;
-    // z_j, w (double or float) and the FP32 vector of the largest simulation
+    // z_j, w (double or float) and the FP32 vector of the largest simulation, where the shared memory for
+    // them does not cost the SM its second CTA while simulations wait for one (512 nets of 20 x 20: Krylov
+    // 20.0 -> 15.6 ms a step); reductions of four inner products make room for both
     const int vec = (int)((nmax * (fp32 ? 3 : 5) + 3) / 4 * 4);
     if (sa.team == 1 && sizeof(float) * (size_t)vec <= kGmresVecSmem) {
+      const size_t limit = n_sims > h->sms && gmres_smem_total(sa) <= kGmresTwoPerSm ? kGmresTwoPerSm : kGmresSmemLimit;
+      const int dots = sa.dots;
       sa.vec_smem = vec;
-      if (gmres_smem_total(sa) > kGmresSmemLimit) sa.vec_smem = 0;
+      if (gmres_smem_total(sa) > limit) sa.dots = 4;
+      if (gmres_smem_total(sa) > limit) {
+        sa.vec_smem = 0;
+        sa.dots = dots;
+      }
     }
   }
 
