@@ -14,7 +14,7 @@
 // Cuthill-McKee order.  A 48-wire stent of 8,664 nodes keeps about 250 nodes,
 // and N b² (the band LU's work) falls by two orders of magnitude.
 //
-// When another level pays (cond_cost, in us of one application): a level costs 5 us (about 2.5 in
+// When another level pays (cond_cost, in us of one application): a level costs 5 us, 3 in small systems (about 2.5 in
 // each sweep: a barrier of the team and its instructions' latency) and its blocks' bytes (with 2 us
 // a 33 x 33 net took 2.10 ms a step, with 5 us 1.94, a 48 x 200 stent 11.4 and 10.8; from 6 us on a
 // stent that refactorises twice a step loses 4% to the larger inverse); the explicit inverse reads 4 N² bytes at about 1 TB/s and its 2 N³ operations at 20 TFLOP/s are
@@ -141,6 +141,11 @@ struct CondPlan {
 
 constexpr int kWholeDofs = 200;  // at most this many DOFs: nothing is eliminated
 
+// us of one application that a level costs.  A small system's team is at most four CTAs, whose barriers
+// are cheaper (12 x 12 net, one level instead of none: a step 1.12 -> 1.05 ms, and as 1,024 of them 42.0 -> 36.4; with 3
+// us for every size a 33 x 33 net's step 1.84 -> 1.86).
+inline double level_cost(int nodes) { return 6 * nodes <= 2048 ? 3.0 : 5.0; }
+
 // The cheaper of the two (past max_dense the explicit inverse is still what the next levels aim
 // at); w < 0: the inverse.  stage_b: the widest half bandwidth whose blocks fit in shared memory.
 inline double cond_cost(int nodes, int w, int max_dense, int stage_b) {
@@ -163,6 +168,7 @@ inline void cond_plan_for(const std::vector<std::vector<int>>& adj0, int max_w, 
   std::vector<int> left(n);
   std::iota(left.begin(), left.end(), 0);
   P.lev_ptr.assign(1, 0);
+  const double level = level_cost(n);
 
   // One level: a greedy independent set of the nodes of degree <= cap, lowest degree first.
   auto pick = [&](int cap) {
@@ -201,7 +207,7 @@ inline void cond_plan_for(const std::vector<std::vector<int>>& adj0, int max_w, 
   };
   auto commit = [&](std::vector<int>& set) {
     std::sort(set.begin(), set.end());
-    P.cost += 5.0;
+    P.cost += level;
     for (int v : set) {
       P.cost += 144e-6 * (1.0 + 2.0 * adj[v].size());
       nb[v] = adj[v];
@@ -252,7 +258,7 @@ inline void cond_plan_for(const std::vector<std::vector<int>>& adj0, int max_w, 
       }
       // past max_dense there is no inverse yet: go on towards it
       if ((max_dense <= 0 || 6 * m <= max_dense) &&
-          cond_cost(m2, w2, max_dense, stage_b) + 5.0 + 144e-6 * blocks > cond_cost(m, w, max_dense, stage_b))
+          cond_cost(m2, w2, max_dense, stage_b) + level + 144e-6 * blocks > cond_cost(m, w, max_dense, stage_b))
         break;
       commit(set);
       w = w2;

@@ -25,7 +25,7 @@ extern "C" void host_grid_plan(int a, int b, int max_w, int max_dense, int stage
   out[2] = (int)P.lev_ptr.size() - 1;
   std::vector<int> pos;
   const int w = rcm_order(adj, pos);
-  cost[0] = 5.0 * out[2] + 144e-6 * P.red0 +
+  cost[0] = level_cost(a * b) * out[2] + 144e-6 * P.red0 +
             cond_cost(kept, P.w, 6 * kept <= max_dense ? max_dense : 0, stage_b);
   cost[1] = cond_cost(a * b, w, 0, stage_b);
 }
