@@ -363,6 +363,7 @@ struct eb_handle {
   BandDev band{};
   CondFactor cond{};
   DenseWork dense_work{};
+  std::vector<int> dense_side;         // dense_grids of the simulations
   std::vector<int64_t> cond_elim_off, cond_tgt_off;  // per level (all simulations): offsets of its lists
   std::vector<int> band_b;  // per sim half bandwidth of the kept nodes (0: block-Jacobi)
   std::vector<int> dense_n; // per sim kept DOFs of its explicit inverse (0: band LU)
@@ -458,7 +459,7 @@ int launch_solve(eb_handle* h, bool refactor, const int* refactor_src, PhaseTime
     CK(cudaMemcpyAsync(h->d_refactor, refactor_src, sizeof(int) * h->n_sims, cudaMemcpyHostToDevice, h->stream));
     const CondLevels lv{h->cond_elim_off.data(), h->cond_tgt_off.data(), (int)h->cond_elim_off.size() - 1};
     launch_cond_factor(h->d, h->cond, lv, h->d_refactor, h->stream);
-    launch_dense_inverse(h->d, h->sa.dense, h->dense_work, h->cond, h->d_refactor, h->stream);
+    launch_dense_inverse(h->d, h->sa.dense, h->dense_work, h->cond, h->dense_side, h->d_refactor, h->stream);
     if (h->max_b > 0) {
       launch_band_fill(h->d, h->band, h->cond, h->stream);
       if (h->tc_lu) CK(launch_band_lu_tc(h->d, h->band, h->max_b, h->band.lu_fail, h->stream));
@@ -1328,6 +1329,9 @@ int eb_create(const eb_params* p, int32_t n_sims, const eb_sim_desc* sims, eb_ha
     sa.dense.n = p_dn;
     int* p_db;
     CK(A.upload(&p_db, h->band_b));
+    std::vector<int> blocks(h->dense_n);  // blocks a side, 0 = not dense
+    for (int& n : blocks) n = dense_ld(n) / kDenseTile;
+    h->dense_side = dense_grids(blocks, h->band_b);
     sa.dense.b = p_db;
     sa.dense_ld = h->dense_work.max_ld;
     CK(A.alloc(&h->dense_work.Ct, (size_t)panel_off[n_sims]));

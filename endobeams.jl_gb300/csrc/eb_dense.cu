@@ -182,16 +182,15 @@ __global__ void __launch_bounds__(kMm) k_dense_panel(Dev d, DenseDev g, DenseWor
 
 // CTA (tile, s) of step k; the next diagonal block's tile comes first, so that its inversion
 // runs beside the other tiles.
-__global__ void __launch_bounds__(kMm) k_dense_update(Dev d, DenseDev g, DenseWork w, const int* refactor, int k, int per) {
+__global__ void __launch_bounds__(kMm) k_dense_update(Dev d, DenseDev g, DenseWork w, const int* refactor, int k, int side) {
   int at;
-  const int s = sim_of(per, &at);
+  const int s = sim_of(side * side, &at);
   if (!marked(d, g, refactor, s)) return;
-  const int ld = dense_ld(g.n[s]), nb = ld / kT;
-  if (k >= nb || at >= nb * nb) return;
-  const int first = k + 1 < nb ? (k + 1) * nb + k + 1 : 0;
+  const int ld = dense_ld(g.n[s]), nb = ld / kT, reach = min(nb, dense_reach(k, g.b[s]));
+  if (k >= nb || at >= reach * reach) return;  // beyond the reach C_i or O_j is zero
+  const int first = k + 1 < nb ? (k + 1) * reach + k + 1 : 0;
   const int tile = at == 0 ? first : (at <= first ? at - 1 : at);
-  const int i = tile / nb, j = tile - i * nb, reach = dense_reach(k, g.b[s]);
-  if (i >= reach || j >= reach) return;  // C_i or O_j is zero
+  const int i = tile / reach, j = tile - i * reach;
   __shared__ __align__(16) float At[kT * kLd], B[kT * kLd];
   __shared__ __align__(16) float rows[2 * kT];
   float* A = g.G + g.off[s] + (int64_t)kT * i * ld + kT * j;
@@ -243,8 +242,8 @@ __global__ void __launch_bounds__(kMm) k_dense_update(Dev d, DenseDev g, DenseWo
   store_inverse(v, w.D + ((int64_t)s * 2 + ((k + 1) & 1)) * kT * kT);
 }
 
-void launch_dense_inverse(const Dev& d, const DenseDev& g, const DenseWork& w, const CondFactor& f, const int* refactor,
-                          cudaStream_t s) {
+void launch_dense_inverse(const Dev& d, const DenseDev& g, const DenseWork& w, const CondFactor& f,
+                          const std::vector<int>& grids, const int* refactor, cudaStream_t s) {
   if (w.max_ld == 0) return;
   const unsigned S = (unsigned)d.n_sims;
   const int nb = w.max_ld / kT, zero = std::max(1, nb * nb / 2);
@@ -253,8 +252,9 @@ void launch_dense_inverse(const Dev& d, const DenseDev& g, const DenseWork& w, c
   if (f.red_n) k_dense_fill<<<nblocks(f.red_n * 36, 256), 256, 0, s>>>(d, g, f, refactor);
   k_dense_first<<<S, kMm, 0, s>>>(d, g, w, refactor);
   for (int k = 0; k < nb; ++k) {
-    if (nb > 1) k_dense_panel<<<nb * S, kMm, 0, s>>>(d, g, w, refactor, k, nb);
-    k_dense_update<<<nb * nb * S, kMm, 0, s>>>(d, g, w, refactor, k, nb * nb);
+    const int side = grids[k];
+    if (nb > 1) k_dense_panel<<<side * S, kMm, 0, s>>>(d, g, w, refactor, k, side);
+    k_dense_update<<<side * side * S, kMm, 0, s>>>(d, g, w, refactor, k, side);
   }
 }
 

@@ -9,6 +9,8 @@
 // operations of the inversion grow past the band LU's latency beyond it, and its memory
 // (4 N^2 bytes) past the band's.
 #pragma once
+#include <vector>
+
 #include "eb_cond.cuh"
 
 namespace eb {
@@ -32,8 +34,9 @@ struct DenseWork {
   int max_ld;           // largest ld of the handle, 0 = no dense simulation
 };
 
-void launch_dense_inverse(const Dev& d, const DenseDev& g, const DenseWork& w, const CondFactor& f, const int* refactor,
-                          cudaStream_t s);
+// grids: dense_grids of the handle's simulations.
+void launch_dense_inverse(const Dev& d, const DenseDev& g, const DenseWork& w, const CondFactor& f,
+                          const std::vector<int>& grids, const int* refactor, cudaStream_t s);
 
 // Rows of z = G x by whole warps, four rows at a time (x in shared memory, ld entries, zero
 // beyond N); a row's sum has one order, whatever the number of warps.

@@ -74,6 +74,16 @@ __host__ __device__
 #endif
 inline int dense_reach(int k, int b) { return k + 1 + (63 + b) / 64; }
 
+// Per pivot block, the most blocks a side that it can change in any simulation (nb: blocks of 64 a side, b:
+// half bandwidths): the grids of a step.  With grids of the largest matrix whole, half of a step's CTAs on
+// average had nothing to do but to find that out.
+inline std::vector<int> dense_grids(const std::vector<int>& nb, const std::vector<int>& b) {
+  std::vector<int> side(nb.empty() ? 0 : *std::max_element(nb.begin(), nb.end()), 0);
+  for (size_t s = 0; s < nb.size(); ++s)
+    for (int k = 0; k < nb[s]; ++k) side[k] = std::max(side[k], std::min(nb[s], dense_reach(k, b[s])));
+  return side;
+}
+
 // Makes `device` the thread's current one for a scope, for entry points that launch on a handle's
 // stream where the caller may have another device current (copies need no such thing).
 template <typename Api>

@@ -4,6 +4,11 @@
 extern "C" int host_gmres_cta_threads(int asked) { return eb::gmres_cta_threads(asked); }
 extern "C" int host_wide_elements(int64_t n_elem, int sms) { return eb::wide_elements(n_elem, sms); }
 extern "C" int host_dense_reach(int k, int b) { return eb::dense_reach(k, b); }
+extern "C" int host_dense_grids(int n, const int* nb, const int* b, int* side) {
+  const std::vector<int> g = eb::dense_grids(std::vector<int>(nb, nb + n), std::vector<int>(b, b + n));
+  std::copy(g.begin(), g.end(), side);
+  return (int)g.size();
+}
 extern "C" int host_many_elements(int64_t n_elem, int sms) { return eb::many_elements(n_elem, sms); }
 extern "C" int host_side_by_side(int beam_groups, int contact_groups, int64_t n_elem, int sms) {
   return eb::side_by_side(beam_groups, contact_groups, n_elem, sms);

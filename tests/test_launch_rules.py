@@ -105,3 +105,15 @@ def test_inversion_leaves_out_zero_blocks_only(rules, n, b):
                         blk(M, r, c)[:] -= C[r] @ O[c]
     assert np.array_equal(full, cut)
     assert np.abs(cut - want).max() <= 1e-12 * np.abs(want).max() * n
+
+
+@pytest.mark.parametrize("sims", [[(1, 5)], [(15, 125), (30, 479)], [(30, 479), (0, 593), (3, 11), (9, 1000)], [(0, 0)], [(32, 2041)]])
+def test_grids_of_the_inversion_hold_every_simulations_blocks(rules, sims):
+    """sims: blocks a side (0: not inverted) and half bandwidth.  Every block that a step changes has a CTA, the next
+    pivot block among them, and a step has no more rows of CTAs than its widest simulation."""
+    n, side = len(sims), (ctypes.c_int * 64)()
+    got = rules.host_dense_grids(n, (ctypes.c_int * n)(*[a for a, _ in sims]), (ctypes.c_int * n)(*[b for _, b in sims]), side)
+    assert got == max(a for a, _ in sims)
+    for k in range(got):
+        rows = [min(a, rules.host_dense_reach(k, b)) for a, b in sims if k < a]
+        assert side[k] == max(rows) and all(r > k + 1 or k + 1 == a for r, (a, _) in zip(rows, [x for x in sims if k < x[0]]))
