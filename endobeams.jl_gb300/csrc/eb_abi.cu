@@ -459,14 +459,14 @@ int launch_solve(eb_handle* h, bool refactor, const int* refactor_src, PhaseTime
     CK(cudaMemcpyAsync(h->d_refactor, refactor_src, sizeof(int) * h->n_sims, cudaMemcpyHostToDevice, h->stream));
     const CondLevels lv{h->cond_elim_off.data(), h->cond_tgt_off.data(), (int)h->cond_elim_off.size() - 1};
     launch_cond_factor(h->d, h->cond, lv, h->d_refactor, h->stream);
-    launch_dense_inverse(h->d, h->sa.dense, h->dense_work, h->cond, h->dense_side, h->d_refactor, h->stream);
+    const int dense = launch_dense_inverse(h->d, h->sa.dense, h->dense_work, h->cond, h->dense_side, h->sms, h->d_refactor,
+                                           h->stream);
     if (h->max_b > 0) {
       launch_band_fill(h->d, h->band, h->cond, h->stream);
       if (h->tc_lu) CK(launch_band_lu_tc(h->d, h->band, h->max_b, h->band.lu_fail, h->stream));
       else CK(launch_band_lu(h->d, h->band, h->max_b, h->stream));
     }
-    T.launches[EB_PHASE_PRECOND] += 2 + 2 * lv.n + (h->max_b > 0 ? 3 : 0) +
-                                    (h->dense_work.max_ld ? 3 + 2 * (h->dense_work.max_ld / kDenseTile) : 0);
+    T.launches[EB_PHASE_PRECOND] += 2 + 2 * lv.n + (h->max_b > 0 ? 3 : 0) + dense;
   }
   CK(cudaGetLastError());
   T.mark(EB_PHASE_PRECOND, h->stream);

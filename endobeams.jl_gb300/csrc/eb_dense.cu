@@ -9,7 +9,8 @@
 // operations instead of 2 N^3, the same values (304 nets of 33 x 33, N = 1,578 and b = 479: 90.9 -> 65.4 ms a
 // factorisation; 512 of 20 x 20: 33.3 -> 23.6; 1,024 of 12 x 12, N = 864 and b = 77: 50.6 -> 30.4).  The
 // chain is N / 64 steps of two launches.  Tiles of 128 x 128 and 128 x 64 outputs (eight by eight and eight by four a
-// thread) were no faster than 64 x 64: shared memory's 16-byte reads bound both (ncu: L1 72%, FP32 41% busy).
+// thread) were no faster than 64 x 64: shared memory's 16-byte reads bound both (ncu: L1 72%, FP32 41% busy).  In
+// launches of many waves a tile has 64 threads with 8 x 8 outputs each (k_dense_update_many).
 #include <algorithm>
 
 #include "eb_dense.cuh"
@@ -21,6 +22,7 @@ namespace {
 
 constexpr int kT = kDenseTile;
 constexpr int kMm = 256;   // threads per CTA: 16 x 16, 4 x 4 outputs each
+constexpr int kMany = 64;  // threads per CTA of k_dense_update_many: 8 x 8, 8 x 8 outputs each
 constexpr int kLd = kT + 4;
 
 // acc (+)= Aᵀ-stored (k, m) times B (k, n), both kT x kT in shared memory with stride kLd
@@ -38,15 +40,19 @@ __device__ __forceinline__ void mm64(const float* At, const float* B, float (&ac
   }
 }
 
-// 64 x 64 tile (row stride ld) into shared memory, as it is or transposed
+// 64 x 64 tile (row stride ld) into shared memory, as it is or transposed, by THR threads
+template <int THR = kMm>
 __device__ __forceinline__ void load_tile(float* sm, const float* g, int64_t ld) {
-  for (int e = threadIdx.x; e < kT * kT / 4; e += kMm) {
+#pragma unroll 8
+  for (int e = threadIdx.x; e < kT * kT / 4; e += THR) {
     const int r = e >> 4, c = 4 * (e & 15);
     *reinterpret_cast<float4*>(sm + r * kLd + c) = *reinterpret_cast<const float4*>(g + r * ld + c);
   }
 }
+template <int THR = kMm>
 __device__ __forceinline__ void load_tile_t(float* sm, const float* g, int64_t ld) {
-  for (int e = threadIdx.x; e < kT * kT / 4; e += kMm) {
+#pragma unroll 8
+  for (int e = threadIdx.x; e < kT * kT / 4; e += THR) {
     const int r = e & 63, c = 4 * (e >> 6);  // lanes along the rows: the transposed stores are conflict free
     const float4 v = *reinterpret_cast<const float4*>(g + r * ld + c);
     sm[c * kLd + r] = v.x; sm[(c + 1) * kLd + r] = v.y; sm[(c + 2) * kLd + r] = v.z; sm[(c + 3) * kLd + r] = v.w;
@@ -242,20 +248,86 @@ __global__ void __launch_bounds__(kMm) k_dense_update(Dev d, DenseDev g, DenseWo
   store_inverse(v, w.D + ((int64_t)s * 2 + ((k + 1) & 1)) * kT * kT);
 }
 
-void launch_dense_inverse(const Dev& d, const DenseDev& g, const DenseWork& w, const CondFactor& f,
-                          const std::vector<int>& grids, const int* refactor, cudaStream_t s) {
-  if (w.max_ld == 0) return;
+// The same for launches of many waves, without the next diagonal block's tile (k_dense_update's): 64 threads of
+// 8 x 8 outputs each, so that a k takes four 16-byte reads of shared memory for 64 multiply-adds instead of two for
+// 16.  Each output's sum has the same order.  Bound by the FP32 pipe and the wait for the tiles (36 TFLOP/s at
+// 48,400 tiles; 304 nets of 33 x 33: a factorisation 62 -> 55 ms).
+__global__ void __launch_bounds__(kMany) k_dense_update_many(Dev d, DenseDev g, DenseWork w, const int* refactor, int k,
+                                                             int side) {
+  int tile;
+  const int s = sim_of(side * side, &tile);
+  if (!marked(d, g, refactor, s)) return;
+  const int ld = dense_ld(g.n[s]), nb = ld / kT, reach = min(nb, dense_reach(k, g.b[s]));
+  const int first = k + 1 < nb ? (k + 1) * reach + k + 1 : 0;
+  if (k >= nb || tile >= reach * reach || tile == first) return;
+  const int i = tile / reach, j = tile - i * reach;
+  __shared__ __align__(16) float At[kT * kLd], B[kT * kLd];
+  float* A = g.G + g.off[s] + (int64_t)kT * i * ld + kT * j;
+  const float* Dk = w.D + ((int64_t)s * 2 + (k & 1)) * kT * kT;
+  const float* Ct = w.Ct + w.poff[s] + kT * i;
+  if (j == k) {  // pivot block column: -C_i, or D⁻¹ itself
+    for (int e = threadIdx.x; e < kT * kT; e += kMany) {
+      const int r = e & 63, c = e >> 6;
+      A[(int64_t)r * ld + c] = i == k ? Dk[r * kT + c] : -Ct[(int64_t)c * ld + r];
+    }
+    return;
+  }
+  if (i == k) load_tile_t<kMany>(At, Dk, kT);  // D⁻¹ O_j
+  else load_tile<kMany>(At, Ct, ld);
+  load_tile<kMany>(B, w.O + w.poff[s] + kT * j, ld);
+  const int tm = threadIdx.x >> 3, tn = threadIdx.x & 7;  // rows and columns 4 t .. + 3 and 32 + 4 t .. + 3
+  float acc[8][8];
+#pragma unroll
+  for (int a = 0; a < 8; ++a)
+#pragma unroll
+    for (int c = 0; c < 8; ++c) acc[a][c] = 0.f;
+  __syncthreads();
+#pragma unroll 4
+  for (int q = 0; q < kT; ++q) {
+    float av[8], bv[8];
+    *reinterpret_cast<float4*>(av) = *reinterpret_cast<const float4*>(At + q * kLd + 4 * tm);
+    *reinterpret_cast<float4*>(av + 4) = *reinterpret_cast<const float4*>(At + q * kLd + 32 + 4 * tm);
+    *reinterpret_cast<float4*>(bv) = *reinterpret_cast<const float4*>(B + q * kLd + 4 * tn);
+    *reinterpret_cast<float4*>(bv + 4) = *reinterpret_cast<const float4*>(B + q * kLd + 32 + 4 * tn);
+#pragma unroll
+    for (int a = 0; a < 8; ++a)
+#pragma unroll
+      for (int c = 0; c < 8; ++c) acc[a][c] = fmaf(av[a], bv[c], acc[a][c]);
+  }
+  const float sg = i == k ? 1.f : -1.f;
+#pragma unroll
+  for (int a = 0; a < 8; ++a)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      float4* p = reinterpret_cast<float4*>(A + (int64_t)(32 * (a >> 2) + 4 * tm + (a & 3)) * ld + 32 * h + 4 * tn);
+      const float4 o = i == k ? make_float4(0.f, 0.f, 0.f, 0.f) : *p;
+      const float* v = &acc[a][4 * h];
+      *p = make_float4(fmaf(sg, v[0], o.x), fmaf(sg, v[1], o.y), fmaf(sg, v[2], o.z), fmaf(sg, v[3], o.w));
+    }
+}
+
+int launch_dense_inverse(const Dev& d, const DenseDev& g, const DenseWork& w, const CondFactor& f,
+                         const std::vector<int>& grids, int sms, const int* refactor, cudaStream_t s) {
+  if (w.max_ld == 0) return 0;
   const unsigned S = (unsigned)d.n_sims;
   const int nb = w.max_ld / kT, zero = std::max(1, nb * nb / 2);
+  int launches = 2;
   // float4 stores of the largest matrix over 256-thread CTAs, eight per thread
   k_dense_zero<<<zero * S, 256, 0, s>>>(d, g, refactor, zero);
-  if (f.red_n) k_dense_fill<<<nblocks(f.red_n * 36, 256), 256, 0, s>>>(d, g, f, refactor);
+  if (f.red_n) {
+    k_dense_fill<<<nblocks(f.red_n * 36, 256), 256, 0, s>>>(d, g, f, refactor);
+    ++launches;
+  }
   k_dense_first<<<S, kMm, 0, s>>>(d, g, w, refactor);
   for (int k = 0; k < nb; ++k) {
     const int side = grids[k];
+    const bool many = dense_many((int64_t)side * side * S, sms);
     if (nb > 1) k_dense_panel<<<side * S, kMm, 0, s>>>(d, g, w, refactor, k, side);
-    k_dense_update<<<side * side * S, kMm, 0, s>>>(d, g, w, refactor, k, side);
+    k_dense_update<<<(many ? 1 : side * side) * S, kMm, 0, s>>>(d, g, w, refactor, k, many ? 1 : side);
+    if (many) k_dense_update_many<<<side * side * S, kMany, 0, s>>>(d, g, w, refactor, k, side);
+    launches += (nb > 1) + 1 + many;
   }
+  return launches;
 }
 
 }  // namespace eb

@@ -34,9 +34,10 @@ struct DenseWork {
   int max_ld;           // largest ld of the handle, 0 = no dense simulation
 };
 
-// grids: dense_grids of the handle's simulations.
-void launch_dense_inverse(const Dev& d, const DenseDev& g, const DenseWork& w, const CondFactor& f,
-                          const std::vector<int>& grids, const int* refactor, cudaStream_t s);
+// grids: dense_grids of the handle's simulations; sms: the device's multiprocessors.
+// Returns the number of launches.
+int launch_dense_inverse(const Dev& d, const DenseDev& g, const DenseWork& w, const CondFactor& f,
+                         const std::vector<int>& grids, int sms, const int* refactor, cudaStream_t s);
 
 // Rows of z = G x by whole warps, four rows at a time (x in shared memory, ld entries, zero
 // beyond N); a row's sum has one order, whatever the number of warps.

@@ -84,6 +84,11 @@ inline std::vector<int> dense_grids(const std::vector<int>& nb, const std::vecto
   return side;
 }
 
+// Steps of an inversion (64 x 64 tiles in all) that run 64 threads a tile: with fewer tiles an SM the
+// 256-thread kernel's shorter chain wins (a factorisation in ms, 256 and 64 threads: 8 nets of 33 x 33, 33 tiles an SM, 2.4 and
+// 2.5; 16, 66 an SM, 3.9 and 4.0; 64 of 20 x 20, 95 an SM, 3.2 and 3.2; 304 of 33 x 33 62 and 55).
+inline bool dense_many(int64_t tiles, int sms) { return tiles > 80 * (int64_t)sms; }
+
 // Makes `device` the thread's current one for a scope, for entry points that launch on a handle's
 // stream where the caller may have another device current (copies need no such thing).
 template <typename Api>

@@ -9,6 +9,7 @@ extern "C" int host_dense_grids(int n, const int* nb, const int* b, int* side) {
   std::copy(g.begin(), g.end(), side);
   return (int)g.size();
 }
+extern "C" int host_dense_many(int64_t tiles, int sms) { return eb::dense_many(tiles, sms); }
 extern "C" int host_many_elements(int64_t n_elem, int sms) { return eb::many_elements(n_elem, sms); }
 extern "C" int host_side_by_side(int beam_groups, int contact_groups, int64_t n_elem, int sms) {
   return eb::side_by_side(beam_groups, contact_groups, n_elem, sms);

@@ -117,3 +117,8 @@ def test_grids_of_the_inversion_hold_every_simulations_blocks(rules, sims):
     for k in range(got):
         rows = [min(a, rules.host_dense_reach(k, b)) for a, b in sims if k < a]
         assert side[k] == max(rows) and all(r > k + 1 or k + 1 == a for r, (a, _) in zip(rows, [x for x in sims if k < x[0]]))
+
+
+@pytest.mark.parametrize("sms", [1, 76, 152])
+def test_inversions_of_many_tiles(rules, sms):
+    assert [bool(rules.host_dense_many(ctypes.c_int64(n), sms)) for n in (1, 80 * sms, 80 * sms + 1)] == [False, False, True]
