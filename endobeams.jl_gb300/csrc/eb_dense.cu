@@ -23,6 +23,7 @@ namespace {
 constexpr int kT = kDenseTile;
 constexpr int kMm = 256;   // threads per CTA: 16 x 16, 4 x 4 outputs each
 constexpr int kMany = 64;  // threads per CTA of k_dense_update_many: 8 x 8, 8 x 8 outputs each
+constexpr int kStages = 4;
 constexpr int kLd = kT + 4;
 
 // acc (+)= Aᵀ-stored (k, m) times B (k, n), both kT x kT in shared memory with stride kLd
@@ -56,6 +57,17 @@ __device__ __forceinline__ void load_tile_t(float* sm, const float* g, int64_t l
     const int r = e & 63, c = 4 * (e >> 6);  // lanes along the rows: the transposed stores are conflict free
     const float4 v = *reinterpret_cast<const float4*>(g + r * ld + c);
     sm[c * kLd + r] = v.x; sm[(c + 1) * kLd + r] = v.y; sm[(c + 2) * kLd + r] = v.z; sm[(c + 3) * kLd + r] = v.w;
+  }
+}
+
+// Rows of group h of a 64 x 64 tile (row stride ld) into shared memory, asynchronously, by kMany threads.
+__device__ __forceinline__ void copy_rows(float* sm, const float* g, int64_t ld, int h) {
+  constexpr int rows = kT / kStages;
+#pragma unroll
+  for (int e = threadIdx.x; e < rows * kT / 4; e += kMany) {
+    const int r = rows * h + (e >> 4), c = 4 * (e & 15);
+    const uint32_t dst = (uint32_t)__cvta_generic_to_shared(sm + r * kLd + c);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(g + r * ld + c) : "memory");
   }
 }
 
@@ -272,27 +284,40 @@ __global__ void __launch_bounds__(kMany) k_dense_update_many(Dev d, DenseDev g, 
     }
     return;
   }
+  // rows of both operands in four asynchronous groups: the products of one run while the next arrive
+  const float* O = w.O + w.poff[s] + kT * j;
   if (i == k) load_tile_t<kMany>(At, Dk, kT);  // D⁻¹ O_j
-  else load_tile<kMany>(At, Ct, ld);
-  load_tile<kMany>(B, w.O + w.poff[s] + kT * j, ld);
+#pragma unroll
+  for (int h = 0; h < kStages; ++h) {
+    if (i != k) copy_rows(At, Ct, ld, h);
+    copy_rows(B, O, ld, h);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
   const int tm = threadIdx.x >> 3, tn = threadIdx.x & 7;  // rows and columns 4 t .. + 3 and 32 + 4 t .. + 3
   float acc[8][8];
 #pragma unroll
   for (int a = 0; a < 8; ++a)
 #pragma unroll
     for (int c = 0; c < 8; ++c) acc[a][c] = 0.f;
-  __syncthreads();
+#pragma unroll
+  for (int h = 0; h < kStages; ++h) {
+    if (h == 0) asm volatile("cp.async.wait_group 3;" ::: "memory");
+    else if (h == 1) asm volatile("cp.async.wait_group 2;" ::: "memory");
+    else if (h == 2) asm volatile("cp.async.wait_group 1;" ::: "memory");
+    else asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
 #pragma unroll 4
-  for (int q = 0; q < kT; ++q) {
-    float av[8], bv[8];
-    *reinterpret_cast<float4*>(av) = *reinterpret_cast<const float4*>(At + q * kLd + 4 * tm);
-    *reinterpret_cast<float4*>(av + 4) = *reinterpret_cast<const float4*>(At + q * kLd + 32 + 4 * tm);
-    *reinterpret_cast<float4*>(bv) = *reinterpret_cast<const float4*>(B + q * kLd + 4 * tn);
-    *reinterpret_cast<float4*>(bv + 4) = *reinterpret_cast<const float4*>(B + q * kLd + 32 + 4 * tn);
+    for (int q = h * (kT / kStages); q < (h + 1) * (kT / kStages); ++q) {
+      float av[8], bv[8];
+      *reinterpret_cast<float4*>(av) = *reinterpret_cast<const float4*>(At + q * kLd + 4 * tm);
+      *reinterpret_cast<float4*>(av + 4) = *reinterpret_cast<const float4*>(At + q * kLd + 32 + 4 * tm);
+      *reinterpret_cast<float4*>(bv) = *reinterpret_cast<const float4*>(B + q * kLd + 4 * tn);
+      *reinterpret_cast<float4*>(bv + 4) = *reinterpret_cast<const float4*>(B + q * kLd + 32 + 4 * tn);
 #pragma unroll
-    for (int a = 0; a < 8; ++a)
+      for (int a = 0; a < 8; ++a)
 #pragma unroll
-      for (int c = 0; c < 8; ++c) acc[a][c] = fmaf(av[a], bv[c], acc[a][c]);
+        for (int c = 0; c < 8; ++c) acc[a][c] = fmaf(av[a], bv[c], acc[a][c]);
+    }
   }
   const float sg = i == k ? 1.f : -1.f;
 #pragma unroll
