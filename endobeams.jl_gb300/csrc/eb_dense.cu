@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(kMm) k_dense_update(Dev d, DenseDev g, DenseWo
 // The same for launches of many waves, without the next diagonal block's tile (k_dense_update's): 64 threads of
 // 8 x 8 outputs each, so that a k takes four 16-byte reads of shared memory for 64 multiply-adds instead of two for
 // 16.  Each output's sum has the same order.  Bound by the FP32 pipe and the wait for the tiles (36 TFLOP/s at
-// 48,400 tiles; 304 nets of 33 x 33: a factorisation 62 -> 55 ms).
+// 48,400 tiles before their rows came in groups; 304 nets of 33 x 33: a factorisation 62 -> 55 ms, with groups 53).
 __global__ void __launch_bounds__(kMany) k_dense_update_many(Dev d, DenseDev g, DenseWork w, const int* refactor, int k,
                                                              int side) {
   int tile;
